@@ -83,6 +83,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// The same by a whole warp, with one answer for all its lanes: what follows stays warp-uniform for the compiler, which then
+// keeps descriptors and addresses in uniform registers.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
+// Looks at a barrier without waiting (whole warp, one answer): asked one block ahead, its latency hides under the current block.
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
+}
+
 // ----- TMA (bulk tensor copies; loads are never cluster-multicast) -----
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* desc) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(desc)) : "memory");
@@ -99,6 +117,30 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* d
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(desc)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
+}
+// A stage of two tiles whose bytes complete on `bar`: optionally arm the barrier and load the first tile (`with_a`), then load the
+// second.  Whole warp, one elected lane issues (see umma_f8f6f4_block for why not `if (lane == 0)`).  `az` < 0: the first tensor
+// is 2-D, else its third coordinate.
+__device__ __forceinline__ void tma_load_stage(uint32_t smem_a, uint32_t smem_b, const CUtensorMap* map_a, const CUtensorMap* map_b,
+                                               uint32_t bar, uint32_t bytes, bool with_a, int x, int ya, int az, int yb) {
+  const uint64_t ma = reinterpret_cast<uint64_t>(map_a), mb = reinterpret_cast<uint64_t>(map_b);
+  if (az < 0) {
+    asm volatile(
+        "{\n\t.reg .pred q, w;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 w, %6, 0, q;\n\t"
+        "@w mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
+        "@w cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%7, %8}], [%4];\n\t"
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%7, %9}], [%4];\n\t}"
+        ::"r"(smem_a), "r"(smem_b), "l"(ma), "l"(mb), "r"(bar), "r"(bytes), "r"(uint32_t(with_a)), "r"(x), "r"(ya), "r"(yb)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred q, w;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 w, %6, 0, q;\n\t"
+        "@w mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
+        "@w cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%7, %8, %10}], [%4];\n\t"
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%7, %9}], [%4];\n\t}"
+        ::"r"(smem_a), "r"(smem_b), "l"(ma), "l"(mb), "r"(bar), "r"(bytes), "r"(uint32_t(with_a)), "r"(x), "r"(ya), "r"(yb), "r"(az)
+        : "memory");
+  }
 }
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -150,6 +192,30 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// One 128-byte K block, four k-steps of 32 bytes each into accumulator `d`, then a commit to each of up to two barriers (shared
+// addresses; 0 = none) -- all issued by ONE elected lane of a warp that runs this converged.  A single lane inside
+// `if (lane == 0)` needs 55 cycles per tcgen05 instruction on a B200 (every operand moves to a uniform register first), four
+// MMAs and their commits 320; issued like this they need 160, below the 256 cycles the tensor core works on a 128 x 128 block.
+// `accumulate` applies to the first step.
+__device__ __forceinline__ void umma_f8f6f4_block(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate,
+                                                  uint32_t bar0, uint32_t bar1) {
+  asm volatile(
+      "{\n\t.reg .pred q, f, t, u, v;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 f, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\t"
+      "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.and.b32 u, %5, 0, q;\n\tsetp.ne.and.b32 v, %6, 0, q;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, f;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a1, b1, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a2, b2, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a3, b3, %3, t;\n\t"
+      "@u tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+      "@v tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1)
       : "memory");
 }
 
@@ -208,6 +274,13 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
 }
 
 // ----- misc -----
+// c += {a0, a1} * s, two fp32 multiply-adds in one instruction
+__device__ __forceinline__ void fma2(float& c0, float& c1, uint32_t a0, uint32_t a1, float s) {
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmov.b64 z, {%0, %1};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "+f"(c0), "+f"(c1)
+      : "r"(a0), "r"(a1), "f"(s));
+}
 __device__ __forceinline__ float bf16_to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 struct alignas(16) U4 { uint32_t x, y, z, w; };

@@ -178,7 +178,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   float* xs_smem = reinterpret_cast<float*>(tiles + stages * Cfg::kStageBytes + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
   const int lane = threadIdx.x & 31;
   const bool gather = p.ag.world > 1;
   pdl_trigger();
@@ -284,34 +284,35 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // Weights are never written by a kernel of the same stream, so the plain GEMM starts the weight tiles of its first
   // ring pass BEFORE it waits for its predecessor: under programmatic dependent launch this CTA is resident while the
   // short kernel that produces its activations (a norm, a quantization) still runs, and the weight stream -- all of it
   // for a short K range -- arrives under that kernel instead of after it.  The activation tiles follow the wait.
   int w_ahead = 0;
   if (!early_inputs) {
+    w_ahead = min(nkb, stages);
     if (warp == 0 && lane == 0) {
       tma_prefetch_desc(&tmap_w);
       tma_prefetch_desc(&tmap_x);
-      w_ahead = min(nkb, stages);
       for (int i = 0; i < w_ahead; ++i) {
         mbar_expect_tx(&full[i], Cfg::kStageBytes);
         tma_load_2d(tiles + i * Cfg::kStageBytes, &tmap_w, &full[i], (kb0 + i) * kBlockK, n0);
       }
     }
+    __syncwarp();
     pdl_wait();
   }
 
   if (warp == 0) {
-    if (lane == 0) {
-      if (early_inputs) {
-        tma_prefetch_desc(&tmap_w);
-        tma_prefetch_desc(&tmap_x);
-      }
-      const CUtensorMap* xmap = (gather && (ag_epoch & 1u)) ? &tmap_x_alt : &tmap_x;
-      bool shard_ready = true;
-      if (gather) {
+    if (early_inputs && lane == 0) {
+      tma_prefetch_desc(&tmap_w);
+      tma_prefetch_desc(&tmap_x);
+    }
+    const CUtensorMap* xmap = (gather && (ag_epoch & 1u)) ? &tmap_x_alt : &tmap_x;
+    bool shard_ready = true;
+    if (gather) {
+      if (lane == 0) {
         // both shards that a token tile may straddle are awaited (tiles are aligned to shards in practice)
         const int first = t0 / p.ag.shard_rows, last = min(p.ag.world - 1, (t0 + BT - 1) / p.ag.shard_rows);
         const unsigned long long t_start = globaltimer_ns();
@@ -329,52 +330,44 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             }
           }
         }
-        fence_proxy_async_smem();
-        asm volatile("fence.proxy.async.global;" ::: "memory");  // peers' generic-proxy stores -> my TMA reads
       }
-      int s = 0;
-      uint32_t ring_phase = 0;  // ring position and wrap parity, kept incrementally: the depth is a run-time value
-      for (int i = 0; shard_ready && i < nkb; ++i, s = (s + 1 == stages ? 0 : s + 1), ring_phase ^= (s == 0 ? 1u : 0u)) {
-        uint8_t* a = tiles + s * Cfg::kStageBytes;
-        uint8_t* b = a + kTileN * kBlockK;
-        if (i >= w_ahead) {  // the first pass of the plain mode is armed and its weight tile on the way already
-          if (!mbar_wait(&empty[s], ring_phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer)) break;
-          mbar_expect_tx(&full[s], Cfg::kStageBytes);
-          if (p.tile_map) tma_load_3d(a, &tmap_w, &full[s], (kb0 + i) * kBlockK, n0, expert);
-          else tma_load_2d(a, &tmap_w, &full[s], (kb0 + i) * kBlockK, n0);
-        }
-        tma_load_2d(b, xmap, &full[s], (kb0 + i) * kBlockK, t0);
-      }
+      shard_ready = __shfl_sync(0xffffffffu, int(shard_ready), 0) != 0;
+      __syncwarp();  // whichever lane is elected below issues the loads: what lane 0 acquired holds for the warp
+      fence_proxy_async_smem();
+      asm volatile("fence.proxy.async.global;" ::: "memory");  // peers' generic-proxy stores -> the warp's TMA reads
+    }
+    __syncwarp();
+    const uint32_t tiles_addr = smem_u32(tiles), full_addr = smem_u32(full);
+    const int third = p.tile_map ? expert : -1;
+    int s = 0;
+    uint32_t ring_phase = 0;  // ring position and wrap parity, kept incrementally: the depth is a run-time value
+    for (int i = 0; shard_ready && i < nkb; ++i) {
+      const bool fresh = i >= w_ahead;  // the first pass of the plain mode is armed and its weight tile on the way already
+      if (fresh && !mbar_wait_warp(&empty[s], ring_phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer)) break;
+      const uint32_t a = tiles_addr + s * Cfg::kStageBytes;
+      tma_load_stage(a, a + kTileN * kBlockK, &tmap_w, xmap, full_addr + s * 8, Cfg::kStageBytes, fresh, (kb0 + i) * kBlockK, n0, third, t0);
+      if (++s == stages) { s = 0; ring_phase ^= 1u; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // This one thread's loop is the pace of a weight-streaming CTA whose tiles are already in shared memory, so it
-      // carries no work that can be left out: descriptors advance by a constant per stage (the ring is contiguous and
-      // stays inside the 14-bit address field), a fresh accumulator is not waited for, and a stage that no later K
-      // block reuses is not handed back.
-      constexpr uint32_t idesc = umma_idesc(kTileN, BT, 0, 0);
-      constexpr uint64_t kStageStep = uint64_t(Cfg::kStageBytes >> 4);
-      const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(tiles));
-      const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(tiles) + kTileN * kBlockK);
-      int s = 0;
-      uint32_t ring_phase = 0;
-      for (int i = 0; i < nkb; ++i, s = (s + 1 == stages ? 0 : s + 1), ring_phase ^= (s == 0 ? 1u : 0u)) {
-        const int buf = i % Cfg::kAcc;
-        if (i >= Cfg::kAcc &&
-            !mbar_wait(&acc_empty[buf], ((i / Cfg::kAcc) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma)) break;
-        if (!mbar_wait(&full[s], ring_phase, abort_flag, p.status, kStatusTimeoutMma)) break;
-        tc_fence_after();
-        const uint64_t a_desc = a_desc0 + uint64_t(s) * kStageStep;
-        const uint64_t b_desc = b_desc0 + uint64_t(s) * kStageStep;
-        const uint32_t d = tmem_base + buf * BT;
-#pragma unroll
-        for (int k = 0; k < kBlockK / 32; ++k) {
-          // advancing 32 bytes along K inside the swizzle row = +2 in the 16-byte address field
-          umma_f8f6f4(d, a_desc + uint64_t(k * 2), b_desc + uint64_t(k * 2), idesc, k > 0 ? 1u : 0u);
-        }
-        if (i + stages < nkb) tc_commit(&empty[s]);  // smem stage reusable once these MMAs have read it
-        tc_commit(&acc_full[buf]);                   // accumulator block complete
-      }
+    // This warp's loop is the pace of a weight-streaming CTA whose tiles are already in shared memory, so it carries no work that
+    // can be left out: descriptors advance by a constant per stage (the ring is contiguous and stays inside the 14-bit address
+    // field), a fresh accumulator is not waited for, and a stage that no later K block reuses is not handed back.
+    constexpr uint32_t idesc = umma_idesc(kTileN, BT, 0, 0);
+    constexpr uint64_t kStageStep = uint64_t(Cfg::kStageBytes >> 4);
+    const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(tiles));
+    const uint64_t b_desc0 = umma_desc_k_sw128(smem_u32(tiles) + kTileN * kBlockK);
+    const uint32_t empty_addr = smem_u32(empty), acc_full_addr = smem_u32(acc_full);
+    int s = 0, buf = 0;
+    uint32_t ring_phase = 0, acc_phase = 1;
+    for (int i = 0; i < nkb; ++i) {
+      if (i >= Cfg::kAcc && !mbar_wait_warp(&acc_empty[buf], acc_phase, abort_flag, p.status, kStatusTimeoutMma)) break;
+      if (!mbar_wait_warp(&full[s], ring_phase, abort_flag, p.status, kStatusTimeoutMma)) break;
+      tc_fence_after();
+      // smem stage reusable once these MMAs have read it; accumulator block complete
+      umma_f8f6f4_block(tmem_base + buf * BT, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc, 0u,
+                        i + stages < nkb ? empty_addr + s * 8 : 0u, acc_full_addr + buf * 8);
+      if (++s == stages) { s = 0; ring_phase ^= 1u; }
+      if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
     }
   } else {
     // ----- epilogue warps: thread owns output feature n0 + q*32 + lane and CW token columns from col0 -----
@@ -402,40 +395,38 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       for (int j = lane; j < nkb; j += 32) ws_w[j] = __ldg(wsc + kb0 + j);
     }
     __syncwarp();
-    bool ok = true;
+    constexpr int kChunk = CW < 32 ? CW : 32, kChunks = CW / kChunk;
+    const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + col0;
+    bool ok = true, ready = false;
+    int buf = 0;
+    uint32_t phase = 0;
     for (int i = 0; i < nkb; ++i) {
-      const int buf = i % Cfg::kAcc;
-      ok = mbar_wait(&acc_full[buf], (i / Cfg::kAcc) & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
-      ok = __all_sync(0xffffffffu, ok);
+      if (!ready) ok = mbar_wait_warp(&acc_full[buf], phase, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (!ok) break;
       tc_fence_after();
       const float s = ws_cached ? ws_w[i] : __ldg(wsc + kb0 + i);
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BT + col0;
-      if constexpr (CW == 64) {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(taddr, r0);        // both loads in flight before the single wait
-        tmem_ld_32x32(taddr + 32, r1);
+      const uint32_t taddr = lane_base + buf * BT;
+      uint32_t r[2][kChunk];
+      auto load_chunk = [&](int c) {
+        if constexpr (kChunk == 32) tmem_ld_32x32(taddr + c * 32, r[c & 1]);
+        else tmem_ld_32x16(taddr, r[0]);
+      };
+      load_chunk(0);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
         tmem_wait_ld();
+        if (c + 1 < kChunks) {
+          load_chunk(c + 1);  // in flight under the multiply-adds of this chunk
+        } else {  // all columns are in registers: hand the accumulator back and look at the next one
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[buf]);
+          if (++buf == Cfg::kAcc) { buf = 0; phase ^= 1u; }
+          ready = i + 1 < nkb && mbar_test_warp(&acc_full[buf], phase);
+        }
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = fmaf(__uint_as_float(r0[j]), s, acc[j]);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[32 + j] = fmaf(__uint_as_float(r1[j]), s, acc[32 + j]);
-      } else if constexpr (CW == 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr, r);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = fmaf(__uint_as_float(r[j]), s, acc[j]);
-      } else {
-        uint32_t r[16];
-        tmem_ld_32x16(taddr, r);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] = fmaf(__uint_as_float(r[j]), s, acc[j]);
+        for (int j = 0; j < kChunk; j += 2) fma2(acc[c * kChunk + j], acc[c * kChunk + j + 1], r[c & 1][j], r[c & 1][j + 1], s);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
     }
     if (ok) {
       const int tl = min(BT, row_end - t0);

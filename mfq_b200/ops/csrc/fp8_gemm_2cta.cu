@@ -1,11 +1,10 @@
 // Block-scaled FP8 GEMM for wide batches on PAIRS of SMs:  out[M, N] = X[M, K] * W[N, K]^T  (prefill shapes)
 //
-// The one-CTA kernel (fp8_gemm.cu) streams 32 KB of operands from L2 per 128 x 128 x 128 block of products; at
-// 4096^3 that is ~1 GB through the L2 -> SM path in 164 us, which is what bounds it (tensor pipe 20 % busy).  Here two
-// CTAs of a cluster work on one 256 x BT tile with `tcgen05.mma.cta_group::2`: each CTA stages ITS 128 weight rows
-// (UMMA A operand, M = 256 over the pair) and only HALF of the BT token rows (B operand, N = BT: the tensor core
-// reads the other half from the peer CTA's shared memory), so a CTA loads 16 KB + BT/2 * 128 B per K block for
-// 128 x BT x 128 products: 1.33x (BT = 128) and 2x (BT = 256) the products per byte of the one-CTA kernel.
+// The one-CTA kernel (fp8_gemm.cu) streams 32 KB of operands from L2 per 128 x 128 x 128 block of products.  Here two CTAs of a
+// cluster work on one 256 x BT tile with `tcgen05.mma.cta_group::2`: each CTA stages ITS 128 weight rows (UMMA A operand, M = 256
+// over the pair) and only HALF of the BT token rows (B operand, N = BT: the tensor core reads the other half from the peer CTA's
+// shared memory), so a CTA loads 16 KB + BT/2 * 128 B per K block for 128 x BT x 128 products: 1.33x (BT = 128) and 2x (BT = 256)
+// the products per byte of the one-CTA kernel.
 //
 // Roles per CTA: warp 0 = TMA producer, warp 1 = TMEM owner (and, in the leader CTA only, the MMA issuer), warps 2, 3
 // idle (they complete the control warp group, which gives its registers away with `setmaxnreg`), warps 4..11 =
@@ -14,9 +13,18 @@
 // multiplier, into registers while the tensor cores run the next block.  Cross-CTA signalling:
 //   full[s]      lives in the leader; both CTAs' TMA loads complete their bytes on it (`.cta_group::2` loads may
 //                signal the peer's barrier), the leader's producer arms it with the bytes of BOTH CTAs;
-//   empty[s]     one per CTA; the leader commits to its own and to the peer's after the MMAs of the stage;
-//   acc_full[b]  one per CTA, same pair of commits; acc_empty[b] lives in the leader and counts the epilogue warps of
-//                both CTAs (the peer's arrive through the cluster address of the leader's barrier).
+//   empty[s]     one per CTA; one commit of the leader arrives on both after the MMAs of the stage;
+//   acc_full[b]  one per CTA, same; acc_empty[b] lives in the leader and counts the epilogue warps of both CTAs (the
+//                peer's arrive through the cluster address of the leader's barrier).
+// What bounds it: a K block is 512 cycles of tensor-core work (BT = 256) and the loop  issue -> complete -> fold -> hand back ->
+// issue  has to fit twice that, TMEM holding two accumulators.  So the issuing and loading warps run converged with one elected
+// lane (common.cuh: umma_f8f6f4_block says why), the fold keeps the TMEM load of one 32-column chunk in flight under the
+// multiply-adds (two per instruction) of the chunk before, an accumulator is handed back as soon as its last column is in
+// registers, and the epilogue looks at its next barrier one step ahead.  Measured on a B200 (operands rotated over more than the
+// L2, before: this kernel as it was with one issuing lane and cluster-scope releases | the one-SM kernel | now):
+//   4096 x 28672 x 4096   1084 (BT = 256) | 1096 | 593 us (1.62 PFLOP/s)     4096 x 4096 x 14336   550 | 420 | 252 us (1.91 PFLOP/s)
+//   357 x 28672 x 4096     115 (one-SM)          | 62 us                     357 x 4096 x 14336     89 (one-SM) | 39 us
+// Without the fold the same loads and MMAs run at 2.3 to 3.1 PFLOP/s, without the loads the fold and its hand-shakes at 2.1.
 // The kernel is persistent: one pair per two SMs walks the tiles, all roles with continuing barrier phases, so a tile's
 // prologue (first loads) and epilogue (store) hide under its neighbours' main loops; with one tile per launched CTA
 // the fixed cost per tile was ~9 us of a 23 us tile at K = 4096.
@@ -25,8 +33,6 @@
 //
 // The reference has no FP8 tensor-core path (mfq/kernels/cuda/fp8_sq.cu:564-592 decodes to fp16 for wmma / cuBLAS).
 #include "common.cuh"
-
-#include <cstdlib>
 
 namespace mfq {
 namespace {
@@ -47,11 +53,6 @@ struct PairCfg {
 };
 
 struct PairParams {
-  // Measurement switches (wrong numbers unless 0).  1: one accumulator over the whole K range, folded once -- the time
-  // of the TMA + MMA pipeline alone, the bound for any way of folding.  2: the epilogue hands every accumulator back
-  // without reading it (the cost of the hand-shakes alone).  4: it reads the accumulators but skips the FMAs.
-  int single_fold;
-  int fold_mode;
   const float* w_scale;
   const float* x_scale;
   __nv_bfloat16* out;
@@ -84,59 +85,42 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// 2-D tile load whose bytes complete on a barrier given by its cluster address (the leader's, from either CTA).
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* desc, uint32_t bar_cluster_addr, int x,
-                                                 int y) {
+// One stage: the weight tile and the token half-tile, both completing on the barrier at `bar_cluster_addr` (the leader's, from
+// either CTA), which the leader arms with `bytes` (0: the peer's call, it does not arm).  Whole warp, one elected lane issues.
+__device__ __forceinline__ void tma_load_stage_pair(uint32_t smem_a, uint32_t smem_b, const CUtensorMap* map_a, const CUtensorMap* map_b,
+                                                    uint32_t bar_cluster_addr, uint32_t bar_local, uint32_t bytes, int x, int ya, int yb) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(desc)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      "{\n\t.reg .pred q, e;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 e, %6, 0, q;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%5], %6;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%7, %8}], [%4];\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%7, %9}], [%4];\n\t}"
+      ::"r"(smem_a), "r"(smem_b), "l"(reinterpret_cast<uint64_t>(map_a)), "l"(reinterpret_cast<uint64_t>(map_b)), "r"(bar_cluster_addr),
+        "r"(bar_local), "r"(bytes), "r"(x), "r"(ya), "r"(yb)
       : "memory");
 }
-__device__ __forceinline__ void umma_f8f6f4_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+// The pair's form of umma_f8f6f4_block: four k-steps into a fresh accumulator, then two commits, each of which arrives on the
+// barrier at that offset in BOTH CTAs once these MMAs have retired.
+__device__ __forceinline__ void umma_f8f6f4_block_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t bar0, uint32_t bar1) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred q, f, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t.reg .b16 both;\n\tmov.b16 both, 3;\n\t"
+      "setp.ne.b32 f, 0, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\t"
+      "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, f;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a1, b1, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a2, b2, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a3, b3, %3, t;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%4], both;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], both;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(bar0), "r"(bar1)
       : "memory");
 }
-// Arrives on the barrier at `bar_cluster_addr` (any CTA of the cluster) once the MMAs issued so far have retired.
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
+// Relaxed: what it orders are tensor-memory reads, which have completed (wait::ld, fence::before_thread_sync) before it; a
+// release at cluster scope would also drain this warp's global accesses, about a microsecond per block.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
-
-// Latency-critical waits (accumulator hand-over in both directions) poll with mbarrier.test_wait, which returns at once;
-// try_wait may park the thread for a system-chosen time and was measured to add about a microsecond per hand-over.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (mbar_test(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  uint32_t spins = 0;
-  while (!mbar_test(bar, parity)) {
-    if ((++spins & 0xFF) == 0) {
-      if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > kWaitBudgetNs) {
-        *abort_flag = 1;
-        if (status) atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-  return true;
-}
-
-__device__ unsigned long long g_stamp_issue;  // measurement switch 64: issue time of the stamped K block
 
 template <int BT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BT>::kThreads, 1)
@@ -150,12 +134,11 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   uint64_t* empty = bars + Cfg::kStages;       // one set per CTA
   uint64_t* acc_full = bars + 2 * Cfg::kStages;
   uint64_t* acc_empty = acc_full + Cfg::kAcc;  // used in the leader only
-  uint64_t* dummy_bar = acc_empty + Cfg::kAcc;  // measurement switch 16 only
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dummy_bar + 1);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + Cfg::kAcc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* xs_smem = reinterpret_cast<float*>(tiles + Cfg::kStages * Cfg::kStageBytes + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();  // 0 = leader
   const bool leader = rank == 0;
   const int nkb = p.K / kBK;
@@ -172,7 +155,6 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   if (threadIdx.x == 0) {
     for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < Cfg::kAcc; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 2 * Cfg::kEpiWarps); }
-    mbar_init(dummy_bar, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -184,83 +166,61 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anybody signals across
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  pdl_trigger();  // TMEM is held by now: a successor that wants some waits for it, not the other way round
   // The register file is the scarce resource of the fold: the control warp group hands its registers to the epilogue
-  // groups, which then hold a thread's accumulators plus the raw columns of TWO K blocks at once.
+  // groups, which then hold a thread's accumulators plus two chunks of raw columns.
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+  pdl_wait();
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmap_w);
       tma_prefetch_desc(&tmap_x);
-      int s = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
-        const int n0 = tile_n0(tile), t0 = tile_t0(tile);
-        for (int i = 0; i < nkb; ++i, s = (s + 1 == Cfg::kStages ? 0 : s + 1), phase ^= (s == 0 ? 1u : 0u)) {
-          if (!mbar_wait(&empty[s], phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer)) { ok = false; break; }
-          uint8_t* a = tiles + s * Cfg::kStageBytes;
-          uint8_t* b = a + kRows * kBK;
-          if (leader) mbar_expect_tx(&full[s], 2 * Cfg::kStageBytes);  // the bytes of both CTAs land on this barrier
-          const uint32_t bar = map_to_cta(&full[s], 0);
-          tma_load_2d_pair(a, &tmap_w, bar, i * kBK, n0);
-          tma_load_2d_pair(b, &tmap_x, bar, i * kBK, t0 + int(rank) * (BT / 2));
-        }
+    }
+    __syncwarp();
+    const uint32_t tiles_addr = smem_u32(tiles), full_local = smem_u32(full), full_leader = map_to_cta(full, 0);
+    const uint32_t bytes = leader ? 2u * Cfg::kStageBytes : 0u;  // the bytes of both CTAs land on the leader's barrier
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
+      const int n0 = tile_n0(tile), t0 = tile_t0(tile) + int(rank) * (BT / 2);
+      for (int i = 0; i < nkb; ++i) {
+        ok = mbar_wait_warp(&empty[s], phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer);
+        if (!ok) break;
+        const uint32_t a = tiles_addr + s * Cfg::kStageBytes;
+        tma_load_stage_pair(a, a + kRows * kBK, &tmap_w, &tmap_x, full_leader + s * 8, full_local + s * 8, bytes, i * kBK, n0, t0);
+        if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
       }
     }
-  } else if (warp == 1) {
-    if (leader && lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(2 * kRows, BT, 0, 0);
-      int s = 0;
-      uint32_t phase = 0, it = 0;  // it: accumulator blocks issued so far, over all tiles
-      bool ok = true;
-      for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
-        for (int i = 0; i < nkb; ++i, s = (s + 1 == Cfg::kStages ? 0 : s + 1), phase ^= (s == 0 ? 1u : 0u)) {
-          const bool fresh = !p.single_fold || i == 0;  // this K block opens a new accumulator
-          const uint32_t buf = it % Cfg::kAcc;
-          if (fresh && !mbar_wait(&acc_empty[buf], ((it / Cfg::kAcc) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma)) { ok = false; break; }
-          const bool stamp = (p.fold_mode & 64) && blockIdx.x == 0 && tile == cluster;
-          if (stamp && i == 10 + Cfg::kAcc) p.status[3] = int(globaltimer_ns() - g_stamp_issue);  // its accumulator came back
-          if (stamp && i == 10) { *reinterpret_cast<volatile unsigned long long*>(&g_stamp_issue) = globaltimer_ns(); __threadfence(); }
-          if (!mbar_wait(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + s * Cfg::kStageBytes);
-          const uint64_t a_desc = umma_desc_k_sw128(a_addr);
-          const uint64_t b_desc = umma_desc_k_sw128(a_addr + kRows * kBK);
-          // measurement switch 8 (with the single-accumulator switch): rotate the accumulator per K block all the same
-          const bool rotate = p.single_fold && (p.fold_mode & 8);
-          const uint32_t d = tmem_base + (rotate ? uint32_t(i % Cfg::kAcc) : buf) * BT;
-#pragma unroll
-          for (int k = 0; k < kBK / 32; ++k)
-            umma_f8f6f4_pair(d, a_desc + uint64_t(k * 2), b_desc + uint64_t(k * 2), idesc, (k > 0 || (!fresh && !rotate)) ? 1u : 0u);
-          // the stage is free, and the accumulator complete, in BOTH CTAs once these MMAs have retired
-          tc_commit_pair(map_to_cta(&empty[s], 0));
-          tc_commit_pair(map_to_cta(&empty[s], 1));
-          if (p.fold_mode & 16) {  // measurement: two more commits per K block, nobody waits on them
-            tc_commit_pair(map_to_cta(dummy_bar, 0));
-            tc_commit_pair(map_to_cta(dummy_bar, 1));
-          }
-          const long long t_commit = clock64();
-          if (!p.single_fold || i == nkb - 1) {
-            tc_commit_pair(map_to_cta(&acc_full[buf], 0));
-            tc_commit_pair(map_to_cta(&acc_full[buf], 1));
-            if ((p.fold_mode & 32) && !p.single_fold) {
-              // measurement: issue -> completion latency of one K block, seen by the issuing thread (unpipelined)
-              while (!mbar_test(&acc_full[buf], (it / Cfg::kAcc) & 1)) {
-              }
-              if (blockIdx.x == 0 && tile == cluster && i == 10) p.status[2] = int(clock64() - t_commit);
-            }
-            ++it;
-          }
-        }
+  } else if (warp == 1 && leader) {
+    constexpr uint32_t idesc = umma_idesc(2 * kRows, BT, 0, 0);
+    constexpr uint64_t kStageStep = uint64_t(Cfg::kStageBytes >> 4);
+    const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(tiles)), b_desc0 = umma_desc_k_sw128(smem_u32(tiles) + kRows * kBK);
+    const uint32_t empty_addr = smem_u32(empty), acc_full_addr = smem_u32(acc_full);
+    int s = 0;
+    uint32_t phase = 0, buf = 0, acc_phase = 1;  // the first pass over the accumulators finds them free
+    bool ok = true;
+    for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
+      for (int i = 0; i < nkb; ++i) {
+        ok = mbar_wait_warp(&acc_empty[buf], acc_phase, abort_flag, p.status, kStatusTimeoutMma) &&
+             mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma);
+        if (!ok) break;
+        tc_fence_after();
+        umma_f8f6f4_block_pair(tmem_base + buf * BT, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc,
+                               empty_addr + s * 8, acc_full_addr + buf * 8);
+        if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
+        if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
       }
     }
   }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    pdl_wait();
     // ----- epilogue warps: thread owns weight row n0 + q*32 + lane and CW token columns from col0 -----
     constexpr int CW = Cfg::kCols;
+    constexpr int kChunks = CW / 32;
     const int q = warp & 3;
     const int col0 = ((warp - 4) >> 2) * CW;
     const int row = q * 32 + lane;
@@ -268,8 +228,9 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     float* ws_w = xs_smem + Cfg::kEpiWarps * CW + (warp - 4) * Cfg::kWsMax;
     const bool ws_cached = nkb <= Cfg::kWsMax;
     const uint32_t acc_empty_leader0 = map_to_cta(&acc_empty[0], 0);
-    bool ok = true;
-    uint32_t it = 0;
+    const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + col0;
+    bool ok = true, ready = false;
+    uint32_t buf = 0, phase = 0;
     for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
       const int n0 = tile_n0(tile), t0 = tile_t0(tile);
       const int n = n0 + row;
@@ -282,74 +243,28 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       if (ws_cached)
         for (int j = lane; j < nkb; j += 32) ws_w[j] = __ldg(wsc + j);
       __syncwarp();
-      const int folds = p.single_fold ? 1 : nkb;
-      int i = 0;
-      if constexpr (CW <= 64) {
-        // Two K blocks per TMEM round trip: the loads of both are in flight under ONE wait, so a warp pays the load
-        // latency (the longest link of the wait -> load -> FMA chain) once per two blocks.  The accumulators are handed
-        // back as soon as their columns sit in registers, before the FMAs.
-        for (; ok && i + 1 < folds; i += 2, it += 2) {
-          const uint32_t buf_a = it % Cfg::kAcc, buf_b = (it + 1) % Cfg::kAcc;
-          // one lane polls (every poll is a shared-memory access, and shared memory is what the tensor cores stream from)
-          if (lane == 0)
-            ok = mbar_wait(&acc_full[buf_a], (it / Cfg::kAcc) & 1, abort_flag, p.status, kStatusTimeoutEpilogue) &&
-                 mbar_wait(&acc_full[buf_b], ((it + 1) / Cfg::kAcc) & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
-          ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
-          if (!ok) break;
-          tc_fence_after();
-          const float sa = ws_cached ? ws_w[i] : __ldg(wsc + i), sb = ws_cached ? ws_w[i + 1] : __ldg(wsc + i + 1);
-          const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + col0;
-          uint32_t ra[CW], rb[CW];
-          if (p.fold_mode & 2) {
-#pragma unroll
-            for (int c = 0; c < CW; ++c) ra[c] = rb[c] = 0u;
-          } else {
-#pragma unroll
-            for (int c = 0; c < CW; c += 32) {
-              tmem_ld_32x32(lane_base + buf_a * BT + c, *reinterpret_cast<uint32_t(*)[32]>(ra + c));
-              tmem_ld_32x32(lane_base + buf_b * BT + c, *reinterpret_cast<uint32_t(*)[32]>(rb + c));
-            }
-            tmem_wait_ld();
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive_cluster(acc_empty_leader0 + buf_a * 8);
-            mbar_arrive_cluster(acc_empty_leader0 + buf_b * 8);
-          }
-          if (p.fold_mode & 4) {
-            acc[0] += __uint_as_float(ra[0] ^ rb[CW - 1]);  // keeps the loads alive
-          } else {
-#pragma unroll
-            for (int j = 0; j < CW; ++j) acc[j] = fmaf(__uint_as_float(rb[j]), sb, fmaf(__uint_as_float(ra[j]), sa, acc[j]));
-          }
-        }
-      }
-      for (; ok && i < folds; ++i, ++it) {
-        const uint32_t buf = it % Cfg::kAcc;
-        if (lane == 0) ok = mbar_wait(&acc_full[buf], (it / Cfg::kAcc) & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
-        ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
-        if ((p.fold_mode & 64) && blockIdx.x < 2 && tile == cluster && i == 10 && warp == 4 && lane == 0)
-          p.status[1 + blockIdx.x] = int(globaltimer_ns() - *reinterpret_cast<volatile unsigned long long*>(&g_stamp_issue));
+      for (int i = 0; i < nkb; ++i) {
+        if (!ready) ok = mbar_wait_warp(&acc_full[buf], phase, abort_flag, p.status, kStatusTimeoutEpilogue);
         if (!ok) break;
         tc_fence_after();
         const float s = ws_cached ? ws_w[i] : __ldg(wsc + i);
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BT + col0;
+        const uint32_t taddr = lane_base + buf * BT;
+        uint32_t r[2][32];
+        tmem_ld_32x32(taddr, r[0]);
 #pragma unroll
-        for (int c = 0; c < CW; c += 64) {
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32(taddr + c, r0);
-          tmem_ld_32x32(taddr + c + 32, r1);
+        for (int c = 0; c < kChunks; ++c) {
           tmem_wait_ld();
-          if (c + 64 >= CW) {  // all columns of this block are in registers: hand the accumulator back
+          if (c + 1 < kChunks) {
+            tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
+          } else {  // all columns of this block are in registers: hand the accumulator back, look at the next one
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty_leader0 + buf * 8);
+            if (++buf == Cfg::kAcc) { buf = 0; phase ^= 1u; }
+            ready = mbar_test_warp(&acc_full[buf], phase);
           }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[c + j] = fmaf(__uint_as_float(r0[j]), s, acc[c + j]);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) acc[c + 32 + j] = fmaf(__uint_as_float(r1[j]), s, acc[c + 32 + j]);
+          for (int j = 0; j < 32; j += 2) fma2(acc[c * 32 + j], acc[c * 32 + j + 1], r[c & 1][j], r[c & 1][j + 1], s);
         }
       }
       if (ok && n < p.N) {
@@ -399,14 +314,12 @@ int launch_pair(const void* w, const float* w_scale, const void* x, const float*
       return -6;
     attr_set[dev] = true;
   }
-  static const int single_fold = [] { const char* e = getenv("MFQ_PAIR_SINGLE_FOLD"); return e ? atoi(e) : 0; }();
-  static const int fold_mode = [] { const char* e = getenv("MFQ_PAIR_FOLD_MODE"); return e ? atoi(e) : 0; }();
-  PairParams p{single_fold, fold_mode, w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(residual), status, M, N, K};
+  PairParams p{w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(residual), status, M, N, K};
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles = (N / (2 * kRows)) * ((M + BT - 1) / BT);
   const int clusters = tiles < sms / 2 ? tiles : sms / 2;
-  fp8_gemm_pair_kernel<BT><<<dim3(2 * clusters), Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tw, tx, p);
+  launch_kernel(fp8_gemm_pair_kernel<BT>, dim3(2 * clusters), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 

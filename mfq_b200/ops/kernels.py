@@ -82,20 +82,29 @@ def pick_splits(m: int, n: int, k: int, sms: int = 148) -> int:
 # 144 CTAs in clusters of 3 leave no slack for cluster placement -- and 14.6 us with 4.
 _MEASURED_SPLITS = {(48, 32): 4}
 
-PAIR_MIN_ROWS = 1024  # batches at least this wide take the two-SM GEMM (``csrc/fp8_gemm_2cta.cu``)
+PAIR_MIN_ROWS = 65  # batches at least this wide may take the two-SM GEMM (``csrc/fp8_gemm_2cta.cu``)
 
 
-def pair_tile(m: int, n: int) -> int:
+def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     """Token tile of the two-SM GEMM for this shape, 0 = use the one-SM kernel.  ``MFQ_GEMM_PAIR`` = 0 / 128 / 256
-    overrides the choice."""
+    overrides the choice.
+
+    Its pairs walk tiles of 256 weight rows; on B200 a tile takes 2.9 + 0.306 us per K block with 128 tokens and 6.7 + 0.506 us with
+    256 (fitted to the projections of an 8B layer at 357 .. 4096 tokens), so the better tile is a matter of whole waves: 1000 x 6144 x
+    4096 is 38.6 against 46.9 us, 1000 x 4096 x 14336 73.7 against 64.5.  The one-SM kernel keeps what it is better at: up to 64
+    tokens, rows that are not whole pairs of blocks, and long K ranges over so few tiles that half of the pairs would idle, which it
+    splits (128 x 4096 x 14336: 19.9 against 37.8 us; at 357 tokens, 48 tiles, it takes 83 against 39.5)."""
     forced = os.environ.get("MFQ_GEMM_PAIR")
-    tile = int(forced) if forced not in (None, "") else _PAIR_DEFAULT
-    if tile not in (128, 256) or n % 256 or m < PAIR_MIN_ROWS:
+    if n % 256 or m < PAIR_MIN_ROWS:
         return 0
-    return tile
-
-
-_PAIR_DEFAULT = 0
+    if forced not in (None, ""):
+        return int(forced) if int(forced) in (128, 256) else 0
+    pairs, blocks = sms // 2, k // 128
+    tiles = {t: n // 256 * math.ceil(m / t) for t in (128, 256)}
+    if 2 * tiles[128] <= pairs and blocks > 64:
+        return 0
+    cost = {t: math.ceil(tiles[t] / pairs) * (ramp + per * blocks) for t, ramp, per in ((128, 2.9, 0.306), (256, 6.7, 0.506))}
+    return 128 if cost[128] <= cost[256] else 256
 
 
 def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, *,
@@ -116,7 +125,7 @@ def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scal
         return out
     ws = Workspace.get(x_q.device)
     if pair is None:
-        pair = pair_tile(m, n) if splits is None and token_tile is None else 0
+        pair = pair_tile(m, n, k) if splits is None and token_tile is None else 0
     if pair:
         assert pair in (128, 256) and n % 256 == 0
         rc = lib().mfq_fp8_gemm_pair(ptr(w_q), ptr(w_scale), ptr(x_q), ptr(x_scale), ptr(out), ptr(residual), ptr(ws.status),
