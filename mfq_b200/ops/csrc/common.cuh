@@ -120,25 +120,25 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* d
 }
 // A stage of two tiles whose bytes complete on `bar`: optionally arm the barrier and load the first tile (`with_a`), then load the
 // second.  Whole warp, one elected lane issues (see umma_f8f6f4_block for why not `if (lane == 0)`).  `az` < 0: the first tensor
-// is 2-D, else its third coordinate.
+// is 2-D, else its third coordinate; `x`, `xb`: the tiles' innermost coordinates.
 __device__ __forceinline__ void tma_load_stage(uint32_t smem_a, uint32_t smem_b, const CUtensorMap* map_a, const CUtensorMap* map_b,
-                                               uint32_t bar, uint32_t bytes, bool with_a, int x, int ya, int az, int yb) {
+                                               uint32_t bar, uint32_t bytes, bool with_a, int x, int ya, int az, int yb, int xb) {
   const uint64_t ma = reinterpret_cast<uint64_t>(map_a), mb = reinterpret_cast<uint64_t>(map_b);
   if (az < 0) {
     asm volatile(
         "{\n\t.reg .pred q, w;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 w, %6, 0, q;\n\t"
         "@w mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
         "@w cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%7, %8}], [%4];\n\t"
-        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%7, %9}], [%4];\n\t}"
-        ::"r"(smem_a), "r"(smem_b), "l"(ma), "l"(mb), "r"(bar), "r"(bytes), "r"(uint32_t(with_a)), "r"(x), "r"(ya), "r"(yb)
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%10, %9}], [%4];\n\t}"
+        ::"r"(smem_a), "r"(smem_b), "l"(ma), "l"(mb), "r"(bar), "r"(bytes), "r"(uint32_t(with_a)), "r"(x), "r"(ya), "r"(yb), "r"(xb)
         : "memory");
   } else {
     asm volatile(
         "{\n\t.reg .pred q, w;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 w, %6, 0, q;\n\t"
         "@w mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n\t"
         "@w cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%7, %8, %10}], [%4];\n\t"
-        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%7, %9}], [%4];\n\t}"
-        ::"r"(smem_a), "r"(smem_b), "l"(ma), "l"(mb), "r"(bar), "r"(bytes), "r"(uint32_t(with_a)), "r"(x), "r"(ya), "r"(yb), "r"(az)
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%11, %9}], [%4];\n\t}"
+        ::"r"(smem_a), "r"(smem_b), "l"(ma), "l"(mb), "r"(bar), "r"(bytes), "r"(uint32_t(with_a)), "r"(x), "r"(ya), "r"(yb), "r"(az), "r"(xb)
         : "memory");
   }
 }
@@ -216,6 +216,41 @@ __device__ __forceinline__ void umma_f8f6f4_block(uint32_t d, uint64_t a, uint64
       "@u tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
       "@v tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
       ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1)
+      : "memory");
+}
+
+// The 16-bit form: four k-steps of 16 values; the descriptors advance by kA, kB (16-byte units) from step to step.
+template <int kA = 2, int kB = 2>
+__device__ __forceinline__ void umma_f16_block(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate,
+                                               uint32_t bar0 = 0, uint32_t bar1 = 0) {
+  asm volatile(
+      "{\n\t.reg .pred q, f, t, u, v;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 f, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a1, %1, %7;\n\tadd.s64 a2, %1, %8;\n\tadd.s64 a3, %1, %9;\n\t"
+      "add.s64 b1, %2, %10;\n\tadd.s64 b2, %2, %11;\n\tadd.s64 b3, %2, %12;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.and.b32 u, %5, 0, q;\n\tsetp.ne.and.b32 v, %6, 0, q;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, f;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n\t"
+      "@u tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+      "@v tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1), "n"(kA), "n"(2 * kA), "n"(3 * kA), "n"(kB),
+        "n"(2 * kB), "n"(3 * kB)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_warp(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {  // a single k-step
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_warp(uint64_t* bar) {  // whole warp, one elected lane; arrives when its prior MMAs retire
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
       : "memory");
 }
 

@@ -82,10 +82,6 @@ struct GemmParams {
   int M, N, K;
   int kb_per_split;
   ArParams ar;
-  // Grouped (mixture-of-experts) mode: blockIdx.y indexes tile_map = (expert, token tile inside the expert), rows of
-  // x / out are the expert-sorted token rows, expert e owning rows [expert_offsets[e], expert_offsets[e+1]).
-  const int2* tile_map = nullptr;
-  const int* expert_offsets = nullptr;
   AgParams ag;
   int stages = 0;  // depth of the shared-memory ring actually used (<= GemmCfg::kStages); fewer stages = more CTAs per SM
   // Split-K with the splits of a tile launched as one thread-block cluster: the partial sums meet in distributed shared
@@ -182,9 +178,9 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   const int lane = threadIdx.x & 31;
   const bool gather = p.ag.world > 1;
   pdl_trigger();
-  // Modes whose prologue already reads memory an earlier kernel wrote (the gathered-activation epoch, the route plan
-  // of the grouped mode) wait for their predecessor right away; the plain GEMM first sets up barriers and TMEM.
-  const bool early_inputs = gather || p.tile_map != nullptr;
+  // The all-gather mode's prologue already reads memory an earlier kernel wrote (the epoch) and waits for its predecessor
+  // right away; the plain GEMM first sets up barriers and TMEM.
+  const bool early_inputs = gather;
   if (early_inputs) pdl_wait();
   const uint32_t ag_epoch = gather ? *p.ag.epoch : 0u;
   if (gather && int(blockIdx.x) < p.ag.push_ctas) {
@@ -256,14 +252,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   }
   const int n_tiles_x = int(gridDim.x) - (gather ? p.ag.push_ctas : 0);
   const int n0 = n_tile * kTileN;
-  int t0 = t_tile * BT, row_end = p.M, expert = 0;
-  if (p.tile_map) {
-    const int2 tm = p.tile_map[t_tile];
-    if (tm.x < 0) return;  // padding entry of the tile map: uniform for the whole CTA, nothing allocated yet
-    expert = tm.x;
-    t0 = p.expert_offsets[expert] + tm.y * BT;
-    row_end = p.expert_offsets[expert + 1];
-  }
+  const int t0 = t_tile * BT, row_end = p.M;
   const int kb_total = p.K / kBlockK;
   const int kb0 = split * p.kb_per_split;
   const int kb1 = min(kb_total, kb0 + p.kb_per_split);
@@ -338,14 +327,13 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     }
     __syncwarp();
     const uint32_t tiles_addr = smem_u32(tiles), full_addr = smem_u32(full);
-    const int third = p.tile_map ? expert : -1;
     int s = 0;
     uint32_t ring_phase = 0;  // ring position and wrap parity, kept incrementally: the depth is a run-time value
     for (int i = 0; shard_ready && i < nkb; ++i) {
       const bool fresh = i >= w_ahead;  // the first pass of the plain mode is armed and its weight tile on the way already
       if (fresh && !mbar_wait_warp(&empty[s], ring_phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer)) break;
       const uint32_t a = tiles_addr + s * Cfg::kStageBytes;
-      tma_load_stage(a, a + kTileN * kBlockK, &tmap_w, xmap, full_addr + s * 8, Cfg::kStageBytes, fresh, (kb0 + i) * kBlockK, n0, third, t0);
+      tma_load_stage(a, a + kTileN * kBlockK, &tmap_w, xmap, full_addr + s * 8, Cfg::kStageBytes, fresh, (kb0 + i) * kBlockK, n0, -1, t0, (kb0 + i) * kBlockK);
       if (++s == stages) { s = 0; ring_phase ^= 1u; }
     }
   } else if (warp == 1) {
@@ -379,7 +367,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     float acc[CW];
 #pragma unroll
     for (int tt = 0; tt < CW; ++tt) acc[tt] = 0.f;
-    const float* wsc = p.w_scale + (size_t(expert) * n_tiles_x + n_tile) * kb_total;
+    const float* wsc = p.w_scale + size_t(n_tile) * kb_total;
     // The token multipliers are fetched now, under the main loop, into this warp's own smem slice (no cross-warp
     // sync needed); at the end they cost a broadcast LDS instead of an exposed global load per column.  In gather
     // mode they only exist once the peers' flags arrived, so that mode reads them at the end.
@@ -643,16 +631,10 @@ template <int BT>
 static int launch_gemm(const void* w, const float* w_scale, const void* x, const float* x_scale, void* out,
                        const void* residual, float* ws, size_t ws_bytes, int* counters, int counters_len, int* status,
                        int M, int N, int K, int splits, cudaStream_t stream, const ArParams* ar = nullptr,
-                       int experts = 0, const int2* tile_map = nullptr, const int* expert_offsets = nullptr,
-                       int map_len = 0, const AgParams* ag = nullptr) {
+                       const AgParams* ag = nullptr) {
   using Cfg = GemmCfg<BT>;
   CUtensorMap tw, tx;
-  if (experts > 0) {
-    if (make_tmap_3d(&tw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, K, N, experts, uint64_t(K), uint64_t(K) * N, kBlockK, kTileN, 1))
-      return -2;
-  } else if (make_tmap_2d(&tw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, kTileN, kBlockK)) {
-    return -2;
-  }
+  if (make_tmap_2d(&tw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, kTileN, kBlockK)) return -2;
   CUtensorMap tx_alt;
   if (ag) {  // x = this rank's gathered buffer: one map per half
     if (make_tmap_2d(&tx, ag->x_full[ag->rank], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, K, BT, kBlockK)) return -3;
@@ -661,7 +643,7 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
     if (make_tmap_2d(&tx, x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, K, BT, kBlockK)) return -3;
     tx_alt = tx;
   }
-  const int n_tiles = (N + kTileN - 1) / kTileN, t_tiles = experts > 0 ? map_len : (M + BT - 1) / BT;
+  const int n_tiles = (N + kTileN - 1) / kTileN, t_tiles = (M + BT - 1) / BT;
   const int kb_total = K / kBlockK;
   if (splits < 1) splits = 1;
   if (splits > kb_total) splits = kb_total;
@@ -672,7 +654,7 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
     if (n_tiles * t_tiles > counters_len) return -5;
   }
   GemmParams p{w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(residual),
-               ws, counters, status, M, N, K, kb_per, ArParams{}, tile_map, expert_offsets};
+               ws, counters, status, M, N, K, kb_per};
   if (ar) {
     if (size_t(n_tiles) * t_tiles * BT * kTileN > ar->half_elems) return -8;
     p.ar = *ar;
@@ -689,7 +671,7 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
   }
   if (ag) p.ag = *ag;
   const int extra_x = ag ? ag->push_ctas : 0;
-  // Ring depth.  The fused-collective modes stage their output in the ring and keep all of it.  A plain or grouped
+  // Ring depth.  The fused-collective modes stage their output in the ring and keep all of it.  A plain
   // launch whose grid is larger than one wave of SMs takes a shallower ring instead, so that two or three CTAs share an
   // SM and one CTA's ramp-up and epilogue hide under another's main loop.
   p.stages = Cfg::kStages;
@@ -701,7 +683,7 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
   }
   const int smem_bytes = p.stages * Cfg::kStageBytes + 1024 + 256 + Cfg::kXsBytes + Cfg::kWsBytes;
   static const bool cluster_ok = [] { const char* e = getenv("MFQ_GEMM_CLUSTER_REDUCE"); return !e || atoi(e) != 0; }();
-  if (cluster_ok && !ar && !ag && !tile_map && splits > 1 && splits <= 8) {
+  if (cluster_ok && !ar && !ag && splits > 1 && splits <= 8) {
     // A cluster is placed inside one GPC, so a grid that needs nearly every SM (144 CTAs in clusters of 3, one CTA per
     // SM) does not fit in one wave although the CTA count says it would; the driver is asked how many clusters of this
     // shape can be resident, and the ring is made shallower (more CTAs per SM) until the whole grid is.
@@ -894,32 +876,15 @@ extern "C" int mfq_fp8_gemm_allgather(const void* w, const float* w_scale, const
   ag.push_done = static_cast<uint32_t*>(push_done);
   int rc;
   switch (token_tile) {
-    case 16: rc = mfq::launch_gemm<16>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, 0, nullptr, nullptr, 0, &ag); break;
-    case 32: rc = mfq::launch_gemm<32>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, 0, nullptr, nullptr, 0, &ag); break;
-    case 64: rc = mfq::launch_gemm<64>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, 0, nullptr, nullptr, 0, &ag); break;
-    case 128: rc = mfq::launch_gemm<128>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, 0, nullptr, nullptr, 0, &ag); break;
+    case 16: rc = mfq::launch_gemm<16>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, &ag); break;
+    case 32: rc = mfq::launch_gemm<32>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, &ag); break;
+    case 64: rc = mfq::launch_gemm<64>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, &ag); break;
+    case 128: rc = mfq::launch_gemm<128>(w, w_scale, nullptr, nullptr, out, nullptr, nullptr, 0, nullptr, 0, status, M, N, K, 1, stream, nullptr, &ag); break;
     default: return -1;
   }
   if (rc != 0) return rc;
   bump_epoch_kernel<<<1, 1, 0, stream>>>(static_cast<uint32_t*>(epoch));
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
-}
-
-// Grouped GEMM over expert-sorted token rows (mixture of experts): w [E, N, K] E4M3 with w_scale [E, N/128, K/128];
-// x / out rows are sorted by expert, expert e owning rows [expert_offsets[e], expert_offsets[e+1]); tile_map holds
-// map_len (expert, token-tile) pairs, entries with expert < 0 are padding.  No split-K, no residual.
-extern "C" int mfq_fp8_gemm_grouped(const void* w, const float* w_scale, const void* x, const float* x_scale, void* out,
-                                    int* status, int rows, int N, int K, int experts, const void* tile_map,
-                                    const int* expert_offsets, int map_len, int token_tile, cudaStream_t stream) {
-  if (K % 128 != 0 || rows <= 0 || N <= 0 || experts <= 0 || map_len <= 0 || N % 128 != 0) return -1;
-  const int2* tm = static_cast<const int2*>(tile_map);
-  switch (token_tile) {
-    case 16: return mfq::launch_gemm<16>(w, w_scale, x, x_scale, out, nullptr, nullptr, 0, nullptr, 0, status, rows, N, K, 1, stream, nullptr, experts, tm, expert_offsets, map_len);
-    case 32: return mfq::launch_gemm<32>(w, w_scale, x, x_scale, out, nullptr, nullptr, 0, nullptr, 0, status, rows, N, K, 1, stream, nullptr, experts, tm, expert_offsets, map_len);
-    case 64: return mfq::launch_gemm<64>(w, w_scale, x, x_scale, out, nullptr, nullptr, 0, nullptr, 0, status, rows, N, K, 1, stream, nullptr, experts, tm, expert_offsets, map_len);
-    case 128: return mfq::launch_gemm<128>(w, w_scale, x, x_scale, out, nullptr, nullptr, 0, nullptr, 0, status, rows, N, K, 1, stream, nullptr, experts, tm, expert_offsets, map_len);
-    default: return -1;
-  }
 }
 
 // ---------------------------------------------------------------------------------------------------------
