@@ -32,7 +32,7 @@
 // All waits are bounded; a cluster barrier before the TMEM release keeps a CTA alive while its peer may still read it.
 //
 // The reference has no FP8 tensor-core path (mfq/kernels/cuda/fp8_sq.cu:564-592 decodes to fp16 for wmma / cuBLAS).
-#include "common.cuh"
+#include "pair.cuh"
 
 namespace mfq {
 namespace {
@@ -59,70 +59,12 @@ struct PairParams {
   const __nv_bfloat16* residual;
   int* status;
   int M, N, K;
+  int kb_per_split;  // split sums: K blocks of a partial sum
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t map_to_cta(const void* smem_ptr, uint32_t cta) {  // cluster address of a peer's variable
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(smem_ptr)), "r"(cta));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {  // one warp in EACH CTA of the pair
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// One stage: the weight tile and the token half-tile, both completing on the barrier at `bar_cluster_addr` (the leader's, from
-// either CTA), which the leader arms with `bytes` (0: the peer's call, it does not arm).  Whole warp, one elected lane issues.
-__device__ __forceinline__ void tma_load_stage_pair(uint32_t smem_a, uint32_t smem_b, const CUtensorMap* map_a, const CUtensorMap* map_b,
-                                                    uint32_t bar_cluster_addr, uint32_t bar_local, uint32_t bytes, int x, int ya, int yb) {
-  asm volatile(
-      "{\n\t.reg .pred q, e;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 e, %6, 0, q;\n\t"
-      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%5], %6;\n\t"
-      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%7, %8}], [%4];\n\t"
-      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%3, {%7, %9}], [%4];\n\t}"
-      ::"r"(smem_a), "r"(smem_b), "l"(reinterpret_cast<uint64_t>(map_a)), "l"(reinterpret_cast<uint64_t>(map_b)), "r"(bar_cluster_addr),
-        "r"(bar_local), "r"(bytes), "r"(x), "r"(ya), "r"(yb)
-      : "memory");
-}
-// The pair's form of umma_f8f6f4_block: four k-steps into a fresh accumulator, then two commits, each of which arrives on the
-// barrier at that offset in BOTH CTAs once these MMAs have retired.
-__device__ __forceinline__ void umma_f8f6f4_block_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t bar0, uint32_t bar1) {
-  asm volatile(
-      "{\n\t.reg .pred q, f, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t.reg .b16 both;\n\tmov.b16 both, 3;\n\t"
-      "setp.ne.b32 f, 0, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
-      "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\t"
-      "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, f;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a1, b1, %3, t;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a2, b2, %3, t;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a3, b3, %3, t;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%4], both;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], both;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(bar0), "r"(bar1)
-      : "memory");
-}
-// Relaxed: what it orders are tensor-memory reads, which have completed (wait::ld, fence::before_thread_sync) before it; a
-// release at cluster scope would also drain this warp's global accesses, about a microsecond per block.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
-
-template <int BT>
+// kSplitSums: every kb_per_split K blocks are summed on their own and the partial sums added in order -- what the one-SM kernel's split-K
+// form does, so that a product gives the same bits on either kernel.
+template <int BT, bool kSplitSums>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BT>::kThreads, 1)
 fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                      const PairParams p) {
@@ -208,7 +150,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
              mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma);
         if (!ok) break;
         tc_fence_after();
-        umma_f8f6f4_block_pair(tmem_base + buf * BT, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc,
+        umma_f8f6f4_block_pair(tmem_base + buf * BT, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc, 0u,
                                empty_addr + s * 8, acc_full_addr + buf * 8);
         if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
         if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
@@ -243,7 +185,24 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       if (ws_cached)
         for (int j = lane; j < nkb; j += 32) ws_w[j] = __ldg(wsc + j);
       __syncwarp();
+      float total[kSplitSums ? CW : 1];
+      int left = p.kb_per_split;
+      if constexpr (kSplitSums) {
+#pragma unroll
+        for (int tt = 0; tt < CW; ++tt) total[tt] = 0.f;
+      }
       for (int i = 0; i < nkb; ++i) {
+        if constexpr (kSplitSums) {
+          if (left == 0) {
+#pragma unroll
+            for (int tt = 0; tt < CW; ++tt) {
+              total[tt] += acc[tt];
+              acc[tt] = 0.f;
+            }
+            left = p.kb_per_split;
+          }
+          --left;
+        }
         if (!ready) ok = mbar_wait_warp(&acc_full[buf], phase, abort_flag, p.status, kStatusTimeoutEpilogue);
         if (!ok) break;
         tc_fence_after();
@@ -267,6 +226,10 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           for (int j = 0; j < 32; j += 2) fma2(acc[c * 32 + j], acc[c * 32 + j + 1], r[c & 1][j], r[c & 1][j + 1], s);
         }
       }
+      if constexpr (kSplitSums) {
+#pragma unroll
+        for (int tt = 0; tt < CW; ++tt) acc[tt] = total[tt] + acc[tt];
+      }
       if (ok && n < p.N) {
         const int tl = min(BT, p.M - t0);
         // residual and output may be one buffer: all loads first, or every load would wait behind the store before it
@@ -276,8 +239,13 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 #pragma unroll
           for (int tt = 0; tt < CW; ++tt)
             res[tt] = (col0 + tt < tl) ? __ldcg(rp + size_t(t0 + col0 + tt) * p.N + n) : (unsigned short)0;
+// the roundings of the one-SM kernel: product and sum in one where its splits meet in a cluster (up to 8), else one by one
+          const bool fused = kSplitSums && (nkb + p.kb_per_split - 1) / p.kb_per_split <= 8;
 #pragma unroll
-          for (int tt = 0; tt < CW; ++tt) acc[tt] = fmaf(acc[tt], xs_w[tt], __uint_as_float(uint32_t(res[tt]) << 16));
+          for (int tt = 0; tt < CW; ++tt) {
+            const float add = __uint_as_float(uint32_t(res[tt]) << 16);
+            acc[tt] = fused ? __fmaf_rn(acc[tt], xs_w[tt], add) : __fadd_rn(__fmul_rn(acc[tt], xs_w[tt]), add);
+          }
         } else {
 #pragma unroll
           for (int tt = 0; tt < CW; ++tt) acc[tt] *= xs_w[tt];
@@ -299,9 +267,9 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int BT>
+template <int BT, bool kSplitSums>
 int launch_pair(const void* w, const float* w_scale, const void* x, const float* x_scale, void* out, const void* residual,
-                int* status, int M, int N, int K, cudaStream_t stream) {
+                int* status, int M, int N, int K, int kb_per_split, cudaStream_t stream) {
   using Cfg = PairCfg<BT>;
   CUtensorMap tw, tx;
   if (make_tmap_2d(&tw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, kRows, kBK)) return -2;
@@ -310,28 +278,30 @@ int launch_pair(const void* w, const float* w_scale, const void* x, const float*
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -6;
   if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(fp8_gemm_pair_kernel<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(fp8_gemm_pair_kernel<BT, kSplitSums>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
       return -6;
     attr_set[dev] = true;
   }
-  PairParams p{w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(residual), status, M, N, K};
+  PairParams p{w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(residual), status, M, N, K, kb_per_split};
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles = (N / (2 * kRows)) * ((M + BT - 1) / BT);
   const int clusters = tiles < sms / 2 ? tiles : sms / 2;
-  launch_kernel(fp8_gemm_pair_kernel<BT>, dim3(2 * clusters), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tw, tx, p);
+  launch_kernel(fp8_gemm_pair_kernel<BT, kSplitSums>, dim3(2 * clusters), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 
 }  // namespace
 }  // namespace mfq
 
-// Two-SM form of mfq_fp8_gemm for wide batches.  N % 256 == 0, K % 128 == 0, token_tile in {128, 256}; no split-K.
+// Two-SM form of mfq_fp8_gemm for wide batches.  N % 256 == 0, K % 128 == 0, token_tile in {128, 256}; no split-K.  kb_per_split > 0
+// (tile 128): the sums are formed as by mfq_fp8_gemm with that many K blocks per split, bit for bit.
 extern "C" int mfq_fp8_gemm_pair(const void* w, const float* w_scale, const void* x, const float* x_scale, void* out,
-                                 const void* residual, int* status, int M, int N, int K, int token_tile,
+                                 const void* residual, int* status, int M, int N, int K, int token_tile, int kb_per_split,
                                  cudaStream_t stream) {
-  if (K % 128 != 0 || N % 256 != 0 || M <= 0) return -1;
-  if (token_tile == 128) return mfq::launch_pair<128>(w, w_scale, x, x_scale, out, residual, status, M, N, K, stream);
-  if (token_tile == 256) return mfq::launch_pair<256>(w, w_scale, x, x_scale, out, residual, status, M, N, K, stream);
+  if (K % 128 != 0 || N % 256 != 0 || M <= 0 || kb_per_split < 0 || (kb_per_split && token_tile != 128)) return -1;
+  if (kb_per_split) return mfq::launch_pair<128, true>(w, w_scale, x, x_scale, out, residual, status, M, N, K, kb_per_split, stream);
+  if (token_tile == 128) return mfq::launch_pair<128, false>(w, w_scale, x, x_scale, out, residual, status, M, N, K, 0, stream);
+  if (token_tile == 256) return mfq::launch_pair<256, false>(w, w_scale, x, x_scale, out, residual, status, M, N, K, 0, stream);
   return -1;
 }

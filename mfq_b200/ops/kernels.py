@@ -85,6 +85,19 @@ _MEASURED_SPLITS = {(48, 32): 4}
 PAIR_MIN_ROWS = 65  # batches at least this wide may take the two-SM GEMM (``csrc/fp8_gemm_2cta.cu``)
 
 
+def split_blocks(m: int, n: int, k: int) -> int:
+    """K blocks per split that the one-SM kernel would sum on their own for this shape, 0 if it would not split.  The two-SM kernel
+    forms its sums alike, so the bits of a product do not depend on which of the two a shape takes."""
+    blocks = k // 128
+    per = math.ceil(blocks / pick_splits(m, n, k))
+    splits = math.ceil(blocks / per)
+    partials = splits * math.ceil(n / 128) * math.ceil(m / 128) * 128 * 128 * 4
+    return per if splits > 1 and partials <= SPLIT_SCRATCH_BYTES else 0  # beyond the scratch it cannot split
+
+
+SPLIT_SCRATCH_BYTES = 64 << 20  # the workspace's split-K scratch
+
+
 def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     """Token tile of the two-SM GEMM for this shape, 0 = use the one-SM kernel.  ``MFQ_GEMM_PAIR`` = 0 / 128 / 256
     overrides the choice.
@@ -103,6 +116,8 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     tiles = {t: n // 256 * math.ceil(m / t) for t in (128, 256)}
     if 2 * tiles[128] <= pairs and blocks > 64:
         return 0
+    if split_blocks(m, n, k):
+        return 128
     cost = {t: math.ceil(tiles[t] / pairs) * (ramp + per * blocks) for t, ramp, per in ((128, 2.9, 0.306), (256, 6.7, 0.506))}
     return 128 if cost[128] <= cost[256] else 256
 
@@ -124,12 +139,14 @@ def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scal
         check(rc, "fp8_gemv")
         return out
     ws = Workspace.get(x_q.device)
+    per_split = 0
     if pair is None:
         pair = pair_tile(m, n, k) if splits is None and token_tile is None else 0
+        per_split = split_blocks(m, n, k) if pair == 128 else 0
     if pair:
         assert pair in (128, 256) and n % 256 == 0
         rc = lib().mfq_fp8_gemm_pair(ptr(w_q), ptr(w_scale), ptr(x_q), ptr(x_scale), ptr(out), ptr(residual), ptr(ws.status),
-                                     m, n, k, pair, stream_ptr())
+                                     m, n, k, pair, per_split, stream_ptr())
         check(rc, "fp8_gemm_pair")
         return out
     bt = token_tile or _token_tile(m)

@@ -19,7 +19,7 @@ _vp, _i, _f, _sz = C.c_void_p, C.c_int, C.c_float, C.c_size_t
 
 _SIGNATURES = {
     "mfq_fp8_gemm": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
-    "mfq_fp8_gemm_pair": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "mfq_fp8_gemm_pair": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "mfq_fp8_gemm_allreduce": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp,
                                _vp, _sz, _i, _vp],
     "mfq_fp8_gemm_allgather": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp],
@@ -48,6 +48,7 @@ _SIGNATURES = {
     "mfq_fp8_gemv": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "mfq_fp8_gemv_act": [_vp, _vp, _vp, _i, _vp, _f, _vp, _vp, _i, _i, _i, _i, _vp],
     "mfq_fp8_gemv_grouped": [_vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _vp],
+    "mfq_w4_gemv": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "mfq_attn_prefill_d256": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _vp],
     "mfq_attn_prefill_bf16": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _vp],
 }
