@@ -20,7 +20,7 @@
 // split-K partials are reduced by the last-arriving CTA in split order (deterministic).  Waits are bounded.
 // Reference counterparts: nint_matmul_kernel / nint_matmul_tiled_prefill_kernel (mfq/kernels/cuda/nint_matmul.cu),
 // which decode rows on CUDA cores (wmma for prefill) and have no tensor-memory path.
-#include "common.cuh"
+#include "w4_decode.cuh"
 
 namespace mfq {
 
@@ -74,7 +74,7 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
 
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   const int n_tile = blockIdx.x, t_tile = blockIdx.y, split = blockIdx.z;
   const int n_tiles = gridDim.x;
   const int t0 = t_tile * BT;
@@ -98,7 +98,7 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_acc = *tmem_slot;
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait();
 
   if (warp == 0) {
@@ -127,23 +127,23 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(128, BT, 1, 1, 0, 0);  // bf16 x bf16, both K-major
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % Cfg::kStages, a = i % Cfg::kAStages;
-        if (!mbar_wait(&full[s], (i / Cfg::kStages) & 1, abort_flag, p.status, kStatusTimeoutMma)) break;
-        if (!mbar_wait(&a_ready[a], (i / Cfg::kAStages) & 1, abort_flag, p.status, kStatusTimeoutMma)) break;
-        tc_fence_after();
-        const uint32_t a_addr = smem_u32(a_tiles + a * Cfg::kABytes);
-        const uint32_t b_addr = smem_u32(stages + s * Cfg::kStageBytes + Cfg::kXOffset);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_f16(tmem_acc, umma_desc_k_sw128(a_addr + ks * 32), umma_desc_k_sw128(b_addr + ks * 32), idesc, (i | ks) != 0);
-        tc_commit(&a_free[a]);   // the decoded tile may be overwritten once these MMAs retire
-        tc_commit(&empty[s]);    // ... and so may the activation tile of the stage
-      }
-      tc_commit(acc_done);
+    constexpr uint32_t idesc = umma_idesc(128, BT, 1, 1, 0, 0);  // bf16 x bf16, both K-major
+    constexpr uint64_t kAStep = uint64_t(Cfg::kABytes >> 4), kStageStep = uint64_t(Cfg::kStageBytes >> 4);
+    const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(a_tiles)), b_desc0 = umma_desc_k_sw128(smem_u32(stages) + Cfg::kXOffset);
+    const uint32_t a_free_addr = smem_u32(a_free), empty_addr = smem_u32(empty);
+    int s = 0, a = 0;
+    uint32_t phase = 0, a_phase = 0;
+    for (int i = 0; i < nkb; ++i) {
+      if (!mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma)) break;
+      if (!mbar_wait_warp(&a_ready[a], a_phase, abort_flag, p.status, kStatusTimeoutMma)) break;
+      tc_fence_after();
+      // once these MMAs retire the decoded tile may be overwritten, and so may the activation tile of the stage
+      umma_f16_block(tmem_acc, a_desc0 + uint64_t(a) * kAStep, b_desc0 + uint64_t(s) * kStageStep, idesc, i > 0 ? 1u : 0u, a_free_addr + a * 8,
+                     empty_addr + s * 8);
+      if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
+      if (++a == Cfg::kAStages) { a = 0; a_phase ^= 1u; }
     }
+    tc_commit_warp(acc_done);
   } else {
     // ----- decode warps, then epilogue -----
     // Two teams of four warps (thread = weight row) take alternate K blocks, so two blocks are being converted at
@@ -173,46 +173,12 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
         if (w == 0 || left == 0) {  // a new group starts: fetch (s, s) and (-b, -b) as bf16x2
           if (w != 0) { ++local; left = wpg; }
           const uint32_t g = gsm[local * kW4TileN];
-          asm("prmt.b32 %0, %1, %1, 0x1010;" : "=r"(s2) : "r"(g));
-          asm("prmt.b32 %0, %1, %1, 0x3232;" : "=r"(b2) : "r"(g));
+          w4_params(g, s2, b2);
         }
         --left;
-        uint4 o;
-        uint32_t* ov = reinterpret_cast<uint32_t*>(&o);
-        if constexpr (KIND == 0) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t pair = ((words[w] >> (4 * j)) & 0x000F000Fu) | 0x43004300u;  // bf16 (128 + c, 128 + c')
-            uint32_t qf;  // (c, c') exactly: integers below 256 are exact in bf16, so is the subtraction
-            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(qf) : "r"(pair), "r"(0x43004300u));
-            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(ov[j]) : "r"(qf), "r"(s2), "r"(b2));  // s * c - b, one rounding
-          }
-        } else {
-          // E2M1 magnitudes {0, .5, 1, 1.5, 2, 3, 4, 6} as bf16 = high bytes {00,3F,3F,3F,40,40,40,40}, low bytes
-          // {00,00,80,C0,00,40,80,C0}: byte-permute instructions look four codes up at once (selector = code & 7)
-          const uint32_t idx = words[w] & 0x77777777u;
-          uint32_t hiA, hiB, loA, loB;  // A: nibbles 0..3 (even columns), B: nibbles 4..7 (odd columns)
-          asm("prmt.b32 %0, %1, %2, %3;" : "=r"(hiA) : "r"(0x3F3F3F00u), "r"(0x40404040u), "r"(idx & 0xFFFFu));
-          asm("prmt.b32 %0, %1, %2, %3;" : "=r"(hiB) : "r"(0x3F3F3F00u), "r"(0x40404040u), "r"(idx >> 16));
-          asm("prmt.b32 %0, %1, %2, %3;" : "=r"(loA) : "r"(0xC0800000u), "r"(0xC0804000u), "r"(idx & 0xFFFFu));
-          asm("prmt.b32 %0, %1, %2, %3;" : "=r"(loB) : "r"(0xC0800000u), "r"(0xC0804000u), "r"(idx >> 16));
-          uint32_t a01, a23, b01, b23;  // (bf16 n0, bf16 n1), (n2, n3), (n4, n5), (n6, n7)
-          asm("prmt.b32 %0, %1, %2, 0x5140;" : "=r"(a01) : "r"(loA), "r"(hiA));
-          asm("prmt.b32 %0, %1, %2, 0x7362;" : "=r"(a23) : "r"(loA), "r"(hiA));
-          asm("prmt.b32 %0, %1, %2, 0x5140;" : "=r"(b01) : "r"(loB), "r"(hiB));
-          asm("prmt.b32 %0, %1, %2, 0x7362;" : "=r"(b23) : "r"(loB), "r"(hiB));
-          uint32_t mag[4];  // word j = (column 2j, column 2j+1) = (nibble j, nibble j + 4)
-          asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(mag[0]) : "r"(a01), "r"(b01));
-          asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(mag[1]) : "r"(a01), "r"(b01));
-          asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(mag[2]) : "r"(a23), "r"(b23));
-          asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(mag[3]) : "r"(a23), "r"(b23));
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t sign = ((words[w] >> (4 * j)) & 0x00080008u) << 12;  // code bit 3 -> bf16 sign bit
-            asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(ov[j]) : "r"(mag[j] | sign), "r"(s2));  // exact: s2 is a power of two
-          }
-        }
-        *reinterpret_cast<uint4*>(dst_row + ((w ^ (row & 7)) << 4)) = o;  // 128-byte swizzle: chunk ^= row % 8
+        uint32_t o[4];
+        w4_decode<KIND>(words[w], s2, b2, o);
+        *reinterpret_cast<uint4*>(dst_row + ((w ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);  // 128-byte swizzle: chunk ^= row % 8
       }
       fence_proxy_async_smem();  // generic-proxy stores -> tensor-core (async proxy) reads
       __syncwarp();

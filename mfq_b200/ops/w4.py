@@ -20,6 +20,7 @@ from . import kernels as K
 from .lib import Workspace, check, lib, ptr, stream_ptr
 
 TILE_N, BLOCK_K = 128, 64
+GEMV_ROWS = 16  # up to this many rows the codes are streamed through registers (csrc/w4_gemv.cu)
 _NIBBLE_COLUMN = np.array([0, 2, 4, 6, 1, 3, 5, 7])  # nibble n of a word holds column _NIBBLE_COLUMN[n] of its 8
 
 
@@ -191,6 +192,10 @@ def w4_gemm(x: torch.Tensor, w: W4Weight, *, residual: torch.Tensor | None = Non
             y = y + residual.float()
         return y.to(torch.bfloat16)
     out = torch.empty((m, w.n), dtype=torch.bfloat16, device=x.device) if out is None else out
+    if token_tile is None and splits is None and m <= GEMV_ROWS and K.gemv_enabled():
+        check(lib().mfq_w4_gemv(ptr(w.packed), ptr(w.group), ptr(x), ptr(out), ptr(residual), m, w.n, k, w.group_size, w.kind, stream_ptr()),
+              "w4_gemv")
+        return out
     bt = token_tile or K._token_tile(m)
     sp = K.pick_splits(m, w.n, k // 2) if splits is None else splits  # K blocks are 64 wide here: same work model
     ws = Workspace.get(x.device)

@@ -67,3 +67,41 @@ def test_mxfp4_kind_matches_checkpoint_dequantization(m, n, k):
     check_status()
     want = x.float() @ torch.from_numpy(F.dequantize(t)).cuda().T
     assert_close(got.float(), want, rel=1e-2, what="mxfp4 gemm")
+
+
+@pytest.mark.parametrize("gs", [16, 24, 32, 64])
+@pytest.mark.parametrize("m,n,k", [(1, 128, 192), (3, 200, 960), (8, 264, 4224), (9, 520, 576), (16, 128, 8256)])
+def test_streamed_codes_match_reference(m, n, k, gs):
+    """Up to 16 rows the codes go from memory into MMA fragments: odd counts of K blocks, rows that end inside a CTA, groups that
+    do and do not hold a thread's 32 codes."""
+    require_gpu_lib()
+    if k % gs:
+        k = k // 192 * 192
+    w = _weight(n, k, gs, m + k)
+    g = torch.Generator(device="cuda").manual_seed(k + gs)
+    x = torch.randn((m, k), generator=g, device="cuda").to(torch.bfloat16)
+    res = torch.randn((m, n), generator=g, device="cuda").to(torch.bfloat16)
+    wd = w.to("cuda")
+    want = x.double() @ w4.dequantize(w).cuda().double().T + res.double()
+    got = w4.w4_gemm(x, wd, residual=res)
+    check_status()
+    # fp32 sums of K terms and one rounding to bf16: half an ulp of 2^-8, and K 2^-24 of the terms' size
+    bound = want.abs() * 2.0 ** -8 + (x.double().abs() @ w4.dequantize(w).cuda().double().abs().T) * k * 2.0 ** -24
+    assert bool(((got.double() - want).abs() <= bound).all())
+    h = res.clone()
+    w4.w4_gemm(x, wd, residual=h, out=h)  # residual and output in one buffer
+    assert torch.equal(h, got)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 256, 192), (16, 200, 2048)])
+def test_streamed_mxfp4_codes_match_the_tensor_core_form(m, n, k):
+    require_gpu_lib()
+    rng = np.random.default_rng(m + n)
+    w = w4.repack(rng.integers(0, 16, (n, k)).astype(np.uint8), np.zeros((n, k // 32), np.float32), np.zeros((n, k // 32), np.float32), 32)
+    e = rng.integers(118, 124, w.group.shape).astype(np.int32) << 7
+    w = w4.W4Weight(w.packed, torch.from_numpy(e), n, k, 32, kind=1).to("cuda")
+    x = torch.randn((m, k), device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).to(torch.bfloat16)
+    got, want = w4.w4_gemm(x, w), w4.w4_gemm(x, w, splits=1)
+    check_status()
+    # both multiply the same bf16 weights and round once: the orders of their fp32 sums may differ by one bf16 step
+    assert_close(got.float(), want.float(), rel=2.0 ** -7, what="mxfp4 streamed")
