@@ -20,8 +20,13 @@
 // addition to the fp32 stream, plain fp32) is shared by the three kernels (dense_common.cuh).  Waits are bounded as everywhere (common.cuh).
 #include "dense_common.cuh"
 
+// the same product on pairs of SMs (dense_pair.cu)
+extern "C" int mfq_dense_pair(const void* w, const void* x, int ldx, void* out, int ldo, const float* bias, int M, int N, int K, int epilogue,
+                              float alpha, float limit, const void* table, const int* ids, int token_tile, int* status, cudaStream_t stream);
+
 namespace mfq {
 
+constexpr int kDensePair = -2;  // as a number of splits: the product runs on pairs of SMs
 constexpr int kDnTileN = 128, kDnBlockK = 64, kDnThreads = 256;
 constexpr int kDnABytes = kDnTileN * kDnBlockK * 2;
 
@@ -109,7 +114,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   if (p.tiles) pdl_wait();  // the tile list comes from the kernel before
   DenseAt at;
   if (!dense_locate(p, kDnTileN, BT, at)) return;  // all CTAs of a cluster
@@ -128,44 +133,46 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_acc = *tmem_slot;
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
+  // Loads and MMAs are issued by an elected lane of a converged warp (common.cuh: umma_f8f6f4_block says why).
   if (warp == 0) {
+    const int ahead = min(nkb, Cfg::kStages);
     if (lane == 0) {
       tma_prefetch_desc(&tmap_w);
       tma_prefetch_desc(&tmap_x);
-      const int ahead = min(nkb, Cfg::kStages);
       for (int i = 0; i < ahead; ++i) {  // weights never depend on the previous kernel
         mbar_expect_tx(&full[i], Cfg::kStageBytes);
         tma_load_2d(base + i * Cfg::kStageBytes, &tmap_w, &full[i], (kb0 + i) * kDnBlockK, at.w_row);
       }
-      pdl_wait();
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % Cfg::kStages;
-        uint8_t* st = base + s * Cfg::kStageBytes;
-        if (i >= ahead) {
-          if (!mbar_wait(&empty[s], ((i / Cfg::kStages) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutProducer)) break;
-          mbar_expect_tx(&full[s], Cfg::kStageBytes);
-          tma_load_2d(st, &tmap_w, &full[s], (kb0 + i) * kDnBlockK, at.w_row);
-        }
-        tma_load_2d(st + kDnABytes, &tmap_x, &full[s], at.x_col + (kb0 + i) * kDnBlockK, t0);
-      }
+    }
+    __syncwarp();
+    pdl_wait();
+    const uint32_t base_addr = smem_u32(base), full_addr = smem_u32(full);
+    const int x_col = __shfl_sync(0xffffffffu, at.x_col, 0), w_row = __shfl_sync(0xffffffffu, at.w_row, 0), t_row = __shfl_sync(0xffffffffu, t0, 0);
+    int s = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < nkb; ++i) {
+      if (i >= ahead && !mbar_wait_warp(&empty[s], phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer)) break;
+      const uint32_t st = base_addr + s * Cfg::kStageBytes;
+      const int k = (kb0 + i) * kDnBlockK;
+      tma_load_stage(st, st + kDnABytes, &tmap_w, &tmap_x, full_addr + s * 8, Cfg::kStageBytes, i >= ahead, k, w_row, -1, t_row, x_col + k);
+      if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(128, BT, 1, 1, 0, 0);
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % Cfg::kStages;
-        if (!mbar_wait(&full[s], (i / Cfg::kStages) & 1, abort_flag, p.status, kStatusTimeoutMma)) break;
-        tc_fence_after();
-        const uint32_t a = smem_u32(base + s * Cfg::kStageBytes), b = a + kDnABytes;
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_f16(tmem_acc, umma_desc_k_sw128(a + ks * 32), umma_desc_k_sw128(b + ks * 32), idesc, (i | ks) != 0);
-        tc_commit(&empty[s]);
-      }
-      tc_commit(acc_done);
+    constexpr uint32_t idesc = umma_idesc(128, BT, 1, 1, 0, 0);
+    constexpr uint64_t kStageStep = uint64_t(Cfg::kStageBytes >> 4);
+    const uint64_t a_desc0 = umma_desc_k_sw128(smem_u32(base)), b_desc0 = umma_desc_k_sw128(smem_u32(base) + kDnABytes);
+    const uint32_t empty_addr = smem_u32(empty);
+    int s = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < nkb; ++i) {
+      if (!mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma)) break;
+      tc_fence_after();
+      umma_f16_block(tmem_acc, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc, i > 0 ? 1u : 0u, empty_addr + s * 8);
+      if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
     }
+    tc_commit_warp(acc_done);
   }
   __syncwarp();
   pdl_wait();  // before this thread's first global access
@@ -409,6 +416,11 @@ static int run_dense(const DenseParams& p, const void* w, const void* x, int ldx
     if (!p.tiles && p.M > 16) return -1;
     return !p.tiles && p.M <= 8 ? launch_dense_gemv<1>(w, x, ldx, p, entries, stream) : launch_dense_gemv<2>(w, x, ldx, p, entries, stream);
   }
+  if (splits == kDensePair) {
+    if (p.tiles || p.groups > 1) return -1;
+    return mfq_dense_pair(w, x, ldx, p.epi.out, p.epi.ldo, p.epi.bias, p.M, p.N, p.K, kind, p.epi.alpha, p.epi.limit, p.epi.table, p.epi.ids,
+                          token_tile, p.status, stream);
+  }
   switch (token_tile) {
     case 16: return launch_dense_gemm<16>(p, w, x, ldx, matrices, entries, splits, stream);
     case 32: return launch_dense_gemm<32>(p, w, x, ldx, matrices, entries, splits, stream);
@@ -422,7 +434,8 @@ static int run_dense(const DenseParams& p, const void* w, const void* x, int ldx
 }  // namespace mfq
 
 // w [N, K] row-major, x [M, ldx], both bf16 (fp32 = 0) or fp32 (fp32 = 1).  N a multiple of 16, K and ldx of 8, M > 0; ldo of 8.
-// token_tile 0: the weight-streaming kernel (M <= 16); 16 .. 256: the tcgen05 kernel with that tile and `splits` K splits.
+// token_tile 0: the weight-streaming kernel (M <= 16); 16 .. 256: the tcgen05 kernel with that tile and `splits` K splits;
+// splits -2 with a tile of 128 or 256 and one matrix: the same on pairs of SMs (dense_pair.cu).
 // groups > 1: w [groups, N, K] (bias [groups, N]); matrix g reads x from column g * x_step on and writes out from g * out_step on
 // (multiples of 8).
 extern "C" int mfq_dense_linear(const void* w, const void* x, int ldx, void* out, int ldo, const float* bias, int M, int N, int K,

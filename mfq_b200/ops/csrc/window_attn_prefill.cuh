@@ -103,7 +103,7 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_max = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // max [2 buffers][2 halves][128], sum [2][128]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
@@ -121,7 +121,7 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   // this one, and would hold what this CTA still needs if it came first.  (For the same reason the wait above precedes the
   // allocation.)
   pdl_trigger();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tO = tmem_base + 2 * KB;
 
   if (warp == 0) {
@@ -149,44 +149,48 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc(128, KB, 1, 1, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc(128, 64 * VS, 1, 1, 0, 1);
-      const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
-      const int ksteps = p.dk / 16;
-      auto issue_qk = [&](int j) {
-        const uint32_t k_addr = smem_u32(sKV + (j & 1) * Cfg::kStage);
-        for (int ks = 0; ks < ksteps; ++ks)
-          umma_f16(tmem_base + (j & 1) * KB, umma_desc_k_sw128(q_addr + (ks >> 2) * (kWpRows * 128) + (ks & 3) * 32),
-                   umma_desc_k_sw128(k_addr + (ks >> 2) * Cfg::kKSlab + (ks & 3) * 32), idesc_qk, ks > 0);
-        tc_commit(&s_full[j & 1]);
-      };
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, kStatusTimeoutMma) &&
-                mbar_wait(&kv_full[0], 0, abort_flag, p.status, kStatusTimeoutMma);
-      if (ok) {
-        tc_fence_after();
-        issue_qk(0);
-      }
-      for (int j = 0; ok && j < nblk; ++j) {
-        if (j + 1 < nblk) {
-          const int s1 = (j + 1) & 1;
-          ok = mbar_wait(&kv_full[s1], ((j + 1) >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma) &&
-               mbar_wait(&s_empty[s1], (((j + 1) >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma);
-          if (!ok) break;
-          tc_fence_after();
-          issue_qk(j + 1);
-        }
-        ok = mbar_wait(p_full, j & 1, abort_flag, p.status, kStatusTimeoutMma) &&
-             mbar_wait(o_empty, (j & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma);
+    // issued by an elected lane of the converged warp (common.cuh: umma_f8f6f4_block says why)
+    constexpr uint32_t idesc_qk = umma_idesc(128, KB, 1, 1, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc(128, 64 * VS, 1, 1, 0, 1);
+    constexpr uint64_t kStageStep = uint64_t(Cfg::kStage >> 4), kRowSlab = uint64_t(kWpRows * 128 >> 4), kKeySlab = uint64_t(Cfg::kKSlab >> 4);
+    const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), p_desc = umma_desc_k_sw128(smem_u32(sP));
+    const uint64_t k_desc0 = umma_desc_k_sw128(smem_u32(sKV)), v_desc0 = umma_desc_mn_sw128(smem_u32(sKV) + DS * Cfg::kKSlab, Cfg::kKSlab);
+    const uint32_t kv_empty_addr = smem_u32(kv_empty), pv_full_addr = smem_u32(pv_full);
+    const int slabs = p.dk / 64, rest = (p.dk % 64) / 16;  // k-steps of 16 channels, four to a slab
+    auto issue_qk = [&](int j) {
+      const uint64_t k_desc = k_desc0 + uint64_t(j & 1) * kStageStep;
+      const uint32_t d = tmem_base + uint32_t(j & 1) * KB;
+      for (int n = 0; n < slabs; ++n) umma_f16_block(d, q_desc + n * kRowSlab, k_desc + n * kKeySlab, idesc_qk, n > 0 ? 1u : 0u);
+      for (int n = 0; n < rest; ++n)
+        umma_f16_warp(d, q_desc + slabs * kRowSlab + n * 2, k_desc + slabs * kKeySlab + n * 2, idesc_qk, slabs + n > 0 ? 1u : 0u);
+      tc_commit_warp(&s_full[j & 1]);
+    };
+    bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, kStatusTimeoutMma) &&
+              mbar_wait_warp(&kv_full[0], 0, abort_flag, p.status, kStatusTimeoutMma);
+    if (ok) {
+      tc_fence_after();
+      issue_qk(0);
+    }
+    for (int j = 0; ok && j < nblk; ++j) {
+      if (j + 1 < nblk) {
+        const int s1 = (j + 1) & 1;
+        ok = mbar_wait_warp(&kv_full[s1], ((j + 1) >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma) &&
+             mbar_wait_warp(&s_empty[s1], (((j + 1) >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(sKV + (j & 1) * Cfg::kStage + DS * Cfg::kKSlab);
+        issue_qk(j + 1);
+      }
+      ok = mbar_wait_warp(p_full, j & 1, abort_flag, p.status, kStatusTimeoutMma) &&
+           mbar_wait_warp(o_empty, (j & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t v_desc = v_desc0 + uint64_t(j & 1) * kStageStep;
+      static_assert(KB % 64 == 0, "four k-steps at a time");
 #pragma unroll
-        for (int ks = 0; ks < KB / 16; ++ks)
-          umma_f16(tO, umma_desc_k_sw128(p_addr + (ks >> 2) * (kWpRows * 128) + (ks & 3) * 32),
-                   umma_desc_mn_sw128(v_addr + ks * 2048, Cfg::kKSlab), idesc_pv, ks > 0);
-        tc_commit(pv_full);
-        tc_commit(&kv_empty[j & 1]);
+      for (int n = 0; n < KB / 64; ++n) {
+        const bool last = n + 1 == KB / 64;
+        umma_f16_block<2, 128>(tO, p_desc + n * kRowSlab, v_desc + n * 512, idesc_pv, n > 0 ? 1u : 0u, last ? pv_full_addr : 0u,
+                               last ? kv_empty_addr + (j & 1) * 8 : 0u);
       }
     }
   } else {

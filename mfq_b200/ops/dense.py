@@ -41,11 +41,17 @@ def _most_splits(tiles: int, blocks: int, small: bool, sms: int) -> int:
     return best
 
 
-def plan(m: int, n: int, k: int, sms: int = 148) -> tuple[int, int]:
-    """``(token tile, K splits)`` of a bf16 product ``[m, k] x [n, k]^T``; tile 0 is the weight-streaming kernel.  Fitted to a
+PAIR = -2  # as a number of K splits: the product runs on pairs of SMs (csrc/dense_pair.cu)
+
+
+def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = True) -> tuple[int, int]:
+    """``(token tile, K splits)`` of a bf16 product ``[m, k] x [n, k]^T``; tile 0 is the weight-streaming kernel, splits
+    :data:`PAIR` the kernel on pairs of SMs (``pairs``: it may be chosen; it takes a single matrix).  Fitted to a
     sweep on B200 over the projections of 1B- and 8B-sized layers at 16 .. 4096 tokens: up to 128 tokens the weights are read
     once whatever the split, so the grid is filled; beyond that a wave of 256-token tiles costs about 7 + 0.35 us per K block,
-    of 128-token tiles 5 + 0.30 us, and meeting in a cluster 5 / 3 us."""
+    of 128-token tiles 5 + 0.30 us, and meeting in a cluster 5 / 3 us.  A wave of pairs (256 rows each) costs 2 + 0.40 us per K block
+    with 256 tokens and 0.26 with 128, once 4 us for the launch: 1508 tokens of gate/up 28672 x 4096 take 252 us there against 462 here,
+    of o_proj 4096 x 4096 50 against 64; what stays here are narrow or split products (300 x 4096 x 14336: 52 against 54 us)."""
     if m <= GEMV_ROWS or (m <= GEMV_MID_ROWS and n * k <= GEMV_MID_WEIGHTS):
         return 0, 1
     rows, blocks = math.ceil(n / 128), math.ceil(k / 64)
@@ -59,6 +65,12 @@ def plan(m: int, n: int, k: int, sms: int = 148) -> tuple[int, int]:
             cost = math.ceil(tiles * s / sms) * (ramp + per_block * math.ceil(blocks / s)) + (meet if s > 1 else 0.0)
             if best_cost is None or cost < best_cost:
                 best, best_cost = (tile, s), cost
+    if math.ceil(rows * math.ceil(m / best[0]) * best[1] / sms) > 1:
+        best_cost *= 1.1  # several waves of CTAs: 4096 x 4096 x 14336 takes 434 us, not the 341 of four single ones
+    for tile, ramp, per_block in ((256, 2.0, 0.40), (128, 0.0, 0.26)) if pairs else ():
+        cost = 4.0 + math.ceil(math.ceil(n / 256) * math.ceil(m / tile) / (sms // 2)) * (ramp + per_block * blocks)
+        if cost < best_cost:
+            best, best_cost = (tile, PAIR), cost
     return best
 
 
@@ -117,7 +129,7 @@ class DenseLinear:
         elif table is not None:
             assert table.shape[1] == n and table.is_contiguous() and table.dtype == x.dtype and ids.dtype == torch.int32
             kind = GELU
-        t, s = plan(m, n * g, k)
+        t, s = plan(m, n * g, k, pairs=g == 1 and tile is None)
         t, s = (t if tile is None else tile), (s if splits is None else splits)
         rc = dense_lib().mfq_dense_linear(ptr(self.w), ptr(x), x.stride(0), ptr(out), out.stride(0), ptr(self.bias), m, n, k, g, x_step,
                                           out_step, kind, alpha, limit, ptr(table), ptr(ids), t, s, is_fp32(x.dtype),

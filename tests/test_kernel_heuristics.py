@@ -42,3 +42,17 @@ def test_kernel_choice_by_rows():
     assert not K.use_gemv(4, 100, 4096)  # rows of 16 only
     assert K.act_gemv_ok(4, 4096, 4096) and not K.act_gemv_ok(5, 4096, 4096) and not K.act_gemv_ok(1, 4096, 32768)
     assert not K.act_gemv_pays(1, 4096, 4096)  # measured slower: off unless asked for
+
+
+def test_pair_kernels_are_chosen_only_where_they_run():
+    from mfq_b200.ops import dense
+    from mfq_b200.ops import kernels as K
+    for m in (1, 8, 64, 65, 100, 129, 357, 1000, 4097):
+        for n, k in ((256, 128), (4096, 4096), (6144, 4096), (28672, 4096), (4096, 14336), (128256, 4096), (384, 512)):
+            t = K.pair_tile(m, n, k)
+            assert t in (0, 128, 256) and (t == 0 or (m >= K.PAIR_MIN_ROWS and n % 256 == 0))
+            tile, splits = dense.plan(m, n, k)
+            assert splits >= 1 or (splits == dense.PAIR and tile in (128, 256) and m > 128)
+            assert dense.plan(m, n, k, pairs=False)[1] >= 1
+    assert K.pair_tile(4096, 28672, 4096) and K.pair_tile(357, 4096, 14336)
+    assert not K.pair_tile(128, 4096, 14336)  # few tiles over a long K range: the one-SM kernel splits it
