@@ -1,14 +1,19 @@
 // Causal self-attention for prefill chunks on tcgen05 tensor cores (bf16 in, fp32 accumulate, head dim 128, GQA).
 //
-// One CTA = (128-query block, query head).  Per 128-key block:
+// A CTA works on TWO tiles of 128 queries at a time, A and B: the same queries of two heads that share a KV head (both then read the
+// same keys and values), or, where a KV head has an odd number of query heads, two neighbouring query blocks of one head.  Per tile and
+// 128-key block:
 //   S = Q K^T      tcgen05.mma kind::f16, A = Q tile, B = K tile (both K-major, TMA 128 B swizzle), S in TMEM
-//   P = softmax    8 warps, two threads per query row (64 keys each): two passes over the TMEM row (max, then
-//                  exp2 + sum), row maxima exchanged through shared memory,
-//                  P written as bf16 into shared memory in the swizzled K-major layout the next MMA expects
-//   O_blk = P V    tcgen05.mma with V as an MN-major B operand (the [key][dim] tile exactly as TMA delivers it)
+//   P = softmax    8 warps, two threads per query row (64 keys each): two passes over the TMEM row (max, then exp2 + sum), row maxima
+//                  exchanged through shared memory; P goes back as bf16 pairs into the columns its own scores came from
+//   O_blk = P V    tcgen05.mma with P from TENSOR MEMORY as the A operand and V as an MN-major B operand (the [key][dim] tile exactly
+//                  as TMA delivers it)
 //   O = (O + O_blk(prev)) * alpha   folded in fp32 registers, so TMEM never needs an in-place rescale
-// The MMA warp issues Q K^T of block j+1 before P V of block j (S is double-buffered in TMEM), so the tensor core
-// works while the softmax warps are busy.  Heaviest (latest) query blocks are scheduled first.
+// The chain  S -> softmax -> P V  of one tile is several times as long as its MMAs: with one tile per CTA a block took 5400 cycles of
+// which the tensor core worked 1000.  Here the softmax warps of A compute while the tensor core works for B and the other way round,
+// four warps per scheduler cover each other's latencies, and P no longer passes through shared memory and a proxy fence.
+// 4096 tokens of 32 heads on a B200: 318 -> 197 us; 1000 tokens after 3001: 145 -> 102 us, with the same bits.
+// Heaviest (latest) query blocks are scheduled first, over all heads.
 //
 // The reference's prefill attention is a llama.cpp-derived mma.sync flash-attention (mfq_fattn_mma_f16.cuh) and a
 // wmma D=256 kernel (attention.cu:218).
@@ -21,14 +26,43 @@ namespace mfq {
 constexpr int kQB = 128, kKB = 128, kHD = 128;
 constexpr int kTileBytes = kQB * kHD * 2;       // 32 KB: one [128 x 128] bf16 tile = two 16 KB swizzled halves
 constexpr int kHalfBytes = kTileBytes / 2;
-constexpr int kPrefillThreads = 64 + 8 * 32;  // TMA warp, MMA warp, 8 softmax warps
-constexpr int kPrefillSmem = kTileBytes /*Q*/ + 2 * 2 * kTileBytes /*K,V x 2 stages*/ + kTileBytes /*P*/ + 1024 + 256 + 6 * kQB * 4 /*row max / sum exchange*/;
+constexpr int kPrefillThreads = 128 + 2 * 256;  // TMA warp, MMA warp, two idle warps; eight softmax warps per tile
+constexpr int kExchange = 6 * kQB;              // floats per tile: maxima [2 buffers][2 halves][128 rows], sums [2 halves][128]
+constexpr int kPrefillSmem = 2 * kTileBytes /*Q*/ + 2 * 2 * kTileBytes /*K, V x 2 stages*/ + 1024 + 256 + 2 * kExchange * 4;
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ void tmem_store_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+// D (+)= A B over 64 keys with A [128 x 64] bf16 in tensor memory (two values per column: 8 columns per k-step of 16) and B = 64 keys x
+// 128 dims, MN-major, 2 KB per k-step.  Whole warp, one elected lane issues the four steps.
+__device__ __forceinline__ void umma_pv(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred q, f, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+      "setp.ne.b32 f, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+      "add.s64 b1, %2, 128;\n\tadd.s64 b2, %2, 256;\n\tadd.s64 b3, %2, 384;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, f;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t}"
+      ::"r"(d), "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+template <bool kMasked>
+struct MaskedBlock {
+  static constexpr bool value = kMasked;
+};
 
 struct PrefillParams {
   __nv_bfloat16* out;  // [T, Hq, 128]
@@ -36,6 +70,7 @@ struct PrefillParams {
   int Tk, offset;      // keys available; query row i sees keys 0 .. i + offset (offset = Tk - T: tokens before the chunk)
   float scale_log2;
   int* status;
+  int two_heads;       // tiles A, B: two heads of a KV head at the same queries (1) or two query blocks of a head (0)
 };
 
 __global__ void __launch_bounds__(kPrefillThreads, 1)
@@ -43,38 +78,43 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = base;
-  uint8_t* sKV = base + kTileBytes;                 // stage s: K at sKV + s*2*tile, V right after it
-  uint8_t* sP = sKV + 4 * kTileBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + kTileBytes);
+  uint8_t* sQ = base;                               // tile A, tile B
+  uint8_t* sK = base + 2 * kTileBytes;              // two stages
+  uint8_t* sV = sK + 2 * kTileBytes;                // two stages
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * kTileBytes);
   uint64_t* q_full = bars;            // 1
-  uint64_t* kv_full = bars + 1;       // [2]
-  uint64_t* kv_empty = bars + 3;      // [2]
-  uint64_t* s_full = bars + 5;        // [2]
-  uint64_t* s_empty = bars + 7;       // [2] (8 arrivals: one per softmax warp)
-  uint64_t* p_full = bars + 9;        // 8 arrivals
-  uint64_t* pv_full = bars + 10;      // commit
-  uint64_t* o_empty = bars + 11;      // 8 arrivals
-  uint64_t* x_bar = bars + 12;        // 8 arrivals: row-max exchange, one phase per key block
-  uint64_t* l_bar = bars + 13;        // 8 arrivals: row-sum exchange, once
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* k_full = bars + 1;        // [2] per stage, like the three below
+  uint64_t* k_empty = bars + 3;
+  uint64_t* v_full = bars + 5;
+  uint64_t* v_empty = bars + 7;
+  uint64_t* s_full = bars + 9;        // [2] per tile: S of a block is complete, and with it every MMA issued before
+  uint64_t* p_full = bars + 11;       // [2] per tile, 8 arrivals: P is in TMEM, and O has been read
+  uint64_t* o_full = bars + 13;       // [2] per tile, once
+  uint64_t* x_bar = bars + 15;        // [2] per tile, 8 arrivals: row-maximum exchange, one phase per key block
+  uint64_t* l_bar = bars + 17;        // [2] per tile, 8 arrivals: row-sum exchange, once
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_max = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // max: [2 buffers][2 halves][128 rows]; sum: [2 halves][128 rows]
+  float* exchange = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   const int num_qb = (p.T + kQB - 1) / kQB;
-  const int qb = num_qb - 1 - blockIdx.x;  // heavy blocks first
-  const int hq = blockIdx.y;
-  const int kvh = hq / (p.Hq / p.Hk);
-  // causal with a past: the last query of the block sees keys up to (qb + 1) * kQB - 1 + offset
-  const int nblk = min((p.Tk + kKB - 1) / kKB, ((qb + 1) * kQB + p.offset + kKB - 1) / kKB);
+  const int heavy = int(gridDim.y) - 1 - int(blockIdx.y);  // heavy blocks first
+  const int head_a = p.two_heads ? 2 * blockIdx.x : blockIdx.x, qb_a = p.two_heads ? heavy : 2 * heavy;
+  const int head[2] = {head_a, p.two_heads ? head_a + 1 : head_a};
+  const int qb[2] = {qb_a, p.two_heads ? qb_a : qb_a + 1};
+  const int kvh = head_a / (p.Hq / p.Hk);
+  // causal with a past: the last query of a block sees keys up to (qb + 1) * kQB - 1 + offset
+  const int k_blocks = (p.Tk + kKB - 1) / kKB;
+  const int n_a = min(k_blocks, ((qb[0] + 1) * kQB + p.offset + kKB - 1) / kKB);
+  const int n_b = qb[1] < num_qb ? min(k_blocks, ((qb[1] + 1) * kQB + p.offset + kKB - 1) / kKB) : 0;
+  const int n_max = max(n_a, n_b);
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 8);
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); mbar_init(&o_full[i], 1); mbar_init(&x_bar[i], 8); mbar_init(&l_bar[i], 8);
     }
-    mbar_init(p_full, 8); mbar_init(pv_full, 1); mbar_init(o_empty, 8); mbar_init(x_bar, 8); mbar_init(l_bar, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -82,208 +122,203 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS[2] = {tmem_base, tmem_base + 128};
-  const uint32_t tO = tmem_base + 256;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  // columns: S of A, S of B (P of 64 keys in the first half of each 64 columns), O of A, O of B
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
 
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
-      mbar_expect_tx(q_full, kTileBytes);
-      tma_load_2d(sQ, &tmap_q, q_full, hq * kHD, qb * kQB);
-      tma_load_2d(sQ + kHalfBytes, &tmap_q, q_full, hq * kHD + 64, qb * kQB);
-      for (int j = 0; j < nblk; ++j) {
+      mbar_expect_tx(q_full, 2 * kTileBytes);
+      for (int x = 0; x < 2; ++x)
+        for (int h = 0; h < 2; ++h)
+          tma_load_2d(sQ + x * kTileBytes + h * kHalfBytes, &tmap_q, q_full, head[x] * kHD + 64 * h, qb[x] * kQB);  // past the end: zeros
+      for (int j = 0; j < n_max; ++j) {
         const int s = j & 1;
-        if (!mbar_wait(&kv_empty[s], ((j >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutProducer)) break;
-        uint8_t* k = sKV + s * 2 * kTileBytes;
-        uint8_t* v = k + kTileBytes;
-        mbar_expect_tx(&kv_full[s], 2 * kTileBytes);
-        tma_load_2d(k, &tmap_k, &kv_full[s], kvh * kHD, j * kKB);
-        tma_load_2d(k + kHalfBytes, &tmap_k, &kv_full[s], kvh * kHD + 64, j * kKB);
-        tma_load_2d(v, &tmap_v, &kv_full[s], kvh * kHD, j * kKB);
-        tma_load_2d(v + kHalfBytes, &tmap_v, &kv_full[s], kvh * kHD + 64, j * kKB);
+        const uint32_t parity = ((j >> 1) & 1) ^ 1;
+        uint8_t *k = sK + s * kTileBytes, *v = sV + s * kTileBytes;
+        if (!mbar_wait(&k_empty[s], parity, abort_flag, p.status, kStatusTimeoutProducer)) break;
+        mbar_expect_tx(&k_full[s], kTileBytes);
+        tma_load_2d(k, &tmap_k, &k_full[s], kvh * kHD, j * kKB);
+        tma_load_2d(k + kHalfBytes, &tmap_k, &k_full[s], kvh * kHD + 64, j * kKB);
+        if (!mbar_wait(&v_empty[s], parity, abort_flag, p.status, kStatusTimeoutProducer)) break;
+        mbar_expect_tx(&v_full[s], kTileBytes);
+        tma_load_2d(v, &tmap_v, &v_full[s], kvh * kHD, j * kKB);
+        tma_load_2d(v + kHalfBytes, &tmap_v, &v_full[s], kvh * kHD + 64, j * kKB);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc(128, 128, 1, 1, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc(128, 128, 1, 1, 0, 1);  // B = V is MN-major
-      const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
-      auto issue_qk = [&](int j) {
-        const uint32_t k_addr = smem_u32(sKV + (j & 1) * 2 * kTileBytes);
+    // issued by an elected lane of the converged warp (common.cuh: umma_f8f6f4_block says why)
+    constexpr uint32_t idesc_qk = umma_idesc(128, 128, 1, 1, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc(128, 128, 1, 1, 0, 1);  // B = V is MN-major
+    constexpr uint64_t kTile = kTileBytes >> 4, kHalf = kHalfBytes >> 4;  // dims 64.. of Q and K live in the second swizzled half
+    const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), k_desc0 = umma_desc_k_sw128(smem_u32(sK));
+    const uint64_t v_desc0 = umma_desc_mn_sw128(smem_u32(sV), kHalfBytes);
+    const uint32_t s_full_addr = smem_u32(s_full);
+    auto issue_qk = [&](int x, int j) {  // S of tile x takes the place of its P, which the MMAs before have read
+      const uint64_t a = q_desc + uint64_t(x) * kTile, b = k_desc0 + uint64_t(j & 1) * kTile;
+      const uint32_t d = tmem_base + uint32_t(x) * 128u;
+      umma_f16_block(d, a, b, idesc_qk, 0u);
+      umma_f16_block(d, a + kHalf, b + kHalf, idesc_qk, 1u, s_full_addr + x * 8);
+    };
+    bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, kStatusTimeoutMma) &&
+              mbar_wait_warp(&k_full[0], 0, abort_flag, p.status, kStatusTimeoutMma);
+    if (ok) {
+      tc_fence_after();
+      issue_qk(0, 0);
+      if (n_b > 0) issue_qk(1, 0);
+      tc_commit_warp(&k_empty[0]);
+    }
+    for (int j = 0; ok && j < n_max; ++j) {
+      ok = mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma);
+      if (ok && j + 1 < n_max) ok = mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {  // 8 x 16 dims; dims 64.. live in the second swizzled half
-          const uint32_t off = (ks >> 2) * kHalfBytes + (ks & 3) * 32;
-          umma_f16(tS[j & 1], umma_desc_k_sw128(q_addr + off), umma_desc_k_sw128(k_addr + off), idesc_qk, ks > 0);
-        }
-        tc_commit(&s_full[j & 1]);
-      };
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, kStatusTimeoutMma) &&
-                mbar_wait(&kv_full[0], 0, abort_flag, p.status, kStatusTimeoutMma);
-      if (ok) {
+      for (int x = 0; x < 2; ++x) {
+        const int n = x == 0 ? n_a : n_b;
+        if (!ok || j >= n) continue;
+        ok = mbar_wait_warp(&p_full[x], j & 1, abort_flag, p.status, kStatusTimeoutMma);
+        if (!ok) continue;
         tc_fence_after();
-        issue_qk(0);
+        const uint32_t o_addr = tmem_base + 256u + uint32_t(x) * 128u, p_addr = tmem_base + uint32_t(x) * 128u;
+        const uint64_t v_desc = v_desc0 + uint64_t(j & 1) * kTile;
+        umma_pv(o_addr, p_addr, v_desc, idesc_pv, 0u);
+        umma_pv(o_addr, p_addr + 64u, v_desc + 512, idesc_pv, 1u);
+        if (j + 1 < n) issue_qk(x, j + 1);
+        else tc_commit_warp(&o_full[x]);
       }
-      for (int j = 0; ok && j < nblk; ++j) {
-        if (j + 1 < nblk) {
-          const int s1 = (j + 1) & 1;
-          ok = mbar_wait(&kv_full[s1], ((j + 1) >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma) &&
-               mbar_wait(&s_empty[s1], (((j + 1) >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma);
-          if (!ok) break;
-          tc_fence_after();
-          issue_qk(j + 1);
-        }
-        ok = mbar_wait(p_full, j & 1, abort_flag, p.status, kStatusTimeoutMma) &&
-             mbar_wait(o_empty, (j & 1) ^ 1, abort_flag, p.status, kStatusTimeoutMma);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t v_addr = smem_u32(sKV + (j & 1) * 2 * kTileBytes + kTileBytes);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {  // 8 x 16 keys
-          const uint32_t a_off = (ks >> 2) * kHalfBytes + (ks & 3) * 32;  // P: K-major over keys
-          umma_f16(tO, umma_desc_k_sw128(p_addr + a_off), umma_desc_mn_sw128(v_addr + ks * 2048, kHalfBytes), idesc_pv,
-                   ks > 0);
-        }
-        tc_commit(pv_full);
-        tc_commit(&kv_empty[j & 1]);
+      if (ok) {
+        tc_commit_warp(&v_empty[j & 1]);
+        if (j + 1 < n_max) tc_commit_warp(&k_empty[(j + 1) & 1]);
       }
     }
+  }
   } else {
-    // ----- softmax warps: two threads per query row (TMEM lane); `half` selects 64 of the 128 key columns of S/P
-    // and 64 of the 128 output dims, so every scheduler has two warps to interleave -----
-    const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int row = quarter * 32 + lane;
-    const int q_idx = qb * kQB + row;
-    const uint32_t lane_base = (uint32_t(quarter * 32) << 16) + uint32_t(half * 64);
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    // ----- softmax warps of tile x: two threads per query row (TMEM lane); `half` selects 64 of the 128 keys of a block and 64 of the
+    // 128 output dims -----
+    const int x = (warp - 4) >> 3, half = ((warp - 4) >> 2) & 1, quarter = warp & 3;
+    const int row = quarter * 32 + lane, q_idx = qb[x] * kQB + row;
+    const int n = x == 0 ? n_a : n_b;
+    const uint32_t lane_base = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(x) * 128u + uint32_t(half) * 64u;
+    const uint32_t tS = lane_base, tO = lane_base + 256u;
+    float* s_max = exchange + x * kExchange;
     float o[64];
 #pragma unroll
     for (int d = 0; d < 64; ++d) o[d] = 0.f;
     float m_run = -FLT_MAX, l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < nblk; ++j) {
+    for (int j = 0; j < n; ++j) {
       const int sb = j & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[sb], (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutEpilogue));
+      ok = mbar_wait_warp(&s_full[x], j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (!ok) break;
       tc_fence_after();
       const int key0 = j * kKB + half * 64;
       // masking is needed where the block reaches past the FIRST query's horizon or past the last key
-      const bool diag = ((j + 1) * kKB - 1 > qb * kQB + p.offset) || ((j + 1) * kKB > p.Tk);
+      const bool diag = ((j + 1) * kKB - 1 > qb[x] * kQB + p.offset) || ((j + 1) * kKB > p.Tk);
       // pass 1: maximum over this thread's 64 columns, then exchange with the partner thread of the row
       float mx = -FLT_MAX;
-      {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(tS[sb] + lane_base, r0);
-        tmem_ld_32x32(tS[sb] + lane_base + 32, r1);
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(tS + c, r);
         tmem_wait_ld();
         if (!diag) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fmaxf(__uint_as_float(r0[i]), __uint_as_float(r1[i])));
+          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const int ka = key0 + i, kb = key0 + 32 + i;
-            mx = fmaxf(mx, (ka <= q_idx + p.offset && ka < p.Tk) ? __uint_as_float(r0[i]) : -FLT_MAX);
-            mx = fmaxf(mx, (kb <= q_idx + p.offset && kb < p.Tk) ? __uint_as_float(r1[i]) : -FLT_MAX);
+            const int key = key0 + c + i;
+            mx = fmaxf(mx, (key <= q_idx + p.offset && key < p.Tk) ? __uint_as_float(r[i]) : -FLT_MAX);
           }
         }
       }
       s_max[(sb * 2 + half) * kQB + row] = mx;
       __syncwarp();
-      if (lane == 0) mbar_arrive(x_bar);
-      ok = __all_sync(0xffffffffu, mbar_wait(x_bar, j & 1, abort_flag, p.status, kStatusTimeoutEpilogue));
+      if (lane == 0) mbar_arrive(&x_bar[x]);
+      uint32_t ro[32];  // first half of the previous block's P V, under the exchange (block 0: not used)
+      tmem_ld_32x32(tO, ro);
+      ok = mbar_wait_warp(&x_bar[x], j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (!ok) break;
       mx = fmaxf(mx, s_max[(sb * 2 + (half ^ 1)) * kQB + row]);
       const float m_new = fmaxf(m_run, mx);
       const float alpha = fast_exp2((m_run - m_new) * p.scale_log2);
-      // fold the previous block's P.V (it was computed against m_run), then move to the new maximum
+      // fold the previous block's P V (it was computed against m_run), then move to the new maximum.  It has retired: its MMAs were
+      // issued before those of the S that was waited for.
       if (j > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(pv_full, (j - 1) & 1, abort_flag, p.status, kStatusTimeoutEpilogue));
-        if (!ok) break;
-        tc_fence_after();
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(tO + lane_base, r0);
-        tmem_ld_32x32(tO + lane_base + 32, r1);
-        tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          o[i] = (o[i] + __uint_as_float(r0[i])) * alpha;
-          o[32 + i] = (o[32 + i] + __uint_as_float(r1[i])) * alpha;
+        for (int c = 0; c < 64; c += 32) {
+          if (c > 0) tmem_ld_32x32(tO + c, ro);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[c + i] = (o[c + i] + __uint_as_float(ro[i])) * alpha;
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(o_empty);
       }
       l_run *= alpha;
       m_run = m_new;
-      // pass 2: probabilities -> bf16 -> this thread's half of the swizzled K-major P tile
+      // pass 2: probabilities -> bf16 pairs over the scores that have been read
       const float mb = m_new * p.scale_log2;
       float psum = 0.f;
-      uint8_t* prow = sP + half * kHalfBytes + row * 128;
+      auto probabilities = [&](auto masked) {
 #pragma unroll
-      for (int c = 0; c < 64; c += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tS[sb] + lane_base + c, r);
-        tmem_wait_ld();
-        uint32_t packed[16];
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tS + c, r);
+          tmem_wait_ld();
+          uint32_t packed[16];
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p0 = fast_exp2(fmaf(__uint_as_float(r[i]), p.scale_log2, -mb));
-          float p1 = fast_exp2(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, -mb));
-          if (diag) {
-            const int key = key0 + c + i;
-            if (!(key <= q_idx + p.offset && key < p.Tk)) p0 = 0.f;
-            if (!(key + 1 <= q_idx + p.offset && key + 1 < p.Tk)) p1 = 0.f;
+          for (int i = 0; i < 32; i += 2) {
+            float p0 = fast_exp2(fmaf(__uint_as_float(r[i]), p.scale_log2, -mb));
+            float p1 = fast_exp2(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, -mb));
+            if (decltype(masked)::value) {
+              const int key = key0 + c + i;
+              if (!(key <= q_idx + p.offset && key < p.Tk)) p0 = 0.f;
+              if (!(key + 1 <= q_idx + p.offset && key + 1 < p.Tk)) p1 = 0.f;
+            }
+            psum += p0 + p1;
+            const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+            packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
           }
-          psum += p0 + p1;
-          __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-          packed[i >> 1] = *reinterpret_cast<uint32_t*>(&h);
+          tmem_store_32x16(tS + c / 2, packed);
         }
-        // 32 keys = 4 chunks of 16 bytes; the chunk index within the 128 B row is XORed with (row % 8)
-#pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          const int chunk = ((c >> 3) + ch) ^ (row & 7);
-          *reinterpret_cast<uint4*>(prow + chunk * 16) =
-              make_uint4(packed[ch * 4], packed[ch * 4 + 1], packed[ch * 4 + 2], packed[ch * 4 + 3]);
-        }
-      }
+      };
+      if (diag) probabilities(MaskedBlock<true>());
+      else probabilities(MaskedBlock<false>());
       l_run += psum;
+      tmem_wait_st();
       tc_fence_before();
-      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&s_empty[sb]); mbar_arrive(p_full); }
+      if (lane == 0) mbar_arrive(&p_full[x]);
     }
-    if (ok) {
+    if (ok && n > 0) {
       // total row sum = both halves
       s_max[(4 + half) * kQB + row] = l_run;  // own slots: the last block's maxima may still be read
       __syncwarp();
-      if (lane == 0) mbar_arrive(l_bar);
-      ok = __all_sync(0xffffffffu, mbar_wait(l_bar, 0, abort_flag, p.status, kStatusTimeoutEpilogue)) &&
-           __all_sync(0xffffffffu, mbar_wait(pv_full, (nblk - 1) & 1, abort_flag, p.status, kStatusTimeoutEpilogue));
+      if (lane == 0) mbar_arrive(&l_bar[x]);
+      ok = mbar_wait_warp(&l_bar[x], 0, abort_flag, p.status, kStatusTimeoutEpilogue) &&
+           mbar_wait_warp(&o_full[x], 0, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (ok) {
         tc_fence_after();
         const float l_tot = l_run + s_max[(4 + (half ^ 1)) * kQB + row];
         const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
-        __nv_bfloat16* dst = p.out + (size_t(q_idx) * p.Hq + hq) * kHD + half * 64;
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(tO + lane_base, r0);
-        tmem_ld_32x32(tO + lane_base + 32, r1);
-        tmem_wait_ld();
-        if (q_idx < p.T) {
+        __nv_bfloat16* dst = p.out + (size_t(q_idx) * p.Hq + head[x]) * kHD + half * 64;
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 va, vb;
-            __nv_bfloat162* ha = reinterpret_cast<__nv_bfloat162*>(&va);
-            __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&vb);
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tO + c, r);
+          tmem_wait_ld();
+          if (q_idx < p.T) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              ha[e] = __floats2bfloat162_rn((o[i + 2 * e] + __uint_as_float(r0[i + 2 * e])) * inv,
-                                            (o[i + 2 * e + 1] + __uint_as_float(r0[i + 2 * e + 1])) * inv);
-              hb[e] = __floats2bfloat162_rn((o[32 + i + 2 * e] + __uint_as_float(r1[i + 2 * e])) * inv,
-                                            (o[32 + i + 2 * e + 1] + __uint_as_float(r1[i + 2 * e + 1])) * inv);
+            for (int i = 0; i < 32; i += 8) {
+              uint4 v;
+              __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                h[e] = __floats2bfloat162_rn((o[c + i + 2 * e] + __uint_as_float(r[i + 2 * e])) * inv,
+                                             (o[c + i + 2 * e + 1] + __uint_as_float(r[i + 2 * e + 1])) * inv);
+              *reinterpret_cast<uint4*>(dst + c + i) = v;
             }
-            *reinterpret_cast<uint4*>(dst + i) = va;
-            *reinterpret_cast<uint4*>(dst + 32 + i) = vb;
           }
         }
       }
@@ -312,8 +347,10 @@ extern "C" int mfq_attn_prefill_past(const void* q, const void* k, const void* v
     if (cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem) != cudaSuccess) return -6;
     attr = true;
   }
-  PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status};
-  attn_prefill_kernel<<<dim3((T + kQB - 1) / kQB, Hq), kPrefillThreads, kPrefillSmem, stream>>>(tq, tk, tv, p);
+  const int two_heads = Hq / Hk % 2 == 0, q_blocks = (T + kQB - 1) / kQB;
+  const PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status, two_heads};
+  const dim3 grid(two_heads ? Hq / 2 : Hq, two_heads ? q_blocks : (q_blocks + 1) / 2);
+  attn_prefill_kernel<<<grid, kPrefillThreads, kPrefillSmem, stream>>>(tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 

@@ -129,3 +129,20 @@ def test_prefix_cache_restores_pages_on_gpu(tmp_path):
         n += 1
     assert n >= 5, (first, again)
     pc.close()
+
+
+@pytest.mark.parametrize("t,past,hq,hk,scale", [(1, 0, 2, 1, 0.09), (127, 1, 6, 2, 0.09), (129, 0, 3, 3, 0.09), (257, 126, 3, 1, 0.09), (385, 0, 8, 2, 0.09),
+                                                (256, 130, 4, 1, 0.0)])
+def test_prefill_attention_on_two_tiles(t, past, hq, hk, scale):
+    """Two heads of a KV head, or two query blocks where their number is odd; a last pair without a second block; keys that grow, so
+    that O is rescaled in every block; a scale of zero."""
+    require_gpu_lib()
+    g = torch.Generator(device="cuda").manual_seed(t + past)
+    q = torch.randn((t, hq, 128), generator=g, device="cuda").to(torch.bfloat16)
+    k = torch.randn((past + t, hk, 128), generator=g, device="cuda")
+    k = (k * torch.linspace(0.25, 4.0, past + t, device="cuda")[:, None, None]).to(torch.bfloat16)
+    v = torch.randn((past + t, hk, 128), generator=g, device="cuda").to(torch.bfloat16)
+    got = ops.kernels.attn_prefill_bf16(q, k, v, scale)
+    check_status()
+    # probabilities and the result are rounded to bf16 (2^-9 each, relative): well inside 2 % of (|ref| + rms / 4)
+    assert_close(got, ref.attention(q, k, v, scale, causal_offset=past), rel=2e-2, what=f"two tiles T={t} past={past}")
