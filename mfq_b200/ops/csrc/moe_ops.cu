@@ -295,6 +295,18 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const in
 
 using namespace mfq;
 
+static int select_experts(const RouterParams& p, cudaStream_t stream) {
+  if (p.logits && p.n_group <= 1 && p.E <= 1024 && p.K <= 32) return launch_router_topk_warp(p, stream);
+  const size_t smem = size_t(p.H + 2 * p.E) * sizeof(float);
+  static size_t configured = 0;
+  if (smem > 48 * 1024 && smem > configured) {
+    if (cudaFuncSetAttribute(moe_router_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -6;
+    configured = smem;
+  }
+  launch_kernel(moe_router_topk_kernel, dim3(p.T), dim3(256), smem, stream, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -7;
+}
+
 // ``logits``: optional [T, E] fp32 scratch.  With it (and H a multiple of 32) the dot products run on tensor cores
 // spread over the whole GPU and the per-token CTAs only score and select; without it one CTA per token does everything.
 extern "C" int mfq_moe_router_topk(const void* x, const void* w, const float* bias, int* topk_ids, float* topk_w,
@@ -314,17 +326,15 @@ extern "C" int mfq_moe_router_topk(const void* x, const void* w, const float* bi
     logits = nullptr;
   }
   RouterParams p{xb, wb, bias, topk_ids, topk_w, scores_out, T, H, E, K, sigmoid, norm_topk, scale, n_group, topk_group, logits};
-  if (logits && n_group <= 1 && E <= 1024 && K <= 32) {
-    return launch_router_topk_warp(p, stream);
-  }
-  const size_t smem = size_t(H + 2 * E) * sizeof(float);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    if (cudaFuncSetAttribute(moe_router_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -6;
-    configured = smem;
-  }
-  launch_kernel(moe_router_topk_kernel, dim3(T), dim3(256), smem, stream, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -7;
+  return select_experts(p, stream);
+}
+
+// The same from router logits that are there already ([T, E] fp32): scoring and selection only.
+extern "C" int mfq_moe_router_select(const float* logits, const float* bias, int* topk_ids, float* topk_w, float* scores_out, int T, int H,
+                                     int E, int K, int sigmoid, int norm_topk, float scale, int n_group, int topk_group, cudaStream_t stream) {
+  if (!logits || T <= 0 || E > kMaxExperts || K > kMaxTopK || K > E || H % 2 || n_group > 64 || (n_group > 1 && E % n_group)) return -1;
+  return select_experts(RouterParams{nullptr, nullptr, bias, topk_ids, topk_w, scores_out, T, H, E, K, sigmoid, norm_topk, scale, n_group, topk_group, logits},
+                        stream);
 }
 
 extern "C" int mfq_moe_gather_rows(const void* xq, const float* xs, const int* src_token, const int* totals, void* out_q,

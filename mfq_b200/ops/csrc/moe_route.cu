@@ -103,9 +103,18 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   const int n_local = e_hi - e_lo;
   for (int e = threadIdx.x; e <= n_local; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
-    const int e = topk_ids[i] - e_lo;
-    if (e >= 0 && e < n_local) atomicAdd(&cnt[e], 1);
+  // One CTA reads all routes, twice: kBatch loads of a thread are on the way at a time (one per round trip made 30000 routes 31 us).
+  constexpr int kBatch = 8;
+  for (int i0 = threadIdx.x; i0 < entries; i0 += kBatch * blockDim.x) {
+    int id[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = i0 + u * int(blockDim.x);
+      id[u] = i < entries ? topk_ids[i] - e_lo : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u)
+      if (id[u] >= 0 && id[u] < n_local) atomicAdd(&cnt[id[u]], 1);
   }
   __syncthreads();
   {
@@ -148,14 +157,23 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
-    const int e = topk_ids[i] - e_lo;
-    int row = -1;
-    if (e >= 0 && e < n_local) {
-      row = atomicAdd(&fill[e], 1);
-      src_token[row] = i / K;
+  for (int i0 = threadIdx.x; i0 < entries; i0 += kBatch * blockDim.x) {
+    int id[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = i0 + u * int(blockDim.x);
+      id[u] = i < entries ? topk_ids[i] - e_lo : -1;
     }
-    dest[i] = row;
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = i0 + u * int(blockDim.x);
+      int row = -1;
+      if (id[u] >= 0 && id[u] < n_local) {
+        row = atomicAdd(&fill[id[u]], 1);
+        src_token[row] = i / K;
+      }
+      if (i < entries) dest[i] = row;
+    }
   }
   for (int e = threadIdx.x; e < n_local; e += blockDim.x) {
     const int n = tbase[e + 1] - tbase[e];

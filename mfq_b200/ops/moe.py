@@ -15,11 +15,13 @@ from dataclasses import dataclass
 import torch
 
 from . import kernels as K
+from .dense import DenseLinear
 from .lib import Workspace, check, lib, ptr, stream_ptr
 
 _vp, _i, _f = C.c_void_p, C.c_int, C.c_float
 _SIGS = {
     "mfq_moe_router_topk": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp],
+    "mfq_moe_router_select": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp],
     "mfq_moe_plan": [_vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp],
     "mfq_moe_gather_rows": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
     "mfq_moe_combine": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
@@ -51,6 +53,9 @@ class RoutePlan:
     n_local: int
 
 
+ROUTER_MMA_ROWS = 64  # router logits of more tokens go through the dense product
+
+
 def router_topk(x: torch.Tensor, w: torch.Tensor, k: int, *, bias: torch.Tensor | None = None, sigmoid: bool = False,
                 norm_topk: bool = True, scale: float = 1.0, n_group: int = 1, topk_group: int = 1,
                 want_scores: bool = False):
@@ -59,6 +64,14 @@ def router_topk(x: torch.Tensor, w: torch.Tensor, k: int, *, bias: torch.Tensor 
     ids = torch.empty((t, k), dtype=torch.int32, device=x.device)
     wt = torch.empty((t, k), dtype=torch.float32, device=x.device)
     scores = torch.empty((t, e), dtype=torch.float32, device=x.device) if want_scores else None
+    if t > ROUTER_MMA_ROWS and e % 16 == 0 and h % 32 == 0 and x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == 1 and x.stride(0) % 8 == 0 \
+            and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+        # a prompt's logits are an ordinary product: 3000 x 2048 x 512 takes 137 us in the router's own mma.sync kernel, 12 on tcgen05
+        logits = DenseLinear(w)(x, fp32=True)
+        rc = _lib().mfq_moe_router_select(ptr(logits), ptr(bias), ptr(ids), ptr(wt), ptr(scores), t, h, e, k, int(sigmoid), int(norm_topk),
+                                          float(scale), n_group, topk_group, stream_ptr())
+        check(rc, "moe_router_select")
+        return (ids, wt, scores) if want_scores else (ids, wt)
     logits = torch.empty((t, e), dtype=torch.float32, device=x.device) if h % 32 == 0 else None
     rc = _lib().mfq_moe_router_topk(ptr(x), ptr(w), ptr(bias), ptr(ids), ptr(wt), ptr(scores), ptr(logits), t, h, e, k, int(sigmoid),
                                     int(norm_topk), float(scale), n_group, topk_group, stream_ptr())

@@ -1,0 +1,143 @@
+"""Kernels that wide batches and prompts take: products on pairs of SMs, row quantization in one pass, several heads of a token per
+warp, router logits through the dense product -- at the edges of their tiles and of the rules that choose them."""
+
+import math
+
+import pytest
+import torch
+
+from mfq_b200 import ops
+from mfq_b200.engine.kv_cache import PagedKVCache
+from mfq_b200.ops import dense, moe
+from mfq_b200.ops import kernels as K
+from mfq_b200.ops.dense import DenseLinear
+from gpu_common import check_status, require_gpu_lib
+
+pytestmark = pytest.mark.gpu
+FP8 = torch.float8_e4m3fn
+
+
+def _normal(seed, *shape, std=1.0, dtype=torch.bfloat16):
+    return (torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * std).to(dtype)
+
+
+def _fp8(seed, m, n, k):
+    xq = _normal(seed, m, k, std=60, dtype=torch.float32).clamp(-448, 448).to(FP8)
+    wq = _normal(seed + 1, n, k, std=60, dtype=torch.float32).clamp(-448, 448).to(FP8)
+    g = torch.Generator(device="cuda").manual_seed(seed + 2)
+    return xq, torch.rand(m, generator=g, device="cuda") + 0.1, wq, torch.rand((math.ceil(n / 128), k // 128), generator=g, device="cuda") + 0.1
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 256, 128), (129, 512, 640), (257, 256, 2048), (400, 4096, 256), (1300, 256, 1152), (130, 256, 33 * 1024)])
+def test_fp8_pair_kernel_gives_the_bits_of_the_one_sm_kernel(m, n, k):
+    """Both fold K block after K block into fp32 registers and round the same way, residual included; 33 * 1024 is a K range whose
+    multipliers do not fit the shared-memory copy."""
+    require_gpu_lib()
+    args = _fp8(m + k, m, n, k)
+    res = _normal(m, m, n)
+    want = ops.fp8_gemm(*args, residual=res, splits=1, token_tile=128)
+    for tile in (128, 256):
+        h = res.clone()
+        assert torch.equal(ops.fp8_gemm(*args, residual=h, out=h, pair=tile), want)
+        assert torch.equal(ops.fp8_gemm(*args, pair=tile), ops.fp8_gemm(*args, splits=1, token_tile=128))
+    check_status()
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 256, 4096), (130, 512, 1408), (700, 4096, 4096)])
+def test_fp8_product_of_a_wide_batch_keeps_the_sums_of_the_split_form(m, n, k):
+    """Chosen by itself, the two-SM kernel adds up the partial sums that the one-SM kernel's K splits would."""
+    require_gpu_lib()
+    args = _fp8(m, m, n, k)
+    res = _normal(m, m, n)
+    assert K.pair_tile(m, n, k) == 128 and K.split_blocks(m, n, k)
+    got, want = ops.fp8_gemm(*args, residual=res), ops.fp8_gemm(*args, residual=res, pair=0)
+    check_status()
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("tile", [128, 256])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 8), (129, 272, 72), (257, 512, 4096), (300, 48, 200), (1400, 1040, 64)])
+def test_dense_pair_kernel_on_every_output_stage(m, n, k, tile):
+    """Ragged rows, tokens and K against 64 bits; more tiles than pairs in the last shape, so that accumulators are used again."""
+    require_gpu_lib()
+    w, x, bias = _normal(n, n, k, std=k ** -0.5), _normal(m, m, k), _normal(k, n, dtype=torch.float32)
+    table, ids = _normal(3, 50, n), torch.arange(m, device="cuda", dtype=torch.int32) % 50
+    y = x.double() @ w.double().T
+    slack = (x.double().abs() @ w.double().abs().T) * (k + 8) * 2.0 ** -24
+
+    def check(got, want, factor=1.0):
+        # bf16 results: half a step; factor: how much the output stage can enlarge an error of the sum (plus its own fp32 steps)
+        bound = want.abs() * (2.0 ** -8 if got.dtype == torch.bfloat16 else 2.0 ** -20) + factor * slack.amax() + 1e-5
+        assert bool(((got.double() - want).abs() <= bound).all())
+
+    how = dict(tile=tile, splits=dense.PAIR)
+    check(DenseLinear(w, bias)(x, **how), y + bias.double())
+    check(DenseLinear(w)(x, fp32=True, **how), y)
+    check(DenseLinear(w)(x, softcap=3.0, **how), 3 * torch.tanh(y / 3))
+    check(DenseLinear(w, act="relu2")(x, **how), y.clamp_min(0).square(), 2 * float(y.abs().max()))
+    check(DenseLinear(w)(x, table=table, ids=ids, **how), torch.nn.functional.gelu(y, approximate="tanh") * table[ids.long()].double(), 6.0)
+    stream = _normal(5, m, n, dtype=torch.float32)
+    want = stream.double() + 0.5 * y
+    check(DenseLinear(w)(x, add_to=stream, scale=0.5, **how), want)
+    if n % 16 == 0:
+        gate, up = (y.view(m, n // 16, 2, 8)[:, :, i].reshape(m, n // 2) for i in (0, 1))
+        check(DenseLinear(w, glu="silu")(x, **how), torch.nn.functional.silu(gate) * up, 2 * float(y.abs().max()) + 2)
+    check_status()
+
+
+@pytest.mark.parametrize("m", [3, 511, 512, 1025])
+@pytest.mark.parametrize("k", [8, 520, 4096, 14336, 16384, 16392])
+def test_row_quantization_in_one_pass(m, k):
+    """Rows that are and are not held in registers between the maximum and the encoding: the codes of plain fp32 arithmetic."""
+    require_gpu_lib()
+    x = _normal(m + k, m, 2 * k)
+    x[0] = 0
+    y = x[:, :k].float()
+    q, s = ops.quant_rows(x[:, :k])
+    # quotients through 64 bits: rounded once to fp32, as the kernel's divisions are (torch multiplies by the reciprocal of a scalar)
+    scale = (y.abs().amax(1).clamp_min(1e-12).double() / 448).float()
+    inverse = (1 / scale.double()).float()
+    assert torch.equal(s, scale)
+    assert torch.equal(q.view(torch.uint8), (y * inverse[:, None]).clamp(-448, 448).to(FP8).view(torch.uint8))
+    q, s = ops.silu_mul_quant(x)
+    q1, s1 = ops.silu_mul_quant(x[-1:])  # a single row: another split of the same row
+    assert torch.equal(q[-1:].view(torch.uint8), q1.view(torch.uint8)) and torch.equal(s[-1:], s1)
+    check_status()
+
+
+@pytest.mark.parametrize("rot", [None, 64])
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_rotation_of_many_tokens_gives_the_bits_of_few(d, rot):
+    """Enough tokens that a warp takes several heads, with a count of heads that does not divide: the same pages and queries as from
+    calls that are too small for that."""
+    require_gpu_lib()
+    t, hq, hk = 5003, 7, 2
+    rows = _normal(d, t, (hq + 2 * hk) * d)
+    pos = torch.randint(0, 9000, (t,), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda", dtype=torch.int32)
+    got = []
+    for step in (t, 1000):
+        cache = PagedKVCache(layers=1, kv_heads=hk, head_dim=d, num_pages=t // 16 + 2, max_seqs=1, max_pages_per_seq=t // 16 + 1, device="cuda")
+        cache.assign(0, 0, t)
+        slots = cache.slots(0, 0, t).to("cuda")
+        slots[5] = -1
+        kd, vd = torch.zeros((t, hk, d), device="cuda", dtype=torch.bfloat16), torch.zeros((t, hk, d), device="cuda", dtype=torch.bfloat16)
+        q = torch.cat([ops.rope_kv_write(rows[a : a + step], pos[a : a + step], slots[a : a + step], cache.layer(0), n_q=hq, n_kv=hk, head_dim=d,
+                                         theta=1e4, rot=rot, kd_out=kd[a : a + step], vd_out=vd[a : a + step]) for a in range(0, t, step)])
+        got.append([q, cache.k.view(torch.uint8), cache.v.view(torch.uint8), cache.k_scale, cache.v_scale, kd, vd])
+    check_status()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("t,e", [(65, 16), (200, 512), (700, 48)])
+def test_router_logits_of_a_prompt(t, e):
+    require_gpu_lib()
+    x, w, h = _normal(t, t, 256), _normal(e, e, 256, std=0.1), 256
+    ids, weights, scores = moe.router_topk(x, w, 4, want_scores=True)
+    check_status()
+    want = torch.softmax(x.double() @ w.double().T, -1)
+    # fp32 sums of 256 terms before an exponential: a relative error of their absolute error, and that of exp itself
+    slack = ((x.double().abs() @ w.double().abs().T) * (h + 8) * 2.0 ** -24).amax() * 2 + 2.0 ** -20
+    assert bool(((scores.double() - want).abs() <= want * slack).all())
+    picked = want.gather(1, ids.long())
+    assert bool((picked >= want.topk(4, -1).values * (1 - 2 * slack)).all())
+    assert bool(((weights.double() - picked / picked.sum(1, keepdim=True)).abs() <= 4 * slack).all())
