@@ -504,15 +504,48 @@ __global__ void attn_reduce_log2_kernel(const float* __restrict__ part_acc, cons
                                         __nv_bfloat16* __restrict__ out, int nsplit) {
   pdl_trigger();
   pdl_wait();
+  // Everything a group of kGroup splits contributes is requested before the first of it is used: with a load per loop round a row of
+  // 16 splits cost as many memory round trips one after the other.
+  constexpr int kGroup = 8;
   const size_t hq = blockIdx.x;
   const int d = threadIdx.x;
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + hq * nsplit;
+  const float* acc = part_acc + hq * nsplit * D + d;
   float mm = kNeg;
-  for (int s = 0; s < nsplit; ++s) mm = fmaxf(mm, part_ml[(hq * nsplit + s) * 2]);
+  float2 first[kGroup];
+  float part[kGroup];
+#pragma unroll
+  for (int i = 0; i < kGroup; ++i) {
+    first[i] = i < nsplit ? ml[i] : make_float2(kNeg, 0.f);
+    part[i] = i < nsplit ? acc[size_t(i) * D] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < kGroup; ++i) mm = fmaxf(mm, first[i].x);
+#pragma unroll 8
+  for (int s = kGroup; s < nsplit; ++s) mm = fmaxf(mm, ml[s].x);
   float ll = 0.f, a = 0.f;
-  for (int s = 0; s < nsplit; ++s) {
-    const float cw = exp2f(part_ml[(hq * nsplit + s) * 2] - mm);
-    ll += part_ml[(hq * nsplit + s) * 2 + 1] * cw;
-    a += part_acc[(hq * nsplit + s) * D + d] * cw;
+#pragma unroll
+  for (int i = 0; i < kGroup; ++i) {
+    if (i < nsplit) {
+      const float cw = exp2f(first[i].x - mm);
+      ll += first[i].y * cw;
+      a += part[i] * cw;
+    }
+  }
+  for (int s0 = kGroup; s0 < nsplit; s0 += kGroup) {
+#pragma unroll
+    for (int i = 0; i < kGroup; ++i) {
+      first[i] = s0 + i < nsplit ? ml[s0 + i] : make_float2(kNeg, 0.f);
+      part[i] = s0 + i < nsplit ? acc[size_t(s0 + i) * D] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kGroup; ++i) {
+      if (s0 + i < nsplit) {
+        const float cw = exp2f(first[i].x - mm);
+        ll += first[i].y * cw;
+        a += part[i] * cw;
+      }
+    }
   }
   out[hq * D + d] = __float2bfloat16(ll > 0.f ? a / ll : 0.f);
 }
