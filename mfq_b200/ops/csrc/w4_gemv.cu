@@ -60,6 +60,11 @@ __global__ void __launch_bounds__(256, 2) w4_gemv_kernel(const W4GemvParams p) {
   const __nv_bfloat16* xr[NT];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) xr[nt] = p.x + size_t(min(nt * 8 + g, p.M - 1)) * p.K + block_in_step * 64 + half * 32;
+  // the output of this thread, and what it is added to: requested under the product instead of after it
+  const int t = threadIdx.x >> 4, row = threadIdx.x & 15, n = n0 + row;
+  const bool mine = t < p.M && t < 8 * NT && n < p.N;
+  const size_t at = size_t(t) * p.N + n;
+  const float add = mine && p.residual ? __bfloat162float(p.residual[at]) : 0.f;
   float acc[NT][4] = {};
   for (int s0 = warp; s0 < steps; s0 += 8 * kRing) {
 #pragma unroll
@@ -106,13 +111,11 @@ __global__ void __launch_bounds__(256, 2) w4_gemv_kernel(const W4GemvParams p) {
     red[warp][g + 8][c + 1] = acc[nt][3];
   }
   __syncthreads();
-  const int t = threadIdx.x >> 4, row = threadIdx.x & 15, n = n0 + row;
-  if (t < p.M && t < 8 * NT && n < p.N) {
+  if (mine) {
     float v = 0.f;
 #pragma unroll
     for (int z = 0; z < 8; ++z) v += red[z][row][t];
-    const size_t at = size_t(t) * p.N + n;
-    if (p.residual) v += __bfloat162float(p.residual[at]);
+    if (p.residual) v += add;
     p.out[at] = __float2bfloat16(v);
   }
 }

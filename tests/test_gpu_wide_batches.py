@@ -141,3 +141,14 @@ def test_router_logits_of_a_prompt(t, e):
     picked = want.gather(1, ids.long())
     assert bool((picked >= want.topk(4, -1).values * (1 - 2 * slack)).all())
     assert bool(((weights.double() - picked / picked.sum(1, keepdim=True)).abs() <= 4 * slack).all())
+
+
+@pytest.mark.parametrize("m,i", [(1, 8), (6, 2056), (295, 264), (296, 264)])
+def test_gated_rows_over_one_and_several_blocks(m, i):
+    """The last sizes before and after the rule's line, rows that end in the middle of a block, a batch of rows set apart by padding."""
+    require_gpu_lib()
+    rows = _normal(m, m, 2 * i + 8)[:, :2 * i]
+    a, b = rows[:, :i].double(), rows[:, i:].double()
+    want = a * torch.sigmoid(a) * b
+    # rounded to bf16 once (2^-8); fp32 exponential and divide are far below that
+    assert ((K.silu_mul(rows).double() - want).abs() <= 2.0 ** -7.9 * want.abs() + 1e-30).all()
