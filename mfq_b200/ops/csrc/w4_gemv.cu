@@ -141,6 +141,7 @@ extern "C" int mfq_w4_gemv(const void* packed, const void* group, const void* x,
                            int group_size, int kind, cudaStream_t stream) {
   if (M <= 0 || M > 16 || N <= 0 || K <= 0 || K % 64 || group_size < 16 || group_size % 8 || K % group_size) return -1;
   if (kind != 0 && (kind != 1 || group_size != 32)) return -1;  // MXFP4 blocks are 32 wide
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed)) % 16) return -3;  // read in vectors, as by the TMA of mfq_w4_gemm
   const mfq::W4GemvParams p{static_cast<const uint8_t*>(packed), static_cast<const uint32_t*>(group), static_cast<const __nv_bfloat16*>(x),
                             static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(residual), M, N, K, K / group_size, group_size / 8};
   if (kind == 1) return M <= 8 ? mfq::launch_w4_gemv<1, 1, true>(p, stream) : mfq::launch_w4_gemv<2, 1, true>(p, stream);

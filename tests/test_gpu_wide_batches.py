@@ -8,7 +8,7 @@ import torch
 
 from mfq_b200 import ops
 from mfq_b200.engine.kv_cache import PagedKVCache
-from mfq_b200.ops import dense, moe
+from mfq_b200.ops import dense, moe, w4
 from mfq_b200.ops import kernels as K
 from mfq_b200.ops.dense import DenseLinear
 from gpu_common import check_status, require_gpu_lib
@@ -152,3 +152,13 @@ def test_gated_rows_over_one_and_several_blocks(m, i):
     want = a * torch.sigmoid(a) * b
     # rounded to bf16 once (2^-8); fp32 exponential and divide are far below that
     assert ((K.silu_mul(rows).double() - want).abs() <= 2.0 ** -7.9 * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("m", [1, 16, 17])
+def test_w4_rows_off_a_vector_are_refused(m):
+    """By the host, on either route of the rule on rows."""
+    require_gpu_lib()
+    w = w4.quantize_torch(_normal(1, 128, 256, dtype=torch.float32))
+    x = torch.zeros(m * 256 + 8, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        w4.w4_gemm(x[1:1 + m * 256].view(m, 256), w)
