@@ -331,6 +331,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
   const int heads = Hq + 2 * Hk, groups = (heads + heads_per_warp - 1) / heads_per_warp;
   if (gw >= T * groups) return;
   const int t = gw / groups, h_first = gw % groups * heads_per_warp;
+  const int slot = h_first + heads_per_warp > Hq ? slots[t] : -1;  // requested with the position, not after the rotation
   // The angles of a token are the same for all its heads: a warp that takes several evaluates them once.
   float cs[EPL / 2], sn[EPL / 2];
   if (rot == D) {
@@ -439,7 +440,6 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
     store_half(dst + D / 2 + lane * HP, hi);
     continue;
   }
-  const int slot = slots[t];
   if (slot < 0) continue;
   const int kvh = is_v ? h - Hq - Hk : h - Hq;
   const int page = slot / page_size, off = slot % page_size;
@@ -679,8 +679,8 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
   // Enough tokens to fill the GPU with a warp for several heads each: the angles (sine, cosine and the frequency's power) are a good
   // part of the work of a head.  4096 tokens of 48 heads on a B200: 71 us with one head per warp, 64 with eight (the pages' single-byte
-  // stores take most of that).
-  const int heads = Hq + 2 * Hk, per = long(T) * heads >= 8L * 148 * 32 ? 8 : 1;
+  // stores take most of that); 357 tokens: 11.7 and 10.4, with a warp or two per scheduler left.
+  const int heads = Hq + 2 * Hk, per = long(T) * heads >= 8L * 148 * 8 ? 8 : 1;
   const long warps = long(T) * ((heads + per - 1) / per);
   const int blocks = int((warps + 7) / 8);
   const float l2t = log2f(theta);
