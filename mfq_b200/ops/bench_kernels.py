@@ -171,7 +171,7 @@ def bench_dense(m: int, n: int, k: int, reps: int, stage: str = "", tile=None, s
     add = stage == "add"
     out = torch.zeros((m, lin[0].out_width), device="cuda", dtype=torch.float32 if add else torch.bfloat16)
     ms = time_ms(lambda i: lin[i % copies](x, tile=tile, splits=splits, **{"add_to" if add else "out": out}), reps)
-    t, sp = dense.plan(m, n, k)
+    t, sp = dense.plan(m, n, k, pairs=True)
     return {"kernel": "dense_gemv" if (t if tile is None else tile) == 0 else "dense_gemm", "m": m, "n": n, "k": k, "stage": stage, "us": ms * 1e3,
             "gbs": (2 * (n * k + m * k) + out.numel() * (8 if add else 2)) / ms / 1e6, "tflops": 2 * m * n * k / ms / 1e9,
             "tile": t if tile is None else tile, "splits": sp if splits is None else splits}

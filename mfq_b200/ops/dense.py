@@ -44,7 +44,7 @@ def _most_splits(tiles: int, blocks: int, small: bool, sms: int) -> int:
 PAIR = -2  # as a number of K splits: the product runs on pairs of SMs (csrc/dense_pair.cu)
 
 
-def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = True) -> tuple[int, int]:
+def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[int, int]:
     """``(token tile, K splits)`` of a bf16 product ``[m, k] x [n, k]^T``; tile 0 is the weight-streaming kernel, splits
     :data:`PAIR` the kernel on pairs of SMs (``pairs``: it may be chosen; it takes a single matrix).  Fitted to a
     sweep on B200 over the projections of 1B- and 8B-sized layers at 16 .. 4096 tokens: up to 128 tokens the weights are read
@@ -129,7 +129,7 @@ class DenseLinear:
         elif table is not None:
             assert table.shape[1] == n and table.is_contiguous() and table.dtype == x.dtype and ids.dtype == torch.int32
             kind = GELU
-        t, s = plan(m, n * g, k, pairs=g == 1 and tile is None)
+        t, s = plan(m, n * g, k, pairs=g == 1 and tile is None and splits is None)
         t, s = (t if tile is None else tile), (s if splits is None else splits)
         rc = dense_lib().mfq_dense_linear(ptr(self.w), ptr(x), x.stride(0), ptr(out), out.stride(0), ptr(self.bias), m, n, k, g, x_step,
                                           out_step, kind, alpha, limit, ptr(table), ptr(ids), t, s, is_fp32(x.dtype),

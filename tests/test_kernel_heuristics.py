@@ -51,8 +51,8 @@ def test_pair_kernels_are_chosen_only_where_they_run():
         for n, k in ((256, 128), (4096, 4096), (6144, 4096), (28672, 4096), (4096, 14336), (128256, 4096), (384, 512)):
             t = K.pair_tile(m, n, k)
             assert t in (0, 128, 256) and (t == 0 or (m >= K.PAIR_MIN_ROWS and n % 256 == 0))
-            tile, splits = dense.plan(m, n, k)
+            tile, splits = dense.plan(m, n, k, pairs=True)
             assert splits >= 1 or (splits == dense.PAIR and tile in (128, 256) and m > 128)
-            assert dense.plan(m, n, k, pairs=False)[1] >= 1
+            assert dense.plan(m, n, k)[1] >= 1
     assert K.pair_tile(4096, 28672, 4096) and K.pair_tile(357, 4096, 14336)
     assert not K.pair_tile(128, 4096, 14336)  # few tiles over a long K range: the one-SM kernel splits it
