@@ -93,6 +93,13 @@ def test_streamed_codes_match_reference(m, n, k, gs):
     assert torch.equal(h, got)
 
 
+@pytest.mark.parametrize("gs", [16, 32])
+@pytest.mark.parametrize("m,n,k", [(8, 9440, 192), (7, 9448, 320), (1, 200, 8128), (8, 4744, 8256), (16, 4736, 192), (9, 4744, 320)])
+def test_streamed_codes_by_blocks_of_rows(m, n, k, gs):
+    """Both sides of every line of the rule that gives a CTA one or two blocks of 16 rows, eight or sixteen warps."""
+    test_streamed_codes_match_reference(m, n, k, gs)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 256, 192), (16, 200, 2048)])
 def test_streamed_mxfp4_codes_match_the_tensor_core_form(m, n, k):
     require_gpu_lib()
