@@ -33,7 +33,10 @@ __global__ void embed_scaled_kernel(const int* __restrict__ ids, const T* __rest
   }
 }
 
-template <typename T>
+// kVecs: vectors a thread holds, 1 for rows up to 2048 wide, 2 up to 4096, kStreamVecs beyond.  Bound by its reads in flight: the fewer
+// registers a thread holds, the more rows an SM works on; up to two vectors the weights, which depend on no kernel, are fetched before
+// the wait.
+template <typename T, int kVecs>
 __global__ void __launch_bounds__(512)
 norm_add_kernel(const T* __restrict__ y, const float* __restrict__ w, float* __restrict__ x, T* __restrict__ xa, int W,
                 float inv_width, float eps) {
@@ -41,11 +44,16 @@ norm_add_kernel(const T* __restrict__ y, const float* __restrict__ w, float* __r
   __shared__ float red[33];
   const size_t row = blockIdx.x;
   const int nvec = W / 8;
+  constexpr bool kEarly = kVecs <= 2;
+  float ww[kEarly ? kVecs : 1][8];
+#pragma unroll
+  for (int i = 0; i < (kEarly ? kVecs : 0); ++i)
+    if (int(threadIdx.x + i * blockDim.x) < nvec) load8<float>(w + (threadIdx.x + i * blockDim.x) * 8, ww[i]);
   pdl_wait();
-  float v[kStreamVecs][8], r[kStreamVecs][8];
+  float v[kVecs][8], r[kVecs][8];
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < kStreamVecs; ++i) {
+  for (int i = 0; i < kVecs; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
       load8<T>(y + row * W + vi * 8, v[i]);
@@ -56,13 +64,12 @@ norm_add_kernel(const T* __restrict__ y, const float* __restrict__ w, float* __r
   }
   const float rstd = rsqrtf(dense_block_sum(ss, red) * inv_width + eps);
 #pragma unroll
-  for (int i = 0; i < kStreamVecs; ++i) {
+  for (int i = 0; i < kVecs; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
-      float ww[8];
-      load8<float>(w + vi * 8, ww);
+      if (!kEarly) load8<float>(w + vi * 8, ww[0]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) r[i][j] += v[i][j] * rstd * ww[j];
+      for (int j = 0; j < 8; ++j) r[i][j] += v[i][j] * rstd * ww[kEarly ? i : 0][j];
       store8<float>(x + row * W + vi * 8, r[i]);
       if (xa) store8<T>(xa + row * W + vi * 8, r[i]);
     }
@@ -121,6 +128,7 @@ struct QkvFinishParams {
   const float2* rope;       // (cos, sin)
   const float2* v_rope;
   int v_d, v_table_rows;    // v_d 0: values stay as they are
+  int vectors;              // rotated pairs are whole 8-channel vectors apart, tables 16-byte aligned
   const int* positions;
   const int* slots;
 };
@@ -169,13 +177,33 @@ qkv_finish_kernel(const T* __restrict__ qkv, const T* __restrict__ v_first, T* _
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] *= inv * ww[j];
   }
-  float* mysh = sh[warp] + sub * p.L * 8;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) mysh[c * 8 + j] = v[j];
-  __syncwarp();
-  if (!mine) return;
   const int rot = is_v ? p.v_d : p.rot;
-  if (c * 8 < rot) {
+  // Pairs that are whole vectors apart (half a multiple of 8): the partner vector comes from the lane that holds it and the angles in four
+  // wide loads; else through shared memory, one by one.
+  float* mysh = sh[warp] + sub * p.L * 8;
+  if (p.vectors) {
+    const int half = rot >> 1, step = half >> 3;
+    const bool turns = c * 8 < rot, low = c * 8 < half;
+    float other[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) other[j] = __shfl_sync(0xffffffffu, v[j], turns ? lane + (low ? step : -step) : lane);
+    if (mine && turns) {
+      const int pos = min(p.positions[t], (is_v ? p.v_table_rows : p.table_rows) - 1);
+      const float4* tab = reinterpret_cast<const float4*>((is_v ? p.v_rope : p.rope) + size_t(pos) * half + (low ? c * 8 : c * 8 - half));
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        const float4 cs = tab[j >> 1];  // (cos, sin) of two channels
+        v[j] = v[j] * cs.x + (low ? -other[j] : other[j]) * cs.y;
+        v[j + 1] = v[j + 1] * cs.z + (low ? -other[j + 1] : other[j + 1]) * cs.w;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mysh[c * 8 + j] = v[j];
+    __syncwarp();
+  }
+  if (!mine) return;
+  if (!p.vectors && c * 8 < rot) {
     const int half = rot >> 1, pos = min(p.positions[t], (is_v ? p.v_table_rows : p.table_rows) - 1);
     const float2* tab = (is_v ? p.v_rope : p.rope) + size_t(pos) * half;
     if (p.pairs) {
@@ -343,8 +371,14 @@ extern "C" int mfq_norm_add(const void* y, const float* w, float* x, void* xa, i
                             cudaStream_t stream) {
   const int threads = W > 0 && W % 8 == 0 ? stream_threads(W) : -1;
   if (M <= 0 || threads < 0 || width <= 0 || width > W) return -1;
-  MFQ_BY_TYPE(fp32, launch_kernel(norm_add_kernel<T>, dim3(M), dim3(threads), 0, stream, static_cast<const T*>(y), w, x,
-                                  static_cast<T*>(xa), W, 1.f / float(width), eps));
+  const auto launch = [&](auto kernel, auto* rows, auto* copy) {
+    launch_kernel(kernel, dim3(M), dim3(threads), 0, stream, rows, w, x, copy, W, 1.f / float(width), eps);
+  };
+  // More rows than SMs: several share one.  1508 rows of 4096 on a B200: 17.5 -> 13.5 us.  A few rows are as fast either way on their own
+  // (16: 3.2 us), and a decode step of 16 was 0.5 % slower with the weights asked for ahead of the product it waits for.
+  if (M > 148 && W / 8 <= threads) MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, 1>, static_cast<const T*>(y), static_cast<T*>(xa)));
+  else if (M > 148 && W / 8 <= 2 * threads) MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, 2>, static_cast<const T*>(y), static_cast<T*>(xa)));
+  else MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, kStreamVecs>, static_cast<const T*>(y), static_cast<T*>(xa)));
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 
@@ -399,8 +433,11 @@ extern "C" int mfq_qkv_finish(const void* qkv, int row_stride, const void* v_fir
   if (rot < 0 || rot % 2 || rot > d || (rot > 0 && (!rope || table_rows <= 0))) return -1;
   int L = 1;
   while (L * 8 < max(dk, dv)) L *= 2;
+  const auto aligned = [](const float* t) { return reinterpret_cast<uintptr_t>(t) % 16 == 0; };
+  // 1508 tokens of 48 heads of 128 on a B200: 36.8 -> 21.4 us; a decode step keeps the general form, which it is as fast with.
+  const int vectors = T_ > 148 && !pairs && rot % 16 == 0 && v_d % 16 == 0 && aligned(rope) && aligned(v_rope);
   QkvFinishParams p{T_, Hq, Hk, maps, d, dk, dv, rot, pairs, row_stride, page_size, L, table_rows, eps, lambda, temp, temp_every, first_stride, q_norm, k_norm,
-                    reinterpret_cast<const float2*>(rope), reinterpret_cast<const float2*>(v_rope), v_d, v_table_rows, positions, slots};
+                    reinterpret_cast<const float2*>(rope), reinterpret_cast<const float2*>(v_rope), v_d, v_table_rows, vectors, positions, slots};
   const int heads = Hq + Hk * (maps + 1), per_warp = 32 / L;
   const long long warps = (long long)(T_) * ((heads + per_warp - 1) / per_warp);
   MFQ_BY_TYPE(fp32, launch_kernel(qkv_finish_kernel<T>, dim3(unsigned((warps + 7) / 8)), dim3(256), 0, stream, static_cast<const T*>(qkv),

@@ -7,8 +7,8 @@ import pytest
 import torch
 
 from mfq_b200 import ops
-from mfq_b200.engine.kv_cache import PagedKVCache
-from mfq_b200.ops import dense, moe, w4
+from mfq_b200.engine.kv_cache import PagedKVCache, PlainPagedKVCache
+from mfq_b200.ops import dense, moe, w4, window_attn
 from mfq_b200.ops import kernels as K
 from mfq_b200.ops.dense import DenseLinear
 from gpu_common import check_status, require_gpu_lib
@@ -162,3 +162,48 @@ def test_w4_rows_off_a_vector_are_refused(m):
     x = torch.zeros(m * 256 + 8, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(RuntimeError):
         w4.w4_gemm(x[1:1 + m * 256].view(m, 256), w)
+
+
+@pytest.mark.parametrize("dtype,ulp", [(torch.float32, 2.0 ** -23), (torch.bfloat16, 2.0 ** -7)])
+@pytest.mark.parametrize("d,rot,v_rot", [(128, 128, 0), (128, 64, 0), (16, 16, 16), (256, 256, 128), (80, 48, 0), (96, 0, 32)])
+def test_heads_rotated_by_vectors_agree_with_the_general_form(d, rot, v_rot, dtype, ulp):
+    """A table 8 bytes past a 16-byte boundary takes the general form.  Both evaluate a cos + b sin, a and b at most the row's largest
+    value: each rounds at most twice, so they differ by 4 * 2 * 2^-24 of it, and by one place more where that is rounded to the type."""
+    require_gpu_lib()
+    t, h, g = 149, 6, 2  # the fewest tokens of the rule
+    rows = _normal(1, t, (h + 2 * g) * d, dtype=dtype)
+    pos = torch.randint(0, 900, (t,), device="cuda", dtype=torch.int32)
+    slots = (torch.randperm(160, device="cuda")[:t] + 16).int()
+    slots[5] = -1
+
+    def finish(shift):
+        def table(r):
+            if not r:
+                return None
+            whole = torch.zeros(1000 * r + 4, device="cuda")
+            assert whole.data_ptr() % 16 == 0
+            part = whole[shift:shift + 1000 * r].view(1000, r // 2, 2)
+            return part.copy_(window_attn.rope_table(3e4, r, 1000, "cuda"))
+        cache = PlainPagedKVCache([(g, d, d)], dtype, num_pages=11, max_seqs=1, max_pages_per_seq=11, device="cuda")
+        turn = window_attn.ValueTurn(table(v_rot), v_rot) if v_rot else None
+        norm = _normal(2, d, dtype=torch.float32)
+        q = window_attn.qkv_finish(rows, cache.layer(0), pos, slots, heads=h, kv_heads=g, dim=d, q_norm=norm, k_norm=norm, rope=table(rot),
+                                   rot=rot, eps=1e-5, turn=turn)
+        return q, cache.layer(0).k.clone(), cache.layer(0).v.clone()
+
+    for got, want in zip(finish(0), finish(2)):
+        got, want = got.double(), want.double()
+        assert ((got - want).abs() <= (2.0 ** -21 + ulp) * want.abs().amax(-1, keepdim=True)).all()
+
+
+@pytest.mark.parametrize("m", [148, 149])
+@pytest.mark.parametrize("w", [8, 2048, 2056, 4096, 4104])
+def test_stream_rows_by_vectors_per_thread(m, w):
+    """Widths around one and two vectors per thread, rows around the line of the rule."""
+    require_gpu_lib()
+    y, f, x = _normal(m, m, w), _normal(1, w, dtype=torch.float32), _normal(2, m, w, dtype=torch.float32)
+    want, act = x.double() + y.double() * torch.rsqrt(y.double().square().mean(1, keepdim=True) + 1e-5) * f.double(), torch.empty_like(y)
+    size = x.double().abs() + (want - x.double()).abs()
+    dense.norm_add(y, f, x, act, w, 1e-5)
+    # a tree of w squares, its root and three more roundings: below 32 of 2^-24, of the size of the two terms
+    assert ((x.double() - want).abs() <= 2.0 ** -19 * size).all() and torch.equal(act, x.bfloat16())
