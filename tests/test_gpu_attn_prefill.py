@@ -132,7 +132,8 @@ def test_prefix_cache_restores_pages_on_gpu(tmp_path):
 
 
 @pytest.mark.parametrize("t,past,hq,hk,scale", [(1, 0, 2, 1, 0.09), (127, 1, 6, 2, 0.09), (129, 0, 3, 3, 0.09), (257, 126, 3, 1, 0.09), (385, 0, 8, 2, 0.09),
-                                                (256, 130, 4, 1, 0.0)])
+                                                (256, 130, 4, 1, 0.0), (128, 0, 148, 74, 0.09), (128, 1, 150, 75, 0.09), (257, 126, 51, 17, 0.09),
+                                                (257, 126, 50, 25, 0.0), (385, 0, 45, 15, 0.09)])  # up to 148 tiles: one per CTA
 def test_prefill_attention_on_two_tiles(t, past, hq, hk, scale):
     """Two heads of a KV head, or two query blocks where their number is odd; a last pair without a second block; keys that grow, so
     that O is rescaled in every block; a scale of zero."""
