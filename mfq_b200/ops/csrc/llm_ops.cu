@@ -679,8 +679,8 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
   // Enough tokens to fill the GPU with a warp for several heads each: the angles (sine, cosine and the frequency's power) are a good
   // part of the work of a head.  4096 tokens of 48 heads on a B200: 71 us with one head per warp, 64 with eight (the pages' single-byte
-  // stores take most of that); 357 tokens: 11.7 and 10.4, with a warp or two per scheduler left.
-  const int heads = Hq + 2 * Hk, per = long(T) * heads >= 8L * 148 * 8 ? 8 : 1;
+  // stores take most of that); 357 tokens: 11.7 and 10.4; 200: 7.8 and 9.7.
+  const int heads = Hq + 2 * Hk, per = long(T) * heads >= 8L * 148 * 14 ? 8 : 1;
   const long warps = long(T) * ((heads + per - 1) / per);
   const int blocks = int((warps + 7) / 8);
   const float l2t = log2f(theta);
