@@ -241,6 +241,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       uint32_t ro[32];  // first half of the previous block's P V, under the exchange (block 0: not used)
       tmem_ld_32x32(tO, ro);
       ok = mbar_wait_warp(&x_bar[x], j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
+      tmem_wait_ld();  // on every path: the registers of a load that is not used are the load's all the same until it is complete
       if (!ok) break;
       mx = fmaxf(mx, s_max[(sb * 2 + (half ^ 1)) * kQB + row]);
       const float m_new = fmaxf(m_run, mx);
@@ -250,8 +251,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       if (j > 0) {
 #pragma unroll
         for (int c = 0; c < 64; c += 32) {
-          if (c > 0) tmem_ld_32x32(tO + c, ro);
-          tmem_wait_ld();
+          if (c > 0) {
+            tmem_ld_32x32(tO + c, ro);
+            tmem_wait_ld();
+          }
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[c + i] = (o[c + i] + __uint_as_float(ro[i])) * alpha;
         }

@@ -1,0 +1,23 @@
+"""What the sources of the CUDA kernels promise on every path, where a run cannot show it."""
+
+import re
+
+import pytest
+
+from mfq_b200.ops.build import CSRC
+
+LOADS = re.compile(r"\btmem_ld_\w+\(")
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu*") if p.name != "common.cuh" and LOADS.search(p.read_text())))
+def test_no_path_leaves_between_a_tensor_memory_load_and_its_wait(name):
+    """Until ``tcgen05.wait::ld`` the registers of a load are the load's, whether its values are used or not: a jump out of the
+    sequence would hand them to other values while the load may still write them."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    for load in LOADS.finditer(text):
+        wait = text.find("tmem_wait_ld()", load.end())
+        if wait < 0:  # requested one round ahead: the next round of an unrolled loop begins with the wait
+            assert "#pragma unroll" in text[: load.start()] and "tmem_wait_ld()" in text[: load.start()]
+            continue
+        between = text[load.end() : wait]
+        assert not re.search(r"\b(break|continue|return|goto)\b", between), f"{name}:{text.count(chr(10), 0, load.start()) + 1}"
