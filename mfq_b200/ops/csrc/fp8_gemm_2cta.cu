@@ -183,7 +183,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       for (int tt = 0; tt < CW; ++tt) acc[tt] = 0.f;
       const float* wsc = p.w_scale + size_t(n0 / kRows) * nkb;
       __syncwarp();  // the previous tile's reads of this warp's slices are done
-      for (int j = lane; j < CW; j += 32) xs_w[j] = (t0 + col0 + j < p.M) ? __ldg(p.x_scale + t0 + col0 + j) : 0.f;
+      for (int j = lane; j < CW; j += 32) xs_w[j] = (t0 + col0 + j < p.M) ? p.x_scale[t0 + col0 + j] : 0.f;  // no __ldg: written since this grid began
       if (ws_cached)
         for (int j = lane; j < nkb; j += 32) ws_w[j] = __ldg(wsc + j);
       __syncwarp();

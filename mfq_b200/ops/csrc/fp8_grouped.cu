@@ -72,10 +72,11 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   pdl_wait();
 
   // Tile t = (entry t / n_tiles of the map, weight rows of block t % n_tiles): CTAs at work at the same time share token rows.  Entries
-  // are dense: the first unused one ends the list.
+  // are dense: the first unused one ends the list.  The plan and the row multipliers are read by plain loads: under the programmatic
+  // launch this grid began before they were written, so they are not constant for its life, as __ldg promises (weights are).
   const int n_tiles = p.N / kTileN, nkb = p.K / kBlockK, tiles = p.map_len * n_tiles, step = int(gridDim.x);
   auto entry = [&](int tile) {  // the same for the whole warp
-    const int2 e = tile < tiles ? __ldg(p.tile_map + tile / n_tiles) : make_int2(-1, 0);
+    const int2 e = tile < tiles ? p.tile_map[tile / n_tiles] : make_int2(-1, 0);
     return make_int2(__shfl_sync(0xffffffffu, e.x, 0), __shfl_sync(0xffffffffu, e.y, 0));
   };
 
@@ -90,10 +91,10 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     uint32_t phase = 0;
     bool ok = true;
     int2 e = entry(blockIdx.x);
-    int first = e.x >= 0 ? __ldg(p.offsets + e.x) : 0;
+    int first = e.x >= 0 ? p.offsets[e.x] : 0;
     for (int tile = blockIdx.x; ok && e.x >= 0; tile += step) {
       const int2 next = entry(tile + step);
-      const int next_first = next.x >= 0 ? __ldg(p.offsets + next.x) : 0;
+      const int next_first = next.x >= 0 ? p.offsets[next.x] : 0;
       const int t0 = __shfl_sync(0xffffffffu, first, 0) + e.y * BT, n0 = tile % n_tiles * kTileN;
       for (int i = 0; i < nkb; ++i) {
         ok = mbar_wait_warp(&empty[s], phase ^ 1u, abort_flag, p.status, kStatusTimeoutProducer);
@@ -142,8 +143,8 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     float ws = 0.f;
     auto fetch = [&](int tile, int2 at) {
       if (at.x < 0) return;
-      lo = __ldg(p.offsets + at.x);
-      hi = __ldg(p.offsets + at.x + 1);
+      lo = p.offsets[at.x];
+      hi = p.offsets[at.x + 1];
       if (lane < nkb) ws = __ldg(p.w_scale + (size_t(at.x) * n_tiles + tile % n_tiles) * nkb + lane);
     };
     fetch(blockIdx.x, e);
@@ -153,7 +154,7 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       const float* wsc = p.w_scale + (size_t(e.x) * n_tiles + tile % n_tiles) * nkb;
       float xs[(CW + 31) / 32];  // row multipliers of this warp's columns, one per lane
 #pragma unroll
-      for (int j = 0; j < (CW + 31) / 32; ++j) xs[j] = col0 + j * 32 + lane < tl ? __ldg(p.x_scale + t0 + col0 + j * 32 + lane) : 0.f;
+      for (int j = 0; j < (CW + 31) / 32; ++j) xs[j] = col0 + j * 32 + lane < tl ? p.x_scale[t0 + col0 + j * 32 + lane] : 0.f;
       float acc[CW];
 #pragma unroll
       for (int tt = 0; tt < CW; ++tt) acc[tt] = 0.f;

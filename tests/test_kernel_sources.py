@@ -21,3 +21,11 @@ def test_no_path_leaves_between_a_tensor_memory_load_and_its_wait(name):
             continue
         between = text[load.end() : wait]
         assert not re.search(r"\b(break|continue|return|goto)\b", between), f"{name}:{text.count(chr(10), 0, load.start()) + 1}"
+
+
+@pytest.mark.parametrize("name", ["fp8_grouped.cu", "fp8_gemm_2cta.cu"])
+def test_what_the_kernel_before_wrote_is_not_read_as_constant(name):
+    """Under a programmatic launch a grid begins before its inputs are written: only weights may be read through ``__ldg``, which
+    promises data that stays the same for the life of the kernel."""
+    sources = re.findall(r"__ldg\((?:p\.)?(\w+)", (CSRC / name).read_text())
+    assert sources and set(sources) <= {"wsc", "w_scale"}
