@@ -1,18 +1,17 @@
 // Causal self-attention for prefill chunks on tcgen05 tensor cores (bf16 in, fp32 accumulate, head dim 128, GQA).
 //
-// A CTA works on TWO tiles of 128 queries at a time, A and B: the same queries of two heads that share a KV head (both then read the
-// same keys and values), or, where a KV head has an odd number of query heads, two neighbouring query blocks of one head.  Per tile and
-// 128-key block:
+// One CTA = (128-query block, query head).  Per 128-key block:
 //   S = Q K^T      tcgen05.mma kind::f16, A = Q tile, B = K tile (both K-major, TMA 128 B swizzle), S in TMEM
 //   P = softmax    8 warps, two threads per query row (64 keys each): two passes over the TMEM row (max, then exp2 + sum), row maxima
 //                  exchanged through shared memory; P goes back as bf16 pairs into the columns its own scores came from
 //   O_blk = P V    tcgen05.mma with P from TENSOR MEMORY as the A operand and V as an MN-major B operand (the [key][dim] tile exactly
 //                  as TMA delivers it)
 //   O = (O + O_blk(prev)) * alpha   folded in fp32 registers, so TMEM never needs an in-place rescale
-// The chain  S -> softmax -> P V  of one tile is several times as long as its MMAs: with one tile per CTA a block took 5400 cycles of
-// which the tensor core worked 1000.  Here the softmax warps of A compute while the tensor core works for B and the other way round,
-// four warps per scheduler cover each other's latencies, and P no longer passes through shared memory and a proxy fence.
-// 4096 tokens of 32 heads on a B200: 318 -> 197 us; 1000 tokens after 3001: 145 -> 102 us, with the same bits.
+// The chain  softmax -> P V -> fold  is several times as long as the MMAs, so Q K^T of block j + 1 is issued before P V of block j, into
+// the other of two S buffers, and all of it but the chain itself is hidden; P never passes through shared memory and its proxy fence.
+// What bounds it is the softmax: exponentials, and the two passes over S.  32 heads on a B200, P through shared memory and MMAs issued
+// by one lane | two tiles per CTA on one S buffer each, whose eight more warps leave a thread 104 registers | this, same bits:
+//   120 tokens 8.5 | 13.1 | 6.8 us    512 after 4000  84 | 110 | 55    1000 after 3001  144 | 101 | 90    4096  316 | 197 | 190    16384  3933 | 2533 | 2501
 // Heaviest (latest) query blocks are scheduled first, over all heads.
 //
 // The reference's prefill attention is a llama.cpp-derived mma.sync flash-attention (mfq_fattn_mma_f16.cuh) and a
@@ -26,9 +25,8 @@ namespace mfq {
 constexpr int kQB = 128, kKB = 128, kHD = 128;
 constexpr int kTileBytes = kQB * kHD * 2;       // 32 KB: one [128 x 128] bf16 tile = two 16 KB swizzled halves
 constexpr int kHalfBytes = kTileBytes / 2;
-constexpr int kPrefillThreads = 128 + 2 * 256;  // TMA warp, MMA warp, two idle warps; eight softmax warps per tile
-constexpr int kExchange = 6 * kQB;              // floats per tile: maxima [2 buffers][2 halves][128 rows], sums [2 halves][128]
-constexpr int kPrefillSmem = 2 * kTileBytes /*Q*/ + 2 * 2 * kTileBytes /*K, V x 2 stages*/ + 1024 + 256 + 2 * kExchange * 4;
+constexpr int kPrefillThreads = 128 + 256;  // TMA warp, MMA warp, two idle warps; eight softmax warps
+constexpr int kPrefillSmem = kTileBytes /*Q*/ + 2 * 2 * kTileBytes /*K, V x 2 stages*/ + 1024 + 256 + 6 * kQB * 4 /*row max / sum exchange*/;
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -70,8 +68,6 @@ struct PrefillParams {
   int Tk, offset;      // keys available; query row i sees keys 0 .. i + offset (offset = Tk - T: tokens before the chunk)
   float scale_log2;
   int* status;
-  int two_heads;       // tiles A, B: two heads of a KV head at the same queries (1) or two query blocks of a head (0)
-  int single;     // tile B is absent
 };
 
 __global__ void __launch_bounds__(kPrefillThreads, 1)
@@ -79,8 +75,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = base;                               // tile A, tile B
-  uint8_t* sK = base + 2 * kTileBytes;              // two stages
+  uint8_t* sQ = base;
+  uint8_t* sK = base + kTileBytes;                  // two stages
   uint8_t* sV = sK + 2 * kTileBytes;                // two stages
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * kTileBytes);
   uint64_t* q_full = bars;            // 1
@@ -88,34 +84,27 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   uint64_t* k_empty = bars + 3;
   uint64_t* v_full = bars + 5;
   uint64_t* v_empty = bars + 7;
-  uint64_t* s_full = bars + 9;        // [2] per tile: S of a block is complete, and with it every MMA issued before
-  uint64_t* p_full = bars + 11;       // [2] per tile, 8 arrivals: P is in TMEM, and O has been read
-  uint64_t* o_full = bars + 13;       // [2] per tile, once
-  uint64_t* x_bar = bars + 15;        // [2] per tile, 8 arrivals: row-maximum exchange, one phase per key block
-  uint64_t* l_bar = bars + 17;        // [2] per tile, 8 arrivals: row-sum exchange, once
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* s_full = bars + 9;        // [2] per S buffer
+  uint64_t* p_full = bars + 11;       // 8 arrivals: P is in TMEM, and O has been read
+  uint64_t* o_full = bars + 12;       // P V of a block is complete
+  uint64_t* x_bar = bars + 13;        // 8 arrivals: row-maximum exchange, one phase per key block
+  uint64_t* l_bar = bars + 14;        // 8 arrivals: row-sum exchange, once
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* exchange = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);
+  float* s_max = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // max: [2 buffers][2 halves][128 rows]; sum: [2 halves][128 rows]
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
-  const int num_qb = (p.T + kQB - 1) / kQB;
-  const int heavy = int(gridDim.y) - 1 - int(blockIdx.y);  // heavy blocks first
-  const int head_a = p.two_heads ? 2 * blockIdx.x : blockIdx.x, qb_a = p.two_heads || p.single ? heavy : 2 * heavy;
-  const int head[2] = {head_a, p.two_heads ? head_a + 1 : head_a};
-  const int qb[2] = {qb_a, p.two_heads ? qb_a : p.single ? num_qb : qb_a + 1};
-  const int kvh = head_a / (p.Hq / p.Hk);
-  // causal with a past: the last query of a block sees keys up to (qb + 1) * kQB - 1 + offset
-  const int k_blocks = (p.Tk + kKB - 1) / kKB;
-  const int n_a = min(k_blocks, ((qb[0] + 1) * kQB + p.offset + kKB - 1) / kKB);
-  const int n_b = qb[1] < num_qb ? min(k_blocks, ((qb[1] + 1) * kQB + p.offset + kKB - 1) / kKB) : 0;
-  const int n_max = max(n_a, n_b);
+  const int qb = (p.T + kQB - 1) / kQB - 1 - int(blockIdx.x) / p.Hq;  // heavy blocks first
+  const int head = int(blockIdx.x) % p.Hq, kvh = head / (p.Hq / p.Hk);
+  // causal with a past: the last query of the block sees keys up to (qb + 1) * kQB - 1 + offset
+  const int nblk = min((p.Tk + kKB - 1) / kKB, ((qb + 1) * kQB + p.offset + kKB - 1) / kKB);
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); mbar_init(&o_full[i], 1); mbar_init(&x_bar[i], 8); mbar_init(&l_bar[i], 8);
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); mbar_init(&s_full[i], 1);
     }
+    mbar_init(p_full, 8); mbar_init(o_full, 1); mbar_init(x_bar, 8); mbar_init(l_bar, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -124,18 +113,15 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  // columns: S of A, S of B (P of 64 keys in the first half of each 64 columns), O of A, O of B
-  if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+  // columns: S of even blocks, S of odd blocks (P of 64 keys in the first half of each 64 columns), O
 
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
-      mbar_expect_tx(q_full, 2 * kTileBytes);
-      for (int x = 0; x < 2; ++x)
-        for (int h = 0; h < 2; ++h)
-          tma_load_2d(sQ + x * kTileBytes + h * kHalfBytes, &tmap_q, q_full, head[x] * kHD + 64 * h, qb[x] * kQB);  // past the end: zeros
-      for (int j = 0; j < n_max; ++j) {
+      mbar_expect_tx(q_full, kTileBytes);
+      tma_load_2d(sQ, &tmap_q, q_full, head * kHD, qb * kQB);
+      tma_load_2d(sQ + kHalfBytes, &tmap_q, q_full, head * kHD + 64, qb * kQB);
+      for (int j = 0; j < nblk; ++j) {
         const int s = j & 1;
         const uint32_t parity = ((j >> 1) & 1) ^ 1;
         uint8_t *k = sK + s * kTileBytes, *v = sV + s * kTileBytes;
@@ -157,107 +143,93 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), k_desc0 = umma_desc_k_sw128(smem_u32(sK));
     const uint64_t v_desc0 = umma_desc_mn_sw128(smem_u32(sV), kHalfBytes);
     const uint32_t s_full_addr = smem_u32(s_full);
-    auto issue_qk = [&](int x, int j) {  // S of tile x takes the place of its P, which the MMAs before have read
-      const uint64_t a = q_desc + uint64_t(x) * kTile, b = k_desc0 + uint64_t(j & 1) * kTile;
-      const uint32_t d = tmem_base + uint32_t(x) * 128u;
-      umma_f16_block(d, a, b, idesc_qk, 0u);
-      umma_f16_block(d, a + kHalf, b + kHalf, idesc_qk, 1u, s_full_addr + x * 8);
+    auto issue_qk = [&](int j) {  // S takes the place of P of block j - 2, which the MMAs before have read
+      const uint64_t k_desc = k_desc0 + uint64_t(j & 1) * kTile;
+      const uint32_t d = tmem_base + uint32_t(j & 1) * 128u;
+      umma_f16_block(d, q_desc, k_desc, idesc_qk, 0u);
+      umma_f16_block(d, q_desc + kHalf, k_desc + kHalf, idesc_qk, 1u, s_full_addr + (j & 1) * 8);
+      tc_commit_warp(&k_empty[j & 1]);
     };
     bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, kStatusTimeoutMma) &&
               mbar_wait_warp(&k_full[0], 0, abort_flag, p.status, kStatusTimeoutMma);
     if (ok) {
       tc_fence_after();
-      issue_qk(0, 0);
-      if (n_b > 0) issue_qk(1, 0);
-      tc_commit_warp(&k_empty[0]);
+      issue_qk(0);
     }
-    for (int j = 0; ok && j < n_max; ++j) {
-      ok = mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma);
-      if (ok && j + 1 < n_max) ok = mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma);
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const int n = x == 0 ? n_a : n_b;
-        if (!ok || j >= n) continue;
-        ok = mbar_wait_warp(&p_full[x], j & 1, abort_flag, p.status, kStatusTimeoutMma);
-        if (!ok) continue;
+    for (int j = 0; ok && j < nblk; ++j) {
+      if (j + 1 < nblk) {
+        ok = mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t o_addr = tmem_base + 256u + uint32_t(x) * 128u, p_addr = tmem_base + uint32_t(x) * 128u;
-        const uint64_t v_desc = v_desc0 + uint64_t(j & 1) * kTile;
-        umma_pv(o_addr, p_addr, v_desc, idesc_pv, 0u);
-        umma_pv(o_addr, p_addr + 64u, v_desc + 512, idesc_pv, 1u);
-        if (j + 1 < n) issue_qk(x, j + 1);
-        else tc_commit_warp(&o_full[x]);
+        issue_qk(j + 1);
       }
-      if (ok) {
-        tc_commit_warp(&v_empty[j & 1]);
-        if (j + 1 < n_max) tc_commit_warp(&k_empty[(j + 1) & 1]);
-      }
+      ok = mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutMma) &&
+           mbar_wait_warp(p_full, j & 1, abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t p_addr = tmem_base + uint32_t(j & 1) * 128u;
+      const uint64_t v_desc = v_desc0 + uint64_t(j & 1) * kTile;
+      umma_pv(tmem_base + 256u, p_addr, v_desc, idesc_pv, 0u);
+      umma_pv(tmem_base + 256u, p_addr + 64u, v_desc + 512, idesc_pv, 1u);
+      tc_commit_warp(o_full);
+      tc_commit_warp(&v_empty[j & 1]);
     }
-  }
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
-    // ----- softmax warps of tile x: two threads per query row (TMEM lane); `half` selects 64 of the 128 keys of a block and 64 of the
-    // 128 output dims -----
-    const int x = (warp - 4) >> 3, half = ((warp - 4) >> 2) & 1, quarter = warp & 3;
-    const int row = quarter * 32 + lane, q_idx = qb[x] * kQB + row;
-    const int n = x == 0 ? n_a : n_b;
-    const uint32_t lane_base = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(x) * 128u + uint32_t(half) * 64u;
-    const uint32_t tS = lane_base, tO = lane_base + 256u;
-    float* s_max = exchange + x * kExchange;
+  } else if (warp >= 4) {
+    // ----- softmax warps: two threads per query row (TMEM lane); `half` selects 64 of the 128 keys of a block and 64 of the 128 output
+    // dims -----
+    const int half = (warp - 4) >> 2, quarter = warp & 3;
+    const int row = quarter * 32 + lane, q_idx = qb * kQB + row;
+    const uint32_t lane_base = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(half) * 64u;
+    const uint32_t tO = lane_base + 256u;
     float o[64];
 #pragma unroll
     for (int d = 0; d < 64; ++d) o[d] = 0.f;
     float m_run = -FLT_MAX, l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < n; ++j) {
+    for (int j = 0; j < nblk; ++j) {
       const int sb = j & 1;
-      ok = mbar_wait_warp(&s_full[x], j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
+      const uint32_t tS = lane_base + uint32_t(sb) * 128u;
+      ok = mbar_wait_warp(&s_full[sb], (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (!ok) break;
       tc_fence_after();
       const int key0 = j * kKB + half * 64;
       // masking is needed where the block reaches past the FIRST query's horizon or past the last key
-      const bool diag = ((j + 1) * kKB - 1 > qb[x] * kQB + p.offset) || ((j + 1) * kKB > p.Tk);
+      const bool diag = ((j + 1) * kKB - 1 > qb * kQB + p.offset) || ((j + 1) * kKB > p.Tk);
       // pass 1: maximum over this thread's 64 columns, then exchange with the partner thread of the row
       float mx = -FLT_MAX;
-#pragma unroll
-      for (int c = 0; c < 64; c += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tS + c, r);
+      {
+        uint32_t r[2][32];
+        tmem_ld_32x32(tS, r[0]);
+        tmem_ld_32x32(tS + 32, r[1]);
         tmem_wait_ld();
         if (!diag) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
+          for (int i = 0; i < 64; ++i) mx = fmaxf(mx, __uint_as_float(r[i >> 5][i & 31]));
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = key0 + c + i;
-            mx = fmaxf(mx, (key <= q_idx + p.offset && key < p.Tk) ? __uint_as_float(r[i]) : -FLT_MAX);
-          }
+          for (int i = 0; i < 64; ++i)
+            mx = fmaxf(mx, (key0 + i <= q_idx + p.offset && key0 + i < p.Tk) ? __uint_as_float(r[i >> 5][i & 31]) : -FLT_MAX);
         }
       }
       s_max[(sb * 2 + half) * kQB + row] = mx;
       __syncwarp();
-      if (lane == 0) mbar_arrive(&x_bar[x]);
-      uint32_t ro[32];  // first half of the previous block's P V, under the exchange (block 0: not used)
-      tmem_ld_32x32(tO, ro);
-      ok = mbar_wait_warp(&x_bar[x], j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
-      tmem_wait_ld();  // on every path: the registers of a load that is not used are the load's all the same until it is complete
+      if (lane == 0) mbar_arrive(x_bar);
+      ok = mbar_wait_warp(x_bar, j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (!ok) break;
       mx = fmaxf(mx, s_max[(sb * 2 + (half ^ 1)) * kQB + row]);
       const float m_new = fmaxf(m_run, mx);
       const float alpha = fast_exp2((m_run - m_new) * p.scale_log2);
-      // fold the previous block's P V (it was computed against m_run), then move to the new maximum.  It has retired: its MMAs were
-      // issued before those of the S that was waited for.
+      // fold the previous block's P V (it was computed against m_run), then move to the new maximum
       if (j > 0) {
+        ok = mbar_wait_warp(o_full, (j - 1) & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[2][32];
+        tmem_ld_32x32(tO, r[0]);
+        tmem_ld_32x32(tO + 32, r[1]);
+        tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 64; c += 32) {
-          if (c > 0) {
-            tmem_ld_32x32(tO + c, ro);
-            tmem_wait_ld();
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[c + i] = (o[c + i] + __uint_as_float(ro[i])) * alpha;
-        }
+        for (int i = 0; i < 64; ++i) o[i] = (o[i] + __uint_as_float(r[i >> 5][i & 31])) * alpha;
       }
       l_run *= alpha;
       m_run = m_new;
@@ -293,20 +265,20 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[x]);
+      if (lane == 0) mbar_arrive(p_full);
     }
-    if (ok && n > 0) {
+    if (ok) {
       // total row sum = both halves
       s_max[(4 + half) * kQB + row] = l_run;  // own slots: the last block's maxima may still be read
       __syncwarp();
-      if (lane == 0) mbar_arrive(&l_bar[x]);
-      ok = mbar_wait_warp(&l_bar[x], 0, abort_flag, p.status, kStatusTimeoutEpilogue) &&
-           mbar_wait_warp(&o_full[x], 0, abort_flag, p.status, kStatusTimeoutEpilogue);
+      if (lane == 0) mbar_arrive(l_bar);
+      ok = mbar_wait_warp(l_bar, 0, abort_flag, p.status, kStatusTimeoutEpilogue) &&
+           mbar_wait_warp(o_full, (nblk - 1) & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (ok) {
         tc_fence_after();
         const float l_tot = l_run + s_max[(4 + (half ^ 1)) * kQB + row];
         const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
-        __nv_bfloat16* dst = p.out + (size_t(q_idx) * p.Hq + head[x]) * kHD + half * 64;
+        __nv_bfloat16* dst = p.out + (size_t(q_idx) * p.Hq + head) * kHD + half * 64;
 #pragma unroll
         for (int c = 0; c < 64; c += 32) {
           uint32_t r[32];
@@ -351,13 +323,8 @@ extern "C" int mfq_attn_prefill_past(const void* q, const void* k, const void* v
     if (cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem) != cudaSuccess) return -6;
     attr = true;
   }
-  const int q_blocks = (T + kQB - 1) / kQB;
-  // As long as every tile can have an SM of its own it does, B absent: two tiles of a short prompt only wait for each other (120 tokens of
-  // 32 heads: 13.2 us in pairs, 9.6 alone; 200 tokens: 14.4 and 11.4).
-  const int single = long(Hq) * q_blocks <= 148, two_heads = !single && Hq / Hk % 2 == 0;
-  const PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status, two_heads, single};
-  const dim3 grid(two_heads ? Hq / 2 : Hq, two_heads || single ? q_blocks : (q_blocks + 1) / 2);
-  attn_prefill_kernel<<<grid, kPrefillThreads, kPrefillSmem, stream>>>(tq, tk, tv, p);
+  const PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status};
+  attn_prefill_kernel<<<dim3((T + kQB - 1) / kQB * Hq), kPrefillThreads, kPrefillSmem, stream>>>(tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 

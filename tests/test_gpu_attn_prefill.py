@@ -133,10 +133,10 @@ def test_prefix_cache_restores_pages_on_gpu(tmp_path):
 
 @pytest.mark.parametrize("t,past,hq,hk,scale", [(1, 0, 2, 1, 0.09), (127, 1, 6, 2, 0.09), (129, 0, 3, 3, 0.09), (257, 126, 3, 1, 0.09), (385, 0, 8, 2, 0.09),
                                                 (256, 130, 4, 1, 0.0), (128, 0, 148, 74, 0.09), (128, 1, 150, 75, 0.09), (257, 126, 51, 17, 0.09),
-                                                (257, 126, 50, 25, 0.0), (385, 0, 45, 15, 0.09)])  # up to 148 tiles: one per CTA
-def test_prefill_attention_on_two_tiles(t, past, hq, hk, scale):
-    """Two heads of a KV head, or two query blocks where their number is odd; a last pair without a second block; keys that grow, so
-    that O is rescaled in every block; a scale of zero."""
+                                                (257, 126, 50, 25, 0.0), (385, 0, 45, 15, 0.09), (130, 1000, 2, 1, 0.09)])
+def test_prefill_attention_over_tiles_and_heads(t, past, hq, hk, scale):
+    """One key block up to nine, so that both S buffers and stages come around; odd counts of heads and blocks, more tiles than SMs; keys
+    that grow, so that O is rescaled in every block; a scale of zero."""
     require_gpu_lib()
     g = torch.Generator(device="cuda").manual_seed(t + past)
     q = torch.randn((t, hq, 128), generator=g, device="cuda").to(torch.bfloat16)
@@ -146,4 +146,4 @@ def test_prefill_attention_on_two_tiles(t, past, hq, hk, scale):
     got = ops.kernels.attn_prefill_bf16(q, k, v, scale)
     check_status()
     # probabilities and the result are rounded to bf16 (2^-9 each, relative): well inside 2 % of (|ref| + rms / 4)
-    assert_close(got, ref.attention(q, k, v, scale, causal_offset=past), rel=2e-2, what=f"two tiles T={t} past={past}")
+    assert_close(got, ref.attention(q, k, v, scale, causal_offset=past), rel=2e-2, what=f"T={t} past={past}")
