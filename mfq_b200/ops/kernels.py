@@ -102,11 +102,14 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     """Token tile of the two-SM GEMM for this shape, 0 = use the one-SM kernel.  ``MFQ_GEMM_PAIR`` = 0 / 128 / 256
     overrides the choice.
 
-    Its pairs walk tiles of 256 weight rows; on B200 a tile takes 2.9 + 0.306 us per K block with 128 tokens and 6.7 + 0.506 us with
-    256 (fitted to the projections of an 8B layer at 357 .. 4096 tokens), so the better tile is a matter of whole waves: 1000 x 6144 x
-    4096 is 38.6 against 46.9 us, 1000 x 4096 x 14336 73.7 against 64.5.  The one-SM kernel keeps what it is better at: up to 64
-    tokens, rows that are not whole pairs of blocks, and long K ranges over so few tiles that half of the pairs would idle, which it
-    splits (128 x 4096 x 14336: 19.9 against 37.8 us; at 357 tokens, 48 tiles, it takes 83 against 39.5)."""
+    Both sides by wave models in microseconds, fitted on B200 to 652 shapes of 65 .. 4096 tokens, 256 .. 28672 rows and K 512 .. 14336.
+    Pairs walk tiles of 256 weight rows: a wave takes 2.9 + 0.306 per K block with 128 tokens, 6.7 + 0.506 with 256, and about 1.5 for
+    every split sum beyond two, which one pair works through one after the other; the launch costs 3.2.  A wave of one-SM CTAs takes 6.1 + 0.36
+    per K block of a split, and meeting 4.4 with two splits, 2 in a larger cluster, 10 in memory; clusters in a grid
+    of nearly every SM do not all fit (6).  So few tiles over a range that the one-SM kernel splits stay there (66 x 256 x 2048: 6.2
+    against 20.0 us; 128 x 4096 x 4096: 11.6 against 19.1), full waves come here (1000 x 6144 x 4096: 38.6 with 128 tokens).
+    Where half of the pairs would idle over more than 64 K blocks the one-SM kernel is kept without a sum (128 x 4096 x 14336: 19.9
+    against 37.8 us)."""
     forced = os.environ.get("MFQ_GEMM_PAIR")
     if n % 256 or m < PAIR_MIN_ROWS:
         return 0
@@ -116,10 +119,14 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     tiles = {t: n // 256 * math.ceil(m / t) for t in (128, 256)}
     if 2 * tiles[128] <= pairs and blocks > 64:
         return 0
-    if split_blocks(m, n, k):
-        return 128
-    cost = {t: math.ceil(tiles[t] / pairs) * (ramp + per * blocks) for t, ramp, per in ((128, 2.9, 0.306), (256, 6.7, 0.506))}
-    return 128 if cost[128] <= cost[256] else 256
+    per = split_blocks(m, n, k) or blocks
+    splits = math.ceil(blocks / per)
+    cost = {t: 3.2 + math.ceil(tiles[t] / pairs) * (ramp + step * blocks + 1.5 * max(0, splits - 2))
+            for t, ramp, step in ((128, 2.9, 0.306), (256, 6.7, 0.506))}
+    tile = 128 if splits > 1 or cost[128] <= cost[256] else 256
+    ctas = math.ceil(n / 128) * math.ceil(m / 128) * splits
+    meet = {1: 0.0, 2: 4.4}.get(splits, 2.0 if splits <= 8 else 10.0) + (6.0 if splits > 1 and 128 < ctas <= sms else 0.0)
+    return tile if cost[tile] < math.ceil(ctas / sms) * (6.1 + 0.36 * per + meet) else 0
 
 
 def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, *,
