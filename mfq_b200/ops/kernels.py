@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import math
 import os
+from functools import lru_cache
 
 import torch
 
@@ -46,6 +47,7 @@ def _token_tile(m: int) -> int:
     return 16 if m <= 16 else 32 if m <= 32 else 64 if m <= 64 else 128
 
 
+@lru_cache(maxsize=4096)  # sizes only; a prompt asks for the same few once per layer
 def pick_splits(m: int, n: int, k: int, sms: int = 148) -> int:
     """Split-K factor minimizing a wave model of the weight-streaming GEMM.
 
@@ -85,6 +87,7 @@ _MEASURED_SPLITS = {(48, 32): 4}
 PAIR_MIN_ROWS = 65  # batches at least this wide may take the two-SM GEMM (``csrc/fp8_gemm_2cta.cu``)
 
 
+@lru_cache(maxsize=4096)
 def split_blocks(m: int, n: int, k: int) -> int:
     """K blocks per split that the one-SM kernel would sum on their own for this shape, 0 if it would not split.  The two-SM kernel
     forms its sums alike, so the bits of a product do not depend on which of the two a shape takes."""
@@ -115,6 +118,11 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
         return 0
     if forced not in (None, ""):
         return int(forced) if int(forced) in (128, 256) else 0
+    return _pair_tile_by_cost(m, n, k, sms)
+
+
+@lru_cache(maxsize=4096)
+def _pair_tile_by_cost(m: int, n: int, k: int, sms: int) -> int:
     pairs, blocks = sms // 2, k // 128
     tiles = {t: n // 256 * math.ceil(m / t) for t in (128, 256)}
     if 2 * tiles[128] <= pairs and blocks > 64:

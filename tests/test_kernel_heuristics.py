@@ -65,3 +65,12 @@ def test_pair_kernel_leaves_split_ranges_of_few_tiles_alone():
         assert K.pair_tile(m, n, k) == 0, (m, n, k)
     for m, n, k in ((357, 4096, 14336), (700, 4096, 4096), (1000, 6144, 4096), (500, 2048, 1024), (100, 6144, 2048), (1000, 2560, 14336)):
         assert K.pair_tile(m, n, k), (m, n, k)  # 39.5 against 83 us, 29 against 50, ...
+
+
+def test_the_choice_for_a_shape_is_worked_out_once():
+    """A prompt asks for the same few shapes in every layer, and the wave models cost about as much host time as a launch."""
+    K.pair_tile(777, 4096, 4096), K.split_blocks(777, 4096, 4096)
+    before = K.pick_splits.cache_info().misses, K.split_blocks.cache_info().misses
+    for _ in range(8):
+        K.pair_tile(777, 4096, 4096), K.split_blocks(777, 4096, 4096), K.pick_splits(777, 4096, 4096)
+    assert (K.pick_splits.cache_info().misses, K.split_blocks.cache_info().misses) == before
