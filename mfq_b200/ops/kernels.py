@@ -13,6 +13,7 @@ from .lib import Workspace, check, lib, ptr, stream_ptr
 
 FP8 = torch.float8_e4m3fn
 
+SPLIT_SCRATCH_BYTES = 64 << 20  # the workspace's split-K scratch
 
 GEMV_MAX_ROWS = 8   # up to this many rows the weight-streaming kernel (fp8_gemv.cu) always replaces the tcgen05 GEMM
 GEMV_MID_ROWS = 16  # ... up to this many when the matrix is at most GEMV_MID_WEIGHTS values
@@ -52,8 +53,19 @@ def pick_splits(m: int, n: int, k: int, sms: int = 148) -> int:
     """Split-K factor minimizing a wave model of the weight-streaming GEMM.
 
     cost(s) = waves(s) * (K blocks per CTA + fixed ramp of ~4 blocks) + a small charge for the reduction;
-    it fills the SMs when the (n, token) tile grid alone cannot and avoids a nearly empty last wave.
+    it fills the SMs when the (n, token) tile grid alone cannot and avoids a nearly empty last wave.  Where the partial sums of its
+    choice exceed the scratch (8192 x 640 x 14336: 4 splits, 80 MB) the product is not split.
     """
+    best = _best_splits(m, n, k, sms)
+    if best == 1:
+        return 1
+    per = math.ceil(k // 128 / best)
+    tile = _token_tile(m)
+    partials = math.ceil(k // 128 / per) * math.ceil(n / 128) * math.ceil(m / tile) * tile * 128 * 4
+    return best if partials <= SPLIT_SCRATCH_BYTES else 1
+
+
+def _best_splits(m: int, n: int, k: int, sms: int) -> int:
     tiles = math.ceil(n / 128) * math.ceil(m / _token_tile(m))
     kb = k // 128
     if tiles >= 4 * sms or kb <= 1:
@@ -93,12 +105,7 @@ def split_blocks(m: int, n: int, k: int) -> int:
     forms its sums alike, so the bits of a product do not depend on which of the two a shape takes."""
     blocks = k // 128
     per = math.ceil(blocks / pick_splits(m, n, k))
-    splits = math.ceil(blocks / per)
-    partials = splits * math.ceil(n / 128) * math.ceil(m / 128) * 128 * 128 * 4
-    return per if splits > 1 and partials <= SPLIT_SCRATCH_BYTES else 0  # beyond the scratch it cannot split
-
-
-SPLIT_SCRATCH_BYTES = 64 << 20  # the workspace's split-K scratch
+    return per if math.ceil(blocks / per) > 1 else 0
 
 
 def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:

@@ -59,6 +59,15 @@ def test_fp8_product_of_a_wide_batch_keeps_the_sums_of_the_split_form(m, n, k, m
     assert torch.equal(got, want)
 
 
+def test_fp8_product_whose_partial_sums_exceed_the_scratch():
+    """Rows that are not whole pairs of blocks stay on the one-SM kernel, whose wave model asks for 80 MB of partial sums here."""
+    require_gpu_lib()
+    args = _fp8(1, 8192, 640, 14336)
+    assert K._best_splits(8192, 640, 14336, 148) > 1
+    assert torch.equal(ops.fp8_gemm(*args), ops.fp8_gemm(*args, splits=1, token_tile=128))
+    check_status()
+
+
 @pytest.mark.parametrize("tile", [128, 256])
 @pytest.mark.parametrize("m,n,k", [(1, 16, 8), (129, 272, 72), (257, 512, 4096), (300, 48, 200), (1400, 1040, 64)])
 def test_dense_pair_kernel_on_every_output_stage(m, n, k, tile):

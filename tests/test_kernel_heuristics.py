@@ -74,3 +74,20 @@ def test_the_choice_for_a_shape_is_worked_out_once():
     for _ in range(8):
         K.pair_tile(777, 4096, 4096), K.split_blocks(777, 4096, 4096), K.pick_splits(777, 4096, 4096)
     assert (K.pick_splits.cache_info().misses, K.split_blocks.cache_info().misses) == before
+
+
+def test_splits_fit_the_scratch():
+    """The split-K kernels refuse partial sums beyond the workspace's scratch: no rule may ask for them."""
+    import inspect
+
+    from mfq_b200.ops.lib import Workspace
+    assert inspect.signature(Workspace.__init__).parameters["splitk_bytes"].default == K.SPLIT_SCRATCH_BYTES
+    unsplit = 0
+    for rows in (1, 3, 5, 7, 13, 15, 33, 65, 129, 257, 513):
+        for k in (512, 2048, 4096, 14336, 28672):
+            for m in (1, 64, 65, 129, 700, 1500, 3000, 4096, 8192):
+                s, tile, blocks = K.pick_splits(m, rows * 128, k), K._token_tile(m), k // 128
+                partials = math.ceil(blocks / math.ceil(blocks / s)) * rows * math.ceil(m / tile) * tile * 128 * 4
+                assert s == 1 or partials <= K.SPLIT_SCRATCH_BYTES, (m, rows * 128, k, s)
+                unsplit += s == 1 and K._best_splits(m, rows * 128, k, 148) > 1
+    assert unsplit and K.pick_splits(8192, 640, 14336) == 1
