@@ -313,49 +313,25 @@ __device__ __forceinline__ float rope_inv_freq(float log2_theta, int fi, int rot
   return f;
 }
 
-template <int D>
-__global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
-                                     const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
-                                     uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
-                                     float* __restrict__ k_scale, float* __restrict__ v_scale, int T, int Hq, int Hk,
-                                     int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
-                                     __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
-                                     const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
-                                     const RopeScale ys, int heads_per_warp) {
-  pdl_trigger();
-  pdl_wait();
-  constexpr int EPL = D / 32;  // elements per lane
-  const int warps_per_block = blockDim.x >> 5;
-  const int gw = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const int heads = Hq + 2 * Hk, groups = (heads + heads_per_warp - 1) / heads_per_warp;
-  if (gw >= T * groups) return;
-  const int t = gw / groups, h_first = gw % groups * heads_per_warp;
-  const int slot = h_first + heads_per_warp > Hq ? slots[t] : -1;  // requested with the position, not after the rotation
-  // lane owns EPL/2 rotation pairs: indices j and j + rot/2 for j = lane*EPL/2 .. (only when below rot/2),
-  // plus pass-through of non-rotated dims; simplest uniform scheme: lane handles dims
-  // [lane*EPL/2, lane*EPL/2 + EPL/2) of each half of the head vector.
-  constexpr int HP = EPL / 2;
-  float lo[HP], hi[HP];
-  // explicit vector loads: with a run-time row stride the compiler can no longer prove the alignment itself
-  // (the host entry checks that the stride is a multiple of 8 elements)
-  auto load_half = [&](const __nv_bfloat16* ptr, float (&dst)[HP]) {
-    if constexpr (HP == 2) {
-      const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(ptr);
-      dst[0] = __bfloat162float(v.x);
-      dst[1] = __bfloat162float(v.y);
-    } else if constexpr (HP == 4) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(ptr);
-      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) dst[j] = __bfloat162float(e[j]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < HP; ++j) dst[j] = __bfloat162float(ptr[j]);
-    }
-  };
+// Where a head's rows go.
+struct RopeOut {
+  __nv_bfloat16* q;  // [T, Hq, D]
+  uint8_t *k_cache, *v_cache;
+  float *k_scale, *v_scale;
+  __nv_bfloat16 *kd, *vd;  // [T, Hk, D], optional
+  int Hq, Hk, page_size;
+};
+
+// One head of a token by a warp: `lo`, `hi` are the lane's D / 64 values of either half of `src`.  `angle(j, s, c)`: sine and cosine of
+// the lane's j-th pair (full rotary).  kWide: what a lane writes to q, kd and vd goes out in one store.
+template <int D, bool kWide, typename Angle, typename Slot>
+__device__ __forceinline__ void rope_head(const __nv_bfloat16* __restrict__ src, float (&lo)[D / 64], float (&hi)[D / 64], int t, int h,
+                                          int lane, const int* __restrict__ positions, int rot, float log2_theta, const RopeScale& ys,
+                                          const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float norm_eps,
+                                          const RopeOut& to, const Angle& angle, const Slot& slot_of) {
+  constexpr int HP = D / 64;
   auto store_half = [&](__nv_bfloat16* ptr, const float (&v)[HP]) {
-    if constexpr (HP % 2 == 0) {
+    if constexpr (kWide && HP % 2 == 0) {
       uint32_t packed[HP / 2];
 #pragma unroll
       for (int j = 0; j < HP / 2; ++j) {
@@ -369,27 +345,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
       for (int j = 0; j < HP; ++j) ptr[j] = __float2bfloat16(v[j]);
     }
   };
-  // The first head is requested before the angles: their evaluation hides its way from memory (40 tokens of 48 heads: 3.9 -> 3.5 us).
-  const __nv_bfloat16* row = qkv + size_t(t) * row_stride;  // rows may carry extra trailing columns
-  load_half(row + size_t(h_first) * D + lane * HP, lo);
-  load_half(row + size_t(h_first) * D + D / 2 + lane * HP, hi);
-  // The angles of a token are the same for all its heads: a warp that takes several evaluates them once.
-  float cs[EPL / 2], sn[EPL / 2];
-  if (rot == D && h_first < Hq + Hk) {  // values are not rotated
-    const float pos = float(positions[t]);
-#pragma unroll
-    for (int j = 0; j < EPL / 2; ++j) {
-      sincosf(pos * rope_inv_freq(log2_theta, lane * (EPL / 2) + j, rot, ys), &sn[j], &cs[j]);
-      sn[j] *= ys.mscale;
-      cs[j] *= ys.mscale;
-    }
-  }
-  for (int h = h_first; h < min(h_first + heads_per_warp, heads); ++h) {
-  const __nv_bfloat16* src = row + size_t(h) * D;
-  if (h != h_first) {
-    load_half(src + lane * HP, lo);
-    load_half(src + D / 2 + lane * HP, hi);
-  }
+  const int Hq = to.Hq, Hk = to.Hk, page_size = to.page_size;
   const bool is_v = h >= Hq + Hk;
   // optional per-head RMSNorm of q and k before the rotation (QK-norm); nw_scale folds 1/rms into the partner reads
   const float* nw = is_v ? nullptr : (h < Hq ? q_norm_w : k_norm_w);
@@ -412,13 +368,16 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
     if (rot == D) {
 #pragma unroll
       for (int j = 0; j < HP; ++j) {
+        float s, c;
+        angle(j, s, c);
         const float a = lo[j], b = hi[j];
-        lo[j] = __fmaf_rn(a, cs[j], -__fmul_rn(b, sn[j]));
-        hi[j] = __fmaf_rn(b, cs[j], __fmul_rn(a, sn[j]));
+        lo[j] = __fmaf_rn(a, c, -__fmul_rn(b, s));
+        hi[j] = __fmaf_rn(b, c, __fmul_rn(a, s));
       }
     } else {
       // partial rotary: pairs (i, i + rot/2) live inside the first `rot` dims.  Handle through shared
       // exchange-free recomputation: each lane re-reads its partner element.
+      const float pos = float(positions[t]);
 #pragma unroll
       for (int j = 0; j < HP; ++j) {
         for (int part = 0; part < 2; ++part) {
@@ -427,7 +386,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
             const int fi = idx % half_rot;
             const float inv_freq = rope_inv_freq(log2_theta, fi, rot, ys);
             float s, c;
-            sincosf(float(positions[t]) * inv_freq, &s, &c);
+            sincosf(pos * inv_freq, &s, &c);
             s *= ys.mscale;
             c *= ys.mscale;
             const float self = part ? hi[j] : lo[j];
@@ -441,12 +400,13 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
     }
   }
   if (h < Hq) {
-    __nv_bfloat16* dst = q_out + size_t(t) * Hq * D + size_t(h) * D;
+    __nv_bfloat16* dst = to.q + size_t(t) * Hq * D + size_t(h) * D;
     store_half(dst + lane * HP, lo);
     store_half(dst + D / 2 + lane * HP, hi);
-    continue;
+    return;
   }
-  if (slot < 0) continue;
+  const int slot = slot_of();
+  if (slot < 0) return;
   const int kvh = is_v ? h - Hq - Hk : h - Hq;
   const int page = slot / page_size, off = slot % page_size;
   float amax = 0.f;
@@ -463,7 +423,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
   const size_t ph = size_t(page) * Hk + kvh;
   if (!is_v) {
     // K page: [D/64 chunks][page_size tokens][64 dims]
-    uint8_t* dst = k_cache + ph * (size_t(page_size) * D);
+    uint8_t* dst = to.k_cache + ph * (size_t(page_size) * D);
 #pragma unroll
     for (int j = 0; j < HP; ++j) {
       const int d0 = lane * HP + j, d1 = D / 2 + lane * HP + j;
@@ -472,7 +432,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
     }
   } else {
     // V page: [D dims][page_size tokens in the order 0,1,8,9,2,3,10,11,4,5,12,13,6,7,14,15]
-    uint8_t* dst = v_cache + ph * (size_t(page_size) * D);
+    uint8_t* dst = to.v_cache + ph * (size_t(page_size) * D);
     const int pos = 4 * ((off & 7) >> 1) + 2 * (off >> 3) + (off & 1);
 #pragma unroll
     for (int j = 0; j < HP; ++j) {
@@ -482,7 +442,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
   }
   // Optional contiguous copy of what the pages now hold (code * multiplier), [T, Hk, D] bf16: the prefill attention
   // of this chunk reads it, so prefill and later decode steps see the same FP8-rounded K/V.
-  __nv_bfloat16* dq = is_v ? vd_out : kd_out;
+  __nv_bfloat16* dq = is_v ? to.vd : to.kd;
   if (dq) {
     dq += (size_t(t) * Hk + kvh) * D;
 #pragma unroll
@@ -493,8 +453,106 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
     store_half(dq + lane * HP, lo);
     store_half(dq + D / 2 + lane * HP, hi);
   }
-  if (lane == 0) (is_v ? v_scale : k_scale)[base] = scale;
+  if (lane == 0) (is_v ? to.v_scale : to.k_scale)[base] = scale;
+}
+
+// kHeads: heads of a token that a warp takes.  Several (full rotary only): their angles are evaluated once.
+template <int D, int kHeads>
+__device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+                                          const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
+                                          uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
+                                          float* __restrict__ k_scale, float* __restrict__ v_scale, int T, int Hq, int Hk,
+                                          int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
+                                          __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
+                                          const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
+                                          const RopeScale ys) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int EPL = D / 32;  // elements per lane
+  const int warps_per_block = blockDim.x >> 5;
+  const int gw = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const int heads = Hq + 2 * Hk, groups = (heads + kHeads - 1) / kHeads;
+  if (gw >= T * groups) return;
+  const int t = gw / groups, h_first = gw % groups * kHeads;
+  const __nv_bfloat16* src = qkv + size_t(t) * row_stride + size_t(h_first) * D;  // rows may carry extra trailing columns
+  // lane owns EPL/2 rotation pairs: indices j and j + rot/2 for j = lane*EPL/2 .. (only when below rot/2),
+  // plus pass-through of non-rotated dims; simplest uniform scheme: lane handles dims
+  // [lane*EPL/2, lane*EPL/2 + EPL/2) of each half of the head vector.
+  constexpr int HP = EPL / 2;
+  float lo[HP], hi[HP];
+  // explicit vector loads: with a run-time row stride the compiler can no longer prove the alignment itself
+  // (the host entry checks that the stride is a multiple of 8 elements)
+  auto load_half = [&](const __nv_bfloat16* ptr, float (&dst)[HP]) {
+    if constexpr (HP == 2) {
+      const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(ptr);
+      dst[0] = __bfloat162float(v.x);
+      dst[1] = __bfloat162float(v.y);
+    } else if constexpr (HP == 4) {
+      const uint2 raw = *reinterpret_cast<const uint2*>(ptr);
+      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[j] = __bfloat162float(e[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < HP; ++j) dst[j] = __bfloat162float(ptr[j]);
+    }
+  };
+  load_half(src + lane * HP, lo);
+  load_half(src + D / 2 + lane * HP, hi);
+  const RopeOut to{q_out, k_cache, v_cache, k_scale, v_scale, kd_out, vd_out, Hq, Hk, page_size};
+  auto evaluate = [&](int j, float& s, float& c) {
+    sincosf(float(positions[t]) * rope_inv_freq(log2_theta, lane * HP + j, rot, ys), &s, &c);
+    s *= ys.mscale;
+    c *= ys.mscale;
+  };
+  if constexpr (kHeads == 1) {
+    rope_head<D, false>(src, lo, hi, t, h_first, lane, positions, rot, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to, evaluate,
+                        [&] { return slots[t]; });
+  } else {
+    const int slot = h_first + kHeads > Hq ? slots[t] : -1;  // requested with the position, not after the rotation
+    float cs[HP], sn[HP];
+    if (h_first < Hq + Hk) {  // values are not rotated; the first head is on its way from memory
+#pragma unroll
+      for (int j = 0; j < HP; ++j) evaluate(j, sn[j], cs[j]);
+    }
+    const int h_end = min(h_first + kHeads, heads);
+    for (int h = h_first; h < h_end; ++h, src += D) {
+      if (h != h_first) {
+        load_half(src + lane * HP, lo);
+        load_half(src + D / 2 + lane * HP, hi);
+      }
+      rope_head<D, true>(src, lo, hi, t, h, lane, positions, D, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to,
+                         [&](int j, float& s, float& c) { s = sn[j]; c = cs[j]; }, [&] { return slot; });
+    }
   }
+}
+
+template <int D>
+__global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+                                     const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
+                                     uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
+                                     float* __restrict__ k_scale, float* __restrict__ v_scale, int T, int Hq, int Hk,
+                                     int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
+                                     __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
+                                     const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
+                                     const RopeScale ys) {
+  rope_rows<D, 1>(qkv, positions, slots, q_out, k_cache, v_cache, k_scale, v_scale, T, Hq, Hk, page_size, rot, log2_theta, kd_out, vd_out, q_norm_w, k_norm_w,
+                  norm_eps, row_stride, ys);
+}
+
+constexpr int kRopeHeads = 8;
+template <int D>
+__global__ void __launch_bounds__(256, D <= 128 ? 6 : 4) rope_kv_write_heads_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+                                     const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
+                                     uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
+                                     float* __restrict__ k_scale, float* __restrict__ v_scale, int T, int Hq, int Hk,
+                                     int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
+                                     __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
+                                     const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
+                                     const RopeScale ys) {
+  rope_rows<D, kRopeHeads>(qkv, positions, slots, q_out, k_cache, v_cache, k_scale, v_scale, T, Hq, Hk, page_size, rot, log2_theta, kd_out, vd_out, q_norm_w, k_norm_w,
+                       norm_eps, row_stride, ys);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -683,19 +741,21 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
                                       cudaStream_t stream) {
   if (T <= 0 || row_stride < (Hq + 2 * Hk) * D || row_stride % 8) return -1;
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
-  // Enough tokens to fill the GPU with a warp for several heads each: the angles (sine, cosine and the frequency's power) are a good
-  // part of the work of a head.  4096 tokens of 48 heads on a B200: 71 us with one head per warp, 64 with eight (the pages' single-byte
-  // stores take most of that); 357 tokens: 11.7 and 10.4; 200: 7.3 and 9.7.
-  const int heads = Hq + 2 * Hk, per = long(T) * heads >= 8L * 148 * 14 ? 8 : 1;
-  const long warps = long(T) * ((heads + per - 1) / per);
-  const int blocks = int((warps + 7) / 8);
+  // A warp per head, or one per kRopeHeads heads of a token, whose angles (sine, cosine and the frequency's power, a good part of a head's
+  // work) it evaluates once.  That needs full rotary, enough heads that the fewer and longer warps still fill the GPU, and groups that are
+  // three quarters full.  On a B200, a warp per head | eight heads:  48 heads of 128, 500 tokens 10.3 | 11.4 us, 700 13.4 | 14.5, 800
+  // 15.1 | 14.7, 1000 18.7 | 14.9, 4096 68.5 | 47.0;  36 heads of 64, 800 tokens 6.4 | 6.8, 1000 7.6 | 6.9;  20 of 256, 2000 21.5 | 20.4;
+  // 10 of 128 (two groups), 4096 13.1 | 14.2.
+  const int heads = Hq + 2 * Hk, full_groups = (heads + kRopeHeads - 1) / kRopeHeads;
+  const bool shared = rot == D && long(T) * heads >= 36000 && 4 * heads >= 3 * kRopeHeads * full_groups;
+  const int blocks = int((long(T) * (shared ? full_groups : heads) + 7) / 8);
   const float l2t = log2f(theta);
   const RopeScale ys{yarn_factor, yarn_low, yarn_high, yarn_mscale};
 #define MFQ_ROPE(DD)                                                                                             \
-  launch_kernel(rope_kv_write_kernel<DD>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkv), positions, slots, \
+  launch_kernel(shared ? rope_kv_write_heads_kernel<DD> : rope_kv_write_kernel<DD>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkv), positions, slots, \
       static_cast<__nv_bfloat16*>(q_out), static_cast<uint8_t*>(k_cache), static_cast<uint8_t*>(v_cache),      \
       k_scale, v_scale, T, Hq, Hk, page_size, rot, l2t, static_cast<__nv_bfloat16*>(kd_out),                   \
-      static_cast<__nv_bfloat16*>(vd_out), q_norm_w, k_norm_w, norm_eps, row_stride, ys, per)
+      static_cast<__nv_bfloat16*>(vd_out), q_norm_w, k_norm_w, norm_eps, row_stride, ys)
   if (D == 128) MFQ_ROPE(128);
   else if (D == 64) MFQ_ROPE(64);
   else if (D == 256) MFQ_ROPE(256);

@@ -124,7 +124,7 @@ def test_rotation_of_many_tokens_gives_the_bits_of_few(d, rot):
     """Enough tokens that a warp takes several heads, with a count of heads that does not divide: the same pages and queries as from
     calls that are too small for that."""
     require_gpu_lib()
-    t, hq, hk = 5003, 7, 2
+    t, hq, hk = 5003, 11, 2
     rows = _normal(d, t, (hq + 2 * hk) * d)
     pos = torch.randint(0, 9000, (t,), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda", dtype=torch.int32)
     got = []
