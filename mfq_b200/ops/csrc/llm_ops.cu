@@ -743,11 +743,12 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
   // A warp per head, or one per kRopeHeads heads of a token, whose angles (sine, cosine and the frequency's power, a good part of a head's
   // work) it evaluates once.  That needs full rotary, enough heads that the fewer and longer warps still fill the GPU, and groups that are
-  // three quarters full.  On a B200, a warp per head | eight heads:  48 heads of 128, 500 tokens 10.3 | 11.4 us, 700 13.4 | 14.5, 800
+  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  On a B200, a warp per head | eight heads:  48 heads of 128, 500 tokens 10.3 | 11.4 us, 700 13.4 | 14.5, 800
   // 15.1 | 14.7, 1000 18.7 | 14.9, 4096 68.5 | 47.0;  36 heads of 64, 800 tokens 6.4 | 6.8, 1000 7.6 | 6.9;  20 of 256, 2000 21.5 | 20.4;
   // 10 of 128 (two groups), 4096 13.1 | 14.2.
   const int heads = Hq + 2 * Hk, full_groups = (heads + kRopeHeads - 1) / kRopeHeads;
-  const bool shared = rot == D && long(T) * heads >= 36000 && 4 * heads >= 3 * kRopeHeads * full_groups;
+  const bool aligned = (reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kd_out) | reinterpret_cast<uintptr_t>(vd_out)) % 8 == 0;
+  const bool shared = rot == D && long(T) * heads >= 36000 && 4 * heads >= 3 * kRopeHeads * full_groups && aligned;
   const int blocks = int((long(T) * (shared ? full_groups : heads) + 7) / 8);
   const float l2t = log2f(theta);
   const RopeScale ys{yarn_factor, yarn_low, yarn_high, yarn_mscale};

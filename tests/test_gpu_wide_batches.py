@@ -141,6 +141,25 @@ def test_rotation_of_many_tokens_gives_the_bits_of_few(d, rot):
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("d", [128, 256])
+def test_rotation_into_rows_off_a_vector(d):
+    """Outputs that begin 2 bytes past a vector, as views of a larger buffer may: the same values as in aligned ones."""
+    require_gpu_lib()
+    t, hq, hk = 3003, 12, 2
+    rows, pos = _normal(d, t, (hq + 2 * hk) * d), torch.arange(t, device="cuda", dtype=torch.int32)
+    got = []
+    for shift in (0, 1):
+        cache = PagedKVCache(layers=1, kv_heads=hk, head_dim=d, num_pages=t // 16 + 2, max_seqs=1, max_pages_per_seq=t // 16 + 1, device="cuda")
+        cache.assign(0, 0, t)
+        q, kd, vd = (torch.zeros(t * h * d + 8, device="cuda", dtype=torch.bfloat16)[shift : shift + t * h * d].view(t, h, d) for h in (hq, hk, hk))
+        assert q.data_ptr() % 8 == 2 * shift
+        ops.rope_kv_write(rows, pos, cache.slots(0, 0, t).to("cuda"), cache.layer(0), n_q=hq, n_kv=hk, head_dim=d, theta=1e4, q_out=q, kd_out=kd,
+                          vd_out=vd)
+        got.append([q, kd, vd, cache.k.view(torch.uint8)])
+    check_status()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("t,e", [(65, 16), (200, 512), (700, 48)])
 def test_router_logits_of_a_prompt(t, e):
     require_gpu_lib()
