@@ -183,17 +183,31 @@ __global__ void __launch_bounds__(512) quant_rows_kernel(const __nv_bfloat16* __
   float amax = 0.f;
   if (nvec <= kRowVecs * int(blockDim.x)) {
     uint4 held[kRowVecs];
+    if (kMode == 0 && nvec == kRowVecs * int(blockDim.x)) {
+      // Nothing but the row, and as many vectors as a thread can hold: bound by its loads in flight, so all of a thread's are requested
+      // before the first is used.  4000 rows of 16384: 44.5 us with each load under its condition, 37.5 in two passes of four loads, 30.9 so;
+      // of 4096: 7.9, 20.0, 7.0.
 #pragma unroll
-    for (int i = 0; i < kRowVecs; ++i) {
-      const int vi = threadIdx.x + i * blockDim.x;
-      if (vi < nvec) {
-        float y[8];
-        value(vi, y);
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&held[i]);
+      for (int i = 0; i < kRowVecs; ++i) held[i] = *reinterpret_cast<const uint4*>(xr + (threadIdx.x + i * blockDim.x) * 8);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(y[j]));
+      for (int i = 0; i < kRowVecs; ++i) {
+        const uint32_t w[4] = {held[i].x, held[i].y, held[i].z, held[i].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
+        for (int j = 0; j < 4; ++j) amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[j] << 16)), fabsf(__uint_as_float(w[j] & 0xffff0000u))));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kRowVecs; ++i) {
+        const int vi = threadIdx.x + i * blockDim.x;
+        if (vi < nvec) {
+          float y[8];
+          value(vi, y);
+          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&held[i]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(y[j]));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
+        }
       }
     }
     amax = block_reduce<true>(amax, red);
