@@ -96,7 +96,7 @@ def test_rope_kv_write_and_decode_attention(hq, hk, d):
     q = torch.randn((b, hq, d), device="cuda").to(torch.bfloat16)
     seq_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
     want = ref.paged_attn_decode(q, kv, cache.block_table, seq_lens, 1 / math.sqrt(d))
-    for splits in (1, 3, 8, 40):
+    for splits in (1, 3, 8, 9, 40):
         got = ops.paged_attn_decode(q, kv, cache.block_table, seq_lens, sm_scale=1 / math.sqrt(d), splits=splits)
         assert_close(got, want, rel=2e-2, what=f"decode attention splits={splits}")
 
