@@ -68,3 +68,24 @@ def test_moe_ffn_matches_reference(t, e, k, e_lo, e_hi):
     # the SwiGLU output is re-quantized to E4M3 between the two GEMMs: a bf16 ulp of difference there flips a code now
     # and then, which moves single outputs by more than the element-wise bound
     assert_close(got, want, rel=2e-2, what="moe ffn", outliers=5e-3)
+
+
+@pytest.mark.parametrize("t,k,e,lo,hi", [(12288, 1, 512, 0, 512), (12289, 1, 64, 16, 48), (2500, 10, 512, 0, 512), (5000, 6, 64, 0, 1)])
+def test_route_plan_of_many_routes(t, k, e, lo, hi):
+    """Around the line from which a thread reads eight routes at a time, and several such rounds; routes to nobody and to other ranks."""
+    require_gpu_lib()
+    ids = torch.randint(-1, e, (t, k), generator=torch.Generator(device="cuda").manual_seed(t), device="cuda", dtype=torch.int32)
+    plan = moe.plan_routes(ids, lo, hi, token_tile=32)
+    flat, dest = ids.flatten().long().cpu(), plan.dest.flatten().long().cpu()
+    mine = (flat >= lo) & (flat < hi)
+    counts = torch.bincount(flat[mine] - lo, minlength=hi - lo)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    assert torch.equal(plan.offsets.long().cpu(), offsets) and bool((dest[~mine] == -1).all())
+    assert torch.equal(dest[mine].sort().values, torch.arange(int(mine.sum())))  # every row once ...
+    at, expert = dest[mine], flat[mine] - lo
+    assert bool(((at >= offsets[expert]) & (at < offsets[expert + 1])).all())  # ... among its expert's
+    assert torch.equal(plan.src_token.long().cpu()[at], (torch.arange(t * k) // k)[mine])
+    want = [(x, i) for x in range(hi - lo) for i in range(-(-int(counts[x]) // 32))]
+    tiles = [tuple(r) for r in plan.tile_map.tolist()]
+    assert tiles[: len(want)] == want and all(r[0] < 0 for r in tiles[len(want):])
+    assert plan.totals.tolist() == [int(offsets[-1]), len(want)]
