@@ -114,6 +114,11 @@ def dense_lib() -> C.CDLL:
     return _open(DENSE_LIB_PATH, _DENSE_SIGNATURES)
 
 
+def dense_available() -> bool:
+    """Whether the library of the unquantized path is there: what the FP8 path borrows from it has a kernel of its own to fall back on."""
+    return DENSE_LIB_PATH.exists()
+
+
 def available() -> bool:
     return LIB_PATH.exists() and torch.cuda.is_available()
 

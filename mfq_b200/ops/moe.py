@@ -16,7 +16,7 @@ import torch
 
 from . import kernels as K
 from .dense import DenseLinear
-from .lib import Workspace, check, lib, ptr, stream_ptr
+from .lib import Workspace, check, dense_available, lib, ptr, stream_ptr
 
 _vp, _i, _f = C.c_void_p, C.c_int, C.c_float
 _SIGS = {
@@ -65,7 +65,7 @@ def router_topk(x: torch.Tensor, w: torch.Tensor, k: int, *, bias: torch.Tensor 
     wt = torch.empty((t, k), dtype=torch.float32, device=x.device)
     scores = torch.empty((t, e), dtype=torch.float32, device=x.device) if want_scores else None
     if t > ROUTER_MMA_ROWS and e % 16 == 0 and h % 32 == 0 and x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == 1 and x.stride(0) % 8 == 0 \
-            and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+            and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and dense_available():
         # a prompt's logits are an ordinary product: 3000 x 2048 x 512 takes 137 us in the router's own mma.sync kernel, 12 on tcgen05
         logits = DenseLinear(w)(x, fp32=True)
         rc = _lib().mfq_moe_router_select(ptr(logits), ptr(bias), ptr(ids), ptr(wt), ptr(scores), t, h, e, k, int(sigmoid), int(norm_topk),

@@ -89,3 +89,23 @@ def test_route_plan_of_many_routes(t, k, e, lo, hi):
     tiles = [tuple(r) for r in plan.tile_map.tolist()]
     assert tiles[: len(want)] == want and all(r[0] < 0 for r in tiles[len(want):])
     assert plan.totals.tolist() == [int(offsets[-1]), len(want)]
+
+
+@pytest.mark.parametrize("sig,ng,tg,norm,scale", [(False, 1, 1, True, 1.0), (True, 1, 1, True, 2.5), (True, 8, 4, True, 2.5), (False, 1, 1, False, 1.0)])
+def test_router_of_a_prompt_chooses_what_the_routers_own_kernels_do(sig, ng, tg, norm, scale, monkeypatch):
+    """Beyond 64 tokens logits come from the dense product -- or, where its library is not there, from the router's own kernels."""
+    require_gpu_lib()
+    g = torch.Generator(device="cuda").manual_seed(ng)
+    x, w = torch.randn((201, 1024), generator=g, device="cuda").to(torch.bfloat16), (torch.randn((256, 1024), generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    bias = torch.randn(256, generator=g, device="cuda") * 0.1 if sig else None
+    how = dict(bias=bias, sigmoid=sig, n_group=ng, topk_group=tg, norm_topk=norm, scale=scale, want_scores=True)
+    got = moe.router_topk(x, w, 8, **how)
+    monkeypatch.setattr(moe, "dense_available", lambda: False)
+    monkeypatch.setattr(moe, "DenseLinear", None)
+    want = moe.router_topk(x, w, 8, **how)
+    # fp32 sums of 1024 products in another order before an exponential: their absolute error, on either side
+    slack = float((x.abs().float() @ w.abs().float().T).amax()) * 1032 * 2.0 ** -23
+    assert bool(((got[2] - want[2]).abs() <= slack * want[2]).all())
+    same = (got[0].sort(1).values == want[0].sort(1).values).all(1)
+    assert same.float().mean() > 0.98  # near ties may fall either way
+    assert bool(((got[1][same].sort(1).values - want[1][same].sort(1).values).abs() <= 2 * slack * scale).all())
