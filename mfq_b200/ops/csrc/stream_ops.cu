@@ -374,10 +374,13 @@ extern "C" int mfq_norm_add(const void* y, const float* w, float* x, void* xa, i
   const auto launch = [&](auto kernel, auto* rows, auto* copy) {
     launch_kernel(kernel, dim3(M), dim3(threads), 0, stream, rows, w, x, copy, W, 1.f / float(width), eps);
   };
-  // More rows than SMs: several share one.  1508 rows of 4096 on a B200: 17.5 -> 13.5 us.  A few rows are as fast either way on their own
-  // (16: 3.2 us), and a decode step of 16 was 0.5 % slower with the weights asked for ahead of the product it waits for.
-  if (M > 148 && W / 8 <= threads) MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, 1>, static_cast<const T*>(y), static_cast<T*>(xa)));
-  else if (M > 148 && W / 8 <= 2 * threads) MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, 2>, static_cast<const T*>(y), static_cast<T*>(xa)));
+  // Fewer registers: more rows on an SM.  That pays once the rows no longer fit the general form's first wave or two: on a B200, general |
+  // 1 or 2 vectors, 1500 rows of 4096 17.6 | 14.2 us, 500 7.1 | 5.6, 296 3.4 | 3.7, 200 3.3 | 4.4;  of 2048: 1000 7.7 | 5.1, 600 4.5 | 4.4,
+  // 500 3.6 | 4.2, 260 2.3 | 2.8;  of 1024: 1500 5.0 | 4.6, 1000 3.6 | 3.9;  of 512: 149 1.83 | 1.54.  Up to 148 rows a decode step of
+  // 16 was 0.5 % slower with the weights asked for ahead of the product it waits for.
+  const bool many = M > (W <= 512 ? 148 : W <= 1024 ? 1036 : W <= 2048 ? 592 : 296);
+  if (many && W / 8 <= threads) MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, 1>, static_cast<const T*>(y), static_cast<T*>(xa)));
+  else if (many && W / 8 <= 2 * threads) MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, 2>, static_cast<const T*>(y), static_cast<T*>(xa)));
   else MFQ_BY_TYPE(fp32, launch(norm_add_kernel<T, kStreamVecs>, static_cast<const T*>(y), static_cast<T*>(xa)));
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }

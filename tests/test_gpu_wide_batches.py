@@ -228,10 +228,10 @@ def test_heads_rotated_by_vectors_agree_with_the_general_form(d, rot, v_rot, dty
         assert ((got - want).abs() <= (2.0 ** -21 + ulp) * want.abs().amax(-1, keepdim=True)).all()
 
 
-@pytest.mark.parametrize("m", [148, 149])
-@pytest.mark.parametrize("w", [8, 2048, 2056, 4096, 4104])
+@pytest.mark.parametrize("m", [148, 149, 296, 297, 592, 593, 1036, 1037])
+@pytest.mark.parametrize("w", [8, 512, 520, 1024, 1032, 2048, 2056, 4096, 4104])
 def test_stream_rows_by_vectors_per_thread(m, w):
-    """Widths around one and two vectors per thread, rows around the line of the rule."""
+    """Widths around one and two vectors per thread, rows around the lines of the rule."""
     require_gpu_lib()
     y, f, x = _normal(m, m, w), _normal(1, w, dtype=torch.float32), _normal(2, m, w, dtype=torch.float32)
     want, act = x.double() + y.double() * torch.rsqrt(y.double().square().mean(1, keepdim=True) + 1e-5) * f.double(), torch.empty_like(y)
