@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from mfq_b200.ops import moe
+from mfq_b200.ops import fp8_gemm, moe
 from mfq_b200.ops import reference as ref
 from mfq_b200.quantize.fp8_block import quantize_fp8_block_torch
 from gpu_common import assert_close, check_status, require_gpu_lib
@@ -109,3 +109,29 @@ def test_router_of_a_prompt_chooses_what_the_routers_own_kernels_do(sig, ng, tg,
     same = (got[0].sort(1).values == want[0].sort(1).values).all(1)
     assert same.float().mean() > 0.98  # near ties may fall either way
     assert bool(((got[1][same].sort(1).values - want[1][same].sort(1).values).abs() <= 2 * slack * scale).all())
+
+
+@pytest.mark.parametrize("k", [128, 640, 4224])
+@pytest.mark.parametrize("tile", [16, 32, 64, 128])
+def test_grouped_product_over_several_tiles_per_cta(tile, k):
+    """Empty experts, single rows, whole and ragged tiles; one, a few and more than 32 K blocks per tile: the bits of the product of each
+    expert by itself."""
+    require_gpu_lib()
+    counts = [0, 1, 3 * tile + 5, tile, tile + 1, 0, 2 * tile - 1, 7] * 5 + [0]
+    e, n, rows = len(counts), 1024, sum(counts)
+    g = torch.Generator(device="cuda").manual_seed(k + tile)
+    fp8 = lambda *s: (torch.randn(s, generator=g, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
+    x, w = fp8(rows, k), fp8(e, n, k)
+    xs, ws = torch.rand(rows, generator=g, device="cuda") + 0.1, torch.rand((e, n // 128, k // 128), generator=g, device="cuda") + 0.1
+    ids = torch.repeat_interleave(torch.arange(e), torch.tensor(counts))[torch.randperm(rows, generator=torch.Generator().manual_seed(1))]
+    plan = moe.plan_routes(ids.int()[:, None].cuda(), 0, e, token_tile=tile)
+    assert int(plan.totals[1]) * (n // 128) > 3 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert not moe.grouped_gemv_ok(plan, n)
+    got = moe.fp8_gemm_grouped(x, xs, w, ws, plan)
+    check_status()
+    at = 0
+    for i, c in enumerate(counts):
+        if c:
+            rng = slice(at, at + c)
+            assert torch.equal(got[rng], fp8_gemm(x[rng], xs[rng], w[i], ws[i], splits=1, token_tile=tile)), (i, c)
+        at += c

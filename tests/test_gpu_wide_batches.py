@@ -28,11 +28,15 @@ def _fp8(seed, m, n, k):
     return xq, torch.rand(m, generator=g, device="cuda") + 0.1, wq, torch.rand((math.ceil(n / 128), k // 128), generator=g, device="cuda") + 0.1
 
 
-@pytest.mark.parametrize("m,n,k", [(65, 256, 128), (129, 512, 640), (257, 256, 2048), (400, 4096, 256), (1300, 256, 1152), (130, 256, 33 * 1024)])
+@pytest.mark.parametrize("m,n,k", [(65, 256, 128), (129, 512, 640), (257, 256, 2048), (400, 4096, 256), (1300, 256, 1152), (130, 256, 33 * 1024),
+                                   (2100, 4608, 640)])
 def test_fp8_pair_kernel_gives_the_bits_of_the_one_sm_kernel(m, n, k):
     """Both fold K block after K block into fp32 registers and round the same way, residual included; 33 * 1024 is a K range whose
-    multipliers do not fit the shared-memory copy."""
+    multipliers do not fit the shared-memory copy; in the last shape a pair walks several tiles of either width, of five K blocks each
+    (a number that the stages and the accumulators do not divide), the last ones ragged."""
     require_gpu_lib()
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert m != 2100 or math.ceil(m / 256) * (n // 256) > 2 * pairs
     args = _fp8(m + k, m, n, k)
     res = _normal(m, m, n)
     want = ops.fp8_gemm(*args, residual=res, splits=1, token_tile=128)
@@ -69,10 +73,13 @@ def test_fp8_product_whose_partial_sums_exceed_the_scratch():
 
 
 @pytest.mark.parametrize("tile", [128, 256])
-@pytest.mark.parametrize("m,n,k", [(1, 16, 8), (129, 272, 72), (257, 512, 4096), (300, 48, 200), (1400, 1040, 64)])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 8), (129, 272, 72), (257, 512, 4096), (300, 48, 200), (1400, 1040, 64), (4100, 2832, 72)])
 def test_dense_pair_kernel_on_every_output_stage(m, n, k, tile):
-    """Ragged rows, tokens and K against 64 bits; more tiles than pairs in the last shape, so that accumulators are used again."""
+    """Ragged rows, tokens and K against 64 bits; in the last shape a pair walks more tiles than it has accumulators, so that they are
+    handed back and used again."""
     require_gpu_lib()
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert m != 4100 or math.ceil(m / tile) * math.ceil(n / 256) > 512 // tile * pairs
     w, x, bias = _normal(n, n, k, std=k ** -0.5), _normal(m, m, k), _normal(k, n, dtype=torch.float32)
     table, ids = _normal(3, 50, n), torch.arange(m, device="cuda", dtype=torch.int32) % 50
     y = x.double() @ w.double().T
