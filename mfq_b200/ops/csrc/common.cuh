@@ -176,16 +176,7 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {  // one thread; arriv
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, fp8/fp6/fp4 element kinds, fp32 accumulate.  One thread issues.
-__device__ __forceinline__ void umma_f8f6f4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Same for f16/bf16 inputs.
+// D[tmem] (+)= A[smem] * B[smem]^T, f16/bf16 inputs, fp32 accumulate.  One thread issues.
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
@@ -195,8 +186,8 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
       : "memory");
 }
 
-// One 128-byte K block, four k-steps of 32 bytes each into accumulator `d`, then a commit to each of up to two barriers (shared
-// addresses; 0 = none) -- all issued by ONE elected lane of a warp that runs this converged.  A single lane inside
+// fp8/fp6/fp4 element kinds: one 128-byte K block, four k-steps of 32 bytes each into accumulator `d`, then a commit to each of up to
+// two barriers (shared addresses; 0 = none) -- all issued by ONE elected lane of a warp that runs this converged.  A single lane inside
 // `if (lane == 0)` needs 55 cycles per tcgen05 instruction on a B200 (every operand moves to a uniform register first), four
 // MMAs and their commits 320; issued like this they need 160, below the 256 cycles the tensor core works on a 128 x 128 block.
 // `accumulate` applies to the first step.
