@@ -117,7 +117,7 @@ def test_grouped_product_over_several_tiles_per_cta(tile, k):
     """Empty experts, single rows, whole and ragged tiles; one, a few and more than 32 K blocks per tile: the bits of the product of each
     expert by itself."""
     require_gpu_lib()
-    counts = [0, 1, 3 * tile + 5, tile, tile + 1, 0, 2 * tile - 1, 7] * 5 + [0]
+    counts = [0, 1, 3 * tile + 5, tile, tile + 1, 0, 2 * tile - 1, 7] * 6 + [0]
     e, n, rows = len(counts), 1024, sum(counts)
     g = torch.Generator(device="cuda").manual_seed(k + tile)
     fp8 = lambda *s: (torch.randn(s, generator=g, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
