@@ -66,7 +66,8 @@ def bench_gemm(m: int, n: int, k: int, reps: int, splits=None, tile=None) -> dic
     ms = time_ms(lambda i: K.fp8_gemm(x, xs, w[i % copies], ws, out=out, splits=splits, token_tile=tile), reps)
     byt = n * k + m * k + 2 * m * n
     gemv = splits is None and tile is None and K.use_gemv(m, n, k)
-    return {"kernel": "fp8_gemv" if gemv else "fp8_gemm", "m": m, "n": n, "k": k, "us": ms * 1e3, "gbs": byt / ms / 1e6,
+    pair = K.pair_tile(m, n, k) if splits is None and tile is None else 0
+    return {"kernel": "fp8_gemv" if gemv else "fp8_gemm_pair" if pair else "fp8_gemm", "pair": pair, "m": m, "n": n, "k": k, "us": ms * 1e3, "gbs": byt / ms / 1e6,
             "tflops": 2 * m * n * k / ms / 1e9, "splits": splits if splits else K.pick_splits(m, n, k)}
 
 
@@ -80,7 +81,7 @@ def bench_w4_gemm(m: int, n: int, k: int, reps: int, splits=None) -> dict:
     out = torch.empty((m, n), device="cuda", dtype=torch.bfloat16)
     ms = time_ms(lambda i: w4.w4_gemm(x, ws[i % copies], out=out, splits=splits), reps)
     byt = n * k * 5 // 8 + 2 * m * k + 2 * m * n
-    return {"kernel": "w4_gemm", "m": m, "n": n, "k": k, "us": ms * 1e3, "gbs": byt / ms / 1e6, "tflops": 2 * m * n * k / ms / 1e9}
+    return {"kernel": "w4_gemv" if splits is None and m <= w4.GEMV_ROWS else "w4_gemm", "m": m, "n": n, "k": k, "us": ms * 1e3, "gbs": byt / ms / 1e6, "tflops": 2 * m * n * k / ms / 1e9}
 
 
 def bench_attn(batch: int, ctx: int, hq: int, hk: int, d: int, splits: int, reps: int) -> dict:
