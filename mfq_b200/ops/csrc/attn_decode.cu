@@ -498,33 +498,32 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
   }
 }
 
-// Combine the split partials (running max in the log2 domain).
-template <int D>
+// Combine the split partials (running max in the log2 domain).  kFew: at most kMergeGroup of them, and everything they contribute is
+// requested before the first of it is used (a decode step's attention of one sequence of 600 tokens in 8 splits on a B200: 6.7 -> 6.1
+// us).  More are read in a loop: in groups of eight they took longer (4096 tokens in 32 splits: 10.7 us with the loop, 11.3 in groups).
+constexpr int kMergeGroup = 8;
+template <int D, bool kFew>
 __global__ void attn_reduce_log2_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                         __nv_bfloat16* __restrict__ out, int nsplit) {
   pdl_trigger();
   pdl_wait();
-  // Up to kGroup splits: everything they contribute is requested before the first of it is used (a decode step's attention of one
-  // sequence of 600 tokens in 8 splits on a B200: 6.7 -> 6.1 us).  More are read in a loop: in groups of eight they took longer (4096
-  // tokens in 32 splits: 10.7 us with the loop, 11.3 in groups; 16 splits 8.6, 8.7).
-  constexpr int kGroup = 8;
   const size_t hq = blockIdx.x;
   const int d = threadIdx.x;
-  const float2* ml = reinterpret_cast<const float2*>(part_ml) + hq * nsplit;
-  const float* acc = part_acc + hq * nsplit * D + d;
   float mm = kNeg, ll = 0.f, a = 0.f;
-  if (nsplit <= kGroup) {
-    float2 of[kGroup];
-    float part[kGroup];
+  if constexpr (kFew) {
+    const float2* ml = reinterpret_cast<const float2*>(part_ml) + hq * nsplit;
+    const float* acc = part_acc + hq * nsplit * D + d;
+    float2 of[kMergeGroup];
+    float part[kMergeGroup];
 #pragma unroll
-    for (int i = 0; i < kGroup; ++i) {
+    for (int i = 0; i < kMergeGroup; ++i) {
       of[i] = i < nsplit ? ml[i] : make_float2(kNeg, 0.f);
       part[i] = i < nsplit ? acc[size_t(i) * D] : 0.f;
     }
 #pragma unroll
-    for (int i = 0; i < kGroup; ++i) mm = fmaxf(mm, of[i].x);
+    for (int i = 0; i < kMergeGroup; ++i) mm = fmaxf(mm, of[i].x);
 #pragma unroll
-    for (int i = 0; i < kGroup; ++i) {
+    for (int i = 0; i < kMergeGroup; ++i) {
       if (i < nsplit) {
         const float cw = exp2f(of[i].x - mm);
         ll += of[i].y * cw;
@@ -532,11 +531,11 @@ __global__ void attn_reduce_log2_kernel(const float* __restrict__ part_acc, cons
       }
     }
   } else {
-    for (int s = 0; s < nsplit; ++s) mm = fmaxf(mm, ml[s].x);
+    for (int s = 0; s < nsplit; ++s) mm = fmaxf(mm, part_ml[(hq * nsplit + s) * 2]);
     for (int s = 0; s < nsplit; ++s) {
-      const float cw = exp2f(ml[s].x - mm);
-      ll += ml[s].y * cw;
-      a += acc[size_t(s) * D] * cw;
+      const float cw = exp2f(part_ml[(hq * nsplit + s) * 2] - mm);
+      ll += part_ml[(hq * nsplit + s) * 2 + 1] * cw;
+      a += part_acc[(hq * nsplit + s) * D + d] * cw;
     }
   }
   out[hq * D + d] = __float2bfloat16(ll > 0.f ? a / ll : 0.f);
@@ -566,7 +565,7 @@ static int launch_attn_v(const void* q, const void* k_cache, const void* v_cache
                 seq_lens, static_cast<__nv_bfloat16*>(out), part_acc, part_ml, Hq, Hk, max_pages, scale_log2, q_len, status);
   if (cudaGetLastError() != cudaSuccess) return -7;
   if (splits > 1) {
-    launch_kernel(attn_reduce_log2_kernel<D>, dim3(B * q_len * Hq), dim3(D), 0, stream, part_acc, part_ml, static_cast<__nv_bfloat16*>(out), splits);
+    launch_kernel(splits <= kMergeGroup ? attn_reduce_log2_kernel<D, true> : attn_reduce_log2_kernel<D, false>, dim3(B * q_len * Hq), dim3(D), 0, stream, part_acc, part_ml, static_cast<__nv_bfloat16*>(out), splits);
     if (cudaGetLastError() != cudaSuccess) return -7;
   }
   return 0;

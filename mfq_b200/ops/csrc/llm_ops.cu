@@ -520,11 +520,14 @@ __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv,
     s *= ys.mscale;
     c *= ys.mscale;
   };
+  // The slot is requested with the position, not after the rotation (0.4 us of a decode step's launch), but for one head of 64, where it
+  // costs a block per SM (36 registers instead of 32: 500 tokens of 36 heads 4.6 -> 4.8 us).
+  constexpr bool kEarlySlot = kHeads > 1 || D > 64;
+  const int slot_early = kEarlySlot && h_first + kHeads > Hq ? slots[t] : -1;
+  const auto slot = [&] { return kEarlySlot ? slot_early : slots[t]; };
   if constexpr (kHeads == 1) {
-    rope_head<D, false>(src, lo, hi, t, h_first, lane, positions, rot, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to, evaluate,
-                        [&] { return slots[t]; });
+    rope_head<D, false>(src, lo, hi, t, h_first, lane, positions, rot, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to, evaluate, slot);
   } else {
-    const int slot = h_first + kHeads > Hq ? slots[t] : -1;  // requested with the position, not after the rotation
     float cs[HP], sn[HP];
     if (h_first < Hq + Hk) {  // values are not rotated; the first head is on its way from memory
 #pragma unroll
@@ -537,7 +540,7 @@ __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv,
         load_half(src + D / 2 + lane * HP, hi);
       }
       rope_head<D, true>(src, lo, hi, t, h, lane, positions, D, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to,
-                         [&](int j, float& s, float& c) { s = sn[j]; c = cs[j]; }, [&] { return slot; });
+                         [&](int j, float& s, float& c) { s = sn[j]; c = cs[j]; }, slot);
     }
   }
 }
@@ -757,9 +760,9 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
   // A warp per head, or one per kRopeHeads heads of a token, whose angles (sine, cosine and the frequency's power, a good part of a head's
   // work) it evaluates once.  That needs full rotary, enough heads that the fewer and longer warps still fill the GPU, and groups that are
-  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  On a B200, a warp per head | eight heads:  48 heads of 128, 500 tokens 10.3 | 11.4 us, 700 13.4 | 14.5, 800
-  // 15.1 | 14.7, 1000 18.7 | 14.9, 4096 68.5 | 47.0;  36 heads of 64, 800 tokens 6.4 | 6.8, 1000 7.6 | 6.9;  20 of 256, 2000 21.5 | 20.4;
-  // 10 of 128 (two groups), 4096 13.1 | 14.2.
+  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  On a B200, a warp per
+  // head | eight heads:  48 heads of 128, 500 tokens 10.3 | 12.6 us, 700 13.5 | 14.5, 800 15.2 | 14.8, 1000 18.8 | 15.2, 4096 68.7 | 47.0;
+  // 36 heads of 64, 800 tokens 6.5 | 6.8, 1000 7.6 | 6.9;  20 of 256, 2000 21.5 | 20.1;  10 of 128 (two groups), 4096 13.1 | 14.2.
   const int heads = Hq + 2 * Hk, full_groups = (heads + kRopeHeads - 1) / kRopeHeads;
   const bool aligned = (reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kd_out) | reinterpret_cast<uintptr_t>(vd_out)) % 8 == 0;
   const bool shared = rot == D && long(T) * heads >= 36000 && 4 * heads >= 3 * kRopeHeads * full_groups && aligned;
