@@ -862,8 +862,8 @@ __global__ void silu_mul_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_b
 extern "C" int mfq_silu_mul_bf16(const void* x, void* out, int M, int I, int in_stride, cudaStream_t stream) {
   if (M <= 0 || I % 8 || in_stride % 8) return -1;
   // Fewer rows than two waves of CTAs: a row over several of them, a vector per thread, instead of up to seven vectors one after the
-  // other (6 rows of 14336 took 6.8 us with a CTA each).
-  const int parts = M >= 296 ? 1 : (I / 8 + 255) / 256;
+  // other (6 rows of 14336 took 6.8 us with a CTA each).  Rows of no width keep one: a grid has no empty dimension.
+  const int parts = M >= 296 ? 1 : max(1, (I / 8 + 255) / 256);
   mfq::launch_kernel(mfq::silu_mul_bf16_kernel, dim3(M, parts), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(x),
                      static_cast<__nv_bfloat16*>(out), I, in_stride);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;

@@ -182,9 +182,10 @@ def test_router_logits_of_a_prompt(t, e):
     assert bool(((weights.double() - picked / picked.sum(1, keepdim=True)).abs() <= 4 * slack).all())
 
 
-@pytest.mark.parametrize("m,i", [(1, 8), (6, 2056), (295, 264), (296, 264)])
+@pytest.mark.parametrize("m,i", [(1, 8), (6, 2056), (295, 264), (296, 264), (3, 0)])
 def test_gated_rows_over_one_and_several_blocks(m, i):
-    """The last sizes before and after the rule's line, rows that end in the middle of a block, a batch of rows set apart by padding."""
+    """The last sizes before and after the rule's line, rows that end in the middle of a block, a batch of rows set apart by padding, rows
+    of no width."""
     require_gpu_lib()
     rows = _normal(m, m, 2 * i + 8)[:, :2 * i]
     a, b = rows[:, :i].double(), rows[:, i:].double()
