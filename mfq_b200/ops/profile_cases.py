@@ -4,7 +4,8 @@ Each case launches one kernel three times on inputs of a few hundred MB (larger 
 for a multi-pass capture to finish in about a minute) and exits.  Cases: ``gemm_prefill`` (M=4096, N=K=4096),
 ``gemm_decode`` (M=64, N=28672, K=4096), ``attn_decode`` (64 sequences x 4096 tokens), ``attn_prefill`` (T=2048),
 ``w4_decode`` / ``w4_prefill`` (the 4-bit in-pipeline-decode GEMM at the same shapes), ``gdn_decode`` (Gated DeltaNet step,
-64 sequences), ``moe_dispatch`` (expert-parallel dispatch + combine kernels at world 1, 4096 tokens), ``gemv_decode``
+64 sequences), ``w4_decode_bs6`` (the weight-streaming 4-bit kernel), ``experts_prefill`` (grouped FP8 product, 3000 tokens x top-10 of
+512 experts of 1024 x 2048), ``moe_dispatch`` (expert-parallel dispatch + combine kernels at world 1, 4096 tokens), ``gemv_decode``
 (the weight-streaming FP8 kernel, M=1, N=28672, K=4096), ``attn_prefill_d256`` (T=2048, 16 query / 2 KV heads of 256),
 ``gdn_prefill`` (the long-row Gated DeltaNet path, 2048 tokens, 32 heads), ``mla_decode`` (latent-cache decode attention), ``packed_decode`` / ``packed_decode_bs1`` (the
 packed-expert product at 64 tokens / one token, 512 experts), ``window_decode`` / ``window_prefill`` (attention over
@@ -172,6 +173,18 @@ def packed_decode(tokens: int = 64) -> None:
         packed.packed_gemv_grouped(pe, x, plan, gather=True)
 
 
+def experts_prefill() -> None:
+    """The gate/up product of a 512-expert layer: 3000 tokens x top-10 routes, 1.1 GB of weights."""
+    from . import moe
+    t, e, k, n, h = 3000, 512, 10, 1024, 2048
+    ids = torch.stack([torch.randperm(e, device="cuda")[:k] for _ in range(t)]).to(torch.int32)
+    plan = moe.plan_routes(ids, 0, e)
+    w, x, xs = _fp8((e, n, h)), _fp8((t * k, h)), torch.rand(t * k, device="cuda")
+    ws = torch.rand((e, n // 128, h // 128), device="cuda") * 0.01 + 0.001
+    for _ in range(3):
+        moe.fp8_gemm_grouped(x, xs, w, ws, plan)
+
+
 def window_decode() -> None:
     from . import bench_kernels, window_attn
     cache = bench_kernels._plain_cache(64, 4096, 8, 128, 128, 3)  # 1 GB of pages per launch, a quarter of it inside the window
@@ -271,6 +284,7 @@ CASES = {"ssd_decode": lambda: ssd_case(1, 64), "ssd_prefill": lambda: ssd_case(
          "gla_prefill": lambda: gla_case(2048, 1), "gemm_prefill": lambda: gemm(4096, 4096, 4096), "gemm_decode": lambda: gemm(64, 28672, 4096),
          "gemm_decode_splitk": lambda: gemm(64, 4096, 14336),
          "attn_decode": attn_decode, "attn_prefill": attn_prefill, "w4_decode": lambda: w4_gemm(64, 28672, 4096),
+         "w4_decode_bs6": lambda: w4_gemm(6, 28672, 4096), "experts_prefill": experts_prefill,
          "w4_prefill": lambda: w4_gemm(4096, 4096, 4096), "gdn_decode": gdn_decode, "moe_dispatch": moe_dispatch,
          "gemv_decode": lambda: gemm(1, 28672, 4096), "packed_decode": packed_decode, "packed_decode_bs1": lambda: packed_decode(1), "attn_prefill_d256": attn_prefill_d256, "gdn_prefill": gdn_prefill, "mla_decode": mla_decode,
          "window_decode": window_decode, "window_prefill": window_prefill, "dense_prefill": dense_prefill}
