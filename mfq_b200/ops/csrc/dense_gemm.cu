@@ -22,11 +22,11 @@
 
 // the same product on pairs of SMs (dense_pair.cu)
 extern "C" int mfq_dense_pair(const void* w, const void* x, int ldx, void* out, int ldo, const float* bias, int M, int N, int K, int epilogue,
-                              float alpha, float limit, const void* table, const int* ids, int token_tile, int* status, cudaStream_t stream);
+                              float alpha, float limit, const void* table, const int* ids, int token_tile, int parts, int* status, cudaStream_t stream);
 
 namespace mfq {
 
-constexpr int kDensePair = -2;  // as a number of splits: the product runs on pairs of SMs
+constexpr int kDensePair = -2;  // as a number of splits: the product runs on pairs of SMs, in one sum; -1 - s: in s parts along K
 constexpr int kDnTileN = 128, kDnBlockK = 64, kDnThreads = 256;
 constexpr int kDnABytes = kDnTileN * kDnBlockK * 2;
 
@@ -416,10 +416,10 @@ static int run_dense(const DenseParams& p, const void* w, const void* x, int ldx
     if (!p.tiles && p.M > 16) return -1;
     return !p.tiles && p.M <= 8 ? launch_dense_gemv<1>(w, x, ldx, p, entries, stream) : launch_dense_gemv<2>(w, x, ldx, p, entries, stream);
   }
-  if (splits == kDensePair) {
+  if (splits <= kDensePair) {
     if (p.tiles || p.groups > 1) return -1;
     return mfq_dense_pair(w, x, ldx, p.epi.out, p.epi.ldo, p.epi.bias, p.M, p.N, p.K, kind, p.epi.alpha, p.epi.limit, p.epi.table, p.epi.ids,
-                          token_tile, p.status, stream);
+                          token_tile, -1 - splits, p.status, stream);
   }
   switch (token_tile) {
     case 16: return launch_dense_gemm<16>(p, w, x, ldx, matrices, entries, splits, stream);
@@ -435,7 +435,7 @@ static int run_dense(const DenseParams& p, const void* w, const void* x, int ldx
 
 // w [N, K] row-major, x [M, ldx], both bf16 (fp32 = 0) or fp32 (fp32 = 1).  N a multiple of 16, K and ldx of 8, M > 0; ldo of 8.
 // token_tile 0: the weight-streaming kernel (M <= 16); 16 .. 256: the tcgen05 kernel with that tile and `splits` K splits;
-// splits -2 with a tile of 128 or 256 and one matrix: the same on pairs of SMs (dense_pair.cu).
+// splits -1 - s with a tile of 128 or 256 and one matrix: the same on pairs of SMs (dense_pair.cu), its sums in s parts along K.
 // groups > 1: w [groups, N, K] (bias [groups, N]); matrix g reads x from column g * x_step on and writes out from g * out_step on
 // (multiples of 8).
 extern "C" int mfq_dense_linear(const void* w, const void* x, int ldx, void* out, int ldo, const float* bias, int M, int N, int K,

@@ -10,6 +10,9 @@
 // warp % 4, two warps per quarter split the tokens).  Barriers as in fp8_gemm_2cta.cu, except that an accumulator is complete once per
 // tile.  A warp of the output stage turns 32 rows x 16 tokens through its own 2 KB of shared memory, so that a lane holds 8
 // consecutive rows of a token: 16-byte stores, and the pairs of 8 gate and 8 up rows of a gated unit in one thread.
+// A product that the one-SM kernel would split along K is summed in the same parts (kParts): each gets an accumulator of its own, and the
+// output stage adds them up in order, so that the sums and their rounding are the split form's.  In one accumulator 200 x 6144 x 4096 was
+// twice as far from 64 bits (4.4e-6 instead of 2.1e-6 of the result).
 // 1508 tokens on a B200, one-SM kernel -> this one: 28672 x 4096 gated 462 -> 252 us (1.40 PFLOP/s), 6144 x 4096 73 -> 53, 4096 x 4096
 // 64 -> 50, 4096 x 14336 211 -> 170; 4096 tokens of the first 1225 -> 687.
 #include "dense_common.cuh"
@@ -34,9 +37,10 @@ struct DensePairParams {
   DenseEpilogue epi;
   int* status;
   int M, N, K;
+  int kb_per_part;  // kParts: K blocks of a part
 };
 
-template <int BT>
+template <int BT, bool kParts>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DensePairCfg<BT>::kThreads, 1)
 dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const DensePairParams p) {
   using Cfg = DensePairCfg<BT>;
@@ -53,7 +57,7 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();  // 0 = leader
   const bool leader = rank == 0;
-  const int nkb = (p.K + kBK - 1) / kBK;
+  const int nkb = (p.K + kBK - 1) / kBK, per_part = kParts ? p.kb_per_part : nkb, parts = kParts ? (nkb + per_part - 1) / per_part : 1;
   const int clusters = int(gridDim.x) / 2, cluster = int(blockIdx.x) / 2;
   // token tiles innermost: pairs at work at the same time share the weight rows in L2
   const int t_tiles = (p.M + BT - 1) / BT, tiles_total = t_tiles * ((p.N + 2 * kRows - 1) / (2 * kRows));
@@ -108,16 +112,19 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     uint32_t phase = 0, buf = 0, acc_phase = 1;  // the first pass over the accumulators finds them free
     bool ok = true;
     for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
-      ok = mbar_wait_warp(&acc_empty[buf], acc_phase, abort_flag, p.status, kStatusTimeoutMma);
-      for (int i = 0; ok && i < nkb; ++i) {
-        ok = mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma);
-        if (!ok) break;
-        tc_fence_after();
-        umma_f16_block_pair(tmem_base + buf * BT, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc,
-                            i > 0 ? 1u : 0u, empty_addr + s * 8, i + 1 == nkb ? acc_full_addr + buf * 8 : 0u);
-        if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
+      for (int first = 0; ok && first < nkb; first += per_part) {
+        const int end = min(nkb, first + per_part);
+        ok = mbar_wait_warp(&acc_empty[buf], acc_phase, abort_flag, p.status, kStatusTimeoutMma);
+        for (int i = first; ok && i < end; ++i) {
+          ok = mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma);
+          if (!ok) break;
+          tc_fence_after();
+          umma_f16_block_pair(tmem_base + buf * BT, a_desc0 + uint64_t(s) * kStageStep, b_desc0 + uint64_t(s) * kStageStep, idesc,
+                              i > first ? 1u : 0u, empty_addr + s * 8, i + 1 == end ? acc_full_addr + buf * 8 : 0u);
+          if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
+        }
+        if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
       }
-      if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;
@@ -128,14 +135,31 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     bool ok = true;
     for (int tile = cluster; ok && tile < tiles_total; tile += clusters) {
       const int n0 = tile_n0(tile) + q * 32, t0 = tile_t0(tile) + half * (BT / 2);
-      ok = mbar_wait_warp(&acc_full[buf], phase, abort_flag, p.status, kStatusTimeoutEpilogue);
+      uint32_t after = buf, after_phase = phase;  // past the parts of this tile, at most kAcc of them
+      for (int z = 0; ok && z < parts; ++z) {
+        ok = mbar_wait_warp(&acc_full[after], after_phase, abort_flag, p.status, kStatusTimeoutEpilogue);
+        if (++after == Cfg::kAcc) { after = 0; after_phase ^= 1u; }
+      }
       if (!ok) break;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BT + half * (BT / 2);
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + half * (BT / 2);
       for (int c = 0; c < BT / 2; c += 16) {
         uint32_t r[16];
-        tmem_ld_32x16(taddr + c, r);
+        tmem_ld_32x16(taddr + buf * BT + c, r);
         tmem_wait_ld();
+        if constexpr (kParts) {
+          float sum[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sum[j] = 0.f + __uint_as_float(r[j]);
+          for (int z = 1; z < parts; ++z) {
+            tmem_ld_32x16(taddr + (buf + z) % Cfg::kAcc * BT + c, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[j] += __uint_as_float(r[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(sum[j]);
+        }
         __syncwarp();  // the chunk before has been read
 #pragma unroll
         for (int j = 0; j < 16; ++j) turn[j * 32 + lane] = __uint_as_float(r[j]);
@@ -148,8 +172,10 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(acc_empty_leader + buf * 8);
-      if (++buf == Cfg::kAcc) { buf = 0; phase ^= 1u; }
+      if (lane == 0)
+        for (int z = 0; z < parts; ++z) mbar_arrive_cluster(acc_empty_leader + (buf + z) % Cfg::kAcc * 8);
+      buf = after;
+      phase = after_phase;
     }
   }
 
@@ -162,7 +188,7 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int BT>
+template <int BT, bool kParts>
 int launch_dense_pair(const DensePairParams& p, const void* w, const void* x, int ldx, cudaStream_t stream) {
   using Cfg = DensePairCfg<BT>;
   CUtensorMap tw, tx;
@@ -172,25 +198,27 @@ int launch_dense_pair(const DensePairParams& p, const void* w, const void* x, in
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -6;
   if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(dense_pair_kernel<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return -6;
+    if (cudaFuncSetAttribute(dense_pair_kernel<BT, kParts>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return -6;
     attr_set[dev] = true;
   }
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles = (p.N + 2 * kRows - 1) / (2 * kRows) * ((p.M + BT - 1) / BT);
-  launch_kernel(dense_pair_kernel<BT>, dim3(2 * (tiles < sms / 2 ? tiles : sms / 2)), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tw, tx, p);
+  launch_kernel(dense_pair_kernel<BT, kParts>, dim3(2 * (tiles < sms / 2 ? tiles : sms / 2)), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 
 }  // namespace
 }  // namespace mfq
 
-// The plain form of mfq_dense_linear (one matrix, bf16, checked there) on CTA pairs; token_tile 128 or 256.
+// The plain form of mfq_dense_linear (one matrix, bf16, checked there) on CTA pairs; token_tile 128 or 256.  parts: sums along K, as
+// many as there are accumulators (2 with the tile of 256, 4 with 128).
 extern "C" int mfq_dense_pair(const void* w, const void* x, int ldx, void* out, int ldo, const float* bias, int M, int N, int K, int epilogue,
-                              float alpha, float limit, const void* table, const int* ids, int token_tile, int* status, cudaStream_t stream) {
+                              float alpha, float limit, const void* table, const int* ids, int token_tile, int parts, int* status, cudaStream_t stream) {
   using namespace mfq;
-  const DensePairParams p{DenseEpilogue{epilogue, bias, alpha, limit, table, ids, out, ldo}, status, M, N, K};
-  if (token_tile == 128) return launch_dense_pair<128>(p, w, x, ldx, stream);
-  if (token_tile == 256) return launch_dense_pair<256>(p, w, x, ldx, stream);
-  return -1;
+  if ((token_tile != 128 && token_tile != 256) || parts < 1 || parts > 512 / token_tile) return -1;
+  const int nkb = (K + kBK - 1) / kBK, per_part = (nkb + parts - 1) / parts;
+  const DensePairParams p{DenseEpilogue{epilogue, bias, alpha, limit, table, ids, out, ldo}, status, M, N, K, per_part};
+  if (per_part < nkb) return token_tile == 128 ? launch_dense_pair<128, true>(p, w, x, ldx, stream) : launch_dense_pair<256, true>(p, w, x, ldx, stream);
+  return token_tile == 128 ? launch_dense_pair<128, false>(p, w, x, ldx, stream) : launch_dense_pair<256, false>(p, w, x, ldx, stream);
 }

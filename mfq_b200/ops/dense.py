@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -44,6 +45,7 @@ def _most_splits(tiles: int, blocks: int, small: bool, sms: int) -> int:
 PAIR = -2  # as a number of K splits: the product runs on pairs of SMs (csrc/dense_pair.cu)
 
 
+@lru_cache(maxsize=4096)  # sizes only; a prompt asks for the same few once per layer
 def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[int, int]:
     """``(token tile, K splits)`` of a bf16 product ``[m, k] x [n, k]^T``; tile 0 is the weight-streaming kernel, splits
     :data:`PAIR` the kernel on pairs of SMs (``pairs``: it may be chosen; it takes a single matrix).  Fitted to a
@@ -51,7 +53,9 @@ def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[i
     once whatever the split, so the grid is filled; beyond that a wave of 256-token tiles costs about 7 + 0.35 us per K block,
     of 128-token tiles 5 + 0.30 us, and meeting in a cluster 5 / 3 us.  A wave of pairs (256 rows each) costs 2 + 0.40 us per K block
     with 256 tokens and 0.26 with 128, once 4 us for the launch: 1508 tokens of gate/up 28672 x 4096 take 252 us there against 462 here,
-    of o_proj 4096 x 4096 50 against 64; what stays here are narrow or split products (300 x 4096 x 14336: 52 against 54 us)."""
+    of o_proj 4096 x 4096 50 against 64; what stays here are narrow or split products (300 x 4096 x 14336: 52 against 54 us).
+    Sums in parts (:func:`pair_sums`), as many as there are accumulators, cost a pair 0.5 to 1 us: 300 x 4096 x 4096 in two 19.5 us there
+    against 21.2 here, 200 x 1536 x 1536 in three 10.05 against 9.95, the least favourable."""
     if m <= GEMV_ROWS or (m <= GEMV_MID_ROWS and n * k <= GEMV_MID_WEIGHTS):
         return 0, 1
     rows, blocks = math.ceil(n / 128), math.ceil(k / 64)
@@ -67,11 +71,20 @@ def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[i
                 best, best_cost = (tile, s), cost
     if math.ceil(rows * math.ceil(m / best[0]) * best[1] / sms) > 1:
         best_cost *= 1.1  # several waves of CTAs: 4096 x 4096 x 14336 takes 434 us, not the 341 of four single ones
+    sums = best[1]  # a pair forms them too, in an accumulator each
     for tile, ramp, per_block in ((256, 2.0, 0.40), (128, 0.0, 0.26)) if pairs else ():
+        if sums > 512 // tile:
+            continue
         cost = 4.0 + math.ceil(math.ceil(n / 256) * math.ceil(m / tile) / (sms // 2)) * (ramp + per_block * blocks)
         if cost < best_cost:
             best, best_cost = (tile, PAIR), cost
     return best
+
+
+def pair_sums(m: int, n: int, k: int) -> int:
+    """Parts along K that the one-SM kernel would sum on their own for this shape.  The kernel on pairs forms its sums alike, so that a
+    product that moves there is no further from the exact one and keeps its bits."""
+    return plan(m, n, k)[1]
 
 
 @dataclass
@@ -131,6 +144,8 @@ class DenseLinear:
             kind = GELU
         t, s = plan(m, n * g, k, pairs=g == 1 and tile is None and splits is None)
         t, s = (t if tile is None else tile), (s if splits is None else splits)
+        if s == PAIR and splits is None:
+            s = -1 - pair_sums(m, n, k)
         rc = dense_lib().mfq_dense_linear(ptr(self.w), ptr(x), x.stride(0), ptr(out), out.stride(0), ptr(self.bias), m, n, k, g, x_step,
                                           out_step, kind, alpha, limit, ptr(table), ptr(ids), t, s, is_fp32(x.dtype),
                                           ptr(Workspace.get(x.device).status), stream_ptr())

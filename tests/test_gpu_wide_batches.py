@@ -105,6 +105,21 @@ def test_dense_pair_kernel_on_every_output_stage(m, n, k, tile):
     check_status()
 
 
+@pytest.mark.parametrize("m,n,k,tile,sums", [(200, 6144, 4096, 128, 2), (129, 2560, 1536, 128, 3), (300, 1040, 1104, 128, 4), (1300, 2832, 1096, 128, 3),
+                                             (1500, 4112, 520, 256, 2)])
+def test_dense_pair_kernel_keeps_the_sums_of_the_split_form(m, n, k, tile, sums):
+    """The first two are taken by themselves; in the last two a pair walks several tiles of several accumulators each, over a K range that
+    the parts do not divide."""
+    require_gpu_lib()
+    x, w = _normal(m, m, k), _normal(n, n, k, std=k ** -0.5)
+    want = DenseLinear(w)(x, fp32=True, tile=tile, splits=sums)
+    assert torch.equal(DenseLinear(w)(x, fp32=True, tile=tile, splits=-1 - sums), want)
+    if k in (4096, 1536):
+        assert dense.plan(m, n, k, pairs=True) == (tile, dense.PAIR) and dense.pair_sums(m, n, k) == sums
+        assert torch.equal(DenseLinear(w)(x, fp32=True), want)
+    check_status()
+
+
 @pytest.mark.parametrize("m", [3, 511, 512, 1025])
 @pytest.mark.parametrize("k", [8, 520, 4096, 14336, 16384, 16392])
 def test_row_quantization_in_one_pass(m, k):

@@ -91,3 +91,17 @@ def test_splits_fit_the_scratch():
                 assert s == 1 or partials <= K.SPLIT_SCRATCH_BYTES, (m, rows * 128, k, s)
                 unsplit += s == 1 and K._best_splits(m, rows * 128, k, 148) > 1
     assert unsplit and K.pick_splits(8192, 640, 14336) == 1
+
+
+def test_sums_of_a_dense_pair_product_fit_its_accumulators():
+    from mfq_b200.ops import dense
+    seen = set()
+    for m in (129, 160, 200, 257, 357, 500, 1000, 2048):
+        for n in (256, 1040, 2560, 3072, 4096, 6144, 11008, 28672):
+            for k in (512, 1536, 2048, 4096, 5632, 14336):
+                tile, splits = dense.plan(m, n, k, pairs=True)
+                if splits == dense.PAIR:
+                    sums = dense.pair_sums(m, n, k)
+                    assert 1 <= sums <= 512 // tile and sums == dense.plan(m, n, k)[1]
+                    seen.add(sums)
+    assert seen > {1}
