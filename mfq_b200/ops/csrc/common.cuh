@@ -142,6 +142,15 @@ __device__ __forceinline__ void tma_load_stage(uint32_t smem_a, uint32_t smem_b,
         : "memory");
   }
 }
+// Bulk store of a shared-memory tile (rows and columns beyond the tensor are left out), in the issuing thread's current group.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* desc, uint32_t smem_src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(desc)), "r"(smem_src), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // sources may be written again
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }             // ... and the stores are done
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

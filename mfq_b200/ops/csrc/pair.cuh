@@ -42,10 +42,25 @@ __device__ __forceinline__ void tma_load_stage_pair(uint32_t smem_a, uint32_t sm
         "r"(bar_local), "r"(bytes), "r"(x), "r"(ya), "r"(yb)
       : "memory");
 }
+// One tile of a stage, likewise.
+__device__ __forceinline__ void tma_load_pair(uint32_t smem, const CUtensorMap* map, uint32_t bar_cluster_addr, uint32_t bar_local, uint32_t bytes, int x,
+                                              int y) {
+  asm volatile(
+      "{\n\t.reg .pred q, e;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.and.b32 e, %4, 0, q;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%5, %6}], [%2];\n\t}"
+      ::"r"(smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(bar_local), "r"(bytes), "r"(x), "r"(y)
+      : "memory");
+}
 // Relaxed: what it orders are tensor-memory reads, which have completed (wait::ld, fence::before_thread_sync) before it; a
 // release at cluster scope would also drain this warp's global accesses, about a microsecond per block.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_cluster_warp(uint32_t bar_cluster_addr) {  // whole warp, one elected lane, no branch
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(bar_cluster_addr)
+               : "memory");
 }
 
 // Four k-steps of 32 bytes into accumulator `d`, then up to two commits (shared addresses; 0 = none), each of which arrives on the

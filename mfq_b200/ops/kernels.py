@@ -112,14 +112,15 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     """Token tile of the two-SM GEMM for this shape, 0 = use the one-SM kernel.  ``MFQ_GEMM_PAIR`` = 0 / 128 / 256
     overrides the choice.
 
-    Both sides by wave models in microseconds, fitted on B200 to 652 shapes of 65 .. 4096 tokens, 256 .. 28672 rows and K 512 .. 14336.
-    Pairs walk tiles of 256 weight rows: a wave takes 2.9 + 0.306 per K block with 128 tokens, 6.7 + 0.506 with 256, and about 1.5 for
-    every split sum beyond two, which one pair works through one after the other; the launch costs 3.2.  A wave of one-SM CTAs takes 6.1 + 0.36
+    Both sides by wave models in microseconds, fitted on B200 to 315 shapes of 65 .. 4096 tokens, 256 .. 28672 rows and K 512 .. 14336;
+    over these the choice is 0.3 % slower than the best of the three.
+    Pairs walk tiles of 256 weight rows: a wave takes 1.9 + 0.214 per K block with 128 tokens, 1.95 + 0.38 with 256; in split sums (128
+    tokens) a microsecond more, and 0.5 for every sum beyond two, which one pair works through one after the other; the launch costs
+    4.2 and 3.4.  A wave of one-SM CTAs takes 6.1 + 0.36
     per K block of a split, and meeting 4.4 with two splits, 2 in a larger cluster, 10 in memory; clusters in a grid
-    of nearly every SM do not all fit (6).  So few tiles over a range that the one-SM kernel splits stay there (66 x 256 x 2048: 6.2
-    against 20.0 us; 128 x 4096 x 4096: 11.6 against 19.1), full waves come here (1000 x 6144 x 4096: 38.6 with 128 tokens).
-    Where half of the pairs would idle over more than 64 K blocks the one-SM kernel is kept without a sum (128 x 4096 x 14336: 19.9
-    against 37.8 us)."""
+    of nearly every SM do not all fit (5; 22 clusters of six do).  So few tiles over a range that the one-SM kernel splits stay there (66 x 256 x 2048: 7.0
+    against 12.6 us; 128 x 4096 x 4096: 11.7 against 15.0; 128 x 4096 x 14336: 19.4 against 31.5), full waves come here (1000 x 6144 x 4096:
+    54.5 against 37.8 with 128 tokens and 34.2 with 256)."""
     forced = os.environ.get("MFQ_GEMM_PAIR")
     if n % 256 or m < PAIR_MIN_ROWS:
         return 0
@@ -131,17 +132,17 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
 @lru_cache(maxsize=4096)
 def _pair_tile_by_cost(m: int, n: int, k: int, sms: int) -> int:
     pairs, blocks = sms // 2, k // 128
-    tiles = {t: n // 256 * math.ceil(m / t) for t in (128, 256)}
-    if 2 * tiles[128] <= pairs and blocks > 64:
-        return 0
+    waves = {t: math.ceil(n // 256 * math.ceil(m / t) / pairs) for t in (128, 256)}
     per = split_blocks(m, n, k) or blocks
     splits = math.ceil(blocks / per)
-    cost = {t: 3.2 + math.ceil(tiles[t] / pairs) * (ramp + step * blocks + 1.5 * max(0, splits - 2))
-            for t, ramp, step in ((128, 2.9, 0.306), (256, 6.7, 0.506))}
-    tile = 128 if splits > 1 or cost[128] <= cost[256] else 256
+    if splits > 1:
+        cost = {128: 4.1 + waves[128] * (2.9 + 0.21 * blocks + 0.5 * (splits - 2))}
+    else:
+        cost = {128: 4.2 + waves[128] * (1.9 + 0.214 * blocks), 256: 3.4 + waves[256] * (1.95 + 0.38 * blocks)}
+    tile = min(cost, key=cost.get)
     ctas = math.ceil(n / 128) * math.ceil(m / 128) * splits
-    meet = {1: 0.0, 2: 4.4}.get(splits, 2.0 if splits <= 8 else 10.0) + (6.0 if splits > 1 and 128 < ctas <= sms else 0.0)
-    return tile if cost[tile] < math.ceil(ctas / sms) * (6.1 + 0.36 * per + meet) else 0
+    meet = {1: 0.0, 2: 4.4}.get(splits, 2.0 if splits <= 8 else 10.0) + (5.0 if splits > 1 and (132 if splits == 6 else 128) < ctas <= sms else 0.0)
+    return tile if cost[tile] + 0.3 < math.ceil(ctas / sms) * (6.1 + 0.36 * per + meet) else 0
 
 
 def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, *,

@@ -63,6 +63,26 @@ def test_fp8_product_of_a_wide_batch_keeps_the_sums_of_the_split_form(m, n, k, m
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("m,n,k,tile", [(128, 1536, 1024, 0), (96, 5120, 768, 0), (1300, 2048, 2048, 0), (300, 4608, 1024, 128), (300, 4608, 1024, 256)])
+def test_fp8_pair_kernel_passes_its_output_places_on(m, n, k, tile, monkeypatch):
+    """The output places in shared memory hold, in turn, split sums (tile 0: several of them), the residual and the results, of a token
+    range that ends inside a place; output and residual off a 16-byte boundary go round them."""
+    require_gpu_lib()
+    args = _fp8(m, m, n, k)
+    res = _normal(m, m, n)
+    off = torch.empty(m * n + 1, device="cuda", dtype=torch.bfloat16)[1:].view(m, n)
+    assert off.data_ptr() % 16 and (tile or K.split_blocks(m, n, k))
+    monkeypatch.setattr(K, "pair_tile", lambda *_: tile or 128)
+    one = dict(splits=1, token_tile=128) if tile else dict(pair=0)
+    for r in (None, res) * 3:
+        want = ops.fp8_gemm(*args, residual=r, **one)
+        assert torch.equal(ops.fp8_gemm(*args, residual=r, pair=tile or None), want)
+        assert torch.equal(ops.fp8_gemm(*args, residual=r, out=off, pair=tile or None), want)
+    h = off.copy_(res)
+    assert torch.equal(ops.fp8_gemm(*args, residual=h, out=h, pair=tile or None), want)
+    check_status()
+
+
 def test_fp8_product_whose_partial_sums_exceed_the_scratch():
     """Rows that are not whole pairs of blocks stay on the one-SM kernel, whose wave model asks for 80 MB of partial sums here."""
     require_gpu_lib()
