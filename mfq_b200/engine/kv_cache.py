@@ -165,9 +165,11 @@ class PagedKVCache(PagedTables):
         self.v = torch.zeros((layers, num_pages, kv_heads, head_dim, page_size), dtype=torch.float8_e4m3fn, device=dev)
         self.k_scale = torch.zeros((layers, num_pages, kv_heads, page_size), dtype=torch.float32, device=dev)
         self.v_scale = torch.zeros((layers, num_pages, kv_heads, page_size), dtype=torch.float32, device=dev)
+        # four views a layer, made once: every forward pass asks for every layer's
+        self._by_layer = [LayerKV(self.k[i], self.v[i], self.k_scale[i], self.v_scale[i], page_size) for i in range(layers)]
 
     def layer(self, i: int) -> LayerKV:
-        return LayerKV(self.k[i], self.v[i], self.k_scale[i], self.v_scale[i], self.page_size)
+        return self._by_layer[i]
 
     # -- page export / import (prefix cache, session snapshots) ------------------------------------------------------
     def export_pages(self, page_ids: list[int]):

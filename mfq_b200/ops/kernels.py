@@ -9,6 +9,7 @@ from functools import lru_cache
 
 import torch
 
+from .. import config
 from .lib import Workspace, check, lib, ptr, stream_ptr
 
 FP8 = torch.float8_e4m3fn
@@ -23,8 +24,7 @@ GEMV_WIDE_ROWS = 64  # ... and up to this many when the weight matrix is small (
 
 def gemv_enabled() -> bool:
     """``MFQ_GEMV=0`` in the environment sends every shape through the tcgen05 GEMM (A/B measurements)."""
-    from ..config import current
-    return current().gemv
+    return config.current().gemv
 
 
 def use_gemv(m: int, n: int, k: int) -> bool:
@@ -35,13 +35,13 @@ def use_gemv(m: int, n: int, k: int) -> bool:
     matrix small (a tensor-parallel rank's q/k/v shard), where the tcgen05 path would need a deep split-K whose reduction
     costs more than the product: 768 x 4096 at 64 rows takes 11.1 us here against 14.7 us there; from 3072 x 4096 up the
     tcgen05 path wins (the legacy ``mma.sync`` pipe this kernel uses runs at a fraction of the tcgen05 rate)."""
-    if n % 16 or not gemv_enabled():
+    if m > GEMV_WIDE_ROWS or n % 16 or not gemv_enabled():
         return False
     if m <= GEMV_MAX_ROWS:
         return True
     if m <= GEMV_MID_ROWS and n * k <= GEMV_MID_WEIGHTS:
         return True
-    return m <= GEMV_WIDE_ROWS and n <= 1024 and n * k <= (4 << 20)
+    return n <= 1024 and n * k <= (4 << 20)
 
 
 def _token_tile(m: int) -> int:
@@ -154,9 +154,9 @@ def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scal
     n = w_q.shape[0]
     assert w_q.shape[1] == k and k % 128 == 0 and x_q.dtype == FP8 and w_q.dtype == FP8
     assert x_scale.dtype == torch.float32 and w_scale.dtype == torch.float32 and x_scale.numel() == m
-    assert w_scale.shape == (math.ceil(n / 128), k // 128) and w_scale.is_contiguous()
+    assert w_scale.shape == (-(-n // 128), k // 128) and w_scale.is_contiguous()
     if out is None:
-        out = torch.empty((m, n), dtype=torch.bfloat16, device=x_q.device)
+        out = x_q.new_empty((m, n), dtype=torch.bfloat16)
     if splits is None and token_tile is None and use_gemv(m, n, k):
         rc = lib().mfq_fp8_gemv(ptr(w_q), ptr(w_scale), ptr(x_q), ptr(x_scale), ptr(out), ptr(residual), m, n, k, stream_ptr())
         check(rc, "fp8_gemv")
@@ -186,10 +186,9 @@ def rmsnorm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float, *, residual
                   residual_out=None):
     """(x [+ residual]) -> RMSNorm -> fp8 rows.  Returns ``(q, scale, y, new_residual)`` (unused ones None)."""
     m, h = x.shape
-    dev = x.device
     if want_q:
-        q_out = torch.empty((m, h), dtype=FP8, device=dev) if q_out is None else q_out
-        scale_out = torch.empty(m, dtype=torch.float32, device=dev) if scale_out is None else scale_out
+        q_out = x.new_empty((m, h), dtype=FP8) if q_out is None else q_out
+        scale_out = x.new_empty(m, dtype=torch.float32) if scale_out is None else scale_out
     if want_y and y_out is None:
         y_out = torch.empty_like(x)
     if residual is not None and residual_out is None:
@@ -220,8 +219,7 @@ def act_gemv_pays(m: int, n: int, k: int) -> bool:
     2.92 ms -- three dependent passes over the row with block-wide reductions in between cost more inside every CTA than
     the hand-over to a separate one-CTA kernel.  So the answer is no unless ``MFQ_ACT_GEMV=1`` asks for it; the kernel
     stays for shapes and parts where the balance differs."""
-    from ..config import current
-    return current().act_gemv and act_gemv_ok(m, n, k) and n // 16 <= ACT_GEMV_MAX_CTAS
+    return config.current().act_gemv and act_gemv_ok(m, n, k) and n // 16 <= ACT_GEMV_MAX_CTAS
 
 
 def fp8_gemv_act(x: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, mode: int, *, norm_w: torch.Tensor | None = None,
@@ -244,8 +242,8 @@ def fp8_gemv_act(x: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, mode
 
 def quant_rows(x: torch.Tensor, *, q_out=None, scale_out=None):
     m, k = x.shape
-    q_out = torch.empty((m, k), dtype=FP8, device=x.device) if q_out is None else q_out
-    scale_out = torch.empty(m, dtype=torch.float32, device=x.device) if scale_out is None else scale_out
+    q_out = x.new_empty((m, k), dtype=FP8) if q_out is None else q_out
+    scale_out = x.new_empty(m, dtype=torch.float32) if scale_out is None else scale_out
     check(lib().mfq_quant_rows(ptr(x), ptr(q_out), ptr(scale_out), m, k, x.stride(0), 0, stream_ptr()), "quant_rows")
     return q_out, scale_out
 
@@ -254,8 +252,8 @@ def silu_mul_quant(gate_up: torch.Tensor, *, q_out=None, scale_out=None):
     """``[M, 2I]`` (gate | up) -> fp8 ``silu(gate) * up`` rows ``[M, I]`` + per-row multiplier."""
     m, two_i = gate_up.shape
     i = two_i // 2
-    q_out = torch.empty((m, i), dtype=FP8, device=gate_up.device) if q_out is None else q_out
-    scale_out = torch.empty(m, dtype=torch.float32, device=gate_up.device) if scale_out is None else scale_out
+    q_out = gate_up.new_empty((m, i), dtype=FP8) if q_out is None else q_out
+    scale_out = gate_up.new_empty(m, dtype=torch.float32) if scale_out is None else scale_out
     check(lib().mfq_quant_rows(ptr(gate_up), ptr(q_out), ptr(scale_out), m, i, gate_up.stride(0), 1, stream_ptr()),
           "silu_mul_quant")
     return q_out, scale_out
@@ -289,7 +287,7 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, slots: torch.Tenso
     ``q_norm`` / ``k_norm`` (``[D]`` fp32): per-head RMSNorm before the rotation; ``rot`` < D: partial rotary.
     Rows of ``qkv`` may be wider than the q|k|v heads (e.g. an output gate after v); the row stride is honoured."""
     t = qkv.shape[0]
-    q_out = torch.empty((t, n_q, head_dim), dtype=torch.bfloat16, device=qkv.device) if q_out is None else q_out
+    q_out = qkv.new_empty((t, n_q, head_dim), dtype=torch.bfloat16) if q_out is None else q_out
     if scaling is not None and (scaling.factor != 1.0 or scaling.mscale != 1.0):
         rc = lib().mfq_rope_kv_write_yarn(ptr(qkv), ptr(positions), ptr(slots), ptr(q_out), ptr(kv.k), ptr(kv.v), ptr(kv.k_scale),
                                           ptr(kv.v_scale), t, n_q, n_kv, head_dim, kv.page_size, rot or head_dim, float(theta),
@@ -391,6 +389,8 @@ def kv_gather_dequant(kv, block_row: torch.Tensor, tokens: int):
 def attn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens: list[int], sm_scale: float) -> torch.Tensor:
     """Causal self-attention over a packed chunk (each sequence attends to itself)."""
     out = torch.empty_like(q)
+    if len(cu_seqlens) == 2 and cu_seqlens[0] == 0 and cu_seqlens[1] == q.shape[0] == k.shape[0] == v.shape[0]:  # no slices to make
+        return attn_prefill_bf16(q, k, v, sm_scale, out=out)
     for i in range(len(cu_seqlens) - 1):
         a, b = cu_seqlens[i], cu_seqlens[i + 1]
         attn_prefill_bf16(q[a:b], k[a:b], v[a:b], sm_scale, out=out[a:b])
