@@ -32,7 +32,9 @@ constexpr int kDnABytes = kDnTileN * kDnBlockK * 2;
 
 template <int BT>
 struct DenseCfg {
-  static constexpr int kStages = 4;
+  // As deep as two CTAs per SM have room for: a stream of weights takes its rate from the bytes in flight.  16 tokens, 4 stages | 6:
+  // 4096 x 4096 11.8 | 10.5 us, 4096 x 14336 25.5 | 23.0, 28672 x 4096 38.8 | 37.7; 32 tokens, 4 | 5: 11.4 | 11.0, 25.7 | 24.0, 39.6 | 38.2.
+  static constexpr int kStages = BT == 16 ? 6 : BT == 32 ? 5 : 4;
   static constexpr int kXBytes = BT * kDnBlockK * 2;
   static constexpr int kStageBytes = kDnABytes + kXBytes;
   static constexpr int kTmemCols = BT < 32 ? 32 : BT;
@@ -266,11 +268,14 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int NT>
+// kDeep: for grids that leave SMs idle, where a CTA's time is the latency of its loads: 16 K blocks of a warp's weights are requested at
+// once, ahead of the kernel before, and 8 blocks of the tokens at a time after it.
+template <int NT, bool kDeep>
 __global__ void __launch_bounds__(256)
 dense_gemv_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x, int ldx, const DenseParams p) {
   pdl_trigger();
-  constexpr int kBatch = 4;  // K blocks whose weights are requested before the first MMA of the batch
+  constexpr int kBatch = kDeep ? 16 : 4;  // K blocks whose weights are requested before the first MMA of the batch
+  constexpr int kX = kDeep ? 8 : 1;       // ... and whose tokens are
   __shared__ float red[8][16][8 * NT + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   if (p.tiles) pdl_wait();
@@ -302,13 +307,22 @@ dense_gemv_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __re
   for (int c0 = warp; c0 < blocks; c0 += 8 * kBatch) {
     if (c0 != warp) fetch(c0);
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      const int k = (c0 + j * 8) * 32 + t4 * 8;
+    for (int j0 = 0; j0 < kBatch; j0 += kX) {
+      if (kDeep && c0 + j0 * 8 >= blocks) break;
+      uint4 xv[kX][NT];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const uint4 xv = (k < K && nt * 8 + g < rows) ? *reinterpret_cast<const uint4*>(xr[nt] + k) : zero;
-        mma_bf16_16816(acc[nt], a[j].x, b[j].x, a[j].y, b[j].y, xv.x, xv.y);
-        mma_bf16_16816(acc[nt], a[j].z, b[j].z, a[j].w, b[j].w, xv.z, xv.w);
+      for (int j = 0; j < kX; ++j) {
+        const int k = (c0 + (j0 + j) * 8) * 32 + t4 * 8;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) xv[j][nt] = (k < K && nt * 8 + g < rows) ? *reinterpret_cast<const uint4*>(xr[nt] + k) : zero;
+      }
+#pragma unroll
+      for (int j = 0; j < kX; ++j) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          mma_bf16_16816(acc[nt], a[j0 + j].x, b[j0 + j].x, a[j0 + j].y, b[j0 + j].y, xv[j][nt].x, xv[j][nt].y);
+          mma_bf16_16816(acc[nt], a[j0 + j].z, b[j0 + j].z, a[j0 + j].w, b[j0 + j].w, xv[j][nt].z, xv[j][nt].w);
+        }
       }
     }
   }
@@ -337,18 +351,27 @@ dense_gemv_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __re
   }
 }
 
-template <int NT>
-static int launch_dense_gemv(const void* w, const void* x, int ldx, const DenseParams& p, int entries, cudaStream_t stream) {
+template <int NT, bool kDeep>
+static int launch_dense_gemv_as(const void* w, const void* x, int ldx, const DenseParams& p, int entries, cudaStream_t stream) {
   // The loads in flight live in L1.  On an SM that a kernel with much shared memory leaves behind, L1 would stay small and
   // the stream slow, so this kernel asks for a small shared-memory carve-out.
   static bool set = false;
   if (!set) {
-    if (cudaFuncSetAttribute(dense_gemv_kernel<NT>, cudaFuncAttributePreferredSharedMemoryCarveout, 15 * NT) != cudaSuccess) return -6;
+    if (cudaFuncSetAttribute(dense_gemv_kernel<NT, kDeep>, cudaFuncAttributePreferredSharedMemoryCarveout, 15 * NT) != cudaSuccess) return -6;
     set = true;
   }
-  launch_kernel(dense_gemv_kernel<NT>, dim3(p.N / 16 * p.groups, p.tiles ? entries : 1), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(w),
+  launch_kernel(dense_gemv_kernel<NT, kDeep>, dim3(p.N / 16 * p.groups, p.tiles ? entries : 1), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(w),
                 static_cast<const __nv_bfloat16*>(x), ldx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
+}
+// Up to a CTA per SM, and two batches of the shallow form at least.  Shallow | deep on a B200 (cold weights): 16 x 256 x 4096 10.4 | 8.3 us,
+// 1 x 256 x 4096 6.3 | 4.1, 16 x 2048 x 4096 12.0 | 9.8, 1 x 2048 x 2048 4.2 | 3.8, 16 x 512 x 14336 39.4 | 30.3; but 16 x 256 x 1024 3.2 | 3.7, and
+// with several CTAs per SM 8 x 6144 x 4096 11.9 | 17.4.
+constexpr int kGemvDeepCtas = 148, kGemvDeepK = 2048;
+template <int NT>
+static int launch_dense_gemv(const void* w, const void* x, int ldx, const DenseParams& p, int entries, cudaStream_t stream) {
+  const bool deep = !p.tiles && p.N / 16 * p.groups <= kGemvDeepCtas && p.K >= kGemvDeepK;
+  return deep ? launch_dense_gemv_as<NT, true>(w, x, ldx, p, entries, stream) : launch_dense_gemv_as<NT, false>(w, x, ldx, p, entries, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -52,6 +52,20 @@ def test_products(m, n, k, dtype):
     check_status()
 
 
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(16, 2048), (256, 4096), (2368, 2056), (48, 4104), (32, 14336)])
+def test_streaming_product_of_few_rows_of_weights(m, n, k):
+    """Grids up to a CTA per SM request sixteen K blocks at once: the remainders of a batch, and the bits of the form that a larger grid
+    takes (the same rows of weights, repeated until the grid is larger)."""
+    from mfq_b200.ops import dense
+    x, w = rnd(m, k), rnd(n, k, scale=k ** -0.5)
+    got = dense.DenseLinear(w)(x, fp32=True, tile=0)
+    close(got, (x.double() @ w.double().T).cpu(), 2e-5)
+    many = w.repeat(149 * 16 // n + 1, 1)
+    assert many.shape[0] // 16 > 148 and torch.equal(dense.DenseLinear(many)(x, fp32=True, tile=0)[:, :n], got)
+    check_status()
+
+
 @pytest.mark.parametrize("tile", [16, 32, 64, 128, 256])
 @pytest.mark.parametrize("splits", [1, 2, 3, 5, 8])
 def test_every_tile_and_split(tile, splits):
