@@ -91,6 +91,71 @@ def test_route_plan_of_many_routes(t, k, e, lo, hi):
     assert plan.totals.tolist() == [int(offsets[-1]), len(want)]
 
 
+@pytest.mark.parametrize("t,k,e,lo,hi", [(250, 10, 512, 0, 512), (251, 10, 512, 0, 512), (2501, 1, 3, 0, 3), (8191, 5, 512, 100, 356)])
+def test_route_plan_shared_by_a_cluster(t, k, e, lo, hi):
+    """Around the number of routes from which eight CTAs share the plan, and shares that do not divide: the invariants of the test before."""
+    test_route_plan_of_many_routes(t, k, e, lo, hi)
+
+
+@pytest.mark.parametrize("e,k", [(1, 1), (5, 5), (128, 16), (129, 3), (256, 8), (300, 10), (512, 10)])
+def test_selection_of_ties_and_values_that_cannot_be_chosen(e, k):
+    """Largest first, the lowest index among equals; NaN and minus infinity never, and a token without enough others gets no more."""
+    require_gpu_lib()
+    g = torch.Generator(device="cuda").manual_seed(e)
+    t, none = 37, 0x7FFFFFFF
+    logits = (torch.randn((t, e), generator=g, device="cuda") * 4).round() / 4  # a quarter apart: equal or well apart after the exponential
+    logits[3] = 1.5
+    logits[4] = float("nan")
+    bias = torch.zeros(e, device="cuda")
+    bias[::3] = float("-inf")
+    for b in (None, bias):
+        for sig in (0, 1):
+            ids = torch.full((t, k), -5, dtype=torch.int32, device="cuda")
+            w, scores = torch.empty((t, k), device="cuda"), torch.empty((t, e), device="cuda")
+            rc = moe._lib().mfq_moe_router_select(logits.data_ptr(), b.data_ptr() if b is not None else None, ids.data_ptr(), w.data_ptr(), scores.data_ptr(),
+                                                  t, 64, e, k, sig, 0, 1.0, 1, 1, moe.stream_ptr())
+            assert rc == 0
+            for row in range(t):
+                left = [i for i in range(e) if row != 4 and (b is None or i % 3)]
+                want = sorted(left, key=lambda i: (-float(logits[row, i]), i))[:k] if row in (0, 3, 4, t - 1) else None
+                if want is None:
+                    continue
+                assert ids[row].tolist() == want + [none] * (k - len(want)), (row, sig)
+                assert torch.equal(w[row, : len(want)], scores[row, want]) and not w[row, len(want):].any()
+    check_status()
+
+
+@pytest.mark.parametrize("rows", [1, 1499, 1500, 1503])
+@pytest.mark.parametrize("h", [16, 528, 2048])
+def test_gathered_rows(rows, h):
+    """Around the number of rows from which a warp takes four; the rows that no route fills stay as they are."""
+    require_gpu_lib()
+    xq, xs = torch.randint(0, 127, (97, h), device="cuda", dtype=torch.uint8).view(torch.float8_e4m3fn), torch.rand(97, device="cuda")
+    token = torch.randint(0, 97, (rows,), device="cuda", dtype=torch.int32)
+    live = rows - rows // 5
+    plan = moe.RoutePlan(None, None, token, None, torch.tensor([live, 0], dtype=torch.int32, device="cuda"), 16, rows, 1)
+    q, s = moe.gather_rows(xq, xs, plan)
+    assert torch.equal(q.view(torch.uint8)[:live], xq.view(torch.uint8)[token[:live].long()]) and torch.equal(s[:live], xs[token[:live].long()])
+    check_status()
+
+
+@pytest.mark.parametrize("k", [1, 4, 5, 6, 10, 16])
+def test_combined_rows(k):
+    """Contributions in batches of five and what is left of one, some of other ranks: the sums in slot order, as fp32 gives them."""
+    require_gpu_lib()
+    t, h = 33, 264
+    y, base = torch.randn(t * k, h, device="cuda").bfloat16(), torch.randn(t, h, device="cuda").bfloat16()
+    dest = torch.randperm(t * k, device="cuda").int().view(t, k)
+    dest[torch.rand(t, k, device="cuda") < 0.2] = -1
+    w = torch.rand(t, k, device="cuda")
+    plan = moe.RoutePlan(None, dest, None, None, None, 16, t * k, 1)
+    want = base.double()
+    for j in range(k):  # one rounding per addition, as a fused multiply-add has it
+        want = (want + (w[:, j, None].double() * y[dest[:, j].clamp_min(0).long()].double()) * (dest[:, j, None] >= 0)).float().double()
+    assert torch.equal(moe.combine(y, plan, w, base), want.bfloat16())
+    check_status()
+
+
 @pytest.mark.parametrize("sig,ng,tg,norm,scale", [(False, 1, 1, True, 1.0), (True, 1, 1, True, 2.5), (True, 8, 4, True, 2.5), (False, 1, 1, False, 1.0)])
 def test_router_of_a_prompt_chooses_what_the_routers_own_kernels_do(sig, ng, tg, norm, scale, monkeypatch):
     """Beyond 64 tokens logits come from the dense product -- or, where its library is not there, from the router's own kernels."""
@@ -135,3 +200,19 @@ def test_grouped_product_over_several_tiles_per_cta(tile, k):
             rng = slice(at, at + c)
             assert torch.equal(got[rng], fp8_gemm(x[rng], xs[rng], w[i], ws[i], splits=1, token_tile=tile)), (i, c)
         at += c
+
+
+@pytest.mark.parametrize("tile", [32, 64])
+def test_grouped_product_into_an_unaligned_output(tile):
+    """Results leave in 16-byte stores only where the output allows them."""
+    require_gpu_lib()
+    rows, k, n = 70, 256, 256
+    fp8 = lambda *s: (torch.randn(s, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
+    x, w, xs, ws = fp8(rows, k), fp8(2, n, k), torch.rand(rows, device="cuda"), torch.rand((2, n // 128, k // 128), device="cuda")
+    plan = moe.plan_routes((torch.arange(rows, device="cuda") >= 41).int()[:, None], 0, 2, token_tile=tile)
+    want = moe.fp8_gemm_grouped(x, xs, w, ws, plan)
+    out = torch.zeros(rows * n + 2, device="cuda", dtype=torch.bfloat16)
+    rc = moe._lib().mfq_fp8_gemm_grouped(w.data_ptr(), ws.data_ptr(), x.data_ptr(), xs.data_ptr(), out[1:].data_ptr(), moe.Workspace.get(x.device).status.data_ptr(),
+                                         rows, n, k, 2, plan.tile_map.data_ptr(), plan.offsets.data_ptr(), plan.tile_map.shape[0], tile, moe.stream_ptr())
+    assert rc == 0 and torch.equal(out[1:-1].view(rows, n), want) and not out[0] and not out[-1]
+    check_status()

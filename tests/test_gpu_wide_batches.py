@@ -160,6 +160,13 @@ def test_row_quantization_in_one_pass(m, k):
     check_status()
 
 
+@pytest.mark.parametrize("m", [255, 256, 4999, 5001])
+@pytest.mark.parametrize("k", [8, 248, 264, 512, 520, 1024])
+def test_quantization_of_short_rows(m, k):
+    """A warp or a block per row: the codes of plain fp32 arithmetic, and of a single row."""
+    test_row_quantization_in_one_pass(m, k)
+
+
 @pytest.mark.parametrize("rot", [None, 64])
 @pytest.mark.parametrize("d", [64, 128, 256])
 def test_rotation_of_many_tokens_gives_the_bits_of_few(d, rot):
