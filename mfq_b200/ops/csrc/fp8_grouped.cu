@@ -5,8 +5,11 @@
 // down projection of that layer (2048 x 512) spent 8 us per CTA on four K blocks; here one CTA per SM walks the tiles: the loads of the
 // tiles to come fill the ring while the epilogue warps still fold and store, nothing but the first tile pays for set-up, and what a tile
 // needs from memory to begin (its place, its weight multipliers) is fetched during the one before.
-// 3000 tokens, 512 experts of 3 x 2048 x 512, top 10 on a B200, both products: 421 us (a CTA per tile: 577; the weights alone take 242 at
-// the copy rate); 32 tokens: 129 us (161; 110).
+// What bounds a tile of few K blocks is its end and the next one's beginning: tiles of 32 tokens and more leave through shared memory in
+// 16-byte stores (a thread's own columns are 2 bytes every N), and entries, row ranges and multipliers are requested up to two tiles ahead.
+// 512 experts of 3 x 2048 x 512, top 10 on a B200, gate/up + down (before: 2-byte stores, entries one tile ahead): 3000 tokens 217 + 193 ->
+// 206 + 159 us (what they read and write takes 184 + 104 at the copy rate), 4096 250 + 261 -> 224 + 169, 1500 202 + 178 -> 188 + 144; 200 (tiles
+// of 16, which store their columns themselves: 102 through shared memory) 158 + 90 -> 156 + 91, 32 77 + 46 -> 77 + 44.
 //
 // Roles: warp 0 = TMA, warp 1 = TMEM owner + MMA issuer, warps 2.. = epilogue (TMEM lane quarter = warp % 4; tiles of 64 and 128 tokens
 // use two warps per quarter, each taking half of the token columns).  Per 128-wide K block a fresh TMEM accumulator, folded with the
@@ -27,7 +30,11 @@ struct GroupedCfg {
   static constexpr int kEpiWarps = BT >= 64 ? 8 : 4;
   static constexpr int kCols = BT / (kEpiWarps / 4);  // token columns per epilogue thread
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+  static constexpr bool kTurned = BT >= 32;           // whether results leave through shared memory
+  static constexpr int kGroups = kEpiWarps / 4;       // of four warps: 128 weight rows x kCols tokens
+  static constexpr int kTurnBytes = kCols * kTileN * 2;  // their results on the way out
+  static constexpr int kTurnAt = kStages * kStageBytes, kBarsAt = kTurnAt + (kTurned ? kGroups * kTurnBytes : 0);
+  static constexpr int kSmemBytes = kBarsAt + 1024 + 256;
 };
 
 struct GroupedParams {
@@ -38,6 +45,7 @@ struct GroupedParams {
   const int* offsets;     // expert e owns rows [offsets[e], offsets[e + 1])
   int* status;
   int N, K, map_len;
+  int direct;             // output off a 16-byte boundary: plain stores
 };
 
 template <int BT>
@@ -46,17 +54,20 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   using Cfg = GroupedCfg<BT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(ring + Cfg::kStages * Cfg::kStageBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + Cfg::kBarsAt);
   uint64_t* empty = full + Cfg::kStages;
   uint64_t* acc_full = empty + Cfg::kStages;
   uint64_t* acc_empty = acc_full + Cfg::kAcc;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + Cfg::kAcc);
+  uint64_t* turn_full = acc_empty + Cfg::kAcc;  // [kGroups] the four warps' results are in shared memory
+  uint64_t* turn_free = turn_full + 2;          // ... and have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(turn_free + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < Cfg::kAcc; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], Cfg::kEpiWarps); }
+    for (int i = 0; i < Cfg::kGroups; ++i) { mbar_init(&turn_full[i], 4); mbar_init(&turn_free[i], 4); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -75,10 +86,10 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   // are dense: the first unused one ends the list.  The plan and the row multipliers are read by plain loads: under the programmatic
   // launch this grid began before they were written, so they are not constant for its life, as __ldg promises (weights are).
   const int n_tiles = p.N / kTileN, nkb = p.K / kBlockK, tiles = p.map_len * n_tiles, step = int(gridDim.x);
-  auto entry = [&](int tile) {  // the same for the whole warp
-    const int2 e = tile < tiles ? p.tile_map[tile / n_tiles] : make_int2(-1, 0);
-    return make_int2(__shfl_sync(0xffffffffu, e.x, 0), __shfl_sync(0xffffffffu, e.y, 0));
-  };
+  // What a tile starts from is requested two tiles ahead (its entry) and one (rows of its expert, multipliers), and looked at only then:
+  // a tile of four K blocks is 1500 cycles, a load 700.
+  auto request = [&](int tile) { return tile < tiles ? p.tile_map[tile / n_tiles] : make_int2(-1, 0); };
+  auto same = [&](int2 e) { return make_int2(__shfl_sync(0xffffffffu, e.x, 0), __shfl_sync(0xffffffffu, e.y, 0)); };  // for the whole warp
 
   if (warp == 0) {
     if (lane == 0) {
@@ -90,10 +101,10 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     int s = 0;
     uint32_t phase = 0;
     bool ok = true;
-    int2 e = entry(blockIdx.x);
+    int2 e = same(request(blockIdx.x)), next = same(request(blockIdx.x + step));
     int first = e.x >= 0 ? p.offsets[e.x] : 0;
     for (int tile = blockIdx.x; ok && e.x >= 0; tile += step) {
-      const int2 next = entry(tile + step);
+      const int2 after = request(tile + 2 * step);
       const int next_first = next.x >= 0 ? p.offsets[next.x] : 0;
       const int t0 = __shfl_sync(0xffffffffu, first, 0) + e.y * BT, n0 = tile % n_tiles * kTileN;
       for (int i = 0; i < nkb; ++i) {
@@ -104,6 +115,7 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
       }
       e = next;
+      next = same(after);
       first = next_first;
     }
   } else if (warp == 1) {
@@ -114,9 +126,9 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     int s = 0, buf = 0;
     uint32_t phase = 0, acc_phase = 1;  // the first pass over the accumulators finds them free
     bool ok = true;
-    int2 e = entry(blockIdx.x);
+    int2 e = same(request(blockIdx.x));
     for (int tile = blockIdx.x; ok && e.x >= 0; tile += step) {
-      const int2 next = entry(tile + step);
+      const int2 next = request(tile + step);
       for (int i = 0; i < nkb; ++i) {
         ok = mbar_wait_warp(&acc_empty[buf], acc_phase, abort_flag, p.status, kStatusTimeoutMma) &&
              mbar_wait_warp(&full[s], phase, abort_flag, p.status, kStatusTimeoutMma);
@@ -127,34 +139,52 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
         if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
       }
-      e = next;
+      e = same(next);
     }
   } else {
     // ----- epilogue warps: thread owns output feature n0 + q*32 + lane and CW token columns from col0 -----
     constexpr int CW = Cfg::kCols, kChunk = CW < 32 ? CW : 32, kChunks = CW / kChunk;
-    const int q = warp & 3, col0 = ((warp - 2) >> 2) * CW;
+    const int q = warp & 3, group = (warp - 2) >> 2, col0 = group * CW;
+    const uint32_t turn = smem_u32(ring) + Cfg::kTurnAt + group * Cfg::kTurnBytes;
+    const bool odd = lane & 1;
+    const uint32_t chunk = q * 4 + (lane >> 3), within = ((lane >> 1) & 3) * 4;
+    const int place = ((warp - 2) & 3) * 32 + lane;  // of the group's 128 threads
+    uint32_t turn_phase = 0;
     const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + col0;
     int buf = 0;
     uint32_t phase = 0;
     bool ok = true, ready = false;
-    // what a tile starts from, fetched while the tile before is stored: row range of its expert and 32 multipliers, one per lane
-    int2 e = entry(blockIdx.x);
-    int lo = 0, hi = 0;
-    float ws = 0.f;
-    auto fetch = [&](int tile, int2 at) {
-      if (at.x < 0) return;
-      lo = p.offsets[at.x];
-      hi = p.offsets[at.x + 1];
-      if (lane < nkb) ws = __ldg(p.w_scale + (size_t(at.x) * n_tiles + tile % n_tiles) * nkb + lane);
+    // row range of a tile's expert, 32 weight multipliers and the row multipliers of this warp's columns, one per lane
+    struct Start {
+      int lo, hi;
+      float ws;
     };
-    fetch(blockIdx.x, e);
-    for (int tile = blockIdx.x; ok && e.x >= 0; tile += step) {
-      const int2 next = entry(tile + step);
-      const int t0 = lo + e.y * BT, tl = min(BT, hi - t0), n = tile % n_tiles * kTileN + q * 32 + lane;
-      const float* wsc = p.w_scale + (size_t(e.x) * n_tiles + tile % n_tiles) * nkb;
-      float xs[(CW + 31) / 32];  // row multipliers of this warp's columns, one per lane
+    auto fetch = [&](int tile, int2 at) {
+      Start r = {0, 0, 0.f};
+      if (at.x < 0) return r;
+      r.lo = p.offsets[at.x];
+      r.hi = p.offsets[at.x + 1];
+      if (lane < nkb) r.ws = __ldg(p.w_scale + (size_t(at.x) * n_tiles + tile % n_tiles) * nkb + lane);
+      return r;
+    };
+    constexpr int kXs = (CW + 31) / 32;
+    float xs[kXs];
+    auto fetch_rows = [&](int2 at, const Start& r) {
 #pragma unroll
-      for (int j = 0; j < (CW + 31) / 32; ++j) xs[j] = col0 + j * 32 + lane < tl ? p.x_scale[t0 + col0 + j * 32 + lane] : 0.f;
+      for (int j = 0; j < kXs; ++j) {
+        const int row = r.lo + at.y * BT + col0 + j * 32 + lane;
+        xs[j] = at.x >= 0 && j * 32 + lane < CW && row < r.hi ? p.x_scale[row] : 0.f;
+      }
+    };
+    int2 e = same(request(blockIdx.x)), next = same(request(blockIdx.x + step));
+    Start now = fetch(blockIdx.x, e);
+    fetch_rows(e, now);
+    for (int tile = blockIdx.x; ok && e.x >= 0; tile += step) {
+      const int2 after = request(tile + 2 * step);
+      const Start then = fetch(tile + step, next);
+      const int t0 = now.lo + e.y * BT, tl = min(BT, now.hi - t0), n = tile % n_tiles * kTileN + q * 32 + lane;
+      const float* wsc = p.w_scale + (size_t(e.x) * n_tiles + tile % n_tiles) * nkb;
+      float ws = now.ws;
       float acc[CW];
 #pragma unroll
       for (int tt = 0; tt < CW; ++tt) acc[tt] = 0.f;
@@ -192,14 +222,50 @@ fp8_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         }
       }
       if (!ok) break;
-      fetch(tile + step, next);
-      __nv_bfloat16* dst = p.out + size_t(t0 + col0) * p.N + n;
 #pragma unroll
-      for (int tt = 0; tt < CW; ++tt) {
-        const float v = acc[tt] * __shfl_sync(0xffffffffu, xs[tt / 32], tt & 31);
-        if (col0 + tt < tl) dst[size_t(tt) * p.N] = __float2bfloat16(v);
+      for (int tt = 0; tt < CW; ++tt) acc[tt] *= __shfl_sync(0xffffffffu, xs[tt / 32], tt & 31);
+      fetch_rows(next, then);
+      if (!Cfg::kTurned || p.direct) {
+        __nv_bfloat16* dst = p.out + size_t(t0 + col0) * p.N + n;
+#pragma unroll
+        for (int tt = 0; tt < CW; ++tt)
+          if (col0 + tt < tl) dst[size_t(tt) * p.N] = __float2bfloat16(acc[tt]);
+      } else {
+        // Through shared memory, 256 swizzled bytes of 128 weight rows per token.  A thread has one weight row of tokens t and t + 4; neighbours
+        // trade halves, so that an even lane has its pair of rows of token t, an odd one of token t + 4, whose chunks of 16 bytes the swizzle
+        // puts beside those of token t.  Out in 16-byte stores, a token's 256 bytes by half a warp.
+        ok = mbar_wait_warp(&turn_free[group], turn_phase ^ 1u, abort_flag, p.status, kStatusTimeoutEpilogue);
+        if (!ok) break;
+#pragma unroll
+        for (int tt = 0; tt < CW; tt += 8) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat162 two = __floats2bfloat162_rn(acc[tt + j], acc[tt + j + 4]);
+            const uint32_t own = *reinterpret_cast<const uint32_t*>(&two), other = __shfl_xor_sync(0xffffffffu, own, 1);
+            const uint32_t row = j + (odd ? 4 : 0);  // of the eight tokens
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(turn + (tt + row) * 256 + ((chunk ^ row) << 4) + within), "r"(__byte_perm(own, other, odd ? 0x3276 : 0x5410))
+                         : "memory");
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&turn_full[group]);
+        ok = mbar_wait_warp(&turn_full[group], turn_phase, abort_flag, p.status, kStatusTimeoutEpilogue);
+        if (!ok) break;
+        __nv_bfloat16* dst = p.out + size_t(t0 + col0) * p.N + tile % n_tiles * kTileN;
+#pragma unroll
+        for (int i = 0; i < CW * 16 / 128; ++i) {
+          const int tt = (i * 128 + place) >> 4, c = place & 15;
+          uint4 v;
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(turn + tt * 256 + ((c ^ (tt & 7)) << 4)));
+          if (col0 + tt < tl) *reinterpret_cast<uint4*>(dst + size_t(tt) * p.N + c * 8) = v;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&turn_free[group]);
+        turn_phase ^= 1u;
       }
       e = next;
+      next = same(after);
+      now = then;
     }
   }
 
@@ -239,7 +305,7 @@ extern "C" int mfq_fp8_gemm_grouped(const void* w, const float* w_scale, const v
                                     int* status, int rows, int N, int K, int experts, const void* tile_map,
                                     const int* expert_offsets, int map_len, int token_tile, cudaStream_t stream) {
   if (K % 128 != 0 || rows <= 0 || N <= 0 || experts <= 0 || map_len <= 0 || N % 128 != 0) return -1;
-  const mfq::GroupedParams p{w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const int2*>(tile_map), expert_offsets, status, N, K, map_len};
+  const mfq::GroupedParams p{w_scale, x_scale, static_cast<__nv_bfloat16*>(out), static_cast<const int2*>(tile_map), expert_offsets, status, N, K, map_len, (reinterpret_cast<uintptr_t>(out) & 15) != 0};
   switch (token_tile) {
     case 16: return mfq::launch_grouped<16>(p, w, x, rows, experts, stream);
     case 32: return mfq::launch_grouped<32>(p, w, x, rows, experts, stream);
