@@ -18,6 +18,8 @@
 //
 // The reference multiplies block-FP8 weights by decoding them to fp16 for wmma or cuBLAS
 // (mfq/kernels/cuda/fp8_sq.cu:42-56,564-592); there the FP8 tensor-core path does not exist.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace mfq {
@@ -37,9 +39,11 @@ struct GemmCfg {
   static constexpr int kCols = BT / (kEpiWarps / 4);   // token columns per epilogue thread
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kXsBytes = kEpiWarps * kCols * 4;  // per-warp copy of the row multipliers of its token columns
-  static constexpr int kWsMax = 256;                      // weight-block multipliers of a CTA's K range kept in smem, per warp
-  static constexpr int kWsBytes = kEpiWarps * kWsMax * 4;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kXsBytes + kWsBytes;
+  static constexpr int kWsMax = 256;                      // weight-block multipliers of a CTA's K range kept in smem
+  static constexpr int kWsBytes = kWsMax * 4;
+  static constexpr int kResBytes = (BT + 1) / 2 * kTileN * 2;  // splits that meet in a cluster: residual of the columns that this CTA finishes
+  static constexpr int kFixedBytes = 1024 /*align slack*/ + 256 /*barriers*/ + kXsBytes + kWsBytes + kResBytes;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kFixedBytes;
 };
 
 // Cross-rank all-reduce context of the fused epilogue (world == 1: disabled).
@@ -88,6 +92,8 @@ struct GemmParams {
   // memory instead of a global scratch buffer with an arrival counter, and every CTA of the cluster finishes a share of
   // the token columns instead of the last arriver finishing all of them.
   int cluster_reduce = 0;
+  int wide_out = 0;    // whole tiles of rows, no residual, output on a 16-byte boundary: results leave through shared memory
+  int res_staged = 0;  // ... and its share of the residual is brought to shared memory under the main loop (16-byte rows)
 };
 
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
@@ -100,57 +106,98 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t cta)
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(cta));
   return r;
 }
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Cluster split-K: CTA r of S finishes the token columns c = r (mod S).  Every CTA lays its partial sums out by destination in its ring,
+// which is free by then, and sends each destination its share with one bulk copy into that CTA's ring, once that CTA has said that its own
+// MMAs are done (peer_free); the copies complete on the destination's recv barrier.  The partials of a column are summed in split order
+// whichever CTA does it, so results do not depend on scheduling.  The first
+// copy of every CTA goes to another destination (all to CTA 0 first: 128 x 1000 x 2048 in eight splits 8.4 us, so 7.3).  Against a barrier of
+// the cluster, loads from its shared memory, of residuals and multipliers, and another barrier before anybody might leave: 64 x 4096 x 4096 in
+// four splits 10.5 -> 9.5 us (in a decode step 9.8 -> 6.9 from its inputs to its end), 64 x 6144 x 4096 without residual 11.7 -> 10.1,
+// 128 x 4096 x 4096 13.1 -> 11.5.
+struct MeetBars {
+  uint64_t *peer_free, *recv, *staged;
+};
+// Columns of CTA r among the first `tl`.
+template <int S>
+__device__ __forceinline__ int meet_columns(int tl, int r) { return tl > r ? (tl - r + S - 1) / S : 0; }
+
+// Epilogue warps.  False: a wait ran out.
+template <int BT, int S>
+__device__ __forceinline__ bool cluster_exchange(const float (&acc)[GemmCfg<BT>::kCols], uint8_t* tiles, int me, int tl, const MeetBars& bars,
+                                                 volatile int* abort_flag, int* status) {
+  using Cfg = GemmCfg<BT>;
+  constexpr int kPer = (BT + S - 1) / S, kColBytes = kTileN * 4;
+  const int e = int(threadIdx.x) - 64, lane = threadIdx.x & 31, row = (int(threadIdx.x) >> 5 & 3) * 32 + lane;  // of the accumulators
+  float* stage = reinterpret_cast<float*>(tiles);
+  auto lay = [&](auto first) {
+#pragma unroll
+    for (int tt = 0; tt < Cfg::kCols; ++tt) {
+      const int c = decltype(first)::value + tt;
+      stage[(c % S * kPer + c / S) * kTileN + row] = acc[tt];
+    }
+  };
+  if (e < 128) lay(std::integral_constant<int, 0>());
+  else lay(std::integral_constant<int, Cfg::kCols>());
+  asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's part of the residual
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bars.staged);
+  bool ok = mbar_wait_warp(bars.staged, 0, abort_flag, status, kStatusTimeoutEpilogue);
+  const int mine = meet_columns<S>(tl, me);
+  if (ok && e < 32) {
+    ok = mbar_wait_warp(bars.peer_free, 0, abort_flag, status, kStatusTimeoutEpilogue);
+    if (ok) {
+      if (lane == me && mine) mbar_expect_tx(bars.recv, uint32_t((S - 1) * mine * kColBytes));
+      const int to = (me + 1 + lane) % S, n = meet_columns<S>(tl, to);  // not all to one destination first
+      if (lane < S - 1 && n) {
+        const uint32_t src = smem_u32(tiles) + to * kPer * kColBytes;
+        const uint32_t slot = map_to_cta(smem_u32(tiles) + (S + (me < to ? me : me - 1)) * kPer * kColBytes, to);
+        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(slot), "r"(src), "r"(uint32_t(n * kColBytes)), "r"(map_to_cta(smem_u32(bars.recv), to))
+                     : "memory");
+      }
+    }
+    __syncwarp();
+  }
+  if (ok && mine) ok = mbar_wait_warp(bars.recv, 0, abort_flag, status, kStatusTimeoutEpilogue);
+  return ok;
 }
 
-// Cluster split-K: CTA r of S finishes the token columns c = r (mod S); a thread owns one output row and every kSel-th
-// of those columns.  The S partials of a column are summed in split order whichever CTA does it, so results do not
-// depend on scheduling.  Every load of the thread -- S remote partials per column, multipliers, residual values -- leaves
-// before the first sum, so the round trips through the cluster's shared memory overlap (in groups of at most kLoads
-// partials to bound the registers).  Fetching multipliers and residuals ahead of the barrier measured slower: the values
-// have to be held across it, and the registers for that spill.
 template <int BT, int S>
-__device__ __forceinline__ void cluster_sum_columns(const GemmParams& p, const uint8_t* tiles, int t0, int tl, int n0) {
+__device__ __forceinline__ void cluster_finish(const GemmParams& p, const uint8_t* tiles, const float* xs, const __nv_bfloat16* res_smem, int me,
+                                               int t0, int tl, int n0) {
   using Cfg = GemmCfg<BT>;
-  constexpr int kSel = Cfg::kEpiWarps / 4;
-  constexpr int kLoads = 32;
-  constexpr int kGroup = kLoads / S < 1 ? 1 : kLoads / S;
-  const int e = int(threadIdx.x) - 64, row = e & 127, sel = e >> 7;
-  const int r = int(cluster_cta_rank());
-  const int n = n0 + row;
-  const uint32_t mine = smem_u32(tiles) + uint32_t(row) * 4u;
-  uint32_t base[S];
-#pragma unroll
-  for (int z = 0; z < S; ++z) base[z] = map_to_cta(mine, uint32_t(z));
+  constexpr int kPer = (BT + S - 1) / S, kSel = Cfg::kEpiWarps / 4, kEach = (kPer + kSel - 1) / kSel, kGroup = kEach < 32 / S ? kEach : 32 / S;
+  const int e = int(threadIdx.x) - 64, row = e & 127, sel = e >> 7, n = n0 + row;
+  const float* stage = reinterpret_cast<const float*>(tiles) + row;
+  const int mine = meet_columns<S>(tl, me);
   const unsigned short* rp = reinterpret_cast<const unsigned short*>(p.residual);
-  constexpr int step = S * kSel;
-  for (int c0 = r + S * sel; c0 < tl; c0 += step * kGroup) {
-    float v[kGroup][S], xm[kGroup];
+  for (int i0 = sel; i0 < mine; i0 += kSel * kGroup) {
+    float v[kGroup][S];
     unsigned short res[kGroup];
 #pragma unroll
     for (int j = 0; j < kGroup; ++j) {
-      const int c = c0 + j * step;
-      const bool live = c < tl;
-      xm[j] = live ? __ldg(p.x_scale + t0 + c) : 0.f;
-      res[j] = (live && rp && n < p.N) ? __ldcg(rp + size_t(t0 + c) * p.N + n) : (unsigned short)0;
+      const int i = min(i0 + j * kSel, mine - 1);
+      res[j] = 0;
+      if (rp) res[j] = p.res_staged ? reinterpret_cast<const unsigned short*>(res_smem)[i * kTileN + row]
+                                    : n < p.N ? __ldcg(rp + size_t(t0 + me + i * S) * p.N + n) : (unsigned short)0;
 #pragma unroll
-      for (int z = 0; z < S; ++z) v[j][z] = live ? ld_cluster_f32(base[z] + uint32_t(c) * (kTileN * 4u)) : 0.f;
+      for (int z = 0; z < S; ++z) v[j][z] = stage[((z == me ? me : S + (z < me ? z : z - 1)) * kPer + i) * kTileN];
     }
 #pragma unroll
     for (int j = 0; j < kGroup; ++j) {
-      const int c = c0 + j * step;
+      const int i = i0 + j * kSel, c = me + i * S;
       float sum = 0.f;
 #pragma unroll
       for (int z = 0; z < S; ++z) sum += v[j][z];  // split order
-      sum = sum * xm[j] + __uint_as_float(uint32_t(res[j]) << 16);
-      if (c < tl && n < p.N) p.out[size_t(t0 + c) * p.N + n] = __float2bfloat16(sum);
+      if (i < mine && n < p.N) {
+        sum = sum * xs[c / Cfg::kCols * 4 * Cfg::kCols + c % Cfg::kCols] + __uint_as_float(uint32_t(res[j]) << 16);
+        p.out[size_t(t0 + c) * p.N + n] = __float2bfloat16(sum);
+      }
     }
   }
 }
@@ -169,7 +216,9 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   uint64_t* acc_full = bars + 2 * stages;
   uint64_t* acc_empty = acc_full + Cfg::kAcc;
   uint64_t* epi_bar = acc_empty + Cfg::kAcc;  // four one-shot barriers among the epilogue warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_bar + 4);
+  uint64_t* peer_free = epi_bar + 4;  // cluster_reduce: the other splits' rings may be written
+  uint64_t* recv = peer_free + 1;     // ... and their partial sums are here
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(recv + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   float* xs_smem = reinterpret_cast<float*>(tiles + stages * Cfg::kStageBytes + 256);
@@ -262,6 +311,10 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     for (int i = 0; i < stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < Cfg::kAcc; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], Cfg::kEpiWarps); }
     for (int i = 0; i < 4; ++i) mbar_init(&epi_bar[i], Cfg::kEpiWarps);
+    if (p.cluster_reduce) {
+      mbar_init(peer_free, gridDim.z - 1);
+      mbar_init(recv, 1);
+    }
     *abort_flag = 0;
     *last_flag = 0;
     mbar_fence_init();
@@ -270,10 +323,19 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  // The weight-block multipliers of this CTA's K range, under the kernel before: a global load per K block would sit, exposed, on
+  // the chain wait -> TMEM load -> FMA that every block goes through (it was the longest link of that chain).
+  const float* wsc = p.w_scale + size_t(n_tile) * kb_total;
+  float* ws_smem = xs_smem + Cfg::kEpiWarps * Cfg::kCols;
+  __nv_bfloat16* res_smem = reinterpret_cast<__nv_bfloat16*>(ws_smem + Cfg::kWsMax);
+  const bool ws_cached = nkb <= Cfg::kWsMax;
+  if (ws_cached)
+    for (int j = int(threadIdx.x) - 64; j >= 0 && j < nkb; j += Cfg::kThreads - 64) ws_smem[j] = __ldg(wsc + kb0 + j);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  if (p.cluster_reduce) cluster_arrive();  // this CTA's barriers exist
   // Weights are never written by a kernel of the same stream, so the plain GEMM starts the weight tiles of its first
   // ring pass BEFORE it waits for its predecessor: under programmatic dependent launch this CTA is resident while the
   // short kernel that produces its activations (a norm, a quantization) still runs, and the weight stream -- all of it
@@ -336,6 +398,11 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       tma_load_stage(a, a + kTileN * kBlockK, &tmap_w, xmap, full_addr + s * 8, Cfg::kStageBytes, fresh, (kb0 + i) * kBlockK, n0, -1, t0, (kb0 + i) * kBlockK);
       if (++s == stages) { s = 0; ring_phase ^= 1u; }
     }
+    if (p.cluster_reduce) {
+      __syncwarp();
+      cluster_wait();
+      cluster_arrive_relaxed();
+    }
   } else if (warp == 1) {
     // This warp's loop is the pace of a weight-streaming CTA whose tiles are already in shared memory, so it carries no work that
     // can be left out: descriptors advance by a constant per stage (the ring is contiguous and stays inside the 14-bit address
@@ -357,6 +424,17 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       if (++s == stages) { s = 0; ring_phase ^= 1u; }
       if (++buf == Cfg::kAcc) { buf = 0; acc_phase ^= 1u; }
     }
+    if (p.cluster_reduce) {
+      cluster_wait();  // the other CTAs' barriers exist
+      const int last = (nkb - 1) % Cfg::kAcc;
+      if (mbar_wait_warp(&acc_full[last], uint32_t((nkb - 1) / Cfg::kAcc) & 1u, abort_flag, p.status, kStatusTimeoutMma)) {
+        const uint32_t me = cluster_cta_rank();  // nothing reads or fills this ring any more
+        if (lane < int(gridDim.z) && lane != int(me))
+          asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(smem_u32(peer_free), lane)) : "memory");
+      }
+      __syncwarp();
+      cluster_arrive_relaxed();
+    }
   } else {
     // ----- epilogue warps: thread owns output feature n0 + q*32 + lane and CW token columns from col0 -----
     constexpr int CW = Cfg::kCols;
@@ -367,20 +445,22 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     float acc[CW];
 #pragma unroll
     for (int tt = 0; tt < CW; ++tt) acc[tt] = 0.f;
-    const float* wsc = p.w_scale + size_t(n_tile) * kb_total;
     // The token multipliers are fetched now, under the main loop, into this warp's own smem slice (no cross-warp
     // sync needed); at the end they cost a broadcast LDS instead of an exposed global load per column.  In gather
     // mode they only exist once the peers' flags arrived, so that mode reads them at the end.
     float* xs_w = xs_smem + (warp - 2) * CW;
+    const int splits = gridDim.z, me = p.cluster_reduce ? int(cluster_cta_rank()) : 0;
+    if (p.cluster_reduce && p.res_staged) {
+      const int mine = min(BT, row_end - t0) > me ? (min(BT, row_end - t0) - me + splits - 1) / splits : 0;
+      for (int j = int(threadIdx.x) - 64; j < mine * 16; j += 32 * Cfg::kEpiWarps) {
+        const int c = me + (j >> 4) * splits, off = (j & 15) * 8;
+        if (n0 + off < p.N)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(res_smem) + j * 16), "l"(p.residual + size_t(t0 + c) * p.N + n0 + off)
+                       : "memory");
+      }
+    }
     if (!gather) {
       for (int j = lane; j < CW; j += 32) xs_w[j] = (t0 + col0 + j < row_end) ? __ldg(p.x_scale + t0 + col0 + j) : 0.f;
-    }
-    // The weight-block multipliers of this CTA's K range, likewise: a global load per K block would sit, exposed, on
-    // the chain wait -> TMEM load -> FMA that every block goes through (it was the longest link of that chain).
-    float* ws_w = xs_smem + Cfg::kEpiWarps * CW + (warp - 2) * Cfg::kWsMax;
-    const bool ws_cached = nkb <= Cfg::kWsMax;
-    if (ws_cached) {
-      for (int j = lane; j < nkb; j += 32) ws_w[j] = __ldg(wsc + kb0 + j);
     }
     __syncwarp();
     constexpr int kChunk = CW < 32 ? CW : 32, kChunks = CW / kChunk;
@@ -392,7 +472,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       if (!ready) ok = mbar_wait_warp(&acc_full[buf], phase, abort_flag, p.status, kStatusTimeoutEpilogue);
       if (!ok) break;
       tc_fence_after();
-      const float s = ws_cached ? ws_w[i] : __ldg(wsc + kb0 + i);
+      const float s = ws_cached ? ws_smem[i] : __ldg(wsc + kb0 + i);
       const uint32_t taddr = lane_base + buf * BT;
       uint32_t r[2][kChunk];
       auto load_chunk = [&](int c) {
@@ -416,19 +496,34 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         for (int j = 0; j < kChunk; j += 2) fma2(acc[c * kChunk + j], acc[c * kChunk + j + 1], r[c & 1][j], r[c & 1][j + 1], s);
       }
     }
-    if (ok) {
+    if (p.cluster_reduce) {
+      const int tl = min(BT, row_end - t0);
+      const MeetBars bars{peer_free, recv, &epi_bar[0]};
+      __syncwarp();
+      cluster_wait();
+      // the split count as a constant: all partials of a thread's columns are loaded at once
+      auto meet = [&](auto count) {
+        constexpr int S = decltype(count)::value;
+        if (ok) ok = cluster_exchange<BT, S>(acc, tiles, me, tl, bars, abort_flag, p.status);
+        __syncwarp();
+        cluster_arrive_relaxed();  // nothing more comes from this warp; what it sent has arrived before its receivers say so
+        if (ok) cluster_finish<BT, S>(p, tiles, xs_smem, res_smem, me, t0, tl, n0);
+      };
+      switch (splits) {
+        case 2: meet(std::integral_constant<int, 2>()); break;
+        case 3: meet(std::integral_constant<int, 3>()); break;
+        case 4: meet(std::integral_constant<int, 4>()); break;
+        case 5: meet(std::integral_constant<int, 5>()); break;
+        case 6: meet(std::integral_constant<int, 6>()); break;
+        case 7: meet(std::integral_constant<int, 7>()); break;
+        default: meet(std::integral_constant<int, 8>()); break;
+      }
+    } else if (ok) {
       const int tl = min(BT, row_end - t0);
       const int tiles_nt = n_tiles_x * gridDim.y;
       const int tile_id = t_tile * n_tiles_x + n_tile;
       bool owner = true;  // this CTA holds the tile's complete local sum in `acc`
-      if (p.cluster_reduce) {
-        // The ring is free (the last MMA has completed, so every tile that was loaded has been read): the partial
-        // goes there as [token column][128 rows] fp32 and is summed after the cluster barrier below.
-        owner = false;
-        float* stage = reinterpret_cast<float*>(tiles);
-#pragma unroll
-        for (int tt = 0; tt < CW; ++tt) stage[(col0 + tt) * kTileN + row] = acc[tt];
-      } else if (gridDim.z > 1) {
+      if (gridDim.z > 1) {
         owner = false;
         float* mine = p.ws + (size_t(split) * tiles_nt + tile_id) * (BT * kTileN);
 #pragma unroll
@@ -578,7 +673,38 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           }
           }  // all-reduce
         }
-        if (owner && n < p.N) {
+        if (owner && p.wide_out) {
+          // Through the ring, which is free (the last MMA has completed), 256 swizzled bytes of 128 weight rows per token: neighbours trade
+          // halves of tokens t and t + 4 (fp8_grouped.cu: the same), and a token's 256 bytes leave in 16-byte stores by half a warp.
+          // 64 x 28672 x 4096: 23.5 us with 2-byte stores, so 22.7; 21 tokens 21.6 -> 21.1.
+          const uint32_t turn = smem_u32(tiles) + ((warp - 2) >> 2) * (CW * kTileN * 2);
+          const bool odd = lane & 1;
+          const uint32_t chunk = q * 4 + (lane >> 3), within = ((lane >> 1) & 3) * 4;
+#pragma unroll
+          for (int tt = 0; tt < CW; tt += 8) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const __nv_bfloat162 two = __floats2bfloat162_rn(acc[tt + j], acc[tt + j + 4]);
+              const uint32_t own = *reinterpret_cast<const uint32_t*>(&two), other = __shfl_xor_sync(0xffffffffu, own, 1);
+              const uint32_t at = j + (odd ? 4 : 0);  // of the eight tokens
+              asm volatile("st.shared.b32 [%0], %1;" ::"r"(turn + (tt + at) * 256 + ((chunk ^ at) << 4) + within), "r"(__byte_perm(own, other, odd ? 0x3276 : 0x5410))
+                           : "memory");
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&epi_bar[2]);
+          if (mbar_wait_warp(&epi_bar[2], 0, abort_flag, p.status, kStatusTimeoutEpilogue)) {
+            __nv_bfloat16* dst = p.out + size_t(t0 + col0) * p.N + n0;
+            const int place = ((warp - 2) & 3) * 32 + lane, c = place & 15;
+#pragma unroll
+            for (int i = 0; i < CW / 8; ++i) {
+              const int tt = i * 8 + (place >> 4);
+              uint4 v;
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(turn + tt * 256 + ((c ^ (tt & 7)) << 4)));
+              if (col0 + tt < tl) *reinterpret_cast<uint4*>(dst + size_t(tt) * p.N + c * 8) = v;
+            }
+          }
+        } else if (owner && n < p.N) {
           // The residual may be the output buffer itself (in-place add), so the compiler keeps every load behind the
           // store before it: one exposed memory round trip per token column.  All loads of the thread are issued
           // first (each element is read and written by this thread only), then the sums are stored.
@@ -601,23 +727,10 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   }
 
   if (p.cluster_reduce) {
-    // Every thread of every CTA of the cluster gets here (all waits above are bounded), so the barriers cannot hang.
+    // Every thread of every CTA of the cluster has arrived or will (all waits above are bounded): nobody's shared memory goes away while
+    // partial sums are on their way from it or to it.
     __syncwarp();
-    cluster_barrier();  // all partials are in place
-    if (warp >= 2 && !*abort_flag) {
-      const int tl = min(BT, row_end - t0);
-      switch (int(gridDim.z)) {  // the split count as a constant: all partials of a thread's columns are loaded at once
-        case 2: cluster_sum_columns<BT, 2>(p, tiles, t0, tl, n0); break;
-        case 3: cluster_sum_columns<BT, 3>(p, tiles, t0, tl, n0); break;
-        case 4: cluster_sum_columns<BT, 4>(p, tiles, t0, tl, n0); break;
-        case 5: cluster_sum_columns<BT, 5>(p, tiles, t0, tl, n0); break;
-        case 6: cluster_sum_columns<BT, 6>(p, tiles, t0, tl, n0); break;
-        case 7: cluster_sum_columns<BT, 7>(p, tiles, t0, tl, n0); break;
-        default: cluster_sum_columns<BT, 8>(p, tiles, t0, tl, n0); break;
-      }
-    }
-    __syncwarp();
-    cluster_barrier();  // nobody's shared memory goes away while a peer still reads it
+    cluster_wait();
   }
 
   // ----- teardown: every thread arrives here, also after an aborted wait -----
@@ -670,6 +783,7 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
     attr_set[dev] = true;
   }
   if (ag) p.ag = *ag;
+  p.wide_out = BT >= 32 && !ar && !residual && N % kTileN == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const int extra_x = ag ? ag->push_ctas : 0;
   // Ring depth.  The fused-collective modes stage their output in the ring and keep all of it.  A plain
   // launch whose grid is larger than one wave of SMs takes a shallower ring instead, so that two or three CTAs share an
@@ -681,7 +795,7 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
     if (forced > 0) p.stages = forced < Cfg::kStages ? (forced < 2 ? 2 : forced) : Cfg::kStages;
     else if (ctas > 148 && BT <= 64) p.stages = kb_per < 4 ? (kb_per < 2 ? 2 : kb_per) : 4;
   }
-  const int smem_bytes = p.stages * Cfg::kStageBytes + 1024 + 256 + Cfg::kXsBytes + Cfg::kWsBytes;
+  const int smem_bytes = p.stages * Cfg::kStageBytes + Cfg::kFixedBytes;
   static const bool cluster_ok = [] { const char* e = getenv("MFQ_GEMM_CLUSTER_REDUCE"); return !e || atoi(e) != 0; }();
   if (cluster_ok && !ar && !ag && splits > 1 && splits <= 8) {
     // A cluster is placed inside one GPC, so a grid that needs nearly every SM (144 CTAs in clusters of 3, one CTA per
@@ -689,8 +803,10 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
     // shape can be resident, and the ring is made shallower (more CTAs per SM) until the whole grid is.
     static int resident[64][9][Cfg::kStages + 1] = {};  // [device][cluster size][stages]: 0 = not asked yet
     const int clusters = n_tiles * t_tiles;
-    const int min_stages = (BT * kTileN * 4 + Cfg::kStageBytes - 1) / Cfg::kStageBytes < 2 ? 2 : (BT * kTileN * 4 + Cfg::kStageBytes - 1) / Cfg::kStageBytes;
-    auto smem_for = [](int st) { return st * Cfg::kStageBytes + 1024 + 256 + Cfg::kXsBytes + Cfg::kWsBytes; };
+    // the ring holds this CTA's partial sums by destination and those that come from the others
+    const int exchange = (2 * splits - 1) * ((BT + splits - 1) / splits) * kTileN * 4;
+    const int min_stages = max(2, (exchange + Cfg::kStageBytes - 1) / Cfg::kStageBytes);
+    auto smem_for = [](int st) { return st * Cfg::kStageBytes + Cfg::kFixedBytes; };
     auto fits = [&](int st) {
       int& known = resident[dev][splits][st];
       if (known == 0) {
@@ -709,11 +825,12 @@ static int launch_gemm(const void* w, const float* w_scale, const void* x, const
       }
       return known >= clusters;
     };
-    int st = p.stages;
+    int st = max(p.stages, min_stages);
     while (st > min_stages && st > 2 && !fits(st)) st = st > 4 ? 4 : st - 1;
     if (st >= min_stages) {
       p.stages = st;
       p.cluster_reduce = 1;
+      p.res_staged = residual && N % 8 == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0;
       launch_kernel_clustered(fp8_gemm_kernel<BT>, dim3(n_tiles, t_tiles, splits), dim3(Cfg::kThreads), dim3(1, 1, splits),
                               smem_for(st), stream, tw, tx, tx_alt, p);
       return cudaGetLastError() == cudaSuccess ? 0 : -7;

@@ -129,3 +129,38 @@ def test_gemv_with_folded_activation_preparation_is_bit_identical(m, n, k):
     assert torch.equal(got, want)
     check_status()
     assert_close(got, ref.fp8_gemm(*ref.silu_mul_quant(gu), wq, ws, residual=res), what="against the fp32 restatement")
+
+
+@pytest.mark.parametrize("splits", range(2, 9))
+@pytest.mark.parametrize("m", [1, 5, 16, 17, 33, 64, 100])
+def test_splits_that_meet_in_a_cluster(m, splits):
+    """Every count of splits over every token tile, columns that the splits do not divide or that some of them have none of, rows that end
+    inside a tile: against 64 bits, and the same bits with a residual that cannot be copied in 16-byte pieces or that is the output."""
+    require_gpu_lib()
+    n, k = 328, 128 * (3 * splits - 1)
+    xq, xs, wq, ws = make(m, n, k, seed=m + splits)
+    x, w = xq.double() * xs.double()[:, None], wq.double() * ws.double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)
+    want, slack = x @ w.T, (x.abs() @ w.abs().T) * (k + 8) * 2.0 ** -24  # sums of k products in fp32, whatever their order
+    got = ops.fp8_gemm(xq, xs, wq, ws, splits=splits)
+    assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-30).all())
+    res = torch.randn((m, n), device="cuda").bfloat16()
+    got = ops.fp8_gemm(xq, xs, wq, ws, residual=res, splits=splits)
+    total = want + res.double()
+    assert bool(((got.double() - total).abs() <= total.abs() * 2.0 ** -8 + 2 * slack + 1e-30).all())
+    off = torch.empty(m * n + 1, device="cuda", dtype=torch.bfloat16)[1:].view(m, n).copy_(res)
+    assert torch.equal(ops.fp8_gemm(xq, xs, wq, ws, residual=off, splits=splits), got)
+    assert torch.equal(ops.fp8_gemm(xq, xs, wq, ws, residual=res, out=res, splits=splits), got)
+    check_status()
+
+
+@pytest.mark.parametrize("m", [17, 33, 64, 65, 128, 200])
+def test_whole_tiles_of_rows_in_wide_stores(m):
+    """Results through shared memory, and column by column where the output is off a 16-byte boundary: the same bits."""
+    require_gpu_lib()
+    xq, xs, wq, ws = make(m, 384, 256, seed=m)
+    want = ref.fp8_gemm(xq, xs, wq, ws)
+    got = ops.fp8_gemm(xq, xs, wq, ws, splits=1, token_tile=32 if m <= 32 else 64 if m <= 64 else 128)
+    assert_close(got, want, what="wide")
+    off = torch.empty(m * 384 + 1, device="cuda", dtype=torch.bfloat16)[1:].view(m, 384)
+    assert torch.equal(ops.fp8_gemm(xq, xs, wq, ws, out=off, splits=1, token_tile=32 if m <= 32 else 64 if m <= 64 else 128), got)
+    check_status()
