@@ -29,7 +29,7 @@ from ..engine.recurrent_state import RecurrentState
 from ..ops import gdn
 from ..ops import reference as ref
 from ..utils.profiler import scope
-from .llama import Fp8Linear, LlamaLayer, StepBuffers
+from .llama import Fp8Linear, LlamaLayer, StepBuffers, _own_rows
 from .moe_decoder import MoeDecoderConfig, MoeDecoderModel, MoeFfn, MoeLayer, MoeWeights, _to_float
 
 
@@ -432,10 +432,9 @@ class HybridModel(MoeDecoderModel):
         if qkv.is_cuda:
             kd = vd = None
             if prefill:
-                kd = torch.empty((t, self.hk, d), dtype=torch.bfloat16, device=qkv.device)
-                vd = torch.empty_like(kd)
+                kd, vd = self._chunk_kv(qkv, step)
             q = ops.rope_kv_write(qkv, step.positions, step.slots, kv, n_q=self.hq, n_kv=self.hk, head_dim=d, theta=cfg.rope_theta,
-                                  rot=self.rot, kd_out=kd, vd_out=vd, q_norm=layer.q_norm, k_norm=layer.k_norm,
+                                  rot=self.rot, kd_out=_own_rows(kd, step), vd_out=_own_rows(vd, step), q_norm=layer.q_norm, k_norm=layer.k_norm,
                                   norm_eps=cfg.rms_eps, scaling=self.rope_scaling)
             if prefill:
                 o = self._prefill_attention(q, kd, vd, kv, step)

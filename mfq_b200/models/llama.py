@@ -250,6 +250,11 @@ class StepBuffers:
     plans: dict = field(default_factory=dict)  # what layers derive from the portions, kept for the layers alike
 
 
+def _own_rows(kv: torch.Tensor | None, step: StepBuffers) -> torch.Tensor | None:
+    """The rows of a chunk in what :meth:`LlamaModel._chunk_kv` made."""
+    return kv[step.past_len :] if kv is not None and step.past_len else kv
+
+
 class LlamaModel:
     """Stateless forward over :class:`LlamaWeights`; KV state lives in a :class:`PagedKVCache`."""
 
@@ -315,10 +320,9 @@ class LlamaModel:
         kd = vd = None
         if qkv.is_cuda:
             if prefill:
-                kd = torch.empty((t, self.hk, d), dtype=torch.bfloat16, device=qkv.device)
-                vd = torch.empty_like(kd)
-            q = ops.rope_kv_write(qkv, step.positions, step.slots, kv, n_q=self.hq, n_kv=self.hk, head_dim=d,
-                                  theta=cfg.rope_theta, rot=self.attn_rot, kd_out=kd, vd_out=vd, scaling=self.rope_scaling)
+                kd, vd = self._chunk_kv(qkv, step)
+            q = ops.rope_kv_write(qkv, step.positions, step.slots, kv, n_q=self.hq, n_kv=self.hk, head_dim=d, theta=cfg.rope_theta,
+                                  rot=self.attn_rot, kd_out=_own_rows(kd, step), vd_out=_own_rows(vd, step), scaling=self.rope_scaling)
         else:
             q3 = qkv.view(t, self.hq + 2 * self.hk, d)
             q = ref.rope(q3[:, : self.hq], step.positions, cfg.rope_theta, self.attn_rot, self.rope_scaling)
@@ -333,15 +337,21 @@ class LlamaModel:
             return o.reshape(t, self.hq * d)
         return self._prefill_attention(q, kd, vd, kv, step).reshape(t, self.hq * d)
 
+    def _chunk_kv(self, qkv, step: StepBuffers):
+        """Keys and values that a prefill chunk attends to, ``[past + T, Hk, D]`` each: the chunk's own rows come last (:func:`_own_rows`),
+        the cached past is put before them by :meth:`_prefill_attention`."""
+        kd = qkv.new_empty((step.past_len + qkv.shape[0], self.hk, self.cfg.head_dim), dtype=torch.bfloat16)
+        return kd, torch.empty_like(kd)
+
     def _prefill_attention(self, q, kd, vd, kv, step: StepBuffers):
         """Causal attention of a prefill chunk, ``[T, Hq, D]``.  Each sequence of a packed chunk attends to itself,
         through the same FP8 rounding of K/V that later decode steps read back from the pages (``kd`` / ``vd`` on the
-        GPU); a chunk with ``past_len`` > 0 also attends to the sequence's cached past."""
+        GPU, from :meth:`_chunk_kv`); a chunk with ``past_len`` > 0 also attends to the sequence's cached past."""
         if step.past_len > 0:
             row = step.block_table[0]
             if q.is_cuda:
-                kp, vp = ops.kernels.kv_gather_dequant(kv, row, step.past_len)
-                return ops.kernels.attn_prefill_bf16(q, torch.cat([kp, kd], 0), torch.cat([vp, vd], 0), self.sm_scale)
+                ops.kernels.kv_gather_dequant(kv, row, step.past_len, kd, vd)
+                return ops.kernels.attn_prefill_bf16(q, kd, vd, self.sm_scale)
             ps = kv.page_size
             past = torch.arange(step.past_len)
             kp, vp = ref.gather_slots(kv, row[(past // ps).long()] * ps + past % ps)

@@ -113,6 +113,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  pdl_trigger();  // TMEM is held by now
+  pdl_wait();
   // columns: S of even blocks, S of odd blocks (P of 64 keys in the first half of each 64 columns), O
 
   if (warp == 0) {
@@ -324,7 +326,7 @@ extern "C" int mfq_attn_prefill_past(const void* q, const void* k, const void* v
     attr = true;
   }
   const PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status};
-  attn_prefill_kernel<<<dim3((T + kQB - 1) / kQB * Hq), kPrefillThreads, kPrefillSmem, stream>>>(tq, tk, tv, p);
+  launch_kernel(attn_prefill_kernel, dim3((T + kQB - 1) / kQB * Hq), dim3(kPrefillThreads), kPrefillSmem, stream, tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 

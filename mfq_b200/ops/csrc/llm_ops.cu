@@ -23,6 +23,8 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+// Largest of 32 values that are not negative (and not NaN, as results of fmaxf with one that is not): their bits are in the same order.
+__device__ __forceinline__ float warp_max_abs(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
 // Block-wide reductions over <= 1024 threads; `red` is 33 floats of shared memory.
 template <bool kMax>
 __device__ __forceinline__ float block_reduce(float v, float* red) {
@@ -62,6 +64,8 @@ __device__ __forceinline__ float from_e4m3(uint8_t c) {
 // ---------------------------------------------------------------------------------------------
 constexpr int kNormVecs = 8;
 
+// Where a thread holds several vectors they wait as the bf16 values that they are, four registers a vector: 4096 rows of 4096 on a B200 with
+// eight registers a vector (84 a thread) 18.6 us, so 12.8; 2000 rows 12.8 -> 8.5.
 template <int kNormVecs>
 __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                                      __nv_bfloat16* __restrict__ residual_out, const __nv_bfloat16* __restrict__ w,
@@ -72,31 +76,51 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
   __shared__ float red[33];
   const size_t row = blockIdx.x;
   const int nvec = H / 8;
-  float v[kNormVecs][8];
+  uint4 held[kNormVecs];
+  auto load8 = [](const uint4& a, float (&v)[8]) {
+    const uint32_t u[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[2 * j] = __uint_as_float(u[j] << 16);
+      v[2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+    }
+  };
+  auto pack8 = [](const float (&v)[8]) {
+    uint4 a;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&a);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+    return a;
+  };
+#pragma unroll
+  for (int i = 0; i < kNormVecs; ++i) {
+    const int vi = threadIdx.x + i * blockDim.x;
+    if (vi < nvec) held[i] = *reinterpret_cast<const uint4*>(x + row * H + vi * 8);
+  }
+  if (residual) {
+#pragma unroll
+    for (int i = 0; i < kNormVecs; ++i) {
+      const int vi = threadIdx.x + i * blockDim.x;
+      if (vi < nvec) {
+        float a[8], r[8];
+        load8(held[i], a);
+        load8(*reinterpret_cast<const uint4*>(residual + row * H + vi * 8), r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] += r[j];
+        held[i] = pack8(a);
+        *reinterpret_cast<uint4*>(residual_out + row * H + vi * 8) = held[i];
+      }
+    }
+  }
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < kNormVecs; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
-      uint4 a = *reinterpret_cast<const uint4*>(x + row * H + vi * 8);
-      const __nv_bfloat16* ab = reinterpret_cast<const __nv_bfloat16*>(&a);
-      if (residual) {
-        uint4 r = *reinterpret_cast<const uint4*>(residual + row * H + vi * 8);
-        const __nv_bfloat16* rb = reinterpret_cast<const __nv_bfloat16*>(&r);
-        uint4 o;
-        __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(&o);
+      float v[8];
+      load8(held[i], v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          ob[j] = __float2bfloat16(__bfloat162float(ab[j]) + __bfloat162float(rb[j]));
-          v[i][j] = __bfloat162float(ob[j]);
-        }
-        *reinterpret_cast<uint4*>(residual_out + row * H + vi * 8) = o;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[i][j] = __bfloat162float(ab[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
+      for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
     }
   }
   const float rstd = rsqrtf(block_reduce<false>(ss, red) / float(H) + eps);
@@ -105,14 +129,16 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
   for (int i = 0; i < kNormVecs; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
-      uint4 ww = *reinterpret_cast<const uint4*>(w + vi * 8);
-      const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(&ww);
+      float v[8], wv[8];
+      load8(held[i], v);
+      load8(*reinterpret_cast<const uint4*>(w + vi * 8), wv);
+      // round through bf16 like an unfused norm would, so fused and unfused paths agree bit for bit
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        // round through bf16 like an unfused norm would, so fused and unfused paths agree bit for bit
-        v[i][j] = __bfloat162float(__float2bfloat16(v[i][j] * rstd * __bfloat162float(wb[j])));
-        amax = fmaxf(amax, fabsf(v[i][j]));
-      }
+      for (int j = 0; j < 8; ++j) v[j] = v[j] * rstd * wv[j];
+      held[i] = pack8(v);
+      load8(held[i], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
     }
   }
   amax = block_reduce<true>(amax, red);
@@ -123,14 +149,12 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
   for (int i = 0; i < kNormVecs; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
-      if (q_out) *reinterpret_cast<uint2*>(q_out + row * H + vi * 8) = to_e4m3x8(v[i], inv);
-      if (y_out) {
-        uint4 o;
-        __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(&o);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ob[j] = __float2bfloat16(v[i][j]);
-        *reinterpret_cast<uint4*>(y_out + row * H + vi * 8) = o;
+      if (q_out) {
+        float v[8];
+        load8(held[i], v);
+        *reinterpret_cast<uint2*>(q_out + row * H + vi * 8) = to_e4m3x8(v, inv);
       }
+      if (y_out) *reinterpret_cast<uint4*>(y_out + row * H + vi * 8) = held[i];
     }
   }
 }
@@ -468,7 +492,7 @@ __device__ __forceinline__ void rope_head(const __nv_bfloat16* __restrict__ src,
     hi[j] = __bfloat162float(__float2bfloat16(hi[j]));
     amax = fmaxf(amax, fmaxf(fabsf(lo[j]), fabsf(hi[j])));
   }
-  amax = warp_max(amax);
+  amax = warp_max_abs(amax);
   const float scale = fmaxf(amax, 1e-12f) / kE4M3Max;
   const float inv = 1.f / scale;
   const size_t base = ((size_t(page) * Hk + kvh) * page_size + off);
@@ -476,11 +500,19 @@ __device__ __forceinline__ void rope_head(const __nv_bfloat16* __restrict__ src,
   if (!is_v) {
     // K page: [D/64 chunks][page_size tokens][64 dims]
     uint8_t* dst = to.k_cache + ph * (size_t(page_size) * D);
+    if constexpr (HP == 2) {  // neighbouring dims of a chunk: one store of two
+      const int d0 = lane * HP, d1 = D / 2 + lane * HP;
+      *reinterpret_cast<__nv_fp8x2_storage_t*>(dst + (d0 >> 6) * (page_size * 64) + off * 64 + (d0 & 63)) =
+          __nv_cvt_float2_to_fp8x2(make_float2(lo[0] * inv, lo[1] * inv), __NV_SATFINITE, __NV_E4M3);
+      *reinterpret_cast<__nv_fp8x2_storage_t*>(dst + (d1 >> 6) * (page_size * 64) + off * 64 + (d1 & 63)) =
+          __nv_cvt_float2_to_fp8x2(make_float2(hi[0] * inv, hi[1] * inv), __NV_SATFINITE, __NV_E4M3);
+    } else {
 #pragma unroll
-    for (int j = 0; j < HP; ++j) {
-      const int d0 = lane * HP + j, d1 = D / 2 + lane * HP + j;
-      dst[(d0 >> 6) * (page_size * 64) + off * 64 + (d0 & 63)] = to_e4m3(lo[j] * inv);
-      dst[(d1 >> 6) * (page_size * 64) + off * 64 + (d1 & 63)] = to_e4m3(hi[j] * inv);
+      for (int j = 0; j < HP; ++j) {
+        const int d0 = lane * HP + j, d1 = D / 2 + lane * HP + j;
+        dst[(d0 >> 6) * (page_size * 64) + off * 64 + (d0 & 63)] = to_e4m3(lo[j] * inv);
+        dst[(d1 >> 6) * (page_size * 64) + off * 64 + (d1 & 63)] = to_e4m3(hi[j] * inv);
+      }
     }
   } else {
     // V page: [D dims][page_size tokens in the order 0,1,8,9,2,3,10,11,4,5,12,13,6,7,14,15]
@@ -508,6 +540,94 @@ __device__ __forceinline__ void rope_head(const __nv_bfloat16* __restrict__ src,
   if (lane == 0) (is_v ? to.v_scale : to.k_scale)[base] = scale;
 }
 
+// The values of sixteen tokens and one head, the tokens of one page where a prompt fills whole ones: a page holds a dim's sixteen tokens side
+// by side, so token by token every byte goes to a sector of its own.  A lane has D / 32 neighbouring dims of all sixteen tokens: the bytes
+// of a dim come together in its registers and leave as one store.  The tokens of other groups (a page's part, slots in another order, none)
+// are left to the warps that go token by token.
+constexpr int kGroupTokens = 16;
+// First token of a group: groups are the pages of a prompt in one piece that begins at slots[0].  Whether token t0's group is one whole page,
+// the same for the warp; `slot`: the lane's (lane & 15).
+__device__ __forceinline__ int group_shift(const int* __restrict__ slots) { return slots[0] >= 0 ? slots[0] & 15 : 0; }
+__device__ __forceinline__ bool whole_page(const int* __restrict__ slots, int t0, int T, int lane, int& slot) {
+  const int mine = t0 + (lane & 15);
+  slot = mine >= 0 && mine < T ? slots[mine] : -1;
+  const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
+  return __all_sync(0xffffffffu, slot >= 0 && slot == slot0 + (lane & 15)) && (slot0 & 15) == 0;
+}
+template <int D>
+__device__ __forceinline__ void value_group(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ slots, const RopeOut& to, int T, int row_stride,
+                                            int block) {
+  constexpr int VPL = D / 32, W = VPL / 4;  // dims of a lane, words of their codes
+  const int lane = threadIdx.x & 31, head_blocks = (to.Hk + 7) / 8;
+  const int h = block % head_blocks * 8 + (threadIdx.x >> 5);
+  if (h >= to.Hk) return;
+  const int t0 = block / head_blocks * kGroupTokens - group_shift(slots);
+  int slot;
+  if (t0 < 0 || t0 + kGroupTokens > T || !whole_page(slots, t0, T, lane, slot)) return;
+  const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
+  const __nv_bfloat16* src = qkv + size_t(to.Hq + to.Hk + h) * D + lane * VPL;
+  uint2 raw[kGroupTokens][W];
+#pragma unroll
+  for (int i = 0; i < kGroupTokens; ++i) {
+    const int t = t0 + i;
+#pragma unroll
+    for (int w = 0; w < W; ++w) raw[i][w] = *reinterpret_cast<const uint2*>(src + size_t(t) * row_stride + w * 4);
+  }
+  uint32_t code[kGroupTokens][W];
+  float my_scale = 0.f;
+#pragma unroll
+  for (int i = 0; i < kGroupTokens; ++i) {
+    float v[VPL], amax = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      v[4 * w] = __uint_as_float(raw[i][w].x << 16);
+      v[4 * w + 1] = __uint_as_float(raw[i][w].x & 0xffff0000u);
+      v[4 * w + 2] = __uint_as_float(raw[i][w].y << 16);
+      v[4 * w + 3] = __uint_as_float(raw[i][w].y & 0xffff0000u);
+    }
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) amax = fmaxf(amax, fabsf(v[j]));
+    amax = warp_max_abs(amax);
+    const float scale = fmaxf(amax, 1e-12f) / kE4M3Max, inv = 1.f / scale;
+    if (lane == i) my_scale = scale;
+    const int t = t0 + i;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * w] * inv, v[4 * w + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+      const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * w + 2] * inv, v[4 * w + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+      code[i][w] = lo | hi << 16;
+    }
+    if (to.vd) {
+      __nv_bfloat16* dst = to.vd + (size_t(t) * to.Hk + h) * D + lane * VPL;
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        float d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[j] = from_e4m3(uint8_t(code[i][w] >> (8 * j))) * scale;
+        const __nv_bfloat162 a = __floats2bfloat162_rn(d[0], d[1]), b = __floats2bfloat162_rn(d[2], d[3]);
+        *reinterpret_cast<uint2*>(dst + w * 4) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+      }
+    }
+  }
+  if (lane < kGroupTokens) to.v_scale[(size_t(slot >> 4) * to.Hk + h) * 16 + (slot & 15)] = my_scale;
+  uint4* dst = reinterpret_cast<uint4*>(to.v_cache + (size_t(slot0 >> 4) * to.Hk + h) * (size_t(16) * D) + lane * VPL * 16);
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    uint32_t out[4][4];  // [dim][word]: word g of a page's row holds tokens 2g, 2g + 1, 2g + 8, 2g + 9
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint32_t a = code[2 * g][w], b = code[2 * g + 1][w], c = code[2 * g + 8][w], d = code[2 * g + 9][w];
+      const uint32_t ab0 = __byte_perm(a, b, 0x5140), ab1 = __byte_perm(a, b, 0x7362), cd0 = __byte_perm(c, d, 0x5140), cd1 = __byte_perm(c, d, 0x7362);
+      out[0][g] = __byte_perm(ab0, cd0, 0x5410);
+      out[1][g] = __byte_perm(ab0, cd0, 0x7632);
+      out[2][g] = __byte_perm(ab1, cd1, 0x5410);
+      out[3][g] = __byte_perm(ab1, cd1, 0x7632);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dst[w * 4 + j] = make_uint4(out[j][0], out[j][1], out[j][2], out[j][3]);
+  }
+}
+
 // kHeads: heads of a token that a warp takes.  Several (full rotary only): their angles are evaluated once.
 template <int D, int kHeads>
 __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
@@ -517,12 +637,19 @@ __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv,
                                           int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
                                           __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
                                           const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
-                                          const RopeScale ys) {
+                                          const RopeScale ys, int value_blocks) {
   pdl_trigger();
   pdl_wait();
+  const RopeOut to{q_out, k_cache, v_cache, k_scale, v_scale, kd_out, vd_out, Hq, Hk, page_size};
+  if constexpr (kHeads > 1 && D >= 128) {
+    if (int(blockIdx.x) < value_blocks) {
+      value_group<D>(qkv, slots, to, T, row_stride, blockIdx.x);
+      return;
+    }
+  }
   constexpr int EPL = D / 32;  // elements per lane
   const int warps_per_block = blockDim.x >> 5;
-  const int gw = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
+  const int gw = (int(blockIdx.x) - value_blocks) * warps_per_block + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int heads = Hq + 2 * Hk, groups = (heads + kHeads - 1) / kHeads;
   if (gw >= T * groups) return;
@@ -550,9 +677,25 @@ __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv,
       for (int j = 0; j < HP; ++j) dst[j] = __bfloat162float(ptr[j]);
     }
   };
-  load_half(src + lane * HP, lo);
-  load_half(src + D / 2 + lane * HP, hi);
-  const RopeOut to{q_out, k_cache, v_cache, k_scale, v_scale, kd_out, vd_out, Hq, Hk, page_size};
+  constexpr bool kAhead = kHeads > 1 && HP <= 2;  // all heads of the warp requested before the first is used
+  const int h_end = min(h_first + kHeads, heads);
+  uint32_t raw[kAhead ? kHeads : 1][2];
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int i = 0; i < kHeads; ++i) {
+      const __nv_bfloat16* at = src + (h_first + i < h_end ? i * D : 0) + lane * HP;
+      if constexpr (HP == 2) {
+        raw[i][0] = *reinterpret_cast<const uint32_t*>(at);
+        raw[i][1] = *reinterpret_cast<const uint32_t*>(at + D / 2);
+      } else {
+        raw[i][0] = *reinterpret_cast<const unsigned short*>(at);
+        raw[i][1] = *reinterpret_cast<const unsigned short*>(at + D / 2);
+      }
+    }
+  } else {
+    load_half(src + lane * HP, lo);
+    load_half(src + D / 2 + lane * HP, hi);
+  }
   auto evaluate = [&](int j, float& s, float& c) {
     sincosf(float(positions[t]) * rope_inv_freq(log2_theta, lane * HP + j, rot, ys), &s, &c);
     s *= ys.mscale;
@@ -571,14 +714,32 @@ __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv,
 #pragma unroll
       for (int j = 0; j < HP; ++j) evaluate(j, sn[j], cs[j]);
     }
-    const int h_end = min(h_first + kHeads, heads);
-    for (int h = h_first; h < h_end; ++h, src += D) {
-      if (h != h_first) {
-        load_half(src + lane * HP, lo);
-        load_half(src + D / 2 + lane * HP, hi);
+    bool values_done = false;  // by the warps that take whole pages
+    if (value_blocks && h_end > Hq + Hk) {
+      int unused;
+      values_done = whole_page(slots, t - ((t + group_shift(slots)) & 15), T, lane, unused);
+    }
+    const auto shared_angle = [&](int j, float& s, float& c) { s = sn[j]; c = cs[j]; };
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int i = 0; i < kHeads; ++i) {
+        if (h_first + i >= h_end || (values_done && h_first + i >= Hq + Hk)) break;
+#pragma unroll
+        for (int j = 0; j < HP; ++j) {
+          lo[j] = __uint_as_float(j ? raw[i][0] & 0xffff0000u : raw[i][0] << 16);
+          hi[j] = __uint_as_float(j ? raw[i][1] & 0xffff0000u : raw[i][1] << 16);
+        }
+        rope_head<D, true>(src + i * D, lo, hi, t, h_first + i, lane, positions, D, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to, shared_angle, slot);
       }
-      rope_head<D, true>(src, lo, hi, t, h, lane, positions, D, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to,
-                         [&](int j, float& s, float& c) { s = sn[j]; c = cs[j]; }, slot);
+    } else {
+      for (int h = h_first; h < h_end; ++h, src += D) {
+        if (values_done && h >= Hq + Hk) break;
+        if (h != h_first) {
+          load_half(src + lane * HP, lo);
+          load_half(src + D / 2 + lane * HP, hi);
+        }
+        rope_head<D, true>(src, lo, hi, t, h, lane, positions, D, log2_theta, ys, q_norm_w, k_norm_w, norm_eps, to, shared_angle, slot);
+      }
     }
   }
 }
@@ -591,23 +752,23 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
                                      int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
                                      __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
                                      const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
-                                     const RopeScale ys) {
+                                     const RopeScale ys, int value_blocks) {
   rope_rows<D, 1>(qkv, positions, slots, q_out, k_cache, v_cache, k_scale, v_scale, T, Hq, Hk, page_size, rot, log2_theta, kd_out, vd_out, q_norm_w, k_norm_w,
-                  norm_eps, row_stride, ys);
+                  norm_eps, row_stride, ys, value_blocks);
 }
 
 constexpr int kRopeHeads = 8;
 template <int D>
-__global__ void __launch_bounds__(256, D <= 128 ? 6 : 4) rope_kv_write_heads_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+__global__ void __launch_bounds__(256, 4) rope_kv_write_heads_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
                                      const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
                                      uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
                                      float* __restrict__ k_scale, float* __restrict__ v_scale, int T, int Hq, int Hk,
                                      int page_size, int rot, float log2_theta, __nv_bfloat16* __restrict__ kd_out,
                                      __nv_bfloat16* __restrict__ vd_out, const float* __restrict__ q_norm_w,
                                      const float* __restrict__ k_norm_w, float norm_eps, int row_stride,
-                                     const RopeScale ys) {
+                                     const RopeScale ys, int value_blocks) {
   rope_rows<D, kRopeHeads>(qkv, positions, slots, q_out, k_cache, v_cache, k_scale, v_scale, T, Hq, Hk, page_size, rot, log2_theta, kd_out, vd_out, q_norm_w, k_norm_w,
-                       norm_eps, row_stride, ys);
+                       norm_eps, row_stride, ys, value_blocks);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -794,6 +955,7 @@ extern "C" int mfq_gate_quant_rows(const void* x, const void* gate, void* q_out,
 // q_norm_w / k_norm_w ([D] fp32, may be null): per-head RMSNorm of q / k before the rotation; row_stride: elements
 // between token rows of qkv (>= (Hq + 2 Hk) * D; an attention output gate may follow the v heads).
 // yarn_*: context extension (see RopeScale); factor 1 and mscale 1 are the plain rotation.
+constexpr long kSharedFrom = 18000;
 extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, const int* slots, void* q_out, void* k_cache,
                                       void* v_cache, float* k_scale, float* v_scale, int T, int Hq, int Hk, int D,
                                       int page_size, int rot, float theta, void* kd_out, void* vd_out,
@@ -804,20 +966,24 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
   // A warp per head, or one per kRopeHeads heads of a token, whose angles (sine, cosine and the frequency's power, a good part of a head's
   // work) it evaluates once.  That needs full rotary, enough heads that the fewer and longer warps still fill the GPU, and groups that are
-  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  On a B200, a warp per
-  // head | eight heads:  48 heads of 128, 500 tokens 10.3 | 12.6 us, 700 13.5 | 14.5, 800 15.2 | 14.8, 1000 18.8 | 15.2, 4096 68.7 | 47.0;
-  // 36 heads of 64, 800 tokens 6.5 | 6.8, 1000 7.6 | 6.9;  20 of 256, 2000 21.5 | 20.1;  10 of 128 (two groups), 4096 13.1 | 14.2.
+  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  The eight heads of a warp
+  // are requested together, and the values of whole pages go by themselves (value_group).  48 heads of 128 on a B200, a warp per head | eight
+  // heads | and values by pages: 200 tokens 5.9 | 6.9 | 7.4 us, 357 8.1 | 8.4 | 8.2, 512 10.5 | 9.8 | 9.6, 700 13.4 | 10.5 | 10.3, 1000 18.8 | 14.5 |
+  // 12.9, 4096 68.7 | 43.4 | 39.3 (each head loaded after the one before, eight heads took 15.2 and 47.0).
   const int heads = Hq + 2 * Hk, full_groups = (heads + kRopeHeads - 1) / kRopeHeads;
   const bool aligned = (reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kd_out) | reinterpret_cast<uintptr_t>(vd_out)) % 8 == 0;
-  const bool shared = rot == D && long(T) * heads >= 36000 && 4 * heads >= 3 * kRopeHeads * full_groups && aligned;
-  const int blocks = int((long(T) * (shared ? full_groups : heads) + 7) / 8);
+  const bool shared = rot == D && long(T) * heads >= kSharedFrom && 4 * heads >= 3 * kRopeHeads * full_groups && aligned;
+  // values of whole pages sixteen tokens at a time
+  const bool grouped = shared && D >= 128 && page_size == 16 && reinterpret_cast<uintptr_t>(qkv) % 8 == 0 && row_stride % 4 == 0 && reinterpret_cast<uintptr_t>(v_cache) % 16 == 0;
+  const int value_blocks = grouped ? (T + 15 + kGroupTokens - 1) / kGroupTokens * ((Hk + 7) / 8) : 0;
+  const int blocks = value_blocks + int((long(T) * (shared ? full_groups : heads) + 7) / 8);
   const float l2t = log2f(theta);
   const RopeScale ys{yarn_factor, yarn_low, yarn_high, yarn_mscale};
 #define MFQ_ROPE(DD)                                                                                             \
   launch_kernel(shared ? rope_kv_write_heads_kernel<DD> : rope_kv_write_kernel<DD>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkv), positions, slots, \
       static_cast<__nv_bfloat16*>(q_out), static_cast<uint8_t*>(k_cache), static_cast<uint8_t*>(v_cache),      \
       k_scale, v_scale, T, Hq, Hk, page_size, rot, l2t, static_cast<__nv_bfloat16*>(kd_out),                   \
-      static_cast<__nv_bfloat16*>(vd_out), q_norm_w, k_norm_w, norm_eps, row_stride, ys)
+      static_cast<__nv_bfloat16*>(vd_out), q_norm_w, k_norm_w, norm_eps, row_stride, ys, value_blocks)
   if (D == 128) MFQ_ROPE(128);
   else if (D == 64) MFQ_ROPE(64);
   else if (D == 256) MFQ_ROPE(256);
@@ -915,30 +1081,68 @@ extern "C" int mfq_silu_mul_bf16(const void* x, void* out, int M, int I, int in_
 
 // ---------------------------------------------------------------------------------------------
 // Past K/V of one sequence out of the FP8 pages into contiguous bf16 [T, Hk, D] (code * multiplier): the keys /
-// values a later prefill chunk attends to (chunked prefill, restored prefix).  One warp per (token, KV head).
+// values a later prefill chunk attends to (chunked prefill, restored prefix).  A warp takes one head's page: its rows by 16 bytes, and of the
+// values, which lie dim by dim, the four dims of a lane, turned in registers.  8 heads of 128 on a B200, before a warp per token and head
+// that reads byte by byte (4001 tokens 10.3 us, 357 2.9), so 7.8 and 3.1.
 // ---------------------------------------------------------------------------------------------
 namespace mfq {
 template <int D>
-__global__ void kv_gather_dequant_kernel(const uint8_t* __restrict__ k_cache, const uint8_t* __restrict__ v_cache,
+__global__ void __launch_bounds__(256) kv_gather_dequant_kernel(const uint8_t* __restrict__ k_cache, const uint8_t* __restrict__ v_cache,
                                          const float* __restrict__ k_scale, const float* __restrict__ v_scale,
                                          const int* __restrict__ block_row, __nv_bfloat16* __restrict__ kd,
-                                         __nv_bfloat16* __restrict__ vd, int T, int Hk, int page_size) {
+                                         __nv_bfloat16* __restrict__ vd, int T, int Hk) {
   pdl_trigger();
   pdl_wait();
+  constexpr int P = 16;  // tokens of a page
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (gw >= T * Hk) return;
-  const int t = gw / Hk, h = gw % Hk;
-  const int page = block_row[t / page_size], off = t % page_size;
-  const size_t ph = size_t(page) * Hk + h;
-  const float ks = k_scale[ph * page_size + off], vs = v_scale[ph * page_size + off];
-  const uint8_t* kp = k_cache + ph * (size_t(page_size) * D);
-  const uint8_t* vp = v_cache + ph * (size_t(page_size) * D);
-  const int pos = 4 * ((off & 7) >> 1) + 2 * (off >> 3) + (off & 1);  // slot of the token inside a V page
-  __nv_bfloat16* ko = kd + (size_t(t) * Hk + h) * D;
-  __nv_bfloat16* vo = vd + (size_t(t) * Hk + h) * D;
-  for (int d = lane; d < D; d += 32) {
-    ko[d] = __float2bfloat16(from_e4m3(kp[(d >> 6) * (page_size * 64) + off * 64 + (d & 63)]) * ks);
-    vo[d] = __float2bfloat16(from_e4m3(vp[d * page_size + pos]) * vs);
+  const int pages = (T + P - 1) / P, side = gw / (pages * Hk), at = gw - side * (pages * Hk);  // keys, then values
+  if (side > 1) return;
+  const int pi = at / Hk, h = at - pi * Hk, t0 = pi * P, rows = min(P, T - t0);
+  const size_t ph = size_t(block_row[pi]) * Hk + h;
+  const float my_scale = (side ? v_scale : k_scale)[ph * P + (lane & 15)];
+  auto two = [](uint32_t codes, int j, float s) {  // codes j and j + 1 of a word
+    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(__nv_fp8x2_storage_t(codes >> (8 * j)), __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    const __nv_bfloat162 r = __floats2bfloat162_rn(f.x * s, f.y * s);
+    return *reinterpret_cast<const uint32_t*>(&r);
+  };
+  if (side == 0) {  // [D / 64 chunks][16 tokens][64 dims]
+    const uint4* src = reinterpret_cast<const uint4*>(k_cache + ph * (size_t(P) * D));
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) {
+      const int v = i * 32 + lane, chunk = v >> 6, t = (v >> 2) & 15, dim = chunk * 64 + (v & 3) * 16;
+      const uint4 c = src[v];
+      const float s = __shfl_sync(0xffffffffu, my_scale, t);
+      if (t < rows) {
+        uint4* dst = reinterpret_cast<uint4*>(kd + (size_t(t0 + t) * Hk + h) * D + dim);
+        dst[0] = make_uint4(two(c.x, 0, s), two(c.x, 2, s), two(c.y, 0, s), two(c.y, 2, s));
+        dst[1] = make_uint4(two(c.z, 0, s), two(c.z, 2, s), two(c.w, 0, s), two(c.w, 2, s));
+      }
+    }
+    return;
+  }
+  constexpr int VPL = D / 32;  // dims of a lane
+  const uint4* src = reinterpret_cast<const uint4*>(v_cache + ph * (size_t(P) * D) + lane * VPL * P);
+  uint4 c[VPL];
+#pragma unroll
+  for (int j = 0; j < VPL; ++j) c[j] = src[j];
+#pragma unroll
+  for (int t = 0; t < P; ++t) {
+    const float s = __shfl_sync(0xffffffffu, my_scale, t);
+    const int word = (t & 7) >> 1, byte = 8 * (2 * (t >> 3) + (t & 1));  // word g of a dim holds tokens 2g, 2g + 1, 2g + 8, 2g + 9
+    uint32_t out[VPL / 2];
+#pragma unroll
+    for (int j = 0; j < VPL; j += 2) {
+      const uint32_t a = word == 0 ? c[j].x : word == 1 ? c[j].y : word == 2 ? c[j].z : c[j].w;
+      const uint32_t b = word == 0 ? c[j + 1].x : word == 1 ? c[j + 1].y : word == 2 ? c[j + 1].z : c[j + 1].w;
+      out[j / 2] = two(__byte_perm(a, b, (byte >> 3) | (4 + (byte >> 3)) << 4), 0, s);
+    }
+    if (t < rows) {
+      __nv_bfloat16* dst = vd + (size_t(t0 + t) * Hk + h) * D + lane * VPL;
+      if constexpr (VPL == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+      else if constexpr (VPL == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(out[0], out[1]);
+      else *reinterpret_cast<uint32_t*>(dst) = out[0];
+    }
   }
 }
 }  // namespace mfq
@@ -948,11 +1152,12 @@ extern "C" int mfq_kv_gather_dequant(const void* k_cache, const void* v_cache, c
                                      const int* block_row, void* kd, void* vd, int T, int Hk, int D, int page_size,
                                      cudaStream_t stream) {
   if (T <= 0 || Hk <= 0 || page_size != 16) return -1;
-  const int blocks = (T * Hk + 7) / 8;
+  if ((reinterpret_cast<uintptr_t>(kd) | reinterpret_cast<uintptr_t>(vd) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) return -1;
+  const int blocks = (2 * ((T + 15) / 16) * Hk + 7) / 8;
 #define MFQ_GATHER(DD)                                                                                              \
   mfq::launch_kernel(mfq::kv_gather_dequant_kernel<DD>, dim3(blocks), dim3(256), 0, stream,                        \
                      static_cast<const uint8_t*>(k_cache), static_cast<const uint8_t*>(v_cache), k_scale, v_scale,  \
-                     block_row, static_cast<__nv_bfloat16*>(kd), static_cast<__nv_bfloat16*>(vd), T, Hk, page_size)
+                     block_row, static_cast<__nv_bfloat16*>(kd), static_cast<__nv_bfloat16*>(vd), T, Hk)
   if (D == 128) MFQ_GATHER(128);
   else if (D == 64) MFQ_GATHER(64);
   else if (D == 256) MFQ_GATHER(256);

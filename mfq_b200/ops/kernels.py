@@ -376,11 +376,14 @@ def attn_prefill_bf16(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, sm_scal
     return out
 
 
-def kv_gather_dequant(kv, block_row: torch.Tensor, tokens: int):
-    """The first ``tokens`` cached K/V rows of one sequence (its page ids in ``block_row``) as bf16 ``[tokens, Hk, D]``."""
+def kv_gather_dequant(kv, block_row: torch.Tensor, tokens: int, k_out: torch.Tensor | None = None, v_out: torch.Tensor | None = None):
+    """The first ``tokens`` cached K/V rows of one sequence (its page ids in ``block_row``) as bf16 ``[tokens, Hk, D]``, or in the first rows
+    of ``k_out`` / ``v_out`` (contiguous, at least as long)."""
     hk, d = kv.k.shape[1], kv.k.shape[2] * kv.k.shape[4]
-    kd = torch.empty((tokens, hk, d), dtype=torch.bfloat16, device=block_row.device)
-    vd = torch.empty_like(kd)
+    kd = torch.empty((tokens, hk, d), dtype=torch.bfloat16, device=block_row.device) if k_out is None else k_out
+    vd = torch.empty_like(kd) if v_out is None else v_out
+    for t in (kd, vd):
+        assert t.shape[0] >= tokens and t.shape[1:] == (hk, d) and t.dtype == torch.bfloat16 and t.is_contiguous()
     check(lib().mfq_kv_gather_dequant(ptr(kv.k), ptr(kv.v), ptr(kv.k_scale), ptr(kv.v_scale), ptr(block_row), ptr(kd), ptr(vd),
                                       tokens, hk, d, kv.page_size, stream_ptr()), "kv_gather_dequant")
     return kd, vd

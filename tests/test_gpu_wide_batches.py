@@ -289,3 +289,37 @@ def test_stream_rows_by_vectors_per_thread(m, w):
     dense.norm_add(y, f, x, act, w, 1e-5)
     # a tree of w squares, its root and three more roundings: below 32 of 2^-24, of the size of the two terms
     assert ((x.double() - want).abs() <= 2.0 ** -19 * size).all() and torch.equal(act, x.bfloat16())
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("how", ["pages", "offset", "mixed", "none first"])
+def test_values_that_go_to_whole_pages_together(d, how):
+    """Slots in one piece from a page's start or from inside one, in pieces that change places, and slots that take nothing: the pages and rows
+    that calls too small for whole pages write, and what reading the pages back gives."""
+    require_gpu_lib()
+    t, hq, hk, first = 1100, 12, 4, 5 if how == "offset" else 0
+    rows = _normal(d, t, (hq + 2 * hk) * d)
+    pos = torch.arange(t, device="cuda", dtype=torch.int32)
+    slots = torch.arange(first, first + t, dtype=torch.int32) + 16
+    if how == "mixed":
+        slots = torch.cat([slots[40:300], slots[:40], slots[300:301], slots[302:], slots[301:302]])
+    if how == "none first":
+        slots[0], slots[500:520] = -1, -1
+    slots = slots.cuda()
+    got = []
+    for step in (t, 300):
+        cache = PagedKVCache(layers=1, kv_heads=hk, head_dim=d, num_pages=90, max_seqs=1, max_pages_per_seq=80, device="cuda")
+        kd, vd = torch.zeros((t, hk, d), device="cuda", dtype=torch.bfloat16), torch.zeros((t, hk, d), device="cuda", dtype=torch.bfloat16)
+        assert (step * (hq + 2 * hk) >= 18000) == (step == t)
+        q = torch.cat([ops.rope_kv_write(rows[a : a + step], pos[a : a + step], slots[a : a + step], cache.layer(0), n_q=hq, n_kv=hk, head_dim=d, theta=1e4,
+                                         kd_out=kd[a : a + step], vd_out=vd[a : a + step]) for a in range(0, t, step)])
+        got.append([q, cache.k.view(torch.uint8), cache.v.view(torch.uint8), cache.k_scale, cache.v_scale, kd, vd])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    table = torch.arange(1, 80, device="cuda", dtype=torch.int32)
+    for n in (1, 15, 16, 17, 333, 1100):
+        kr, vr = K.kv_gather_dequant(cache.layer(0), table, n)
+        for i, s in enumerate(slots.tolist()):
+            if 0 <= s - 16 < n and i % 7 == 0:
+                assert torch.equal(kr[s - 16], kd[i]) and torch.equal(vr[s - 16], vd[i])
+    check_status()
