@@ -130,23 +130,30 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       mbar_expect_tx(q_full, uint32_t(DS) * p.per * p.tokens * 128u);  // boxes are always full: rows past the tensor are zeros
       for (int d = 0; d < DS; ++d)
         tma_load_3d(sQ + d * (kWpRows * 128), &tmap_q, q_full, d * 64, q_group * p.per, row0 + tok0);
-      for (int j = 0; j < nblk; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&kv_empty[s], ((j >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutProducer)) break;
-        uint8_t* k = sKV + s * Cfg::kStage;
-        uint8_t* v = k + DS * Cfg::kKSlab;
-        mbar_expect_tx(&kv_full[s], Cfg::kStage);
-#pragma unroll 1
-        for (int i = 0; i < KB / kWpPage; ++i) {
-          const int nth = j * (KB / kWpPage) + i;
-          const int nth_page = min(nth < kept ? nth : nth + skip, last_page), page = table ? table[nth_page] : nth_page + shift;
-          const int row = page * p.page_rows + kvh * p.head_rows;
+    }
+    // A lane per page of a block: it looks its page up while the block before is on its way (one lookup after the other, each a trip to memory,
+    // was the pace of the whole kernel) and issues that page's loads.
+    constexpr int kPages = KB / kWpPage;
+    auto lookup = [&](int j) {
+      const int nth = j * kPages + (lane & (kPages - 1)), nth_page = min(nth < kept ? nth : nth + skip, last_page);
+      return table ? table[nth_page] : nth_page + shift;
+    };
+    int page = lookup(0);
+    for (int j = 0; j < nblk; ++j) {
+      const int s = j & 1, row = page * p.page_rows + kvh * p.head_rows;
+      if (j + 1 < nblk) page = lookup(j + 1);
+      if (!mbar_wait_warp(&kv_empty[s], ((j >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutProducer)) break;
+      uint8_t* k = sKV + s * Cfg::kStage + lane * (kWpPage * 128);
+      uint8_t* v = k + DS * Cfg::kKSlab;
+      if (lane == 0) mbar_expect_tx(&kv_full[s], Cfg::kStage);
+      __syncwarp();
+      if (lane < kPages) {
 #pragma unroll
-          for (int d = 0; d < DS; ++d) tma_load_2d(k + d * Cfg::kKSlab + i * (kWpPage * 128), &tmap_k, &kv_full[s], k_x + d * 64, row);
+        for (int d = 0; d < DS; ++d) tma_load_2d(k + d * Cfg::kKSlab, &tmap_k, &kv_full[s], k_x + d * 64, row);
 #pragma unroll
-          for (int d = 0; d < VS; ++d) tma_load_2d(v + d * Cfg::kKSlab + i * (kWpPage * 128), &tmap_v, &kv_full[s], v_x + d * 64, row);
-        }
+        for (int d = 0; d < VS; ++d) tma_load_2d(v + d * Cfg::kKSlab, &tmap_v, &kv_full[s], v_x + d * 64, row);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // issued by an elected lane of the converged warp (common.cuh: umma_f8f6f4_block says why)
