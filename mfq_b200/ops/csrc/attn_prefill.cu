@@ -9,9 +9,13 @@
 //   O = (O + O_blk(prev)) * alpha   folded in fp32 registers, so TMEM never needs an in-place rescale
 // The chain  softmax -> P V -> fold  is several times as long as the MMAs, so Q K^T of block j + 1 is issued before P V of block j, into
 // the other of two S buffers, and all of it but the chain itself is hidden; P never passes through shared memory and its proxy fence.
-// What bounds it is the softmax: exponentials, and the two passes over S.  32 heads on a B200, P through shared memory and MMAs issued
-// by one lane | two tiles per CTA on one S buffer each, whose eight more warps leave a thread 104 registers | this, same bits:
-//   120 tokens 8.5 | 13.1 | 6.8 us    512 after 4000  84 | 110 | 55    1000 after 3001  144 | 101 | 90    4096  316 | 197 | 190    16384  3933 | 2533 | 2501
+// What bounds it is the softmax: exponentials, and the two passes over S.
+// Grids that fill two CTAs per SM take the pair form: K and V in one stage each, one S buffer (P lies in S, so Q K^T of block j + 1 follows
+// P V of block j), a thread per query row with all 128 of its outputs in registers, no exchange of maxima.  Its chain per block is half as long
+// again, but two CTAs hide each other's waits.  O alpha + O_blk is formed as a product while P V runs and a sum while the next Q K^T does, by
+// two values per instruction in either form.  32 heads on a B200, one CTA per SM one value per instruction | two | pair form, same bits:
+//   120 tokens 8.7 | 7.0 | 7.7 us    512 after 4000 (128 CTAs) 61 | 58 | 88    700 (192) 18.9 | 15.9 | 19.3    1000 after 3001 (256) 95 | 90 | 85
+//   1500 43.5 | 40.1 | 36.1    2048 65 | 62 | 51    4096 199 | 192 | 161    8192 688 | 665 | 570
 // Heaviest (latest) query blocks are scheduled first, over all heads.
 //
 // The reference's prefill attention is a llama.cpp-derived mma.sync flash-attention (mfq_fattn_mma_f16.cuh) and a
@@ -27,6 +31,8 @@ constexpr int kTileBytes = kQB * kHD * 2;       // 32 KB: one [128 x 128] bf16 t
 constexpr int kHalfBytes = kTileBytes / 2;
 constexpr int kPrefillThreads = 128 + 256;  // TMA warp, MMA warp, two idle warps; eight softmax warps
 constexpr int kPrefillSmem = kTileBytes /*Q*/ + 2 * 2 * kTileBytes /*K, V x 2 stages*/ + 1024 + 256 + 6 * kQB * 4 /*row max / sum exchange*/;
+constexpr int kPairThreads = 128 + 128;     // two CTAs per SM: four softmax warps each
+constexpr int kPairSmem = 3 * kTileBytes /*Q, K, V*/ + 1024 + 256;
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -231,7 +237,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tmem_ld_32x32(tO + 32, r[1]);
         tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 64; ++i) o[i] = (o[i] + __uint_as_float(r[i >> 5][i & 31])) * alpha;
+        for (int i = 0; i < 64; i += 2) {
+          add2(o[i], o[i + 1], r[i >> 5][i & 31], r[i >> 5][(i & 31) + 1]);
+          scale2(o[i], o[i + 1], alpha);
+        }
       }
       l_run *= alpha;
       m_run = m_new;
@@ -247,8 +256,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           uint32_t packed[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            float p0 = fast_exp2(fmaf(__uint_as_float(r[i]), p.scale_log2, -mb));
-            float p1 = fast_exp2(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, -mb));
+            const float2 e = fma_f2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), both(p.scale_log2), both(-mb));
+            float p0 = fast_exp2(e.x), p1 = fast_exp2(e.y);
             if (decltype(masked)::value) {
               const int key = key0 + c + i;
               if (!(key <= q_idx + p.offset && key < p.Tk)) p0 = 0.f;
@@ -308,7 +317,211 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
+// The same with two CTAs per SM, for grids that fill them (the head of this file says how).
+__global__ void __launch_bounds__(kPairThreads, 2)
+attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                    const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = base;
+  uint8_t* sK = base + kTileBytes;
+  uint8_t* sV = sK + kTileBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kTileBytes);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;
+  uint64_t* k_empty = bars + 2;
+  uint64_t* v_full = bars + 3;
+  uint64_t* v_empty = bars + 4;
+  uint64_t* s_full = bars + 5;
+  uint64_t* p_full = bars + 6;  // 4 arrivals: P is in TMEM, and O of the block before has been read
+  uint64_t* o_full = bars + 7;  // P V of a block is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
+  const int qb = (p.T + kQB - 1) / kQB - 1 - int(blockIdx.x) / p.Hq;  // heavy blocks first
+  const int head = int(blockIdx.x) % p.Hq, kvh = head / (p.Hq / p.Hk);
+  // causal with a past: the last query of the block sees keys up to (qb + 1) * kQB - 1 + offset
+  const int nblk = min((p.Tk + kKB - 1) / kKB, ((qb + 1) * kQB + p.offset + kKB - 1) / kKB);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 6; ++i) mbar_init(&bars[i], 1);
+    mbar_init(p_full, 4);
+    mbar_init(o_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);  // columns: S (P of 64 keys in the first half of each 64 columns), O
+  pdl_trigger();  // TMEM is held by now
+  // a softmax thread holds a row of O: 128 registers of its own
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  pdl_wait();
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
+      mbar_expect_tx(q_full, kTileBytes);
+      tma_load_2d(sQ, &tmap_q, q_full, head * kHD, qb * kQB);
+      tma_load_2d(sQ + kHalfBytes, &tmap_q, q_full, head * kHD + 64, qb * kQB);
+      for (int j = 0; j < nblk; ++j) {
+        if (!mbar_wait(k_empty, (j & 1) ^ 1, abort_flag, p.status, kStatusTimeoutProducer)) break;
+        mbar_expect_tx(k_full, kTileBytes);
+        tma_load_2d(sK, &tmap_k, k_full, kvh * kHD, j * kKB);
+        tma_load_2d(sK + kHalfBytes, &tmap_k, k_full, kvh * kHD + 64, j * kKB);
+        if (!mbar_wait(v_empty, (j & 1) ^ 1, abort_flag, p.status, kStatusTimeoutProducer)) break;
+        mbar_expect_tx(v_full, kTileBytes);
+        tma_load_2d(sV, &tmap_v, v_full, kvh * kHD, j * kKB);
+        tma_load_2d(sV + kHalfBytes, &tmap_v, v_full, kvh * kHD + 64, j * kKB);
+      }
+    }
+  } else if (warp == 1) {
+    // issued by an elected lane of the converged warp (common.cuh: umma_f8f6f4_block says why)
+    constexpr uint32_t idesc_qk = umma_idesc(128, 128, 1, 1, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc(128, 128, 1, 1, 0, 1);  // B = V is MN-major
+    constexpr uint64_t kHalf = kHalfBytes >> 4;  // dims 64.. of Q and K live in the second swizzled half
+    const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), k_desc = umma_desc_k_sw128(smem_u32(sK));
+    const uint64_t v_desc = umma_desc_mn_sw128(smem_u32(sV), kHalfBytes);
+    auto issue_qk = [&] {  // S takes the place of P of the block before, which the MMAs before have read
+      umma_f16_block(tmem_base, q_desc, k_desc, idesc_qk, 0u);
+      umma_f16_block(tmem_base, q_desc + kHalf, k_desc + kHalf, idesc_qk, 1u, smem_u32(s_full), smem_u32(k_empty));
+    };
+    bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, kStatusTimeoutMma) &&
+              mbar_wait_warp(k_full, 0, abort_flag, p.status, kStatusTimeoutMma);
+    if (ok) {
+      tc_fence_after();
+      issue_qk();
+    }
+    for (int j = 0; ok && j < nblk; ++j) {
+      ok = mbar_wait_warp(v_full, j & 1, abort_flag, p.status, kStatusTimeoutMma) &&
+           (j + 1 == nblk || mbar_wait_warp(k_full, (j + 1) & 1, abort_flag, p.status, kStatusTimeoutMma)) &&
+           mbar_wait_warp(p_full, j & 1, abort_flag, p.status, kStatusTimeoutMma);
+      if (!ok) break;
+      tc_fence_after();
+      umma_pv(tmem_base + 128u, tmem_base, v_desc, idesc_pv, 0u);
+      umma_pv(tmem_base + 128u, tmem_base + 64u, v_desc + 512, idesc_pv, 1u);
+      tc_commit_warp(o_full);
+      tc_commit_warp(v_empty);
+      if (j + 1 < nblk) issue_qk();
+    }
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    pdl_wait();
+    // ----- softmax warps: a thread per query row (TMEM lane) -----
+    const int quarter = warp & 3;
+    const int row = quarter * 32 + lane, q_idx = qb * kQB + row;
+    const uint32_t tS = tmem_base + (uint32_t(quarter * 32) << 16), tO = tS + 128u;
+    float o[128];
+#pragma unroll
+    for (int d = 0; d < 128; ++d) o[d] = 0.f;
+    float m_run = -FLT_MAX, l_run[2] = {0.f, 0.f};  // sums of the first and the second 64 keys of the blocks
+    bool ok = true;
+    for (int j = 0; j < nblk; ++j) {
+      ok = mbar_wait_warp(s_full, j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
+      if (!ok) break;
+      tc_fence_after();
+      const int key0 = j * kKB;
+      // masking is needed where the block reaches past the FIRST query's horizon or past the last key
+      const bool diag = ((j + 1) * kKB - 1 > qb * kQB + p.offset) || ((j + 1) * kKB > p.Tk);
+      const int last = min(q_idx + p.offset, p.Tk - 1) - key0;  // last key of the block that this query sees
+      float mx[2] = {-FLT_MAX, -FLT_MAX};
+      {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32(tS + c * 32, r);
+          tmem_wait_ld();
+          if (!diag) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) mx[i & 1] = fmaxf(mx[i & 1], __uint_as_float(r[i]));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) mx[i & 1] = fmaxf(mx[i & 1], c * 32 + i <= last ? __uint_as_float(r[i]) : -FLT_MAX);
+          }
+        }
+      }
+      const float m_new = fmaxf(m_run, fmaxf(mx[0], mx[1]));
+      const float alpha = fast_exp2((m_run - m_new) * p.scale_log2);
+      m_run = m_new;
+      // probabilities -> bf16 pairs over the scores that have been read
+      const float mb = m_new * p.scale_log2;
+      auto probabilities = [&](auto masked) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float psum = 0.f;
+#pragma unroll
+          for (int c = 0; c < 64; c += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(tS + half * 64 + c, r);
+            tmem_wait_ld();
+            uint32_t packed[16];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              const float2 e = fma_f2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), both(p.scale_log2), both(-mb));
+              float p0 = fast_exp2(e.x), p1 = fast_exp2(e.y);
+              if (decltype(masked)::value) {
+                if (half * 64 + c + i > last) p0 = 0.f;
+                if (half * 64 + c + i + 1 > last) p1 = 0.f;
+              }
+              psum += p0 + p1;
+              const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+              packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            tmem_store_32x16(tS + half * 64 + c / 2, packed);
+          }
+          l_run[half] = __fadd_rn(__fmul_rn(l_run[half], alpha), psum);
+        }
+      };
+      if (diag) probabilities(MaskedBlock<true>());
+      else probabilities(MaskedBlock<false>());
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      if (j > 0) {
+#pragma unroll
+        for (int d = 0; d < 128; d += 2) scale2(o[d], o[d + 1], alpha);
+      }
+      ok = mbar_wait_warp(o_full, j & 1, abort_flag, p.status, kStatusTimeoutEpilogue);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 128; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(tO + c, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) add2(o[c + i], o[c + i + 1], r[i], r[i + 1]);
+      }
+    }
+    if (ok && q_idx < p.T) {
+      const float l_tot = l_run[0] + l_run[1];
+      const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
+      __nv_bfloat16* dst = p.out + (size_t(q_idx) * p.Hq + head) * kHD;
+#pragma unroll
+      for (int c = 0; c < 128; c += 8) {
+        uint4 v;
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(o[c + 2 * e] * inv, o[c + 2 * e + 1] * inv);
+        *reinterpret_cast<uint4*>(dst + c) = v;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem_base, 256);
+}
+
 }  // namespace mfq
+
+// Grids from this size on take the pair form: fewer leave SMs with one CTA, whose longer chain nothing hides.
+constexpr int kPairCtas = 250;
 
 // q: [T, Hq, 128] bf16, k/v: [Tk, Hk, 128] bf16 (contiguous), out: [T, Hq, 128] bf16.  Tk >= T: the first Tk - T keys
 // are the sequence's past (earlier chunks / a restored prefix); query i attends to keys 0 .. i + (Tk - T).
@@ -322,11 +535,15 @@ extern "C" int mfq_attn_prefill_past(const void* q, const void* k, const void* v
   if (make_tmap_2d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, uint64_t(Hk) * D, uint64_t(Hk) * D * 2, kKB, 64)) return -4;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem) != cudaSuccess) return -6;
+    if (cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(attn_prefill_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess)
+      return -6;
     attr = true;
   }
   const PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status};
-  launch_kernel(attn_prefill_kernel, dim3((T + kQB - 1) / kQB * Hq), dim3(kPrefillThreads), kPrefillSmem, stream, tq, tk, tv, p);
+  const int ctas = (T + kQB - 1) / kQB * Hq;
+  if (ctas >= kPairCtas) launch_kernel(attn_prefill_pair_kernel, dim3(ctas), dim3(kPairThreads), kPairSmem, stream, tq, tk, tv, p);
+  else launch_kernel(attn_prefill_kernel, dim3(ctas), dim3(kPrefillThreads), kPrefillSmem, stream, tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 

@@ -316,6 +316,20 @@ __device__ __forceinline__ void fma2(float& c0, float& c1, uint32_t a0, uint32_t
       : "+f"(c0), "+f"(c1)
       : "r"(a0), "r"(a1), "f"(s));
 }
+// Two fp32 operations per instruction, each rounded as by itself: {a, b} * s, {a, b} + {c, d}, {a0, a1} * {b0, b1} + {c0, c1}.
+__device__ __forceinline__ void scale2(float& a, float& b, float s) {
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+f"(a), "+f"(b) : "f"(s));
+}
+__device__ __forceinline__ void add2(float& a, float& b, uint32_t c, uint32_t d) {
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+f"(a), "+f"(b) : "r"(c), "r"(d));
+}
+__device__ __forceinline__ float2 fma_f2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float bf16_to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 struct alignas(16) U4 { uint32_t x, y, z, w; };

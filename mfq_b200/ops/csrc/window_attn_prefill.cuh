@@ -281,7 +281,10 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
           tmem_ld_32x32(tO + lane_base + half * kOut + c, r);
           tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[c + i] = (o[c + i] + __uint_as_float(r[i])) * alpha;
+          for (int i = 0; i < 32; i += 2) {
+            add2(o[c + i], o[c + i + 1], r[i], r[i + 1]);
+            scale2(o[c + i], o[c + i + 1], alpha);
+          }
         }
         tc_fence_before();
         __syncwarp();
@@ -299,13 +302,22 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         float pr[32];
         if (p.cap.out == 0.f) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) pr[i] = fmaf(__uint_as_float(r[i]), p.cap.scale_log2, -m_new);
+          for (int i = 0; i < 32; i += 2) {
+            const float2 e = fma_f2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), both(p.cap.scale_log2), both(-m_new));
+            pr[i] = e.x;
+            pr[i + 1] = e.y;
+          }
         } else if (small) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float s = __uint_as_float(r[i]), t = s * s;
-            const float f = fmaf(t, fmaf(t, fmaf(t, fmaf(t, p.cap.c[4], p.cap.c[3]), p.cap.c[2]), p.cap.c[1]), p.cap.c[0]);
-            pr[i] = fmaf(s, f, -m_new);
+          for (int i = 0; i < 32; i += 2) {  // two scores per instruction
+            const float2 s = make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), t = fma_f2(s, s, both(-0.f));
+            float2 f = fma_f2(t, both(p.cap.c[4]), both(p.cap.c[3]));
+            f = fma_f2(t, f, both(p.cap.c[2]));
+            f = fma_f2(t, f, both(p.cap.c[1]));
+            f = fma_f2(t, f, both(p.cap.c[0]));
+            f = fma_f2(s, f, both(-m_new));
+            pr[i] = f.x;
+            pr[i + 1] = f.y;
           }
         } else {
 #pragma unroll

@@ -147,3 +147,20 @@ def test_prefill_attention_over_tiles_and_heads(t, past, hq, hk, scale):
     check_status()
     # probabilities and the result are rounded to bf16 (2^-9 each, relative): well inside 2 % of (|ref| + rms / 4)
     assert_close(got, ref.attention(q, k, v, scale, causal_offset=past), rel=2e-2, what=f"T={t} past={past}")
+
+
+@pytest.mark.parametrize("t,past,hq,hk", [(257, 0, 84, 21), (385, 126, 64, 16), (1000, 130, 32, 8), (100, 1000, 256, 64)])
+def test_grids_that_fill_two_ctas_per_sm(t, past, hq, hk):
+    """All heads in one call, and a few at a time, which leave SMs free and take the other form: the same bits, with keys that grow."""
+    require_gpu_lib()
+    g = torch.Generator(device="cuda").manual_seed(t)
+    q = torch.randn((t, hq, 128), generator=g, device="cuda").to(torch.bfloat16)
+    k = (torch.randn((past + t, hk, 128), generator=g, device="cuda") * torch.linspace(0.25, 4.0, past + t, device="cuda")[:, None, None]).to(torch.bfloat16)
+    v = torch.randn((past + t, hk, 128), generator=g, device="cuda").to(torch.bfloat16)
+    blocks, per = -(-t // 128), hq // hk
+    assert blocks * hq >= 250 > blocks * per
+    got = ops.kernels.attn_prefill_bf16(q, k, v, 0.09)
+    for h in range(hk):
+        want = ops.kernels.attn_prefill_bf16(q[:, h * per : (h + 1) * per].contiguous(), k[:, h : h + 1].contiguous(), v[:, h : h + 1].contiguous(), 0.09)
+        assert torch.equal(got[:, h * per : (h + 1) * per], want), h
+    check_status()
