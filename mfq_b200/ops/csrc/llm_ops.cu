@@ -58,6 +58,22 @@ __device__ __forceinline__ float from_e4m3(uint8_t c) {
   return __half2float(*reinterpret_cast<__half*>(&h));
 }
 
+// g / (1 + exp(-g)) of two values, rounded as the division rounds it.  A division by itself is most of a gated row's instructions, and for
+// these operands, whose quotient neither over- nor underflows, it needs no cases: a reciprocal by a Newton step, the quotient from
+// it, and two corrections by the remainder, which a fused multiply-add gives exactly (P. Markstein, IBM J. Res. Dev. 34 (1990) 111), two values
+// per instruction.  Others -- large, infinite, NaN, zero and what is nearly that -- divide.
+__device__ __forceinline__ float2 silu2(float2 g) {
+  const float2 d = make_float2(1.f + __expf(-g.x), 1.f + __expf(-g.y));
+  if (!(fabsf(g.x) < 64.f && fabsf(g.y) < 64.f && fabsf(g.x) > 1e-30f && fabsf(g.y) > 1e-30f)) return make_float2(g.x / d.x, g.y / d.y);
+  float2 r, minus = make_float2(-d.x, -d.y);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
+  r = fma_f2(r, fma_f2(minus, r, both(1.f)), r);
+  float2 q = fma_f2(g, r, both(-0.f));
+  q = fma_f2(fma_f2(minus, q, g), r, q);
+  return fma_f2(fma_f2(minus, q, g), r, q);
+}
+
 // ---------------------------------------------------------------------------------------------
 // (x [+ residual]) -> RMSNorm * w -> per-row FP8.  One CTA per row.  Values stay in registers
 // (up to 8 x 8 elements per thread => H <= 8 * 8 * blockDim), so the row is read once.
@@ -164,8 +180,9 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
 // mode 2 (attention output gate): y = x[row, :K] * sigmoid(x2[row, :K]) with x2 a second, separately strided tensor.
 // Up to kRowVecs vectors per thread stay in registers between the maximum and the encoding (every value is a bf16 by then, so a
 // vector is four registers); longer rows are read, and their gates evaluated, a second time.  One pass instead of two, and two
-// values per conversion: 4096 rows of 14336 on a B200 go from 129 to 80 us (reading and writing alone: 44; the gates' exponentials and
-// divisions keep the issue slots two thirds busy), 1000 rows from 36 to 23.
+// values per conversion: 4096 rows of 14336 on a B200 went from 129 to 80 us (reading and writing alone: 44; the gates' exponentials and
+// divisions kept the issue slots two thirds busy), 1000 rows from 36 to 20.  With the gates by silu2 74 and 19, with all loads of a full row
+// requested before the first is used 69 and 18.
 // ---------------------------------------------------------------------------------------------
 constexpr int kRowVecs = 4;
 template <int kMode>
@@ -197,10 +214,10 @@ __global__ void __launch_bounds__(512) quant_rows_kernel(const __nv_bfloat16* __
       uint4 b = *reinterpret_cast<const uint4*>(xr + K + vi * 8);
       const __nv_bfloat16* bb = reinterpret_cast<const __nv_bfloat16*>(&b);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float g = __bfloat162float(ab[j]);
-        const float h = g / (1.f + __expf(-g)) * __bfloat162float(bb[j]);
-        y[j] = __bfloat162float(__float2bfloat16(h));
+      for (int j = 0; j < 8; j += 2) {
+        const float2 h = silu2(make_float2(__bfloat162float(ab[j]), __bfloat162float(ab[j + 1])));
+        y[j] = __bfloat162float(__float2bfloat16(h.x * __bfloat162float(bb[j])));
+        y[j + 1] = __bfloat162float(__float2bfloat16(h.y * __bfloat162float(bb[j + 1])));
       }
     }
   };
@@ -218,6 +235,25 @@ __global__ void __launch_bounds__(512) quant_rows_kernel(const __nv_bfloat16* __
         const uint32_t w[4] = {held[i].x, held[i].y, held[i].z, held[i].w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[j] << 16)), fabsf(__uint_as_float(w[j] & 0xffff0000u))));
+      }
+    } else if (kMode == 1 && nvec == kRowVecs * int(blockDim.x)) {  // likewise, gates and values
+      uint4 up[kRowVecs];
+#pragma unroll
+      for (int i = 0; i < kRowVecs; ++i) {
+        held[i] = *reinterpret_cast<const uint4*>(xr + (threadIdx.x + i * blockDim.x) * 8);
+        up[i] = *reinterpret_cast<const uint4*>(xr + K + (threadIdx.x + i * blockDim.x) * 8);
+      }
+#pragma unroll
+      for (int i = 0; i < kRowVecs; ++i) {
+        const uint32_t a[4] = {held[i].x, held[i].y, held[i].z, held[i].w}, b[4] = {up[i].x, up[i].y, up[i].z, up[i].w};
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&held[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 s = silu2(make_float2(__uint_as_float(a[j] << 16), __uint_as_float(a[j] & 0xffff0000u)));
+          h[j] = __floats2bfloat162_rn(s.x * __uint_as_float(b[j] << 16), s.y * __uint_as_float(b[j] & 0xffff0000u));
+          const float2 y = __bfloat1622float2(h[j]);
+          amax = fmaxf(amax, fmaxf(fabsf(y.x), fabsf(y.y)));
+        }
       }
     } else {
 #pragma unroll
@@ -272,7 +308,7 @@ __global__ void __launch_bounds__(512) quant_rows_kernel(const __nv_bfloat16* __
 
 
 // Many short rows (routed experts' halves): a warp per row and no block, all its vectors requested together.  A block | a warp per row on a
-// B200: 30000 rows of 512 gated values 31.5 | 18.8 us (reading and writing alone: 12), 10000 10.9 | 7.7, 2000 4.0 | 4.3; gated rows of 1024
+// B200: 30000 rows of 512 gated values 31.5 | 17.0 us (reading and writing alone: 12), 10000 10.9 | 6.9, 2000 4.0 | 4.3; gated rows of 1024
 // 30000 39.4 | 37.1, 5120 8.5 | 8.8; plain rows of 1024 30000 31.6 | 11.3, 320 2.0 | 1.7, 80 1.5 | 1.6.
 template <int kMode, int kVecs>
 __global__ void __launch_bounds__(256) quant_short_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out,
@@ -293,12 +329,14 @@ __global__ void __launch_bounds__(256) quant_short_rows_kernel(const __nv_bfloat
 #pragma unroll
   for (int i = 0; i < kVecs; ++i)
     if (lane + i * 32 < nvec) {
-      const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16*>(&a[i]), *bb = reinterpret_cast<const __nv_bfloat16*>(&b[i]);
+      const uint32_t gate[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, up[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float g = __bfloat162float(ab[j]);
-        y[i][j] = kMode == 1 ? __bfloat162float(__float2bfloat16(g / (1.f + __expf(-g)) * __bfloat162float(bb[j]))) : g;
-        amax = fmaxf(amax, fabsf(y[i][j]));
+      for (int j = 0; j < 4; ++j) {
+        const float2 g = make_float2(__uint_as_float(gate[j] << 16), __uint_as_float(gate[j] & 0xffff0000u));
+        const float2 s = kMode == 1 ? silu2(g) : g;
+        y[i][2 * j] = kMode == 1 ? __bfloat162float(__float2bfloat16(s.x * __uint_as_float(up[j] << 16))) : s.x;
+        y[i][2 * j + 1] = kMode == 1 ? __bfloat162float(__float2bfloat16(s.y * __uint_as_float(up[j] & 0xffff0000u))) : s.y;
+        amax = fmaxf(amax, fmaxf(fabsf(y[i][2 * j]), fabsf(y[i][2 * j + 1])));
       }
     }
   amax = warp_max(amax);
@@ -311,53 +349,60 @@ __global__ void __launch_bounds__(256) quant_short_rows_kernel(const __nv_bfloat
 
 // SwiGLU + row quantization for decode-sized batches, one ROW PER CLUSTER of kSplit CTAs: with one CTA per row a batch
 // of 64 rows occupies 64 of 148 SMs and every thread walks its slice twice (amax, then encode, the SiLU evaluated both
-// times).  Here a CTA owns 1/kSplit of the row, keeps its products in registers, and the row maximum is met through
-// distributed shared memory (one float per CTA, two cluster barriers).
+// times).  Here a CTA owns 1/kSplit of the row, keeps its products in registers, and puts its maximum into every CTA's shared memory: the
+// barrier that says that all have is the only one on the way (that all CTAs run, which remote stores need, is asked for before the wait for
+// the kernel before).  64 rows of 14336 on a B200, maxima fetched behind one barrier and kept alive by another: 4.9 us, so 4.3.
 constexpr int kSwigluSplit = 4;
 constexpr int kSwigluVecs = 2;  // 16-byte vectors per thread: covers K <= 8 * 256 * kSwigluVecs * kSwigluSplit
 __global__ void __cluster_dims__(kSwigluSplit, 1, 1) __launch_bounds__(256)
 silu_mul_quant_split_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out, float* __restrict__ scale_out,
                             int K, int in_stride) {
   pdl_trigger();
-  pdl_wait();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   __shared__ float red[33];
-  __shared__ float part_max;
+  __shared__ float maxima[kSwigluSplit];
   const size_t row = blockIdx.x / kSwigluSplit;
   const int part = blockIdx.x % kSwigluSplit;
   const __nv_bfloat16* xr = x + row * in_stride;
   const int nvec = K / 8 / kSwigluSplit, v0 = part * nvec;
+  pdl_wait();
+  uint4 a[kSwigluVecs], b[kSwigluVecs];
+#pragma unroll
+  for (int i = 0; i < kSwigluVecs; ++i) {
+    const int vi = threadIdx.x + i * 256;
+    if (vi < nvec) {
+      a[i] = *reinterpret_cast<const uint4*>(xr + (v0 + vi) * 8);
+      b[i] = *reinterpret_cast<const uint4*>(xr + K + (v0 + vi) * 8);
+    }
+  }
   float y[kSwigluVecs][8];
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < kSwigluVecs; ++i) {
     const int vi = threadIdx.x + i * 256;
     if (vi < nvec) {
-      const uint4 a = *reinterpret_cast<const uint4*>(xr + (v0 + vi) * 8);
-      const uint4 b = *reinterpret_cast<const uint4*>(xr + K + (v0 + vi) * 8);
-      const __nv_bfloat16* ab = reinterpret_cast<const __nv_bfloat16*>(&a);
-      const __nv_bfloat16* bb = reinterpret_cast<const __nv_bfloat16*>(&b);
+      const uint32_t gate[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, up[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float g = __bfloat162float(ab[j]);
-        y[i][j] = __bfloat162float(__float2bfloat16(g / (1.f + __expf(-g)) * __bfloat162float(bb[j])));
-        amax = fmaxf(amax, fabsf(y[i][j]));
+      for (int j = 0; j < 4; ++j) {
+        const float2 s = silu2(make_float2(__uint_as_float(gate[j] << 16), __uint_as_float(gate[j] & 0xffff0000u)));
+        y[i][2 * j] = __bfloat162float(__float2bfloat16(s.x * __uint_as_float(up[j] << 16)));
+        y[i][2 * j + 1] = __bfloat162float(__float2bfloat16(s.y * __uint_as_float(up[j] & 0xffff0000u)));
+        amax = fmaxf(amax, fmaxf(fabsf(y[i][2 * j]), fabsf(y[i][2 * j + 1])));
       }
     }
   }
   amax = block_reduce<true>(amax, red);
-  if (threadIdx.x == 0) part_max = amax;
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  float row_max = 0.f;
-#pragma unroll
-  for (int r = 0; r < kSwigluSplit; ++r) {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x < kSwigluSplit) {
     uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&part_max)), "r"(r));
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-    row_max = fmaxf(row_max, v);
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&maxima[part])), "r"(threadIdx.x));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(amax) : "memory");
   }
-  // nobody leaves (and gives up its shared memory) while a peer may still read it
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  float row_max = maxima[0];
+#pragma unroll
+  for (int r = 1; r < kSwigluSplit; ++r) row_max = fmaxf(row_max, maxima[r]);
   const float scale = fmaxf(row_max, 1e-12f) / kE4M3Max, inv = 1.f / scale;
   if (part == 0 && threadIdx.x == 0) scale_out[row] = scale;
 #pragma unroll

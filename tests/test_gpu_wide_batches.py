@@ -323,3 +323,18 @@ def test_values_that_go_to_whole_pages_together(d, how):
             if 0 <= s - 16 < n and i % 7 == 0:
                 assert torch.equal(kr[s - 16], kd[i]) and torch.equal(vr[s - 16], vd[i])
     check_status()
+
+
+@pytest.mark.parametrize("m,k", [(16, 4096), (600, 4096), (300, 14336), (200, 14336), (5200, 512)])
+def test_gates_of_every_value_round_as_the_division_does(m, k):
+    """All bf16 values as gates, zeros of either sign, subnormal, infinite and NaN among them, through every kernel that quantizes gated rows:
+    the codes of the rows that the plain product of gate and value gives."""
+    require_gpu_lib()
+    g = torch.arange(m * k, device="cuda") % 65521  # a prime: another gate in every place of a row
+    gate = g.to(torch.int32).to(torch.int16).view(torch.bfloat16).view(m, k)
+    gate = torch.where(gate.isfinite() | (torch.arange(m, device="cuda") % 5 == 0)[:, None], gate, torch.ones_like(gate))
+    x = torch.cat([gate, _normal(m, m, k)], 1)
+    q, s = ops.silu_mul_quant(x)
+    want, ws = ops.quant_rows(K.silu_mul(x))
+    assert torch.equal(s.view(torch.int32), ws.view(torch.int32)) and torch.equal(q.view(torch.uint8), want.view(torch.uint8))
+    check_status()
