@@ -65,8 +65,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) w4_gemv_kernel(const W
   const __nv_bfloat16* xr[NT];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) xr[nt] = p.x + size_t(min(nt * 8 + g, p.M - 1)) * p.K + block_in_step * 64 + half * 32;
-  // What this thread's first output is added to: requested under the product instead of after it (it is the only one unless NT * RT is 4
-  // with eight warps).
+  // What this thread's first output is added to: requested under the product instead of after it (it is the only one unless a CTA
+  // has more outputs than threads).
   const int t_first = threadIdx.x / (16 * RT), n_first = n0 + threadIdx.x % (16 * RT);
   const float early = p.residual && t_first < p.M && t_first < 8 * NT && n_first < p.N ? __bfloat162float(p.residual[size_t(t_first) * p.N + n_first]) : 0.f;
   float acc[NT][RT][4] = {};
@@ -154,7 +154,12 @@ static int launch_w4_gemv(const W4GemvParams& p, cudaStream_t stream) {
   // Two blocks of rows per CTA halve the reads of x and the number of CTAs.  Up to 8 tokens that pays where two CTAs per SM are left,
   // or, with 16 warps in one CTA per SM, where K is long: 28672 x 4096 28.0 -> 23.8 us (31.2 with 16 warps), 4096 x 14336 16.0 -> 14.5
   // (20.2 with eight); 6144 x 4096 stays at 9.7.  With 16 tokens, twice the reads, always: 48.4 -> 31.2, 23.7 -> 17.8, 14.3 -> 9.9 us.
+  // Where there are three times as many CTAs as SMs and more, four warps each and four CTAs per SM: a warp has twice the steps, so its
+  // first loads and its CTA's sum are half as much of its time, and they fall under the work of three other CTAs instead of one.
+  // 28672 x 4096 24.3 -> 22.5 us, 128256 x 4096 92.4 -> 82.7 (16 tokens 31.5 -> 28.2, 120 -> 104), 14336 x 2048 7.9 -> 7.1.  Below,
+  // the last wave costs more: 13824 x 5120 15.9 and 16.1 us, 12288 x 4096 11.4 and 13.1.
   const int rows32 = (p.N + 31) / 32, steps = (p.K + 127) / 128;
+  if (rows32 > 3 * 148) return launch_w4_rows<NT, 2, 4, KIND, WHOLE>(p, stream);
   if (rows32 >= 2 * 148 || (NT == 2 && rows32 > 148)) return launch_w4_rows<NT, 2, 8, KIND, WHOLE>(p, stream);
   if (NT == 2 || (rows32 <= 148 && steps >= 64)) return launch_w4_rows<NT, 2, 16, KIND, WHOLE>(p, stream);
   return launch_w4_rows<1, 1, 8, KIND, WHOLE>(p, stream);

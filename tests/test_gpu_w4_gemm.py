@@ -100,6 +100,13 @@ def test_streamed_codes_by_blocks_of_rows(m, n, k, gs):
     test_streamed_codes_match_reference(m, n, k, gs)
 
 
+@pytest.mark.parametrize("m,n,k,gs", [(8, 14208, 64, 32), (8, 14240, 192, 16), (16, 14248, 640, 64)])
+def test_streamed_codes_by_four_warps(m, n, k, gs):
+    """More blocks of 32 rows than three per SM go to CTAs of four warps: the line itself, fewer steps than warps, ragged last rows, and
+    more outputs of a CTA than threads."""
+    test_streamed_codes_match_reference(m, n, k, gs)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 256, 192), (16, 200, 2048)])
 def test_streamed_mxfp4_codes_match_the_tensor_core_form(m, n, k):
     require_gpu_lib()
