@@ -453,7 +453,7 @@ class GogivikModel(RecurrentModel):
             singles = step.num_decode if prefill else t
             out = torch.empty((t, m.heads, kv.v.shape[-1]), dtype=q.dtype, device=q.device)
             if singles:
-                splits = min(self.attn_splits, window_attn.decode_splits(singles, m.kv_heads, m.chunk))
+                splits = min(self.attn_splits, window_attn.decode_splits(singles, m.kv_heads, m.chunk, window_attn.whole_heads(kv)))
                 window_attn.decode(q[:singles], kv, step.block_table[:singles], step.seq_lens[:singles], turn=turn, splits=splits, out=out[:singles], **how)
             if singles < t:
                 window_attn.prefill(q, kv, step.block_table[singles:], step.q_starts[singles:], step.seq_lens[singles:], step.max_q, out=out, **how)

@@ -259,7 +259,7 @@ class TepetarModel(UnquantizedModel):
         singles = step.num_decode if prefill else t
         out = torch.empty((t, l.heads, kv.v.shape[-1]), dtype=q.dtype, device=q.device)
         if singles:
-            splits = min(self.attn_splits, window_attn.decode_splits(singles, l.kv_heads, l.window))
+            splits = min(self.attn_splits, window_attn.decode_splits(singles, l.kv_heads, l.window, window_attn.whole_heads(kv)))
             window_attn.decode(q[:singles], kv, step.block_table[:singles], step.seq_lens[:singles], splits=splits,
                                out=out[:singles], **how)
         if prefill and singles < step.seq_lens.numel():

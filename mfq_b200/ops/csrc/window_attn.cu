@@ -58,6 +58,17 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 }
 
 // DK / DV: upper bounds of the stored widths of a KV head (register arrays); the widths themselves are run-time multiples of 16.
+// Rows of D channels, one after the other, to rows of D + 8: a lane keeps its channels, 32 lanes take 32 * 8 / D rows at a time.
+template <int D>
+__device__ __forceinline__ void copy_page(uint32_t to, const __nv_bfloat16* from, int lane) {
+  constexpr int kLanes = D / 8;  // of a row
+  static_assert(32 % kLanes == 0, "a warp copies whole rows");
+  to += (lane / kLanes * (D + 8) + lane % kLanes * 8) * 2;
+  from += lane * 8;
+#pragma unroll
+  for (int i = 0; i < kWinPage * kLanes / 32; ++i) cp_async16(to + i * (32 / kLanes) * (D + 8) * 2, from + i * 256);
+}
+
 template <int DK, int DV>
 struct WinCfg {
   static constexpr int kStages = 2;  // two pages per warp in flight leave room for three CTAs per SM at 128 + 128 channels
@@ -68,7 +79,11 @@ struct WinCfg {
   }
 };
 
-template <int DK, int DV>
+// kWhole: one map whose widths are the bounds, no bias.  A warp spends some 2 us on a page of 16 keys, with more of them in flight no less:
+// it is bound by what it issues.  The widths known to the compiler leave a copy one instruction, and a page that every query sees whole
+// needs no comparisons.  8 KV heads of 4 queries, 128 channels, 3 splits and their sum, 16 rows of 1024 keys 21.6 -> 20.2 us, of 2000
+// 33.0 -> 32.4; a page that costs less wants fewer splits (decode_splits): 18.6 and 29.8, 64 rows of 2000 115 -> 98, 8 of 900 15.9 -> 13.7.
+template <int DK, int DV, bool kWhole>
 __global__ void __launch_bounds__(kWinWarps * 32)
 window_attn_decode_kernel(const WindowDecodeParams p) {
   pdl_trigger();
@@ -80,7 +95,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
   const int b = bg / p.Hk, g = bg - b * p.Hk, split = blockIdx.y;
   const int per = p.Hq / p.Hk, heads = min(16, per - ht * 16);
   const int head0 = g * per + ht * 16;
-  const int map_dk = p.dk, dk = p.maps * p.dk, dv = p.dv;  // dk: channels of a key row, all maps
+  const int map_dk = kWhole ? DK : p.dk, dk = kWhole ? DK : p.maps * p.dk, dv = kWhole ? DV : p.dv;  // dk: channels of a key row, all maps
   const int pos = p.seq_lens[b] - 1;
   const int lo = first_key(pos, p.window, p.chunk);
   // pages are counted over the visible ones: `kept` pages of first tokens that lie before the window, then the window's
@@ -108,6 +123,11 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
     const uint32_t st = ring + (i % kStages) * stage_bytes;
     const __nv_bfloat16* ks = p.k + (size_t(page) * p.Hk + g) * (kWinPage * dk);
     const __nv_bfloat16* vs = p.v + (size_t(page) * p.Hk + g) * (kWinPage * dv);
+    if constexpr (kWhole) {
+      copy_page<DK>(st, ks, lane);
+      copy_page<DV>(st + kWinPage * kpitch * 2, vs, lane);
+      return;
+    }
     for (int c = lane; c < kWinPage * kch; c += 32) {
       const int row = (c * kinv) >> 16;
       cp_async16(st + (row * kpitch + (c - row * kch) * 8) * 2, ks + c * 8);
@@ -129,7 +149,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
   {
     // a row's own map covers the key channels c0 .. c0 + map_dk - 1
     const int of_map = per / p.maps;
-    const int c0 = (ht * 16 + r0) / of_map * map_dk, c1 = (ht * 16 + r0 + 8) / of_map * map_dk;
+    const int c0 = kWhole ? 0 : (ht * 16 + r0) / of_map * map_dk, c1 = kWhole ? 0 : (ht * 16 + r0 + 8) / of_map * map_dk;
     const __nv_bfloat16* q0 = p.q + (size_t(b) * p.Hq + head0 + r0) * map_dk + t4 * 2 - c0;
     const __nv_bfloat16* q1 = p.q + (size_t(b) * p.Hq + head0 + r0 + 8) * map_dk + t4 * 2 - c1;
 #pragma unroll
@@ -150,7 +170,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
   float m[2] = {-FLT_MAX, -FLT_MAX}, l[2] = {0.f, 0.f};
   const float* bias[2] = {nullptr, nullptr};  // of rows r0 and r0 + 8
   float far[2] = {0.f, 0.f};
-  if (p.extra.bias) {
+  if (!kWhole && p.extra.bias) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       bias[r] = p.extra.bias + size_t(head0 + min(r0 + 8 * r, heads - 1)) * (p.extra.last + 1);
@@ -179,17 +199,47 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
     const int pg = page0 + warp + kWinWarps * i;
     const int key0 = (pg < kept ? pg : pg + skip) * kWinPage + t4 * 2;
     float mx[2] = {-FLT_MAX, -FLT_MAX};
-    const bool near = pos - (key0 - t4 * 2 + kWinPage - 1) < p.extra.last;  // some key of the page is nearer than the last bias
+    if (kWhole) {
+      const bool small = fabsf(s[0][0]) <= p.cap.small && fabsf(s[0][1]) <= p.cap.small && fabsf(s[0][2]) <= p.cap.small && fabsf(s[0][3]) <= p.cap.small &&
+                         fabsf(s[1][0]) <= p.cap.small && fabsf(s[1][1]) <= p.cap.small && fabsf(s[1][2]) <= p.cap.small && fabsf(s[1][3]) <= p.cap.small;
+      if (__all_sync(0xffffffffu, small)) {
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int key = key0 + nt * 8 + (e & 1);
-        float c = score_any(p.cap, s[nt][e]);
-        if (p.extra.bias) c += near ? bias[e >> 1][min(max(pos - key, 0), p.extra.last)] * kLog2e : far[e >> 1];
-        s[nt][e] = (key >= lo || key < p.keep) && key <= pos ? c : -FLT_MAX;
-        mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
+          for (int e = 0; e < 4; ++e) s[nt][e] = score_small(p.cap, s[nt][e]);
+      } else {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[nt][e] = score_any(p.cap, s[nt][e]);
       }
+      const int at = key0 - t4 * 2;
+      if (at + kWinPage - 1 > pos || (at < lo && at + kWinPage > p.keep)) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int key = key0 + nt * 8 + (e & 1);
+            s[nt][e] = (key >= lo || key < p.keep) && key <= pos ? s[nt][e] : -FLT_MAX;
+          }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
+    } else {
+      const bool near = pos - (key0 - t4 * 2 + kWinPage - 1) < p.extra.last;  // some key of the page is nearer than the last bias
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int key = key0 + nt * 8 + (e & 1);
+          float c = score_any(p.cap, s[nt][e]);
+          if (p.extra.bias) c += near ? bias[e >> 1][min(max(pos - key, 0), p.extra.last)] * kLog2e : far[e >> 1];
+          s[nt][e] = (key >= lo || key < p.keep) && key <= pos ? c : -FLT_MAX;
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
+        }
+    }
     float alpha[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -373,18 +423,26 @@ int launch_attn_merge(const float* part, const float* part_ml, const float* sink
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 
-template <int DK, int DV>
-static int launch_window_decode(const WindowDecodeParams& p, const WindowMergeParams& mp, int B, cudaStream_t stream) {
+template <int DK, int DV, bool kWhole>
+static int launch_window_pages(const WindowDecodeParams& p, const WindowMergeParams& mp, int B, cudaStream_t stream) {
   const int smem = WinCfg<DK, DV>::smem_bytes(p.dk * p.maps, p.dv);
   static int allowed = 0;
   if (smem > allowed) {
-    if (cudaFuncSetAttribute(window_attn_decode_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -6;
+    if (cudaFuncSetAttribute(window_attn_decode_kernel<DK, DV, kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -6;
     allowed = smem;
   }
-  launch_kernel(window_attn_decode_kernel<DK, DV>, dim3(B * p.Hk * p.head_tiles, p.splits), dim3(kWinWarps * 32), smem, stream, p);
+  launch_kernel(window_attn_decode_kernel<DK, DV, kWhole>, dim3(B * p.Hk * p.head_tiles, p.splits), dim3(kWinWarps * 32), smem, stream, p);
   if (p.splits > 1 || p.maps > 1)
     launch_kernel(window_attn_merge_kernel, dim3(B * mp.heads), dim3(128), 0, stream, p.part, p.part_ml, p.out, mp);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
+}
+
+template <int DK, int DV>
+static int launch_window_decode(const WindowDecodeParams& p, const WindowMergeParams& mp, int B, cudaStream_t stream) {
+  if constexpr (DK == DV && DK <= 256) {
+    if (p.maps == 1 && p.dk == DK && p.dv == DV && !p.extra.bias) return launch_window_pages<DK, DV, true>(p, mp, B, stream);
+  }
+  return launch_window_pages<DK, DV, false>(p, mp, B, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

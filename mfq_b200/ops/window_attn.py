@@ -160,17 +160,28 @@ def turn_back(o: torch.Tensor, turn: ValueTurn, positions, pairs: bool = False) 
     return o
 
 
-def decode_splits(batch: int, kv_heads: int, keys: int) -> int:
+def whole_heads(kv) -> bool:
+    """Pages of one map whose key and value widths are the bounds of a decode kernel: it takes them without run-time widths."""
+    return kv.k.shape[-1] == kv.v.shape[-1] and kv.k.shape[-1] in (64, 128, 256)
+
+
+def decode_splits(batch: int, kv_heads: int, keys: int, whole: bool = False) -> int:
     """KV splits per (sequence, KV head) over ``keys`` visible keys, fitted to a sweep on B200 (batch 1 .. 128, windows 1024 and
     4096): a batch that leaves SMs free takes the most splits that keep the grid below 400 CTAs (at most 16, 64 keys each); one
     that comes near a wave of three CTAs per SM evens its last wave out with up to 5 splits of at least 256 keys; more is not
-    split."""
+    split.
+
+    ``whole`` (see ``whole_heads``, and no bias): a page costs half as much there, so the sums of the splits count more.  300 CTAs are
+    enough, of 128 keys at least, and a grid of one wave is not split: 128 (sequence, KV head) pairs of 1024 keys 20.2 us in 3
+    splits, 18.6 in 2; 64 of 2048 20.8 in 6, 19.9 in 4; 256 of 2000 56.8 in 5, 51.9 in 1; 512 of 2000 103 in 1, 97.6 in 2."""
     n, slots = max(1, batch * kv_heads), 148 * 3
+    if whole and n <= slots:
+        return max(1, min(300 // n, keys // 128, 16))
     if n <= 200:
         return max(1, min(400 // n, keys // 64, 16))
     if n > 600:
         return 1
-    choices = [s for s in range(1, 6) if s == 1 or keys // s >= 256]
+    choices = [s for s in range(1, 3 if whole else 6) if s == 1 or keys // s >= 256]
     return min(choices, key=lambda s: -(-n * s // slots) * keys / s + 20 * s)
 
 

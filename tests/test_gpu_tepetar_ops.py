@@ -52,6 +52,27 @@ def test_products(m, n, k, dtype):
     check_status()
 
 
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("per,window,keep,chunk,splits,cap", [(1, 1 << 30, 0, 0, 1, 0.0), (4, 40, 0, 0, 3, 50.0), (20, 33, 19, 0, 2, 0.5), (16, 1, 0, 0, 1, 0.0),
+                                                              (8, 1 << 30, 0, 48, 2, 3.0)])
+def test_pages_of_the_bounds_widths(d, per, window, keep, chunk, splits, cap):
+    """Heads of 64, 128 or 256 channels without a bias go through a kernel that knows the widths: the bits of the general one, which a
+    bias of zeros selects.  Lengths at the edges of pages, of the window, of the kept keys and of the splits; an empty row."""
+    from types import SimpleNamespace
+    from mfq_b200.ops import window_attn
+    hk, lens = 2, [0, 1, 15, 16, 17, 33, 48, 49, 64, 100, 257]
+    pages = 17
+    k, v = rnd(len(lens) * pages, hk, 16, d), rnd(len(lens) * pages, hk, 16, d)
+    table = torch.randperm(len(lens) * pages, device="cuda", dtype=torch.int32).view(len(lens), pages)
+    q, n = rnd(len(lens), hk * per, d, scale=3.0), torch.tensor(lens, device="cuda", dtype=torch.int32)
+    how = dict(window=window, keep=keep, chunk=chunk, splits=splits, cap=cap, scale=d ** -0.5)
+    kv = SimpleNamespace(k=k, v=v)
+    got = window_attn.decode(q, kv, table, n, **how)
+    want = window_attn.decode(q, kv, table, n, bias=window_attn.DistanceBias.from_table(torch.zeros(hk * per, 1, device="cuda")), **how)
+    check_status()
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("m", [1, 8, 9, 16])
 @pytest.mark.parametrize("n,k", [(16, 2048), (256, 4096), (2368, 2056), (48, 4104), (32, 14336)])
 def test_streaming_product_of_few_rows_of_weights(m, n, k):
