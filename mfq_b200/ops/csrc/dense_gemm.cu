@@ -270,8 +270,9 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 
 // kDeep: for grids that leave SMs idle, where a CTA's time is the latency of its loads: 16 K blocks of a warp's weights are requested at
 // once, ahead of the kernel before, and 8 blocks of the tokens at a time after it.
+// One CTA per SM is said to the compiler: without it, it keeps to 170 registers and takes the loads of a batch one after the other.
 template <int NT, bool kDeep>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kDeep ? 1 : 0)
 dense_gemv_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x, int ldx, const DenseParams p) {
   pdl_trigger();
   constexpr int kBatch = kDeep ? 16 : 4;  // K blocks whose weights are requested before the first MMA of the batch
@@ -364,13 +365,15 @@ static int launch_dense_gemv_as(const void* w, const void* x, int ldx, const Den
                 static_cast<const __nv_bfloat16*>(x), ldx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
-// Up to a CTA per SM, and two batches of the shallow form at least.  Shallow | deep on a B200 (cold weights): 16 x 256 x 4096 10.4 | 8.3 us,
-// 1 x 256 x 4096 6.3 | 4.1, 16 x 2048 x 4096 12.0 | 9.8, 1 x 2048 x 2048 4.2 | 3.8, 16 x 512 x 14336 39.4 | 30.3; but 16 x 256 x 1024 3.2 | 3.7, and
-// with several CTAs per SM 8 x 6144 x 4096 11.9 | 17.4.
-constexpr int kGemvDeepCtas = 148, kGemvDeepK = 2048;
+// Up to a CTA per SM, and one batch of the shallow form at least; up to two, one after the other, where that is a whole batch of the
+// deep form.  Shallow | deep on a B200 (cold weights): 16 x 256 x 4096 10.4 | 3.5 us, 1 x 256 x 4096 6.3 | 2.3, 16 x 2048 x 4096 12.0 | 5.3,
+// 16 x 512 x 14336 39.4 | 11.2, 16 x 1024 x 1024 3.4 | 2.3, 16 x 256 x 512 2.5 | 2.1; two to an SM 8 x 4096 x 4096 10.4 | 8.8, 8 x 4096 x 14336
+// 32.8 | 24.1, but 8 x 4096 x 2048 5.4 | 5.8, and three 8 x 6144 x 4096 11.8 | 12.3.
+constexpr int kGemvDeepCtas = 2 * 148, kGemvDeepK = 512, kGemvDeepSecondK = 4096;
 template <int NT>
 static int launch_dense_gemv(const void* w, const void* x, int ldx, const DenseParams& p, int entries, cudaStream_t stream) {
-  const bool deep = !p.tiles && p.N / 16 * p.groups <= kGemvDeepCtas && p.K >= kGemvDeepK;
+  const int tiles = p.N / 16 * p.groups;
+  const bool deep = !p.tiles && tiles <= kGemvDeepCtas && p.K >= (tiles <= kGemvDeepCtas / 2 ? kGemvDeepK : kGemvDeepSecondK);
   return deep ? launch_dense_gemv_as<NT, true>(w, x, ldx, p, entries, stream) : launch_dense_gemv_as<NT, false>(w, x, ldx, p, entries, stream);
 }
 

@@ -18,6 +18,7 @@ BIAS, GLU, GELU, GELU_GLU, SOFTCAP, ADD, RELU_GLU, SILU_GLU, FLOAT, RELU2 = rang
 UNITS = {"gelu": GELU_GLU, "relu": RELU_GLU, "silu": SILU_GLU}  # act(gate) * up
 ACTIVATIONS = {"relu2": RELU2}  # max(y, 0)^2
 GEMV_ROWS, GEMV_MID_ROWS, GEMV_MID_WEIGHTS = 8, 16, 8 << 20
+GEMV_FEW_CTAS, GEMV_DEEP_CTAS = 148, 2 * 148  # of 16 weight rows each: one per SM, and where the streaming kernel's deep form ends
 
 
 def up(n: int, m: int = 16) -> int:
@@ -45,6 +46,20 @@ def _most_splits(tiles: int, blocks: int, small: bool, sms: int) -> int:
 PAIR = -2  # as a number of K splits: the product runs on pairs of SMs (csrc/dense_pair.cu)
 
 
+def _streams(m: int, n: int, k: int) -> bool:
+    """Whether up to 16 rows go to the weight-streaming kernel.  On B200 (streaming | tcgen05, cold weights, us): a CTA per SM always does,
+    16 x 2368 x 4096 5.7 | 9.4, 16 x 2048 x 14336 14.0 | 14.9, 1 x 2368 x 18944 16.3 | 17.8; two per SM up to 4096 inputs, 16 x 4096 x 4096
+    10.2 | 10.6, 1 x 4096 x 4096 8.0 | 9.2, but 4096 x 8192 18.0 | 14.9 with 16 rows and 14.1 | 13.8 with one.  Three fit no longer with 16 rows,
+    6144 x 4096 16.1 | 12.4, and with 8 only just: 11.8 | 12.1, 6144 x 8192 20.2 | 19.3.  Wider matrices stream slower than the ring of TMA copies at any
+    length: 1 x 8192 x 4096 17.7 | 13.5, 8 x 28672 x 4096 51.5 | 37.6, 1 x 128256 x 4096 166 | 149, 8 x 32768 x 512 10.6 | 6.8."""
+    ctas = -(-n // 16)
+    if ctas <= GEMV_FEW_CTAS:
+        return True
+    if m > GEMV_ROWS:
+        return n * k <= GEMV_MID_WEIGHTS or (ctas <= GEMV_DEEP_CTAS and k <= 4096)
+    return ctas < 512 and k <= (4096 if ctas <= GEMV_DEEP_CTAS else 6144)
+
+
 @lru_cache(maxsize=4096)  # sizes only; a prompt asks for the same few once per layer
 def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[int, int]:
     """``(token tile, K splits)`` of a bf16 product ``[m, k] x [n, k]^T``; tile 0 is the weight-streaming kernel, splits
@@ -56,7 +71,7 @@ def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[i
     of o_proj 4096 x 4096 50 against 64; what stays here are narrow or split products (300 x 4096 x 14336: 52 against 54 us).
     Sums in parts (:func:`pair_sums`), as many as there are accumulators, cost a pair 0.5 to 1 us: 300 x 4096 x 4096 in two 19.5 us there
     against 21.2 here, 200 x 1536 x 1536 in three 10.05 against 9.95, the least favourable."""
-    if m <= GEMV_ROWS or (m <= GEMV_MID_ROWS and n * k <= GEMV_MID_WEIGHTS):
+    if m <= GEMV_MID_ROWS and _streams(m, n, k):
         return 0, 1
     rows, blocks = math.ceil(n / 128), math.ceil(k / 64)
     for tile in (16, 32, 64, 128):
@@ -142,7 +157,8 @@ class DenseLinear:
         elif table is not None:
             assert table.shape[1] == n and table.is_contiguous() and table.dtype == x.dtype and ids.dtype == torch.int32
             kind = GELU
-        t, s = plan(m, n * g, k, pairs=g == 1 and tile is None and splits is None)
+        # a matrix per head is narrower than a tile of the tensor cores
+        t, s = (0, 1) if g > 1 and m <= GEMV_ROWS else plan(m, n * g, k, pairs=g == 1 and tile is None and splits is None)
         t, s = (t if tile is None else tile), (s if splits is None else splits)
         if s == PAIR and splits is None:
             s = -1 - pair_sums(m, n, k)

@@ -87,6 +87,39 @@ def test_streaming_product_of_few_rows_of_weights(m, n, k):
     check_status()
 
 
+@pytest.mark.parametrize("m", [1, 8, 16])
+@pytest.mark.parametrize("n,k", [(16, 504), (16, 512), (2368, 520), (2384, 4088), (2384, 4096), (4736, 4104)])
+def test_streaming_product_at_the_lines_of_its_deep_form(m, n, k):
+    """Both sides of the sizes from which a warp requests sixteen K blocks at once, against the other form: the bits of a grid too large for it."""
+    from mfq_b200.ops import dense
+    x, w = rnd(m, k), rnd(n, k, scale=k ** -0.5)
+    got = dense.DenseLinear(w)(x, fp32=True, tile=0)
+    close(got, (x.double() @ w.double().T).cpu(), 2e-5)
+    many = w.repeat(297 * 16 // n + 1, 1)
+    assert many.shape[0] // 16 > 296 and torch.equal(dense.DenseLinear(many)(x, fp32=True, tile=0)[:, :n], got)
+    check_status()
+
+
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("n,k,streams", [(8176, 72, True), (8192, 72, False), (8208, 4104, False), (2384, 4104, False), (4752, 4104, True), (2368, 8200, True)])
+def test_few_rows_by_either_kernel(m, n, k, streams):
+    """Up to 16 rows at the lines between the streaming kernel and the tensor cores, ragged K, with each kind of result."""
+    from mfq_b200.ops import dense
+    if m <= 8:
+        assert (dense.plan(m, n, k)[0] == 0) == streams
+    x, w, b = rnd(m, k + 8)[:, :k], rnd(n, k, scale=k ** -0.5), rnd(n, dtype=FP32)
+    want = x.double() @ w.double().T + b.double()
+    close(dense.DenseLinear(w, b)(x, fp32=True), want.cpu(), 2e-5, "fp32")
+    stream = rnd(m, n, dtype=FP32)
+    close(dense.DenseLinear(w, b)(x, add_to=stream.clone(), scale=0.5), (0.5 * want + stream.double()).cpu(), 2e-5, "added")
+    close(dense.DenseLinear(w, b)(x, softcap=30.0), (30 * torch.tanh(want / 30)).cpu(), 2e-2, "capped")
+    gate, up = w[: n // 2], w[n // 2 :]
+    glu = dense.DenseLinear(dense.interleave_glu(gate, up), glu="silu")(x)
+    g, u = x.double() @ gate.double().T, x.double() @ up.double().T
+    close(glu, (torch.nn.functional.silu(g) * u).cpu(), 2e-2, "gated")
+    check_status()
+
+
 @pytest.mark.parametrize("tile", [16, 32, 64, 128, 256])
 @pytest.mark.parametrize("splits", [1, 2, 3, 5, 8])
 def test_every_tile_and_split(tile, splits):
