@@ -1,6 +1,6 @@
 // Paged GQA decode / verify attention over FP8 pages, built to run at HBM speed.
 //
-// One CTA = (sequence, KV head, KV split); its 4 warps take pages round-robin.  Every warp owns a private
+// One CTA = (sequence, KV head, KV split); its warps (4, 8 or 16) take pages round-robin.  Every warp owns a private
 // ring of page buffers in shared memory that it fills with bulk async copies (one 2 KB K block, one 2 KB V
 // block and two 64 B scale rows per page and head; completion on an mbarrier), so dozens of KB are in flight
 // per SM without any CTA-wide synchronisation.  The math is tensor-core `mma.sync.m16n8k16` in f16 with fp32
@@ -47,15 +47,15 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int D, int kAttnStages>
+template <int D, int kAttnStages, int kWarps = 4>
 struct AttnSmem {
   static constexpr int kPageBytes = 16 * D;                    // one head's K (or V) page
   static constexpr int kStageBytes = 2 * kPageBytes + 128;     // K, V, k scales, v scales
   static constexpr int kWarpBytes = kAttnStages * kStageBytes;  // also the merge scratch: needs >= 16*D*4 + 128
-  static constexpr int kTotal = 4 * kWarpBytes + 4 * kAttnStages * 8 + 16;
+  static constexpr int kTotal = kWarps * kWarpBytes + kWarps * kAttnStages * 8 + 16;
 };
 
-// kAttnStages: pages in flight per warp; kMinBlocks: CTAs per SM the register allocation is held to.
+// kAttnStages: pages in flight per warp; kWarps: of a CTA, which take alternate pages; kMinBlocks: CTAs per SM the register allocation is held to.
 template <int D, int kAttnStages, int kMinBlocks>
 __global__ void __launch_bounds__(128, kMinBlocks)
 paged_attn_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* __restrict__ k_cache,
@@ -284,8 +284,8 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
 // Against the 16-row form this halves the MMAs (one 8-wide column block instead of two of which one was dead), the
 // softmax arithmetic (4 scores per thread, none wasted on dead rows) and the output accumulators (D/4 registers), which
 // leaves room for a fourth CTA per SM.
-template <int D, int kAttnStages, int kMinBlocks>
-__global__ void __launch_bounds__(128, kMinBlocks)
+template <int D, int kAttnStages, int kMinBlocks, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, kMinBlocks)
 paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* __restrict__ k_cache,
                            const uint8_t* __restrict__ v_cache, const float* __restrict__ k_scale,
                            const float* __restrict__ v_scale, const int* __restrict__ block_table,
@@ -293,15 +293,22 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
                            float* __restrict__ part_acc, float* __restrict__ part_ml, int Hq, int Hk, int max_pages,
                            float scale_log2, int q_len, int* status) {
   pdl_trigger();
-  pdl_wait();
-  using L = AttnSmem<D, kAttnStages>;
+  using L = AttnSmem<D, kAttnStages, kWarps>;
   constexpr int KSTEPS = D / 16, NBD = D / 16;
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g8 = lane >> 2, c = lane & 3;
   uint8_t* ring = smem + warp * L::kWarpBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 4 * L::kWarpBytes) + warp * kAttnStages;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 4 * L::kWarpBytes + 4 * kAttnStages * 8);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kWarps * L::kWarpBytes) + warp * kAttnStages;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kWarps * L::kWarpBytes + kWarps * kAttnStages * 8);
+
+  if (threadIdx.x == 0) *abort_flag = 0;
+  if (lane == 0) {
+    for (int s = 0; s < kAttnStages; ++s) mbar_init(&bars[s], 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  pdl_wait();
 
   const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z;
   const int G = Hq / Hk;
@@ -311,14 +318,7 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
   const int per_split = (pages_total + nsplit - 1) / nsplit;
   const int page_begin = split * per_split;
   const int page_end = min(pages_total, page_begin + per_split);
-  const int my_pages = page_end > page_begin + warp ? (page_end - page_begin - warp + 3) / 4 : 0;
-
-  if (threadIdx.x == 0) *abort_flag = 0;
-  if (lane == 0) {
-    for (int s = 0; s < kAttnStages; ++s) mbar_init(&bars[s], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
+  const int my_pages = page_end > page_begin + warp ? (page_end - page_begin - warp + kWarps - 1) / kWarps : 0;
 
   const int* bt = block_table + size_t(seq) * max_pages;
   auto issue = [&](int i, int page) {  // lane 0 only: start the copies of this warp's i-th page
@@ -332,9 +332,9 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
     bulk_load(st + 2 * L::kPageBytes + 64, v_scale + ph * 16, 64, &bars[s]);
   };
   if (lane == 0)
-    for (int i = 0; i < min(my_pages, kAttnStages); ++i) issue(i, bt[page_begin + warp + 4 * i]);
+    for (int i = 0; i < min(my_pages, kAttnStages); ++i) issue(i, bt[page_begin + warp + kWarps * i]);
   // the page id of the copy that the next iteration starts is fetched one iteration ahead
-  int next_page = (lane == 0 && kAttnStages < my_pages) ? bt[page_begin + warp + 4 * kAttnStages] : 0;
+  int next_page = (lane == 0 && kAttnStages < my_pages) ? bt[page_begin + warp + kWarps * kAttnStages] : 0;
 
   // ---- Q as the B operand: column g8 = pair (qr, g); dims in the K page's order ----
   uint32_t qb[KSTEPS][2];
@@ -380,7 +380,7 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
     const uint8_t* sV = st + L::kPageBytes;
     const float* sKs = reinterpret_cast<const float*>(st + 2 * L::kPageBytes);
     const float* sVs = sKs + 16;
-    const int tok0 = (page_begin + warp + 4 * i) << 4;
+    const int tok0 = (page_begin + warp + kWarps * i) << 4;
 
     // ---- S^T = K Q^T: rows = tokens g8 and g8 + 8, columns 2c and 2c + 1 ----
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -448,11 +448,11 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
     __syncwarp();
     if (lane == 0 && i + kAttnStages < my_pages) {
       issue(i + kAttnStages, next_page);
-      if (i + 1 + kAttnStages < my_pages) next_page = bt[page_begin + warp + 4 * (i + 1 + kAttnStages)];
+      if (i + 1 + kAttnStages < my_pages) next_page = bt[page_begin + warp + kWarps * (i + 1 + kAttnStages)];
     }
   }
 
-  // ---- merge: the lanes that share a column, then the four warps (the page ring is reused as scratch) ----
+  // ---- merge: the lanes that share a column, then the warps (the page ring is reused as scratch) ----
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 4);
@@ -478,10 +478,10 @@ paged_attn_decode_t_kernel(const __nv_bfloat16* __restrict__ q, const uint8_t* _
     const int r = idx / D, d = idx % D;
     float mm = kNeg;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) mm = fmaxf(mm, reinterpret_cast<const float*>(smem + w * L::kWarpBytes)[16 * D + 2 * r]);
+    for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, reinterpret_cast<const float*>(smem + w * L::kWarpBytes)[16 * D + 2 * r]);
     float ll = 0.f, a = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       const float* wo = reinterpret_cast<const float*>(smem + w * L::kWarpBytes);
       const float cw = exp2f(wo[16 * D + 2 * r] - mm);
       ll += wo[16 * D + 2 * r + 1] * cw;
@@ -541,15 +541,16 @@ __global__ void attn_reduce_log2_kernel(const float* __restrict__ part_acc, cons
   out[hq * D + d] = __float2bfloat16(ll > 0.f ? a / ll : 0.f);
 }
 
-template <int D, int kAttnStages, int kMinBlocks, bool kTokensAsRows>
+template <int D, int kAttnStages, int kMinBlocks, bool kTokensAsRows, int kWarps = 4>
 static int launch_attn_v(const void* q, const void* k_cache, const void* v_cache, const float* k_scale,
                          const float* v_scale, const int* block_table, const int* seq_lens, void* out, float* part_acc,
                          float* part_ml, int B, int Hq, int Hk, int max_pages, float sm_scale, int splits, int q_len,
                          int* status, cudaStream_t stream) {
-  using L = AttnSmem<D, kAttnStages>;
+  using L = AttnSmem<D, kAttnStages, kWarps>;
+  static_assert(kTokensAsRows || kWarps == 4, "the 16-row form has four warps");
   static_assert(L::kWarpBytes >= 16 * D * 4 + 128, "the per-warp ring doubles as the merge scratch");
   auto kernel = [] {
-    if constexpr (kTokensAsRows) return &paged_attn_decode_t_kernel<D, kAttnStages, kMinBlocks>;
+    if constexpr (kTokensAsRows) return &paged_attn_decode_t_kernel<D, kAttnStages, kMinBlocks, kWarps>;
     else return &paged_attn_decode_mma_kernel<D, kAttnStages, kMinBlocks>;
   }();
   static bool attr[64] = {};
@@ -560,7 +561,7 @@ static int launch_attn_v(const void* q, const void* k_cache, const void* v_cache
     attr[dev] = true;
   }
   const float scale_log2 = sm_scale * 1.4426950408889634f;
-  launch_kernel(kernel, dim3(B, Hk, splits), dim3(128), L::kTotal, stream, static_cast<const __nv_bfloat16*>(q),
+  launch_kernel(kernel, dim3(B, Hk, splits), dim3(kWarps * 32), L::kTotal, stream, static_cast<const __nv_bfloat16*>(q),
                 static_cast<const uint8_t*>(k_cache), static_cast<const uint8_t*>(v_cache), k_scale, v_scale, block_table,
                 seq_lens, static_cast<__nv_bfloat16*>(out), part_acc, part_ml, Hq, Hk, max_pages, scale_log2, q_len, status);
   if (cudaGetLastError() != cudaSuccess) return -7;
@@ -584,6 +585,13 @@ static int launch_attn(const void* q, const void* k_cache, const void* v_cache, 
   if constexpr (D <= 128) {
     if (narrow && variant == 2) return launch_attn_v<D, 2, 5, true>(MFQ_ATTN_ARGS);
     if (narrow && variant == 3) return launch_attn_v<D, 4, 3, true>(MFQ_ATTN_ARGS);
+    // A warp takes some 0.8 us for a page whether or not others run beside it, so a grid that leaves room gives its pages to more warps:
+    // as many an SM as four CTAs of four.  Sixteen to a CTA pay where a split has the pages for them.  Four | eight | sixteen warps, the
+    // sum of the splits included: one row of 2048 tokens in 64 CTAs 9.0 | 7.9 | 6.8 us, of 600 in 16 7.9 | 7.9 | 7.0, of 20 in 8 3.3 | 3.1 | 3.9;
+    // 4 of 1024 in 128 9.9 | 7.2 | 7.7, 8 of 1024 in 256 11.1 | 10.0 | 13.1; but 19 of 700 in 304 14.1 | 15.7.
+    const int ctas = B * Hk * splits;
+    if (narrow && variant == 0 && splits > 1 && ctas <= 64) return launch_attn_v<D, 3, 1, true, 16>(MFQ_ATTN_ARGS);
+    if (narrow && variant == 0 && ctas <= 2 * 148) return launch_attn_v<D, 3, 2, true, 8>(MFQ_ATTN_ARGS);
     if (narrow) return launch_attn_v<D, 3, 4, true>(MFQ_ATTN_ARGS);
     return launch_attn_v<D, 3, 3, false>(MFQ_ATTN_ARGS);
   } else {

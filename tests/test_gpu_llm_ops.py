@@ -8,7 +8,7 @@ import torch
 from mfq_b200 import ops
 from mfq_b200.engine.kv_cache import PagedKVCache
 from mfq_b200.ops import reference as ref
-from gpu_common import assert_close, require_gpu_lib
+from gpu_common import assert_close, check_status, require_gpu_lib
 
 pytestmark = pytest.mark.gpu
 
@@ -99,6 +99,28 @@ def test_rope_kv_write_and_decode_attention(hq, hk, d):
     for splits in (1, 3, 8, 9, 40):
         got = ops.paged_attn_decode(q, kv, cache.block_table, seq_lens, sm_scale=1 / math.sqrt(d), splits=splits)
         assert_close(got, want, rel=2e-2, what=f"decode attention splits={splits}")
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,hk,splits", [(8, 8, 1), (32, 1, 2), (33, 1, 2), (37, 8, 1), (37, 4, 2), (37, 2, 4), (149, 2, 1), (1, 1, 32)])
+def test_decode_attention_by_warps_of_a_cta(b, hk, splits, d):
+    """Grids at the lines between sixteen, eight and four warps a CTA; lengths of no page to many for a warp, splits without pages."""
+    require_gpu_lib()
+    cache = make_cache(hk, d, b, 656)
+    kv = cache.layer(0)
+    for pages in (kv.k, kv.v):
+        pages.view(torch.float8_e4m3fn).copy_(torch.randn(pages.shape, device="cuda").mul_(20))
+    kv.k_scale.uniform_(0.001, 0.02)
+    kv.v_scale.uniform_(0.001, 0.02)
+    lens = [(1, 16, 17, 640, 129, 656, 33, 300)[i % 8] for i in range(b)]
+    for i, n in enumerate(lens):
+        cache.assign(i, i, n)
+    q = torch.randn((b, 4 * hk, d), device="cuda").to(torch.bfloat16)
+    seq_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    want = ref.paged_attn_decode(q, kv, cache.block_table, seq_lens, 1 / math.sqrt(d))
+    got = ops.paged_attn_decode(q, kv, cache.block_table, seq_lens, sm_scale=1 / math.sqrt(d), splits=splits)
+    check_status()
+    assert_close(got, want, rel=2e-2, what=f"decode attention of {b} x {hk} in {splits}")
 
 
 @pytest.mark.parametrize("hq,hk,d,ql", [(8, 2, 128, 4), (8, 2, 128, 2), (4, 4, 128, 3), (8, 1, 256, 1), (16, 2, 256, 2)])
