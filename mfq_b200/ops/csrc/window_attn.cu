@@ -5,8 +5,8 @@
 // vector per token; queries are ordered [KV head][map][query head of the KV head].  With one map a head may have a score bias by
 // distance and a sink (window_attn.cuh: ScoreExtra).
 //
-//   window_attn_decode_kernel   bf16, one query per sequence.  A CTA serves one (sequence, KV head, KV split); its four warps
-//                               take alternate pages that hold visible keys through private cp.async rings.  The (up to 16)
+//   window_attn_decode_kernel   bf16, one query per sequence.  A CTA serves one (sequence, KV head, KV split); its four or eight
+//                               warps take alternate pages that hold visible keys through private cp.async rings.  The (up to 16)
 //                               queries of the KV head are the rows of m16n8k16 MMAs: S = Q K^T, probabilities go from
 //                               accumulators straight into the A operand of P V.  Queries of both maps share the rows (and the
 //                               values): a row is zero on the key channels of the other map.  Warps (and splits) merge at the end.
@@ -69,12 +69,12 @@ __device__ __forceinline__ void copy_page(uint32_t to, const __nv_bfloat16* from
   for (int i = 0; i < kWinPage * kLanes / 32; ++i) cp_async16(to + i * (32 / kLanes) * (D + 8) * 2, from + i * 256);
 }
 
-template <int DK, int DV>
+template <int WARPS>
 struct WinCfg {
   static constexpr int kStages = 2;  // two pages per warp in flight leave room for three CTAs per SM at 128 + 128 channels
   static int stage_bytes(int dk, int dv) { return kWinPage * (dk + 8 + dv + 8) * 2; }
   static int smem_bytes(int dk, int dv) {
-    const int ring = kWinWarps * kStages * stage_bytes(dk, dv), merge = kWinWarps * 16 * (dv + 2) * 4;
+    const int ring = WARPS * kStages * stage_bytes(dk, dv), merge = WARPS * 16 * (dv + 2) * 4;
     return ring > merge ? ring : merge;
   }
 };
@@ -82,14 +82,15 @@ struct WinCfg {
 // kWhole: one map whose widths are the bounds, no bias.  A warp spends some 2 us on a page of 16 keys, with more of them in flight no less:
 // it is bound by what it issues.  The widths known to the compiler leave a copy one instruction, and a page that every query sees whole
 // needs no comparisons.  8 KV heads of 4 queries, 128 channels, 3 splits and their sum, 16 rows of 1024 keys 21.6 -> 20.2 us, of 2000
-// 33.0 -> 32.4; a page that costs less wants fewer splits (decode_splits): 18.6 and 29.8, 64 rows of 2000 115 -> 98, 8 of 900 15.9 -> 13.7.
-template <int DK, int DV, bool kWhole>
-__global__ void __launch_bounds__(kWinWarps * 32)
+// 33.0 -> 32.4; a page that costs less wants fewer splits (decode_splits), and with eight warps these are 16.0 and 27.6, 8 of 900 15.9 -> 12.1,
+// 64 of 2000 115 -> 98.
+template <int DK, int DV, bool kWhole, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 window_attn_decode_kernel(const WindowDecodeParams p) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) uint8_t win_smem[];
-  constexpr int kStages = WinCfg<DK, DV>::kStages;
+  constexpr int kStages = WinCfg<WARPS>::kStages;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ht = blockIdx.x % p.head_tiles, bg = blockIdx.x / p.head_tiles;
   const int b = bg / p.Hk, g = bg - b * p.Hk, split = blockIdx.y;
@@ -109,14 +110,14 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
   const int kpitch = dk + 8, vpitch = dv + 8;  // odd multiples of 16 bytes apart modulo 128: ldmatrix without conflicts
   const int stage_bytes = kWinPage * (kpitch + vpitch) * 2;
   const uint32_t ring = smem_u32(win_smem) + warp * kStages * stage_bytes;
-  const int n = max(0, (page1 - page0 - warp + kWinWarps - 1) / kWinWarps);  // my pages: page0 + warp + 4 i
+  const int n = max(0, (page1 - page0 - warp + WARPS - 1) / WARPS);  // my pages: page0 + warp + 4 i
   const int* table = p.table + size_t(b) * p.max_pages;
   const int kch = dk >> 3, vch = dv >> 3;
   const uint32_t kinv = (65536u + kch - 1) / kch, vinv = (65536u + vch - 1) / vch;  // row = i / chunks for i < 512
   int ids = 0;  // lane j holds the id of my page (32 block + j)
   auto fetch = [&](int i) {
     if ((i & 31) == 0) {
-      const int pg = page0 + warp + kWinWarps * (i + lane);
+      const int pg = page0 + warp + WARPS * (i + lane);
       ids = pg < page1 ? table[pg < kept ? pg : pg + skip] : 0;
     }
     const int page = __shfl_sync(0xffffffffu, ids, i & 31);
@@ -196,7 +197,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
         win_mma(s[1], qf[ks], kf[2], kf[3]);
       }
     }
-    const int pg = page0 + warp + kWinWarps * i;
+    const int pg = page0 + warp + WARPS * i;
     const int key0 = (pg < kept ? pg : pg + skip) * kWinPage + t4 * 2;
     float mx[2] = {-FLT_MAX, -FLT_MAX};
     if (kWhole) {
@@ -275,7 +276,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
     }
     __syncwarp();  // the stage is refilled by the next round's fetch
   }
-  // ----- merge the four warps (then the splits, in a second kernel) -----
+  // ----- merge the warps (then the splits, in a second kernel) -----
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
@@ -284,7 +285,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
   cp_async_wait<0>();
   __syncthreads();
   float* acc = reinterpret_cast<float*>(win_smem);              // [warp][16][dv]
-  float* ml = acc + kWinWarps * 16 * dv;                        // [warp][16][2]
+  float* ml = acc + WARPS * 16 * dv;                        // [warp][16][2]
   {
     float* a0 = acc + (warp * 16 + r0) * dv + t4 * 2;
     float* a1 = a0 + 8 * dv;
@@ -301,10 +302,10 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
     }
   }
   __syncthreads();
-  for (int r = warp; r < heads; r += kWinWarps) {
-    float mw[kWinWarps], mt = -FLT_MAX, lt = 0.f;
+  for (int r = warp; r < heads; r += WARPS) {
+    float mw[WARPS], mt = -FLT_MAX, lt = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWinWarps; ++w) { mw[w] = ml[(w * 16 + r) * 2]; mt = fmaxf(mt, mw[w]); }
+    for (int w = 0; w < WARPS; ++w) { mw[w] = ml[(w * 16 + r) * 2]; mt = fmaxf(mt, mw[w]); }
     const bool whole = p.splits == 1 && p.maps == 1;
     if (whole && p.extra.sink) {
       const float sink = p.extra.sink[head0 + r] * kLog2e;
@@ -312,7 +313,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
       lt = window_exp2(sink - mt);
     }
 #pragma unroll
-    for (int w = 0; w < kWinWarps; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       mw[w] = window_exp2(mw[w] - mt);  // a warp without pages: l = 0, o = 0
       lt += ml[(w * 16 + r) * 2 + 1] * mw[w];
     }
@@ -321,7 +322,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
     auto merged = [&](int c) {
       float x = 0.f;
 #pragma unroll
-      for (int w = 0; w < kWinWarps; ++w) x += acc[(w * 16 + r) * dv + c] * mw[w];
+      for (int w = 0; w < WARPS; ++w) x += acc[(w * 16 + r) * dv + c] * mw[w];
       return x * inv;
     };
     if (whole && p.turn.rope) {
@@ -423,15 +424,15 @@ int launch_attn_merge(const float* part, const float* part_ml, const float* sink
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 
-template <int DK, int DV, bool kWhole>
+template <int DK, int DV, bool kWhole, int WARPS = kWinWarps>
 static int launch_window_pages(const WindowDecodeParams& p, const WindowMergeParams& mp, int B, cudaStream_t stream) {
-  const int smem = WinCfg<DK, DV>::smem_bytes(p.dk * p.maps, p.dv);
+  const int smem = WinCfg<WARPS>::smem_bytes(p.dk * p.maps, p.dv);
   static int allowed = 0;
   if (smem > allowed) {
-    if (cudaFuncSetAttribute(window_attn_decode_kernel<DK, DV, kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -6;
+    if (cudaFuncSetAttribute(window_attn_decode_kernel<DK, DV, kWhole, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -6;
     allowed = smem;
   }
-  launch_kernel(window_attn_decode_kernel<DK, DV, kWhole>, dim3(B * p.Hk * p.head_tiles, p.splits), dim3(kWinWarps * 32), smem, stream, p);
+  launch_kernel(window_attn_decode_kernel<DK, DV, kWhole, WARPS>, dim3(B * p.Hk * p.head_tiles, p.splits), dim3(WARPS * 32), smem, stream, p);
   if (p.splits > 1 || p.maps > 1)
     launch_kernel(window_attn_merge_kernel, dim3(B * mp.heads), dim3(128), 0, stream, p.part, p.part_ml, p.out, mp);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
@@ -440,7 +441,16 @@ static int launch_window_pages(const WindowDecodeParams& p, const WindowMergePar
 template <int DK, int DV>
 static int launch_window_decode(const WindowDecodeParams& p, const WindowMergeParams& mp, int B, cudaStream_t stream) {
   if constexpr (DK == DV && DK <= 256) {
-    if (p.maps == 1 && p.dk == DK && p.dv == DV && !p.extra.bias) return launch_window_pages<DK, DV, true>(p, mp, B, stream);
+    if (p.maps == 1 && p.dk == DK && p.dv == DV && !p.extra.bias) {
+      // Grids of about one CTA per SM: eight warps each.  Four | eight, 8 KV heads: 16 rows of 1024 keys 17.6 | 16.0 us, 12 of 2000 26.4 | 22.2,
+      // 4 of 4096 in 4 splits 21.4 | 18.8; a smaller grid has no pages for them (one row of 1024 in 6 splits 8.9 | 9.6), and a larger one
+      // has the warps (19 of 1024 20.2 | 26.8).  At 256 channels the rings of eight do not fit.
+      const int ctas = B * p.Hk * p.head_tiles * p.splits;
+      if constexpr (DK <= 128) {
+        if (ctas > 64 && ctas <= 148) return launch_window_pages<DK, DV, true, 8>(p, mp, B, stream);
+      }
+      return launch_window_pages<DK, DV, true>(p, mp, B, stream);
+    }
   }
   return launch_window_pages<DK, DV, false>(p, mp, B, stream);
 }

@@ -171,12 +171,13 @@ def decode_splits(batch: int, kv_heads: int, keys: int, whole: bool = False) -> 
     that comes near a wave of three CTAs per SM evens its last wave out with up to 5 splits of at least 256 keys; more is not
     split.
 
-    ``whole`` (see ``whole_heads``, and no bias): a page costs half as much there, so the sums of the splits count more.  300 CTAs are
-    enough, of 128 keys at least, and a grid of one wave is not split: 128 (sequence, KV head) pairs of 1024 keys 20.2 us in 3
-    splits, 18.6 in 2; 64 of 2048 20.8 in 6, 19.9 in 4; 256 of 2000 56.8 in 5, 51.9 in 1; 512 of 2000 103 in 1, 97.6 in 2."""
+    ``whole`` (see ``whole_heads``, and no bias): a page costs half as much there and a CTA may have eight warps, so the sums of the splits
+    count more.  A grid of a CTA per SM is enough, of 160 keys at least, and up to one wave of three per SM is not split: 128 (sequence, KV
+    head) pairs of 1024 keys 20.1 us in 3 splits, 18.5 in 2, 16.0 in 1; 64 of 2048 19.9 in 4, 18.0 in 2; 256 of 2000 56.8 in 5, 51.9 in 1; 512
+    of 2000 103 in 1, 97.6 in 2."""
     n, slots = max(1, batch * kv_heads), 148 * 3
     if whole and n <= slots:
-        return max(1, min(300 // n, keys // 128, 16))
+        return max(1, min(148 // n, keys // 160, 16))
     if n <= 200:
         return max(1, min(400 // n, keys // 64, 16))
     if n > 600:

@@ -73,6 +73,23 @@ def test_pages_of_the_bounds_widths(d, per, window, keep, chunk, splits, cap):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("b,hk,splits", [(32, 2, 1), (33, 2, 1), (37, 2, 2), (74, 2, 1), (75, 2, 1)])
+def test_pages_by_warps_of_a_cta(b, hk, splits, d):
+    """Grids at the lines between four and eight warps a CTA, against the general kernel of four (other sums, so a rounding apart)."""
+    from types import SimpleNamespace
+    from mfq_b200.ops import window_attn
+    lens = torch.tensor([(1, 16, 129, 400, 33, 257, 0, 80)[i % 8] for i in range(b)], device="cuda", dtype=torch.int32)
+    kv = SimpleNamespace(k=rnd(b * 25, hk, 16, d), v=rnd(b * 25, hk, 16, d))
+    table = torch.randperm(b * 25, device="cuda", dtype=torch.int32).view(b, 25)
+    q, how = rnd(b, hk * 5, d, scale=3.0), dict(window=300, splits=splits, cap=20.0, scale=d ** -0.5)
+    got = window_attn.decode(q, kv, table, lens, **how)
+    want = window_attn.decode(q, kv, table, lens, bias=window_attn.DistanceBias.from_table(torch.zeros(hk * 5, 1, device="cuda")), **how)
+    check_status()
+    # probabilities are bf16 of the page's own maximum, which differs between warps' pages: half a step of 2^-8 of each, weights summing to one
+    assert bool(((got.double() - want.double()).abs() <= 2.0 ** -8 * (kv.v.double().abs().max() + want.double().abs())).all())
+
+
 @pytest.mark.parametrize("m", [1, 8, 9, 16])
 @pytest.mark.parametrize("n,k", [(16, 2048), (256, 4096), (2368, 2056), (48, 4104), (32, 14336)])
 def test_streaming_product_of_few_rows_of_weights(m, n, k):
