@@ -46,6 +46,11 @@ def _most_splits(tiles: int, blocks: int, small: bool, sms: int) -> int:
 PAIR = -2  # as a number of K splits: the product runs on pairs of SMs (csrc/dense_pair.cu)
 
 
+def _small_tiles(m: int, rows: int, blocks: int, splits: int, sms: int) -> bool:
+    """Whether tiles of 32 tokens are resident at once, one CTA per SM or, with little to stream, two."""
+    return m > 32 and rows * math.ceil(m / 32) * splits <= (2 * sms if blocks <= 16 else sms)
+
+
 def _streams(m: int, n: int, k: int) -> bool:
     """Whether up to 16 rows go to the weight-streaming kernel.  On B200 (streaming | tcgen05, cold weights, us): a CTA per SM always does,
     16 x 2368 x 4096 5.7 | 9.4, 16 x 2048 x 14336 14.0 | 14.9, 1 x 2368 x 18944 16.3 | 17.8; two per SM up to 4096 inputs, 16 x 4096 x 4096
@@ -61,7 +66,7 @@ def _streams(m: int, n: int, k: int) -> bool:
 
 
 @lru_cache(maxsize=4096)  # sizes only; a prompt asks for the same few once per layer
-def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[int, int]:
+def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False, single: bool = True) -> tuple[int, int]:
     """``(token tile, K splits)`` of a bf16 product ``[m, k] x [n, k]^T``; tile 0 is the weight-streaming kernel, splits
     :data:`PAIR` the kernel on pairs of SMs (``pairs``: it may be chosen; it takes a single matrix).  Fitted to a
     sweep on B200 over the projections of 1B- and 8B-sized layers at 16 .. 4096 tokens: up to 128 tokens the weights are read
@@ -70,13 +75,17 @@ def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[i
     with 256 tokens and 0.26 with 128, once 4 us for the launch: 1508 tokens of gate/up 28672 x 4096 take 252 us there against 462 here,
     of o_proj 4096 x 4096 50 against 64; what stays here are narrow or split products (300 x 4096 x 14336: 52 against 54 us).
     Sums in parts (:func:`pair_sums`), as many as there are accumulators, cost a pair 0.5 to 1 us: 300 x 4096 x 4096 in two 19.5 us there
-    against 21.2 here, 200 x 1536 x 1536 in three 10.05 against 9.95, the least favourable."""
+    against 21.2 here, 200 x 1536 x 1536 in three 10.05 against 9.95, the least favourable.
+    A single matrix (``single``) whose grid leaves SMs idle even so takes tiles of 32 tokens, in as many sums (and to the same bits): a CTA's share
+    of the tokens is what its ring waits for.  64 x 256 x 4096 in 8 sums 7.6 us with a tile of 64, 6.3 with two of 32; 128 tokens 10.0 and
+    6.7, 128 x 4096 x 256 5.7 and 3.7, 250 x 2048 x 1024 8.2 and 6.0."""
     if m <= GEMV_MID_ROWS and _streams(m, n, k):
         return 0, 1
     rows, blocks = math.ceil(n / 128), math.ceil(k / 64)
     for tile in (16, 32, 64, 128):
         if m <= tile:
-            return tile, _most_splits(rows, blocks, tile <= 64, sms)
+            s = _most_splits(rows, blocks, tile <= 64, sms)
+            return (32 if single and _small_tiles(m, rows, blocks, s, sms) else tile), s
     best, best_cost = (128, 1), None
     for tile, ramp, per_block, meet in ((128, 5.0, 0.30, 3.0), (256, 7.0, 0.35, 5.0)):
         tiles = rows * math.ceil(m / tile)
@@ -86,6 +95,8 @@ def plan(m: int, n: int, k: int, sms: int = 148, pairs: bool = False) -> tuple[i
                 best, best_cost = (tile, s), cost
     if math.ceil(rows * math.ceil(m / best[0]) * best[1] / sms) > 1:
         best_cost *= 1.1  # several waves of CTAs: 4096 x 4096 x 14336 takes 434 us, not the 341 of four single ones
+    if single and _small_tiles(m, rows, blocks, best[1], sms):
+        return 32, best[1]
     sums = best[1]  # a pair forms them too, in an accumulator each
     for tile, ramp, per_block in ((256, 2.0, 0.40), (128, 0.0, 0.26)) if pairs else ():
         if sums > 512 // tile:
@@ -158,7 +169,8 @@ class DenseLinear:
             assert table.shape[1] == n and table.is_contiguous() and table.dtype == x.dtype and ids.dtype == torch.int32
             kind = GELU
         # a matrix per head is narrower than a tile of the tensor cores
-        t, s = (0, 1) if g > 1 and m <= GEMV_ROWS else plan(m, n * g, k, pairs=g == 1 and tile is None and splits is None)
+        t, s = (0, 1) if g > 1 and m <= GEMV_ROWS else plan(m, n * g, k, pairs=g == 1 and tile is None and splits is None,
+                                                              single=g == 1)
         t, s = (t if tile is None else tile), (s if splits is None else splits)
         if s == PAIR and splits is None:
             s = -1 - pair_sums(m, n, k)

@@ -137,6 +137,20 @@ def test_few_rows_by_either_kernel(m, n, k, streams):
     check_status()
 
 
+@pytest.mark.parametrize("m,n,k,splits", [(33, 256, 4096, 8), (128, 500, 4104, 8), (129, 128, 2048, 4), (100, 2048, 1024, 2), (160, 2048, 1024, 1), (288, 4000, 72, 1)])
+def test_narrow_products_in_tiles_of_32(m, n, k, splits):
+    """Few tiles of weights, or few inputs: small token tiles, to the bits of the large ones."""
+    from mfq_b200.ops import dense
+    n = n // 16 * 16
+    x, w = rnd(m, k), rnd(n, k, scale=k ** -0.5)
+    assert dense.plan(m, n, k, pairs=True) == (32, splits)
+    got = dense.DenseLinear(w)(x, fp32=True)
+    close(got, (x.double() @ w.double().T).cpu(), 2e-5)
+    for tile in (64, 128):
+        assert torch.equal(got, dense.DenseLinear(w)(x, fp32=True, tile=tile, splits=splits))
+    check_status()
+
+
 @pytest.mark.parametrize("tile", [16, 32, 64, 128, 256])
 @pytest.mark.parametrize("splits", [1, 2, 3, 5, 8])
 def test_every_tile_and_split(tile, splits):
