@@ -272,6 +272,9 @@ class LlamaModel:
             self.sm_scale *= self.rope_scaling.softmax_scale_factor
         self.attn_splits = 1
         self.attn_rot = None  # leading dims of a head that are rotated (None: all of them)
+        # no 8-bit rows between the layers: a decode step's attention may round its sums as suits the grid
+        self.more_warps = all(getattr(getattr(l, name, None), "input_kind", "fp8") != "fp8"
+                              for l in weights.layers for name in ("qkv", "o_proj", "gate_up", "down"))
 
     # -- primitive dispatch -------------------------------------------------------------------------------------
     def _norm_quant(self, x, w):
@@ -331,7 +334,7 @@ class LlamaModel:
         if not prefill:
             if qkv.is_cuda:
                 o = ops.paged_attn_decode(q, kv, step.block_table, step.seq_lens, sm_scale=self.sm_scale,
-                                          splits=self.attn_splits, q_len=step.q_len)
+                                          splits=self.attn_splits, q_len=step.q_len, more_warps=self.more_warps)
             else:
                 o = ref.paged_attn_decode(q, kv, step.block_table, step.seq_lens, self.sm_scale, step.q_len)
             return o.reshape(t, self.hq * d)

@@ -19,6 +19,7 @@
 #include "common.cuh"
 
 #include <cfloat>
+#include <climits>
 #include <cuda_fp16.h>
 
 namespace mfq {
@@ -576,7 +577,7 @@ template <int D>
 static int launch_attn(const void* q, const void* k_cache, const void* v_cache, const float* k_scale,
                        const float* v_scale, const int* block_table, const int* seq_lens, void* out, float* part_acc,
                        float* part_ml, int B, int Hq, int Hk, int max_pages, float sm_scale, int splits, int q_len,
-                       int* status, cudaStream_t stream) {
+                       int more_warps, int* status, cudaStream_t stream) {
   // MFQ_ATTN_VARIANT (measurement switch): 0 = by the number of query rows; 1 = always the 16-row form;
   // 2 / 3 = tokens-as-rows form with 2 pages in flight per warp and 5 CTAs per SM / 4 pages and 3 CTAs
   static const int variant = [] { const char* e = getenv("MFQ_ATTN_VARIANT"); return e ? atoi(e) : 0; }();
@@ -589,9 +590,10 @@ static int launch_attn(const void* q, const void* k_cache, const void* v_cache, 
     // as many an SM as four CTAs of four.  Sixteen to a CTA pay where a split has the pages for them.  Four | eight | sixteen warps, the
     // sum of the splits included: one row of 2048 tokens in 64 CTAs 9.0 | 7.9 | 6.8 us, of 600 in 16 7.9 | 7.9 | 7.0, of 20 in 8 3.3 | 3.1 | 3.9;
     // 4 of 1024 in 128 9.9 | 7.2 | 7.7, 8 of 1024 in 256 11.1 | 10.0 | 13.1; but 19 of 700 in 304 14.1 | 15.7.
-    const int ctas = B * Hk * splits;
-    if (narrow && variant == 0 && splits > 1 && ctas <= 64) return launch_attn_v<D, 3, 1, true, 16>(MFQ_ATTN_ARGS);
-    if (narrow && variant == 0 && ctas <= 2 * 148) return launch_attn_v<D, 3, 2, true, 8>(MFQ_ATTN_ARGS);
+    // Their sums are others, so the caller has to ask for them.
+    const int ctas = more_warps && variant == 0 ? B * Hk * splits : INT_MAX;
+    if (narrow && splits > 1 && ctas <= 64) return launch_attn_v<D, 3, 1, true, 16>(MFQ_ATTN_ARGS);
+    if (narrow && ctas <= 2 * 148) return launch_attn_v<D, 3, 2, true, 8>(MFQ_ATTN_ARGS);
     if (narrow) return launch_attn_v<D, 3, 4, true>(MFQ_ATTN_ARGS);
     return launch_attn_v<D, 3, 3, false>(MFQ_ATTN_ARGS);
   } else {
@@ -604,20 +606,22 @@ static int launch_attn(const void* q, const void* k_cache, const void* v_cache, 
 }  // namespace mfq
 
 // q: [B * q_len, Hq, D] bf16; caches in the fragment-friendly page layout described at the top of this file;
-// seq_lens count every token visible to the last query row.  (Hq / Hk) * q_len must be <= 16.
+// seq_lens count every token visible to the last query row.  (Hq / Hk) * q_len must be <= 16.  more_warps: a grid that leaves room may
+// spread its pages over more warps, whose partial sums round differently.
 extern "C" int mfq_paged_attn_decode_mma(const void* q, const void* k_cache, const void* v_cache, const float* k_scale,
                                          const float* v_scale, const int* block_table, const int* seq_lens, void* out,
                                          float* part_acc, float* part_ml, int B, int Hq, int Hk, int D, int max_pages,
-                                         float sm_scale, int splits, int q_len, int* status, cudaStream_t stream) {
+                                         float sm_scale, int splits, int q_len, int more_warps, int* status,
+                                         cudaStream_t stream) {
   if (B <= 0 || Hk <= 0 || Hq % Hk || (Hq / Hk) * q_len > 16 || splits < 1) return -1;
   if (D == 128)
     return mfq::launch_attn<128>(q, k_cache, v_cache, k_scale, v_scale, block_table, seq_lens, out, part_acc, part_ml,
-                                 B, Hq, Hk, max_pages, sm_scale, splits, q_len, status, stream);
+                                 B, Hq, Hk, max_pages, sm_scale, splits, q_len, more_warps, status, stream);
   if (D == 256)
     return mfq::launch_attn<256>(q, k_cache, v_cache, k_scale, v_scale, block_table, seq_lens, out, part_acc, part_ml,
-                                 B, Hq, Hk, max_pages, sm_scale, splits, q_len, status, stream);
+                                 B, Hq, Hk, max_pages, sm_scale, splits, q_len, more_warps, status, stream);
   if (D == 64)
     return mfq::launch_attn<64>(q, k_cache, v_cache, k_scale, v_scale, block_table, seq_lens, out, part_acc, part_ml, B,
-                                Hq, Hk, max_pages, sm_scale, splits, q_len, status, stream);
+                                Hq, Hk, max_pages, sm_scale, splits, q_len, more_warps, status, stream);
   return -1;
 }

@@ -320,8 +320,10 @@ def attn_splits_for(batch: int, kv_heads: int, ctx_len: int, head_dim: int = 128
 
 
 def paged_attn_decode(q: torch.Tensor, kv, block_table: torch.Tensor, seq_lens: torch.Tensor, *, sm_scale: float,
-                      splits: int = 1, q_len: int = 1, out=None) -> torch.Tensor:
-    """``q [B*q_len, Hq, D]`` against the paged fp8 cache; ``seq_lens`` count the query tokens too."""
+                      splits: int = 1, q_len: int = 1, more_warps: bool = False, out=None) -> torch.Tensor:
+    """``q [B*q_len, Hq, D]`` against the paged fp8 cache; ``seq_lens`` count the query tokens too.  ``more_warps``: a grid that leaves room
+    may give its pages to more warps, faster and with other roundings of the sums; a decoder with 8-bit rows between its layers, where
+    one of them moves the logits by 2 %, does without."""
     rows, hq, d = q.shape
     b = rows // q_len
     hk = kv.k.shape[1]
@@ -331,7 +333,7 @@ def paged_attn_decode(q: torch.Tensor, kv, block_table: torch.Tensor, seq_lens: 
         assert rows * hq * splits * d <= ws.attn_acc.numel() and rows * hq * splits * 2 <= ws.attn_ml.numel()
     rc = lib().mfq_paged_attn_decode_mma(ptr(q), ptr(kv.k), ptr(kv.v), ptr(kv.k_scale), ptr(kv.v_scale),
                                          ptr(block_table), ptr(seq_lens), ptr(out), ptr(ws.attn_acc), ptr(ws.attn_ml), b,
-                                         hq, hk, d, block_table.shape[1], float(sm_scale), splits, q_len,
+                                         hq, hk, d, block_table.shape[1], float(sm_scale), splits, q_len, int(more_warps),
                                          ptr(ws.status), stream_ptr())
     check(rc, "paged_attn_decode", 2 if splits > 1 else 1)
     return out

@@ -36,7 +36,7 @@ _SIGNATURES = {
                                _f, _f, _f, _f, _vp],
     "mfq_rope_kv_write": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp],
     
-    "mfq_paged_attn_decode_mma": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _vp],
+    "mfq_paged_attn_decode_mma": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _vp, _vp],
     "mfq_argmax": [_vp, _vp, _i, _i, _i, _vp],
     "mfq_argmax_f32": [_vp, _vp, _i, _i, _i, _vp],
     "mfq_embed": [_vp, _vp, _vp, _i, _i, _vp],

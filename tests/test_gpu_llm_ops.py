@@ -118,7 +118,7 @@ def test_decode_attention_by_warps_of_a_cta(b, hk, splits, d):
     q = torch.randn((b, 4 * hk, d), device="cuda").to(torch.bfloat16)
     seq_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
     want = ref.paged_attn_decode(q, kv, cache.block_table, seq_lens, 1 / math.sqrt(d))
-    got = ops.paged_attn_decode(q, kv, cache.block_table, seq_lens, sm_scale=1 / math.sqrt(d), splits=splits)
+    got = ops.paged_attn_decode(q, kv, cache.block_table, seq_lens, sm_scale=1 / math.sqrt(d), splits=splits, more_warps=True)
     check_status()
     assert_close(got, want, rel=2e-2, what=f"decode attention of {b} x {hk} in {splits}")
 
