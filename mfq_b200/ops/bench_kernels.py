@@ -200,7 +200,7 @@ def bench_window_decode(batch: int, ctx: int, hq: int, hk: int, d: int, window: 
     q = torch.randn((batch, hq, d), device="cuda").to(torch.bfloat16)
     sl = torch.full((batch,), ctx, dtype=torch.int32, device="cuda")
     out = torch.empty_like(q)
-    splits = window_attn.decode_splits(batch, hk, seen) if splits is None else splits
+    splits = window_attn.decode_splits(batch, hk, seen, window_attn.whole_heads(cache.layer(0))) if splits is None else splits
     ms = time_ms(lambda i: window_attn.decode(q, cache.layer(i % layers), cache.block_table, sl, window=window, scale=0.088, cap=cap,
                                               splits=splits, out=out), reps)
     return {"kernel": "window_attn_decode", "batch": batch, "ctx": ctx, "hq": hq, "hk": hk, "d": d, "window": window, "cap": cap,
@@ -496,7 +496,7 @@ def bench_chunks(batch: int, ctx: int, hq: int, hk: int, d: int, size: int, reps
     rows = [{"kernel": f"qkv_finish ({name})", **shape, "us": ms * 1e3, "gbs": n * (hq + 2 * hk) * d * 4 / ms / 1e6}
             for name, ms in (("values normed and rotated", stage(True)), ("plain values", stage(False)))]
     if batch:
-        sl, splits = torch.full((batch,), ctx, dtype=torch.int32, device="cuda"), window_attn.decode_splits(batch, hk, seen)
+        sl, splits = torch.full((batch,), ctx, dtype=torch.int32, device="cuda"), window_attn.decode_splits(batch, hk, seen, window_attn.whole_heads(cache.layer(0)))
         ms = time_ms(lambda i: window_attn.decode(q, cache.layer(i % layers), cache.block_table, sl, splits=splits, turn=turn, out=out, **how), reps)
         return rows + [{"kernel": "window_attn_decode (chunks, turned)", **shape, "splits": splits, "us": ms * 1e3, "gbs": batch * seen * hk * d * 4 / ms / 1e6}]
     starts, lens = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([0, ctx], [ctx]))

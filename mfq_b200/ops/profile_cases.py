@@ -192,7 +192,7 @@ def window_decode() -> None:
     lens = torch.full((64,), 4096, dtype=torch.int32, device="cuda")
     for i in range(3):
         window_attn.decode(q, cache.layer(i), cache.block_table, lens, window=1024, scale=0.088, cap=50.0,
-                           splits=window_attn.decode_splits(64, 8, 1024))
+                           splits=window_attn.decode_splits(64, 8, 1024, True))
 
 
 def window_prefill() -> None:
