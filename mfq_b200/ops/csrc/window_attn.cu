@@ -110,7 +110,7 @@ window_attn_decode_kernel(const WindowDecodeParams p) {
   const int kpitch = dk + 8, vpitch = dv + 8;  // odd multiples of 16 bytes apart modulo 128: ldmatrix without conflicts
   const int stage_bytes = kWinPage * (kpitch + vpitch) * 2;
   const uint32_t ring = smem_u32(win_smem) + warp * kStages * stage_bytes;
-  const int n = max(0, (page1 - page0 - warp + WARPS - 1) / WARPS);  // my pages: page0 + warp + 4 i
+  const int n = max(0, (page1 - page0 - warp + WARPS - 1) / WARPS);  // my pages: page0 + warp + WARPS i
   const int* table = p.table + size_t(b) * p.max_pages;
   const int kch = dk >> 3, vch = dv >> 3;
   const uint32_t kinv = (65536u + kch - 1) / kch, vinv = (65536u + vch - 1) / vch;  // row = i / chunks for i < 512
