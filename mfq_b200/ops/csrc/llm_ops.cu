@@ -184,9 +184,11 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
 // divisions kept the issue slots two thirds busy), 1000 rows from 36 to 20.  With the gates by silu2 74 and 19, with all loads of a full row
 // requested before the first is used 69 and 18.
 // ---------------------------------------------------------------------------------------------
+// kFull: gated rows of kRowVecs vectors for every thread.  They need more registers, which the others do without: with 50 instead of 40 the CTAs of
+// the second product of 320 routes found no room beside this kernel's, and that layer took 148 us instead of 146.
 constexpr int kRowVecs = 4;
-template <int kMode>
-__global__ void __launch_bounds__(512) quant_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out,
+template <int kMode, bool kFull = false>
+__global__ void __launch_bounds__(512, kFull ? 1 : 3) quant_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out,
                                   float* __restrict__ scale_out, int K, int in_stride,
                                   const __nv_bfloat16* __restrict__ x2 = nullptr, int x2_stride = 0) {
   pdl_trigger();
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(512) quant_rows_kernel(const __nv_bfloat16* __
 #pragma unroll
         for (int j = 0; j < 4; ++j) amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[j] << 16)), fabsf(__uint_as_float(w[j] & 0xffff0000u))));
       }
-    } else if (kMode == 1 && nvec == kRowVecs * int(blockDim.x)) {  // likewise, gates and values
+    } else if (kFull) {  // likewise, gates and values
       uint4 up[kRowVecs];
 #pragma unroll
       for (int i = 0; i < kRowVecs; ++i) {
@@ -981,7 +983,7 @@ extern "C" int mfq_quant_rows(const void* x, void* q_out, float* scale_out, int 
     return cudaGetLastError() == cudaSuccess ? 0 : -7;
   }
   if (swiglu)
-    launch_kernel(quant_rows_kernel<1>, dim3(M), dim3(threads), 0, stream, static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q_out), scale_out, K, in_stride, static_cast<const __nv_bfloat16*>(nullptr), 0);
+    launch_kernel(K == 8 * kRowVecs * threads ? quant_rows_kernel<1, true> : quant_rows_kernel<1>, dim3(M), dim3(threads), 0, stream, static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q_out), scale_out, K, in_stride, static_cast<const __nv_bfloat16*>(nullptr), 0);
   else
     launch_kernel(quant_rows_kernel<0>, dim3(M), dim3(threads), 0, stream, static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q_out), scale_out, K, in_stride, static_cast<const __nv_bfloat16*>(nullptr), 0);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
