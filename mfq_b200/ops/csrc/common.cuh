@@ -158,9 +158,13 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // ----- programmatic dependent launch -----
 // Kernels of the decode path are launched with the programmatic-serialization attribute: a kernel may be scheduled
 // while its predecessor in the stream drains, run its prologue (barrier init, TMEM allocation, index math) and
-// then block in pdl_wait() until the predecessor has completed and flushed its writes.  Every such kernel calls
-// pdl_trigger() first thing, so its own successor may be scheduled as early as possible; correctness only depends on
-// pdl_wait() preceding the first access to memory another kernel produced (and the first global write).
+// then block in pdl_wait() until the predecessor has completed and flushed its writes.  Such a kernel calls
+// pdl_trigger() first thing, so its own successor may be scheduled as early as possible, unless it takes tensor memory: then behind the
+// allocation (and the block barrier that publishes it).  The successors may allocate before they wait; were one resident while a CTA
+// of this grid had still to allocate, it could take the columns that this CTA needs and wait, without end, for this grid.  Once all CTAs have
+// triggered, all hold what they need, and a successor that finds too little waits for them, which end without it.
+// Beside that, correctness only depends on pdl_wait() preceding the first access to memory another kernel produced (and the
+// first global write).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

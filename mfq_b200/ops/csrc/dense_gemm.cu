@@ -115,7 +115,6 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  pdl_trigger();
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
   if (p.tiles) pdl_wait();  // the tile list comes from the kernel before
   DenseAt at;
@@ -136,6 +135,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  pdl_trigger();  // TMEM is held by now (common.cuh)
 
   // Loads and MMAs are issued by an elected lane of a converged warp (common.cuh: umma_f8f6f4_block says why).
   if (warp == 0) {

@@ -226,7 +226,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
   const int lane = threadIdx.x & 31;
   const bool gather = p.ag.world > 1;
-  pdl_trigger();
   // The all-gather mode's prologue already reads memory an earlier kernel wrote (the epoch) and waits for its predecessor
   // right away; the plain GEMM first sets up barriers and TMEM.
   const bool early_inputs = gather;
@@ -235,6 +234,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   if (gather && int(blockIdx.x) < p.ag.push_ctas) {
     // ----- push block: copy my shard into every rank's gathered buffer, then announce it -----
     if (blockIdx.y != 0 || blockIdx.z != 0) return;
+    pdl_trigger();  // no tensor memory here
     const AgParams& ag = p.ag;
     const size_t shard_bytes = size_t(ag.shard_rows) * p.K;
     const size_t half = size_t(ag_epoch & 1u) * size_t(p.M) * p.K;
@@ -335,6 +335,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  pdl_trigger();  // TMEM is held by now (common.cuh)
   if (p.cluster_reduce) cluster_arrive();  // this CTA's barriers exist
   // Weights are never written by a kernel of the same stream, so the plain GEMM starts the weight tiles of its first
   // ring pass BEFORE it waits for its predecessor: under programmatic dependent launch this CTA is resident while the

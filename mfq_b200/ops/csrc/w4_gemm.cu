@@ -73,7 +73,6 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
 
-  pdl_trigger();
   // Uniform for the compiler, except beside an epilogue of 128 accumulators per thread: there the uniform copy costs 140 bytes of spills
   // instead of 8 (128 x 256 x 2048: 18.5 against 17.6 us).
   const int warp = BT >= 128 ? int(threadIdx.x) >> 5 : __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
@@ -101,6 +100,7 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  pdl_trigger();  // TMEM is held by now (common.cuh)
   pdl_wait();
 
   if (warp == 0) {

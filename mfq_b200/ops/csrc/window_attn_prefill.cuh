@@ -117,10 +117,7 @@ window_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // Only now may the next kernel be scheduled: a product kernel of the stream takes its tensor memory before it waits for
-  // this one, and would hold what this CTA still needs if it came first.  (For the same reason the wait above precedes the
-  // allocation.)
-  pdl_trigger();
+  pdl_trigger();  // TMEM is held by now (common.cuh)
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tO = tmem_base + 2 * KB;
 

@@ -29,3 +29,25 @@ def test_what_the_kernel_before_wrote_is_not_read_as_constant(name):
     promises data that stays the same for the life of the kernel."""
     sources = re.findall(r"__ldg\((?:p\.)?(\w+)", (CSRC / name).read_text())
     assert sources and set(sources) <= {"wsc", "w_scale"}
+
+
+ALLOCATION = re.compile(r"\btmem_alloc(_pair)?\(")
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu*") if p.name not in ("common.cuh", "pair.cuh") and ALLOCATION.search(p.read_text())))
+def test_tensor_memory_is_held_before_a_successor_may_start(name):
+    """A successor may allocate before it waits.  Resident beside a CTA that has still to allocate, it could take that CTA's columns and wait
+    for its grid for ever, so no path to an allocation passes a trigger, and one comes only after the block barrier behind it."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    kernels = [k for k in text.split("__global__")[1:] if ALLOCATION.search(k)]
+    assert kernels
+    for kernel in kernels:
+        at = ALLOCATION.search(kernel).start()
+        for trigger in re.finditer(r"\bpdl_trigger\(\)", kernel[:at]):  # a branch that leaves the kernel without allocating
+            depth, end = 0, trigger.end()
+            while depth >= 0:
+                depth += {"{": 1, "}": -1}.get(kernel[end], 0)
+                end += 1
+            assert end < at and kernel[:end].rstrip("} \n").endswith("return;"), name
+        behind = kernel[at:].find("pdl_trigger()")
+        assert behind < 0 or "__syncthreads()" in kernel[at : at + behind], name
