@@ -338,6 +338,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll
         for (int tt = 0; tt < CW; ++tt) acc[tt] = add_total(tt);
         if (live && ok) {  // the place is the residual's and the results'; a row of them covers sums of both warps
+          fence_proxy_async_smem();  // the residual comes by TMA where these sums were read and written by plain accesses
           __syncwarp();
           if (lane == 0) mbar_arrive(&turn_done[unit]);
         }

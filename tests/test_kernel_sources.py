@@ -51,3 +51,14 @@ def test_tensor_memory_is_held_before_a_successor_may_start(name):
             assert end < at and kernel[:end].rstrip("} \n").endswith("return;"), name
         behind = kernel[at:].find("pdl_trigger()")
         assert behind < 0 or "__syncthreads()" in kernel[at : at + behind], name
+
+
+def test_an_output_place_is_handed_to_tma_behind_a_proxy_fence():
+    """Warps write sums and results to an output place by plain accesses and read them back; what TMA then reads or writes there is only ordered
+    behind these by a fence of each thread before the arrival that hands the place over."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "fp8_gemm_2cta.cu").read_text())
+    handed = [m.start() for m in re.finditer(r"mbar_arrive\(&turn_done\[", text)]
+    assert len(handed) == 2
+    for at in handed:  # nothing touches the place between the fence and the arrival
+        fence = text.rfind("fence_proxy_async_smem()", 0, at)
+        assert fence >= 0 and not re.search(r"\btotal\(|\bturn_in\(|\.shared\.", text[fence:at])
