@@ -62,3 +62,11 @@ def test_an_output_place_is_handed_to_tma_behind_a_proxy_fence():
     for at in handed:  # nothing touches the place between the fence and the arrival
         fence = text.rfind("fence_proxy_async_smem()", 0, at)
         assert fence >= 0 and not re.search(r"\btotal\(|\bturn_in\(|\.shared\.", text[fence:at])
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu*") if re.search(r"\w*cluster_barrier\(\) \{", p.read_text())))
+def test_warps_are_whole_at_an_aligned_cluster_barrier(name):
+    """``barrier.cluster.*.aligned`` is undefined for a warp whose lanes come one after the other, and lanes need not have met again behind a loop
+    of different lengths or a branch: the barrier brings them together itself."""
+    body = re.search(r"void \w*cluster_barrier\(\) \{\s*(.*)", (CSRC / name).read_text()).group(1)
+    assert body.startswith("__syncwarp();")
