@@ -592,14 +592,21 @@ __device__ __forceinline__ void rope_head(const __nv_bfloat16* __restrict__ src,
 // of a dim come together in its registers and leave as one store.  The tokens of other groups (a page's part, slots in another order, none)
 // are left to the warps that go token by token.
 constexpr int kGroupTokens = 16;
-// First token of a group: groups are the pages of a prompt in one piece that begins at slots[0].  Whether token t0's group is one whole page,
-// the same for the warp; `slot`: the lane's (lane & 15).
-__device__ __forceinline__ int group_shift(const int* __restrict__ slots) { return slots[0] >= 0 ? slots[0] & 15 : 0; }
-__device__ __forceinline__ bool whole_page(const int* __restrict__ slots, int t0, int T, int lane, int& slot) {
-  const int mine = t0 + (lane & 15);
-  slot = mine >= 0 && mine < T ? slots[mine] : -1;
-  const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
-  return __all_sync(0xffffffffu, slot >= 0 && slot == slot0 + (lane & 15)) && (slot0 & 15) == 0;
+// First token of the whole page that begins within sixteen tokens from `from` on, and its slot; -1: none does.  Two cannot: the second would lie
+// inside the first.  So prompts packed one after the other have their pages found wherever they begin.
+__device__ __forceinline__ int whole_page_from(const int* __restrict__ slots, int from, int T, int lane, int& slot0) {
+  const int slot = from + lane < T ? slots[from + lane] : -1;
+  const int next = __shfl_down_sync(0xffffffffu, slot, 1);
+  const uint32_t runs = __ballot_sync(0xffffffffu, lane < 31 && slot >= 0 && next == slot + 1);
+  const uint32_t begins = __ballot_sync(0xffffffffu, lane < 16 && slot >= 0 && (slot & 15) == 0 && (runs >> lane & 0x7fffu) == 0x7fffu);
+  const int at = __ffs(begins) - 1;
+  slot0 = __shfl_sync(0xffffffffu, slot, at & 31);
+  return at < 0 ? -1 : from + at;
+}
+// Whether token t, which goes to `slot`, belongs to such a page.
+__device__ __forceinline__ bool in_whole_page(const int* __restrict__ slots, int t, int slot, int T, int lane) {
+  const int t0 = t - (slot & 15);
+  return slot >= 0 && t0 >= 0 && t0 + kGroupTokens <= T && __all_sync(0xffffffffu, slots[t0 + (lane & 15)] == (slot & ~15) + (lane & 15));
 }
 template <int D>
 __device__ __forceinline__ void value_group(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ slots, const RopeOut& to, int T, int row_stride,
@@ -608,10 +615,9 @@ __device__ __forceinline__ void value_group(const __nv_bfloat16* __restrict__ qk
   const int lane = threadIdx.x & 31, head_blocks = (to.Hk + 7) / 8;
   const int h = block % head_blocks * 8 + (threadIdx.x >> 5);
   if (h >= to.Hk) return;
-  const int t0 = block / head_blocks * kGroupTokens - group_shift(slots);
-  int slot;
-  if (t0 < 0 || t0 + kGroupTokens > T || !whole_page(slots, t0, T, lane, slot)) return;
-  const int slot0 = __shfl_sync(0xffffffffu, slot, 0);
+  int slot0;
+  const int t0 = whole_page_from(slots, block / head_blocks * kGroupTokens, T, lane, slot0);
+  if (t0 < 0) return;
   const __nv_bfloat16* src = qkv + size_t(to.Hq + to.Hk + h) * D + lane * VPL;
   uint2 raw[kGroupTokens][W];
 #pragma unroll
@@ -656,7 +662,7 @@ __device__ __forceinline__ void value_group(const __nv_bfloat16* __restrict__ qk
       }
     }
   }
-  if (lane < kGroupTokens) to.v_scale[(size_t(slot >> 4) * to.Hk + h) * 16 + (slot & 15)] = my_scale;
+  if (lane < kGroupTokens) to.v_scale[(size_t(slot0 >> 4) * to.Hk + h) * 16 + lane] = my_scale;
   uint4* dst = reinterpret_cast<uint4*>(to.v_cache + (size_t(slot0 >> 4) * to.Hk + h) * (size_t(16) * D) + lane * VPL * 16);
 #pragma unroll
   for (int w = 0; w < W; ++w) {
@@ -761,11 +767,8 @@ __device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ qkv,
 #pragma unroll
       for (int j = 0; j < HP; ++j) evaluate(j, sn[j], cs[j]);
     }
-    bool values_done = false;  // by the warps that take whole pages
-    if (value_blocks && h_end > Hq + Hk) {
-      int unused;
-      values_done = whole_page(slots, t - ((t + group_shift(slots)) & 15), T, lane, unused);
-    }
+    // by the warps that take whole pages
+    const bool values_done = value_blocks && h_end > Hq + Hk && in_whole_page(slots, t, slot_early, T, lane);
     const auto shared_angle = [&](int j, float& s, float& c) { s = sn[j]; c = cs[j]; };
     if constexpr (kAhead) {
 #pragma unroll
@@ -805,8 +808,8 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, cons
 }
 
 constexpr int kRopeHeads = 8;
-template <int D>
-__global__ void __launch_bounds__(256, 4) rope_kv_write_heads_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+template <int D, int kPerSm>  // CTAs per SM
+__global__ void __launch_bounds__(256, kPerSm) rope_kv_write_heads_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
                                      const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
                                      uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
                                      float* __restrict__ k_scale, float* __restrict__ v_scale, int T, int Hq, int Hk,
@@ -1002,7 +1005,6 @@ extern "C" int mfq_gate_quant_rows(const void* x, const void* gate, void* q_out,
 // q_norm_w / k_norm_w ([D] fp32, may be null): per-head RMSNorm of q / k before the rotation; row_stride: elements
 // between token rows of qkv (>= (Hq + 2 Hk) * D; an attention output gate may follow the v heads).
 // yarn_*: context extension (see RopeScale); factor 1 and mscale 1 are the plain rotation.
-constexpr long kSharedFrom = 18000;
 extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, const int* slots, void* q_out, void* k_cache,
                                       void* v_cache, float* k_scale, float* v_scale, int T, int Hq, int Hk, int D,
                                       int page_size, int rot, float theta, void* kd_out, void* vd_out,
@@ -1013,21 +1015,27 @@ extern "C" int mfq_rope_kv_write_yarn(const void* qkv, const int* positions, con
   if (!(yarn_factor >= 1.f) || !(yarn_high > yarn_low) || !(yarn_mscale > 0.f)) return -1;
   // A warp per head, or one per kRopeHeads heads of a token, whose angles (sine, cosine and the frequency's power, a good part of a head's
   // work) it evaluates once.  That needs full rotary, enough heads that the fewer and longer warps still fill the GPU, and groups that are
-  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  The eight heads of a warp
-  // are requested together, and the values of whole pages go by themselves (value_group).  48 heads of 128 on a B200, a warp per head | eight
-  // heads | and values by pages: 200 tokens 5.9 | 6.9 | 7.4 us, 357 8.1 | 8.4 | 8.2, 512 10.5 | 9.8 | 9.6, 700 13.4 | 10.5 | 10.3, 1000 18.8 | 14.5 |
-  // 12.9, 4096 68.7 | 43.4 | 39.3 (each head loaded after the one before, eight heads took 15.2 and 47.0).
+  // three quarters full; and its stores are up to 8 bytes wide, where a warp per head writes values one by one.  Up to 128 wide the eight heads
+  // of a warp are requested together, and from 128 on a prompt's values of whole pages go by themselves (value_group).
+  // On a B200, a warp per head | eight heads | and values by pages, one prompt | prompts of 40 to 200 tokens packed:
+  //   48 heads of 128, 378 tokens 8.1 | 8.3 | 8.1 | 8.2 us, 605 11.5 | 10.0 | 9.2 | 9.6, 834 14.9 | 13.5 | 11.9 | 12.3, 2084 32 | 22 | 20.3 | 20.6
+  //   16 of 128, 1132 tokens 6.5 | 7.6 | 5.6 | 6.3, 1813 9.3 | 8.5 | 6.3 | 6.6    16 of 256, 1132 15.4 | 22.8 | 12.3 | 13.6, 2063 24.9 | 26.6 | 17.8 | 17.9
+  // so the line is 18000 heads of work with values by pages, and 36000 without (rows of a decode batch, other pages).
+  // Heads of 64 have no such values: 48 of them, 459 tokens 5.9 | 7.3 us, 605 7.3 | 7.3, 688 8.0 | 7.4.  Their warps are alike in length, so waves
+  // of CTAs are what counts: four CTAs per SM take 7.3 us a wave, 11.8 two, 17.2 three, and six, with 28 bytes of spills, 10.4 and 15.0.
   const int heads = Hq + 2 * Hk, full_groups = (heads + kRopeHeads - 1) / kRopeHeads;
   const bool aligned = (reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kd_out) | reinterpret_cast<uintptr_t>(vd_out)) % 8 == 0;
-  const bool shared = rot == D && long(T) * heads >= kSharedFrom && 4 * heads >= 3 * kRopeHeads * full_groups && aligned;
+  const bool by_pages = D >= 128 && page_size == 16 && reinterpret_cast<uintptr_t>(qkv) % 8 == 0 && row_stride % 4 == 0 && reinterpret_cast<uintptr_t>(v_cache) % 16 == 0;
+  const long shared_from = by_pages && kd_out ? 18000 : D == 64 ? 30000 : 36000;
+  const bool shared = rot == D && long(T) * heads >= shared_from && 4 * heads >= 3 * kRopeHeads * full_groups && aligned;
   // values of whole pages sixteen tokens at a time
-  const bool grouped = shared && D >= 128 && page_size == 16 && reinterpret_cast<uintptr_t>(qkv) % 8 == 0 && row_stride % 4 == 0 && reinterpret_cast<uintptr_t>(v_cache) % 16 == 0;
-  const int value_blocks = grouped ? (T + 15 + kGroupTokens - 1) / kGroupTokens * ((Hk + 7) / 8) : 0;
+  const int value_blocks = shared && by_pages ? (T + kGroupTokens - 1) / kGroupTokens * ((Hk + 7) / 8) : 0;
   const int blocks = value_blocks + int((long(T) * (shared ? full_groups : heads) + 7) / 8);
+  const bool six = D == 64 && (blocks > 8 * 148 || (blocks > 4 * 148 && blocks <= 6 * 148));
   const float l2t = log2f(theta);
   const RopeScale ys{yarn_factor, yarn_low, yarn_high, yarn_mscale};
 #define MFQ_ROPE(DD)                                                                                             \
-  launch_kernel(shared ? rope_kv_write_heads_kernel<DD> : rope_kv_write_kernel<DD>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkv), positions, slots, \
+  launch_kernel(!shared ? rope_kv_write_kernel<DD> : six ? rope_kv_write_heads_kernel<DD, DD == 64 ? 6 : 4> : rope_kv_write_heads_kernel<DD, 4>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkv), positions, slots, \
       static_cast<__nv_bfloat16*>(q_out), static_cast<uint8_t*>(k_cache), static_cast<uint8_t*>(v_cache),      \
       k_scale, v_scale, T, Hq, Hk, page_size, rot, l2t, static_cast<__nv_bfloat16*>(kd_out),                   \
       static_cast<__nv_bfloat16*>(vd_out), q_norm_w, k_norm_w, norm_eps, row_stride, ys, value_blocks)

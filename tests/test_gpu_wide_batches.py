@@ -325,6 +325,31 @@ def test_values_that_go_to_whole_pages_together(d, how):
     check_status()
 
 
+@pytest.mark.parametrize("d,t,hq,hk", [(128, 1200, 12, 2), (128, 400, 32, 8), (256, 1200, 12, 2), (256, 500, 28, 9), (64, 4000, 6, 1), (64, 6000, 6, 1),
+                                       (64, 8000, 6, 1), (64, 10000, 6, 1)])
+def test_rotation_of_prompts_packed_one_after_the_other(d, t, hq, hk):
+    """Pieces of 1 to 90 tokens, each from the start of a page or from inside one, so that whole pages begin at any token of the batch, a page
+    whose tokens are interrupted by another's, and the last page cut short: the pages and rows of calls too small for whole pages."""
+    require_gpu_lib()
+    g, slots, page = torch.Generator().manual_seed(t), [], 1
+    while len(slots) < t:
+        n, inside = (int(torch.randint(a, b, (1,), generator=g)) for a, b in ((1, 90), (0, 5)))
+        slots += range(page * 16 + 3 * inside, page * 16 + 3 * inside + n)
+        page = slots[-1] // 16 + 1
+    slots[100:108], slots[300] = reversed(slots[100:108]), -1
+    slots = torch.tensor(slots[:t], dtype=torch.int32, device="cuda")
+    rows, pos = _normal(d, t, (hq + 2 * hk) * d), torch.arange(t, device="cuda", dtype=torch.int32)
+    got = []
+    for step in (t, 160):
+        cache = PagedKVCache(layers=1, kv_heads=hk, head_dim=d, num_pages=page + 1, max_seqs=1, max_pages_per_seq=page, device="cuda")
+        kd, vd = torch.zeros((t, hk, d), device="cuda", dtype=torch.bfloat16), torch.zeros((t, hk, d), device="cuda", dtype=torch.bfloat16)
+        q = torch.cat([ops.rope_kv_write(rows[a : a + step], pos[a : a + step], slots[a : a + step], cache.layer(0), n_q=hq, n_kv=hk, head_dim=d, theta=1e4,
+                                         kd_out=kd[a : a + step], vd_out=vd[a : a + step]) for a in range(0, t, step)])
+        got.append([q, cache.k.view(torch.uint8), cache.v.view(torch.uint8), cache.k_scale, cache.v_scale, kd, vd])
+    check_status()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("m,k", [(16, 4096), (600, 4096), (300, 14336), (200, 14336), (5200, 512)])
 def test_gates_of_every_value_round_as_the_division_does(m, k):
     """All bf16 values as gates, zeros of either sign, subnormal, infinite and NaN among them, through every kernel that quantizes gated rows:
