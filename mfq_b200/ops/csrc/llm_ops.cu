@@ -1141,7 +1141,31 @@ extern "C" int mfq_silu_mul_bf16(const void* x, void* out, int M, int I, int in_
 // that reads byte by byte (4001 tokens 10.3 us, 357 2.9), so 7.8 and 3.1.
 // ---------------------------------------------------------------------------------------------
 namespace mfq {
-template <int D>
+// kVectors: pages and rows on 16-byte boundaries; else bytes and single values, as a caller's own buffers may need.
+template <bool kVectors>
+__device__ __forceinline__ uint4 load_codes(const uint8_t* from) {
+  if constexpr (kVectors) return *reinterpret_cast<const uint4*>(from);
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = from[4 * i] | uint32_t(from[4 * i + 1]) << 8 | uint32_t(from[4 * i + 2]) << 16 | uint32_t(from[4 * i + 3]) << 24;
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <bool kVectors, int N>
+__device__ __forceinline__ void store_pairs(__nv_bfloat16* to, const uint32_t (&pairs)[N]) {
+  if constexpr (!kVectors) {
+#pragma unroll
+    for (int i = 0; i < 2 * N; ++i) reinterpret_cast<unsigned short*>(to)[i] = static_cast<unsigned short>(pairs[i / 2] >> (16 * (i & 1)));
+  } else if constexpr (N == 1) {
+    *reinterpret_cast<uint32_t*>(to) = pairs[0];
+  } else if constexpr (N == 2) {
+    *reinterpret_cast<uint2*>(to) = make_uint2(pairs[0], pairs[1]);
+  } else {
+    static_assert(N % 4 == 0, "whole vectors");
+#pragma unroll
+    for (int i = 0; i < N; i += 4) reinterpret_cast<uint4*>(to)[i / 4] = make_uint4(pairs[i], pairs[i + 1], pairs[i + 2], pairs[i + 3]);
+  }
+}
+template <int D, bool kVectors>
 __global__ void __launch_bounds__(256) kv_gather_dequant_kernel(const uint8_t* __restrict__ k_cache, const uint8_t* __restrict__ v_cache,
                                          const float* __restrict__ k_scale, const float* __restrict__ v_scale,
                                          const int* __restrict__ block_row, __nv_bfloat16* __restrict__ kd,
@@ -1162,25 +1186,24 @@ __global__ void __launch_bounds__(256) kv_gather_dequant_kernel(const uint8_t* _
     return *reinterpret_cast<const uint32_t*>(&r);
   };
   if (side == 0) {  // [D / 64 chunks][16 tokens][64 dims]
-    const uint4* src = reinterpret_cast<const uint4*>(k_cache + ph * (size_t(P) * D));
+    const uint8_t* src = k_cache + ph * (size_t(P) * D);
 #pragma unroll
     for (int i = 0; i < D / 32; ++i) {
       const int v = i * 32 + lane, chunk = v >> 6, t = (v >> 2) & 15, dim = chunk * 64 + (v & 3) * 16;
-      const uint4 c = src[v];
+      const uint4 c = load_codes<kVectors>(src + v * 16);
       const float s = __shfl_sync(0xffffffffu, my_scale, t);
       if (t < rows) {
-        uint4* dst = reinterpret_cast<uint4*>(kd + (size_t(t0 + t) * Hk + h) * D + dim);
-        dst[0] = make_uint4(two(c.x, 0, s), two(c.x, 2, s), two(c.y, 0, s), two(c.y, 2, s));
-        dst[1] = make_uint4(two(c.z, 0, s), two(c.z, 2, s), two(c.w, 0, s), two(c.w, 2, s));
+        const uint32_t row[8] = {two(c.x, 0, s), two(c.x, 2, s), two(c.y, 0, s), two(c.y, 2, s), two(c.z, 0, s), two(c.z, 2, s), two(c.w, 0, s), two(c.w, 2, s)};
+        store_pairs<kVectors>(kd + (size_t(t0 + t) * Hk + h) * D + dim, row);
       }
     }
     return;
   }
   constexpr int VPL = D / 32;  // dims of a lane
-  const uint4* src = reinterpret_cast<const uint4*>(v_cache + ph * (size_t(P) * D) + lane * VPL * P);
+  const uint8_t* src = v_cache + ph * (size_t(P) * D) + lane * VPL * P;
   uint4 c[VPL];
 #pragma unroll
-  for (int j = 0; j < VPL; ++j) c[j] = src[j];
+  for (int j = 0; j < VPL; ++j) c[j] = load_codes<kVectors>(src + j * P);
 #pragma unroll
   for (int t = 0; t < P; ++t) {
     const float s = __shfl_sync(0xffffffffu, my_scale, t);
@@ -1192,12 +1215,7 @@ __global__ void __launch_bounds__(256) kv_gather_dequant_kernel(const uint8_t* _
       const uint32_t b = word == 0 ? c[j + 1].x : word == 1 ? c[j + 1].y : word == 2 ? c[j + 1].z : c[j + 1].w;
       out[j / 2] = two(__byte_perm(a, b, (byte >> 3) | (4 + (byte >> 3)) << 4), 0, s);
     }
-    if (t < rows) {
-      __nv_bfloat16* dst = vd + (size_t(t0 + t) * Hk + h) * D + lane * VPL;
-      if constexpr (VPL == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
-      else if constexpr (VPL == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(out[0], out[1]);
-      else *reinterpret_cast<uint32_t*>(dst) = out[0];
-    }
+    if (t < rows) store_pairs<kVectors>(vd + (size_t(t0 + t) * Hk + h) * D + lane * VPL, out);
   }
 }
 }  // namespace mfq
@@ -1207,10 +1225,10 @@ extern "C" int mfq_kv_gather_dequant(const void* k_cache, const void* v_cache, c
                                      const int* block_row, void* kd, void* vd, int T, int Hk, int D, int page_size,
                                      cudaStream_t stream) {
   if (T <= 0 || Hk <= 0 || page_size != 16) return -1;
-  if ((reinterpret_cast<uintptr_t>(kd) | reinterpret_cast<uintptr_t>(vd) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) return -1;
+  const bool vectors = ((reinterpret_cast<uintptr_t>(kd) | reinterpret_cast<uintptr_t>(vd) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   const int blocks = (2 * ((T + 15) / 16) * Hk + 7) / 8;
 #define MFQ_GATHER(DD)                                                                                              \
-  mfq::launch_kernel(mfq::kv_gather_dequant_kernel<DD>, dim3(blocks), dim3(256), 0, stream,                        \
+  mfq::launch_kernel(vectors ? mfq::kv_gather_dequant_kernel<DD, true> : mfq::kv_gather_dequant_kernel<DD, false>, dim3(blocks), dim3(256), 0, stream,                        \
                      static_cast<const uint8_t*>(k_cache), static_cast<const uint8_t*>(v_cache), k_scale, v_scale,  \
                      block_row, static_cast<__nv_bfloat16*>(kd), static_cast<__nv_bfloat16*>(vd), T, Hk)
   if (D == 128) MFQ_GATHER(128);

@@ -1,6 +1,7 @@
 """Kernels that wide batches and prompts take: products on pairs of SMs, row quantization in one pass, several heads of a token per
 warp, router logits through the dense product -- at the edges of their tiles and of the rules that choose them."""
 
+import dataclasses
 import math
 
 import pytest
@@ -348,6 +349,34 @@ def test_rotation_of_prompts_packed_one_after_the_other(d, t, hq, hk):
         got.append([q, cache.k.view(torch.uint8), cache.v.view(torch.uint8), cache.k_scale, cache.v_scale, kd, vd])
     check_status()
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_past_rows_off_a_vector(d):
+    """Pages that begin at an odd byte, rows 2 bytes past a vector: the rows that aligned ones give, and nothing beside them."""
+    require_gpu_lib()
+    t, hk = 77, 3
+    cache = PagedKVCache(layers=1, kv_heads=hk, head_dim=d, num_pages=7, max_seqs=1, max_pages_per_seq=6, device="cuda")
+    table = torch.tensor([3, 1, 6, 2, 5], device="cuda", dtype=torch.int32)
+    ops.rope_kv_write(_normal(d, 96, 3 * hk * d), torch.arange(96, device="cuda", dtype=torch.int32), torch.arange(16, 112, device="cuda", dtype=torch.int32),
+                      cache.layer(0), n_q=hk, n_kv=hk, head_dim=d, theta=1e4)
+    kv = cache.layer(0)
+    want = K.kv_gather_dequant(kv, table, t)
+
+    def shifted(x, by):
+        flat = torch.zeros(x.numel() + 16, device="cuda", dtype=x.dtype)[by : by + x.numel()]
+        flat.view(torch.uint8).copy_(x.reshape(-1).view(torch.uint8))
+        return flat.view(x.shape)
+
+    rows = [torch.full((t * hk * d + 16,), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    for pages, row in ((0, 1), (3, 0), (1, 1)):
+        odd = dataclasses.replace(kv, k=shifted(kv.k, pages), v=shifted(kv.v, pages))
+        for r in rows:
+            r.fill_(7.0)
+        got = K.kv_gather_dequant(odd, table, t, *(r[row : row + t * hk * d].view(t, hk, d) for r in rows))
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+        assert all((r[:row] == 7).all() and (r[row + t * hk * d :] == 7).all() for r in rows)
+    check_status()
 
 
 @pytest.mark.parametrize("m,k", [(16, 4096), (600, 4096), (300, 14336), (200, 14336), (5200, 512)])
