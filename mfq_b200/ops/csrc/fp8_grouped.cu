@@ -34,7 +34,8 @@ struct GroupedCfg {
   static constexpr int kGroups = kEpiWarps / 4;       // of four warps: 128 weight rows x kCols tokens
   static constexpr int kTurnBytes = kCols * kTileN * 2;  // their results on the way out
   static constexpr int kTurnAt = kStages * kStageBytes, kBarsAt = kTurnAt + (kTurned ? kGroups * kTurnBytes : 0);
-  static constexpr int kSmemBytes = kBarsAt + 1024 + 256;
+  static constexpr int kBarBytes = (2 * kStages + 2 * kAcc + 4) * 8 + 8;  // two per stage and accumulator, four of the turned results; TMEM slot, abort flag
+  static constexpr int kSmemBytes = kBarsAt + kBarBytes + 1024;           // aligned by hand
 };
 
 struct GroupedParams {

@@ -70,3 +70,17 @@ def test_warps_are_whole_at_an_aligned_cluster_barrier(name):
     of different lengths or a branch: the barrier brings them together itself."""
     body = re.search(r"void \w*cluster_barrier\(\) \{\s*(.*)", (CSRC / name).read_text()).group(1)
     assert body.startswith("__syncwarp();")
+
+
+def test_barriers_of_the_grouped_product_have_their_place():
+    """What the kernel lays out behind the ring is what the configuration sets aside, for every tile: tiles of 16 tokens have ten stages, and
+    their barriers took 264 bytes of 256."""
+    text = (CSRC / "fp8_grouped.cu").read_text()
+    stages = eval(re.sub(r"BT == (\d+) \? (\d+) :", r"\2 if bt == \1 else", re.search(r"kStages = (BT.*?);", text).group(1)), {"bt": 16})
+    acc = int(re.search(r"kAcc = (\d+);", text).group(1))
+    fixed = int(re.search(r"turn_free = turn_full \+ (\d+);", text).group(1)) + int(re.search(r"\(turn_free \+ (\d+)\);", text).group(1))
+    laid_out = 8 * (2 * stages + 2 * acc + fixed) + 2 * 4
+    size = re.search(r"kSmemBytes = kBarsAt \+ (.*?);", text).group(1)
+    scope = {"kStages": stages, "kAcc": acc}
+    scope["kBarBytes"] = eval(m.group(1), scope) if (m := re.search(r"kBarBytes = (.*?);", text)) else 0
+    assert stages == 10 and laid_out <= eval(size, scope) - 1024
