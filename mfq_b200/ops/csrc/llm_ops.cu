@@ -1134,6 +1134,24 @@ extern "C" int mfq_silu_mul_bf16(const void* x, void* out, int M, int I, int in_
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 
+namespace mfq {
+__global__ void __launch_bounds__(256) silu_check_kernel(const float2* __restrict__ g, float2* __restrict__ paired, float2* __restrict__ divided, int pairs) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= pairs) return;
+  const float2 v = g[i];
+  paired[i] = silu2(v);
+  divided[i] = make_float2(v.x / (1.f + __expf(-v.x)), v.y / (1.f + __expf(-v.y)));
+}
+}  // namespace mfq
+
+// silu2 and what it stands for, in fp32: a gated row's bf16 and 8 bits would hide a quotient that is off in its last places.
+extern "C" int mfq_silu_check(const float* gates, float* paired, float* divided, int pairs, cudaStream_t stream) {
+  if (pairs <= 0 || (reinterpret_cast<uintptr_t>(gates) | reinterpret_cast<uintptr_t>(paired) | reinterpret_cast<uintptr_t>(divided)) & 7) return -1;
+  mfq::silu_check_kernel<<<(pairs + 255) / 256, 256, 0, stream>>>(reinterpret_cast<const float2*>(gates), reinterpret_cast<float2*>(paired),
+                                                                  reinterpret_cast<float2*>(divided), pairs);
+  return cudaGetLastError() == cudaSuccess ? 0 : -7;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Past K/V of one sequence out of the FP8 pages into contiguous bf16 [T, Hk, D] (code * multiplier): the keys /
 // values a later prefill chunk attends to (chunked prefill, restored prefix).  A warp takes one head's page: its rows by 16 bytes, and of the

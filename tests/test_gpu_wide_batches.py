@@ -351,6 +351,30 @@ def test_rotation_of_prompts_packed_one_after_the_other(d, t, hq, hk):
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("beside", ["one", "another", "bounds", "any"])
+def test_pairs_of_gates_have_the_bits_of_the_division(beside):
+    """The fp32 quotients themselves: every bf16 gate in either lane of a pair, next to gates of either side of the bounds from which a pair
+    divides (64 and 1e-30), and any bits at all."""
+    require_gpu_lib()
+    gates = torch.arange(1 << 16, device="cuda").to(torch.int32).to(torch.int16).view(torch.bfloat16).float()
+    if beside == "any":
+        g = torch.Generator(device="cuda").manual_seed(0)
+        pairs = [torch.randint(-(1 << 31), 1 << 31, (1 << 22,), generator=g, device="cuda").to(torch.int32).view(torch.float32).view(-1, 2)]
+    elif beside == "bounds":
+        edge = torch.tensor([64.0, 1e-30], device="cuda").view(torch.int32)
+        edge = torch.cat([edge + i for i in range(-2, 3)]).view(torch.float32)
+        edge = torch.cat([edge, -edge])
+        pairs = [torch.stack([gates, e.expand_as(gates)], 1) for e in edge] + [torch.cartesian_prod(edge, edge)]
+    else:
+        other = torch.ones_like(gates) if beside == "one" else gates.roll(12345)
+        pairs = [torch.stack([gates, other], 1)]
+    x = torch.cat(pairs + [p.flip(1) for p in pairs]).contiguous()
+    paired, divided = torch.empty_like(x), torch.empty_like(x)
+    K.check(K.lib().mfq_silu_check(K.ptr(x), K.ptr(paired), K.ptr(divided), x.shape[0], K.stream_ptr()), "silu_check")
+    assert torch.equal(paired.isnan(), divided.isnan())
+    assert torch.equal(paired.view(torch.int32)[~divided.isnan()], divided.view(torch.int32)[~divided.isnan()])
+
+
 @pytest.mark.parametrize("d", [64, 128, 256])
 def test_past_rows_off_a_vector(d):
     """Pages that begin at an odd byte, rows 2 bytes past a vector: the rows that aligned ones give, and nothing beside them."""
