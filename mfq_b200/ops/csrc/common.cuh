@@ -164,7 +164,8 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // of this grid had still to allocate, it could take the columns that this CTA needs and wait, without end, for this grid.  Once all CTAs have
 // triggered, all hold what they need, and a successor that finds too little waits for them, which end without it.
 // Beside that, correctness only depends on pdl_wait() preceding the first access to memory another kernel produced (and the
-// first global write).
+// first global write).  Weights are apart: products and the small router request the first of them ahead of the wait.  No kernel here writes
+// any; whoever changes weights in place on the stream of their product puts a launch without this attribute between the two.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -51,7 +51,7 @@ struct PairCfg {
   static constexpr int kStageBytes = kRows * kBK + (BT / 2) * kBK;
   static constexpr int kEpiWarps = 8;
   static constexpr int kCols = BT / 2;   // accumulator columns per epilogue thread
-  static constexpr int kThreads = 128 + 32 * kEpiWarps;  // warp group 0: TMA, MMA and two idle warps; groups 1, 2: epilogue
+  static constexpr int kThreads = 128 + 32 * kEpiWarps;  // warp group 0: TMA, MMA, output places, multipliers; groups 1, 2: epilogue
   static constexpr int kWsMax = 256;
   // Output places: 32 tokens x 128 weight rows of one warp (kTokenRows), else 64 tokens x 64 weight rows of two.
   static constexpr int kPlaces = kTokenRows ? kEpiWarps : kEpiWarps / 2, kPlaceWarps = kEpiWarps / kPlaces, kPlaceBytes = 8192;

@@ -108,7 +108,7 @@ __device__ __forceinline__ uint32_t plan_peer_load(const int* mine, int cta) {  
   return v;
 }
 
-// Route plan for the experts [e_lo, e_hi) owned by this rank (one CTA).  Row order inside an expert depends on atomic
+// Route plan for the experts [e_lo, e_hi) owned by this rank, by one CTA or a cluster of them.  Row order inside an expert depends on atomic
 // arrival order; results do not, because each row is computed independently and the un-permute sums a token's K
 // contributions in slot order.
 //   offsets[e - e_lo]   first sorted row of local expert e (offsets[n_local] = total rows)

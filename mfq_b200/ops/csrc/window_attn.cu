@@ -57,7 +57,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// DK / DV: upper bounds of the stored widths of a KV head (register arrays); the widths themselves are run-time multiples of 16.
 // Rows of D channels, one after the other, to rows of D + 8: a lane keeps its channels, 32 lanes take 32 * 8 / D rows at a time.
 template <int D>
 __device__ __forceinline__ void copy_page(uint32_t to, const __nv_bfloat16* from, int lane) {
@@ -79,6 +78,7 @@ struct WinCfg {
   }
 };
 
+// DK / DV: upper bounds of the stored widths of a KV head (register arrays); the widths themselves are run-time multiples of 16.
 // kWhole: one map whose widths are the bounds, no bias.  A warp spends some 2 us on a page of 16 keys, with more of them in flight no less:
 // it is bound by what it issues.  The widths known to the compiler leave a copy one instruction, and a page that every query sees whole
 // needs no comparisons.  8 KV heads of 4 queries, 128 channels, 3 splits and their sum, 16 rows of 1024 keys 21.6 -> 20.2 us, of 2000

@@ -149,7 +149,9 @@ def fp8_gemm(x_q: torch.Tensor, x_scale: torch.Tensor, w_q: torch.Tensor, w_scal
              out: torch.Tensor | None = None, residual: torch.Tensor | None = None, splits: int | None = None,
              token_tile: int | None = None, pair: int | None = None) -> torch.Tensor:
     """``out[M, N] = (x_q * x_scale[:, None]) @ (w_q * blockscale(w_scale)).T`` in bf16 (+ residual).
-    ``pair``: token tile (128 / 256) of the two-SM kernel, 0 = never, None = by shape (:func:`pair_tile`)."""
+    ``pair``: token tile (128 / 256) of the two-SM kernel, 0 = never, None = by shape (:func:`pair_tile`).
+    The first weights are requested while the launch before may still run: a kernel that changes ``w_q`` or ``w_scale`` in place is followed by
+    another launch, or a synchronization, before its product."""
     m, k = x_q.shape
     n = w_q.shape[0]
     assert w_q.shape[1] == k and k % 128 == 0 and x_q.dtype == FP8 and w_q.dtype == FP8

@@ -59,6 +59,7 @@ ROUTER_MMA_ROWS = 64  # router logits of more tokens go through the dense produc
 def router_topk(x: torch.Tensor, w: torch.Tensor, k: int, *, bias: torch.Tensor | None = None, sigmoid: bool = False,
                 norm_topk: bool = True, scale: float = 1.0, n_group: int = 1, topk_group: int = 1,
                 want_scores: bool = False):
+    """Expert ids and weights of every token.  As with the products, the first weights are requested while the launch before may still run."""
     t, h = x.shape
     e = w.shape[0]
     ids = torch.empty((t, k), dtype=torch.int32, device=x.device)

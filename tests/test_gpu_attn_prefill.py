@@ -164,3 +164,22 @@ def test_grids_that_fill_two_ctas_per_sm(t, past, hq, hk):
         want = ops.kernels.attn_prefill_bf16(q[:, h * per : (h + 1) * per].contiguous(), k[:, h : h + 1].contiguous(), v[:, h : h + 1].contiguous(), 0.09)
         assert torch.equal(got[:, h * per : (h + 1) * per], want), h
     check_status()
+
+
+@pytest.mark.parametrize("t,past,hq,hk", [(257, 0, 84, 21), (385, 126, 64, 16)])
+def test_infinite_values_by_either_form(t, past, hq, hk):
+    """Keys, queries and values that are infinite or NaN, behind the diagonal and ahead of it: where either form gives NaN, the other does, and the
+    rest are the same bits."""
+    require_gpu_lib()
+    g = torch.Generator(device="cuda").manual_seed(t)
+    q, k, v = (torch.randn((n, h, 128), generator=g, device="cuda").to(torch.bfloat16) for n, h in ((t, hq), (past + t, hk), (past + t, hk)))
+    q[5, 0, 3], k[past + 200, 1, 7], k[130, 2, 0], k[past + t - 1, 3, 9] = float("inf"), -float("inf"), float("inf"), float("nan")
+    v[past + 3, 4, 5], v[past + 250, 5, 6], v[140, 6, 0] = float("inf"), -float("inf"), float("nan")
+    per = hq // hk
+    assert -(-t // 128) * hq >= 250 > -(-t // 128) * per
+    got = ops.kernels.attn_prefill_bf16(q, k, v, 0.09)
+    for h in range(8):
+        want = ops.kernels.attn_prefill_bf16(q[:, h * per : (h + 1) * per].contiguous(), k[:, h : h + 1].contiguous(), v[:, h : h + 1].contiguous(), 0.09)
+        own = got[:, h * per : (h + 1) * per]
+        assert torch.equal(own.isnan(), want.isnan()) and torch.equal(own[~want.isnan()], want[~want.isnan()]), h
+    check_status()
