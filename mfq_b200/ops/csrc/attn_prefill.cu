@@ -10,7 +10,7 @@
 // The chain  softmax -> P V -> fold  is several times as long as the MMAs, so Q K^T of block j + 1 is issued before P V of block j, into
 // the other of two S buffers, and all of it but the chain itself is hidden; P never passes through shared memory and its proxy fence.
 // What bounds it is the softmax: exponentials, and the two passes over S.
-// Grids that fill two CTAs per SM take the pair form: K and V in one stage each, one S buffer (P lies in S, so Q K^T of block j + 1 follows
+// Grids that fill two CTAs per SM (two_ctas_per_sm) take the pair form: K and V in one stage each, one S buffer (P lies in S, so Q K^T of block j + 1 follows
 // P V of block j), a thread per query row with all 128 of its outputs in registers, no exchange of maxima.  Its chain per block is half as long
 // again, but two CTAs hide each other's waits.  O alpha + O_blk is formed as a product while P V runs and a sum while the next Q K^T does, by
 // two values per instruction in either form.  32 heads on a B200, one CTA per SM one value per instruction | two | pair form, same bits:
@@ -520,8 +520,28 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 
 }  // namespace mfq
 
-// Grids from this size on take the pair form: fewer leave SMs with one CTA, whose longer chain nothing hides.
-constexpr int kPairCtas = 250;
+namespace mfq {
+// Which form a grid takes.  Two CTAs per SM share its rate and hide each other's waits (7 to 20 %), but a CTA alone is half as slow again, so the
+// pair form needs company for the longest tiles: enough key blocks in all against those of the first tile, and, in a grid of two
+// or three rounds of one CTA per SM, none of those rounds nearly full of tiles alike, which one CTA per SM works off without a rest.  (With a
+// long past tiles are alike, and then up to two rounds are the other way about: all of them at once by twos.)  One | pair, on a B200:
+//   16 heads: 2028 tokens (256 CTAs) 32.1 | 44.9 us, 2540 (320) 47 | 51, 3052 (384) 62.8 | 61.4, 4076 (512) 94 | 82
+//   32 heads: 1004 tokens (256) 20.9 | 24.9, 1260 (320) 31.0 | 29.3, after 3000 (320) 128 | 127; 1004 after 300 30.7 | 33.1, after 1000 43.6 | 45.3,
+//   after 3000 85.8 | 84.3, after 8000 188 | 178; 1516 after 8000 (384, three rounds nearly full) 289 | 321
+// Over 540 grids of 148 to 1024 CTAs and pasts to 8000 the slower form is taken in 4 by more than 2 % (8 %), and choosing costs 0.7 % on average.
+constexpr int kSms = 148;
+static bool two_ctas_per_sm(int T, int Tk, int Hq) {
+  const long blocks = (T + kQB - 1) / kQB, past = (Tk - T + kKB - 1) / kKB, ctas = blocks * Hq;
+  if (ctas < 250) return false;
+  const auto keys = [&](long cta) { return min((Tk + kKB - 1L) / kKB, blocks - cta / Hq + past); };  // key blocks of the tile of a CTA; heavy ones first
+  const long most = keys(0), all = Hq * (blocks * (blocks + 1) / 2 + blocks * past);
+  if (ctas <= 2 * kSms) return 100 * keys(kSms) >= 87 * most;
+  return 4 * all >= 5 * kSms * most && (ctas > 3 * kSms || 100 * 3 * keys(2 * kSms) * kSms <= 93 * all);
+}
+}  // namespace mfq
+
+// 1: the pair form
+extern "C" int mfq_attn_prefill_form(int T, int Tk, int Hq) { return T > 0 && Tk >= T && Hq > 0 && mfq::two_ctas_per_sm(T, Tk, Hq); }
 
 // q: [T, Hq, 128] bf16, k/v: [Tk, Hk, 128] bf16 (contiguous), out: [T, Hq, 128] bf16.  Tk >= T: the first Tk - T keys
 // are the sequence's past (earlier chunks / a restored prefix); query i attends to keys 0 .. i + (Tk - T).
@@ -542,7 +562,7 @@ extern "C" int mfq_attn_prefill_past(const void* q, const void* k, const void* v
   }
   const PrefillParams p{static_cast<__nv_bfloat16*>(out), T, Hq, Hk, Tk, Tk - T, sm_scale * 1.4426950408889634f, status};
   const int ctas = (T + kQB - 1) / kQB * Hq;
-  if (ctas >= kPairCtas) launch_kernel(attn_prefill_pair_kernel, dim3(ctas), dim3(kPairThreads), kPairSmem, stream, tq, tk, tv, p);
+  if (two_ctas_per_sm(T, Tk, Hq)) launch_kernel(attn_prefill_pair_kernel, dim3(ctas), dim3(kPairThreads), kPairSmem, stream, tq, tk, tv, p);
   else launch_kernel(attn_prefill_kernel, dim3(ctas), dim3(kPrefillThreads), kPrefillSmem, stream, tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }

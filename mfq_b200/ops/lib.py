@@ -28,6 +28,7 @@ _SIGNATURES = {
     "mfq_rmsnorm_quant": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _vp],
     "mfq_quant_rows": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "mfq_kv_gather_dequant": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "mfq_attn_prefill_form": [_i, _i, _i],
     "mfq_attn_prefill_past": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp, _vp],
     "mfq_silu_mul_bf16": [_vp, _vp, _i, _i, _i, _vp],
     "mfq_silu_check": [_vp, _vp, _vp, _i, _vp],

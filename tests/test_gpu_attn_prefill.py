@@ -166,7 +166,36 @@ def test_grids_that_fill_two_ctas_per_sm(t, past, hq, hk):
     check_status()
 
 
-@pytest.mark.parametrize("t,past,hq,hk", [(257, 0, 84, 21), (385, 126, 64, 16)])
+def _form(t, past, hq):
+    return ops.kernels.lib().mfq_attn_prefill_form(t, past + t, hq)
+
+
+@pytest.mark.parametrize("t,past,hq,hk", [(513, 0, 84, 21), (1300, 0, 32, 8), (385, 126, 128, 32), (3100, 0, 16, 4), (200, 8000, 128, 16)])
+def test_two_ctas_per_sm_give_the_bits_of_one(t, past, hq, hk):
+    """Grids that take the pair form, and a few heads of them, which take the other: the same bits."""
+    require_gpu_lib()
+    g = torch.Generator(device="cuda").manual_seed(t)
+    q = torch.randn((t, hq, 128), generator=g, device="cuda").to(torch.bfloat16)
+    k = (torch.randn((past + t, hk, 128), generator=g, device="cuda") * torch.linspace(0.25, 4.0, past + t, device="cuda")[:, None, None]).to(torch.bfloat16)
+    v = torch.randn((past + t, hk, 128), generator=g, device="cuda").to(torch.bfloat16)
+    per = hq // hk
+    assert _form(t, past, hq) and not _form(t, past, per)
+    got = ops.kernels.attn_prefill_bf16(q, k, v, 0.09)
+    for h in range(0, hk, 3):
+        want = ops.kernels.attn_prefill_bf16(q[:, h * per : (h + 1) * per].contiguous(), k[:, h : h + 1].contiguous(), v[:, h : h + 1].contiguous(), 0.09)
+        assert torch.equal(got[:, h * per : (h + 1) * per], want), h
+    check_status()
+
+
+def test_grids_whose_longest_tiles_would_stand_alone_keep_one_cta_per_sm():
+    """Measured on either side: few tiles a head, tiles of many lengths with too few of them for all SMs, and three full rounds of tiles alike."""
+    require_gpu_lib()
+    for t, past, hq, pair in ((2028, 0, 16, 0), (2540, 0, 16, 0), (4076, 0, 16, 1), (1004, 0, 32, 0), (1516, 0, 32, 1), (2028, 0, 32, 1),
+                              (1004, 1000, 32, 0), (1004, 8000, 32, 1), (1516, 8000, 32, 0), (2028, 8000, 32, 1), (120, 0, 32, 0)):
+        assert _form(t, past, hq) == pair, (t, past, hq)
+
+
+@pytest.mark.parametrize("t,past,hq,hk", [(513, 0, 84, 21), (385, 126, 128, 32)])
 def test_infinite_values_by_either_form(t, past, hq, hk):
     """Keys, queries and values that are infinite or NaN, behind the diagonal and ahead of it: where either form gives NaN, the other does, and the
     rest are the same bits."""
@@ -176,7 +205,7 @@ def test_infinite_values_by_either_form(t, past, hq, hk):
     q[5, 0, 3], k[past + 200, 1, 7], k[130, 2, 0], k[past + t - 1, 3, 9] = float("inf"), -float("inf"), float("inf"), float("nan")
     v[past + 3, 4, 5], v[past + 250, 5, 6], v[140, 6, 0] = float("inf"), -float("inf"), float("nan")
     per = hq // hk
-    assert -(-t // 128) * hq >= 250 > -(-t // 128) * per
+    assert _form(t, past, hq) and not _form(t, past, per)
     got = ops.kernels.attn_prefill_bf16(q, k, v, 0.09)
     for h in range(8):
         want = ops.kernels.attn_prefill_bf16(q[:, h * per : (h + 1) * per].contiguous(), k[:, h : h + 1].contiguous(), v[:, h : h + 1].contiguous(), 0.09)
