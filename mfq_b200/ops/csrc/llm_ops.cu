@@ -82,7 +82,11 @@ constexpr int kNormVecs = 8;
 
 // Where a thread holds several vectors they wait as the bf16 values that they are, four registers a vector: 4096 rows of 4096 on a B200 with
 // eight registers a vector (84 a thread) 18.6 us, so 12.8; 2000 rows 12.8 -> 8.5.
-template <int kNormVecs>
+// kAhead: all of the residual and the multipliers are requested before the first of them is used, for 16 to 24 more registers.  That pays where
+// the rows are on the SMs at once either way, and without it they wait longer than with fp32 values.  fp32 | bf16 | requested ahead, in a chain
+// with another kernel: 200 rows of 8192 with residual 5.9 | 7.2 | 5.5 us, 296 of 16384 7.7 | 10.9 | 7.1, 1100 of 4096 10.9 | 12.0 | 9.3; but 900 of 8192
+// 14.1 | 11.4 | 12.6 and 1300 of 8192 21.3 | 13.5 | 14.1.
+template <int kNormVecs, bool kAhead = false>
 __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                                      __nv_bfloat16* __restrict__ residual_out, const __nv_bfloat16* __restrict__ w,
                                      uint8_t* __restrict__ q_out, float* __restrict__ scale_out,
@@ -114,13 +118,22 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
     if (vi < nvec) held[i] = *reinterpret_cast<const uint4*>(x + row * H + vi * 8);
   }
   if (residual) {
+    uint4 add[kAhead ? kNormVecs : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int i = 0; i < kNormVecs; ++i) {
+        const int vi = threadIdx.x + i * blockDim.x;
+        if (vi < nvec) add[i] = *reinterpret_cast<const uint4*>(residual + row * H + vi * 8);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < kNormVecs; ++i) {
       const int vi = threadIdx.x + i * blockDim.x;
       if (vi < nvec) {
         float a[8], r[8];
         load8(held[i], a);
-        load8(*reinterpret_cast<const uint4*>(residual + row * H + vi * 8), r);
+        if constexpr (kAhead) load8(add[i], r);
+        else load8(*reinterpret_cast<const uint4*>(residual + row * H + vi * 8), r);
 #pragma unroll
         for (int j = 0; j < 8; ++j) a[j] += r[j];
         held[i] = pack8(a);
@@ -139,6 +152,14 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
       for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
     }
   }
+  uint4 held_w[kAhead ? kNormVecs : 1];
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int i = 0; i < kNormVecs; ++i) {
+      const int vi = threadIdx.x + i * blockDim.x;
+      if (vi < nvec) held_w[i] = *reinterpret_cast<const uint4*>(w + vi * 8);
+    }
+  }
   const float rstd = rsqrtf(block_reduce<false>(ss, red) / float(H) + eps);
   float amax = 0.f;
 #pragma unroll
@@ -147,7 +168,8 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
     if (vi < nvec) {
       float v[8], wv[8];
       load8(held[i], v);
-      load8(*reinterpret_cast<const uint4*>(w + vi * 8), wv);
+      if constexpr (kAhead) load8(held_w[i], wv);
+      else load8(*reinterpret_cast<const uint4*>(w + vi * 8), wv);
       // round through bf16 like an unfused norm would, so fused and unfused paths agree bit for bit
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = v[j] * rstd * wv[j];
@@ -957,8 +979,8 @@ extern "C" int mfq_rmsnorm_quant(const void* x, const void* residual, void* resi
   };
   // vectors a thread has to hold: registers for no more than that leave room for more rows on an SM
   if (H / 8 <= threads) launch(rmsnorm_quant_kernel<1>);
-  else if (H / 8 <= 4 * threads) launch(rmsnorm_quant_kernel<4>);
-  else launch(rmsnorm_quant_kernel<kNormVecs>);
+  else if (H / 8 <= 4 * threads) launch(M <= 2 * 148 ? rmsnorm_quant_kernel<4, true> : rmsnorm_quant_kernel<4>);
+  else launch(M <= 1600 && H <= 4096 ? rmsnorm_quant_kernel<kNormVecs, true> : rmsnorm_quant_kernel<kNormVecs>);
   return cudaGetLastError() == cudaSuccess ? 0 : -7;
 }
 

@@ -375,6 +375,20 @@ def test_pairs_of_gates_have_the_bits_of_the_division(beside):
     assert torch.equal(paired.view(torch.int32)[~divided.isnan()], divided.view(torch.int32)[~divided.isnan()])
 
 
+@pytest.mark.parametrize("few,many,h", [(296, 297, 4104), (296, 297, 8192), (200, 1000, 16384), (1600, 1601, 2560), (1600, 1601, 4096), (1025, 2000, 2056)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norms_of_few_rows_give_the_bits_of_many(few, many, h, residual):
+    """Either side of the lines from which residual and multipliers are requested ahead."""
+    require_gpu_lib()
+    x, w = _normal(h, many, h), 1 + _normal(1, h, std=0.1)
+    got = []
+    for m in (few, many):
+        r = _normal(h + 1, many, h)[:m] if residual else None
+        got.append([t[:few] for t in K.rmsnorm_quant(x[:m], w, 1e-5, residual=r, want_y=True) if t is not None])
+    check_status()
+    assert len(got[0]) == 3 + residual and all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("d", [64, 128, 256])
 def test_past_rows_off_a_vector(d):
     """Pages that begin at an odd byte, rows 2 bytes past a vector: the rows that aligned ones give, and nothing beside them."""
