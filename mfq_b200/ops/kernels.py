@@ -120,7 +120,8 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
     per K block of a split, and meeting 4.4 with two splits, 2 in a larger cluster, 10 in memory; clusters in a grid
     of nearly every SM do not all fit (5; 22 clusters of six do).  So few tiles over a range that the one-SM kernel splits stay there (66 x 256 x 2048: 7.0
     against 12.6 us; 128 x 4096 x 4096: 11.7 against 15.0; 128 x 4096 x 14336: 19.4 against 31.5), full waves come here (1000 x 6144 x 4096:
-    54.5 against 37.8 with 128 tokens and 34.2 with 256)."""
+    54.5 against 37.8 with 128 tokens and 34.2 with 256).  Up to 128 tokens the model does not see that half of the pairs stream long rows of weights
+    slower than all SMs do (100 x 9216 x 14336: 31.5 against 34.7), so those stay there too."""
     forced = os.environ.get("MFQ_GEMM_PAIR")
     if n % 256 or m < PAIR_MIN_ROWS:
         return 0
@@ -133,6 +134,8 @@ def pair_tile(m: int, n: int, k: int, sms: int = 148) -> int:
 def _pair_tile_by_cost(m: int, n: int, k: int, sms: int) -> int:
     pairs, blocks = sms // 2, k // 128
     waves = {t: math.ceil(n // 256 * math.ceil(m / t) / pairs) for t in (128, 256)}
+    if m <= 128 and blocks > 64 and n // 128 <= pairs:  # half of the pairs, each weight once: these do not draw what all SMs do from memory
+        return 0
     per = split_blocks(m, n, k) or blocks
     splits = math.ceil(blocks / per)
     if splits > 1:
