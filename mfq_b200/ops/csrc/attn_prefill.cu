@@ -12,7 +12,7 @@
 // What bounds it is the softmax: exponentials, and the two passes over S.
 // Grids that fill two CTAs per SM (two_ctas_per_sm) take the pair form: K and V in one stage each, one S buffer (P lies in S, so Q K^T of block j + 1 follows
 // P V of block j), a thread per query row with all 128 of its outputs in registers, no exchange of maxima.  Its chain per block is half as long
-// again, but two CTAs hide each other's waits.  O alpha + O_blk is formed as a product while P V runs and a sum while the next Q K^T does, by
+// again, but two CTAs hide each other's waits.  (The compiler sees 128 registers a thread, of which setmaxnreg makes 200, and spills 124 bytes.)  O alpha + O_blk is formed as a product while P V runs and a sum while the next Q K^T does, by
 // two values per instruction in either form.  32 heads on a B200, one CTA per SM one value per instruction | two | pair form, same bits:
 //   120 tokens 8.7 | 7.0 | 7.7 us    512 after 4000 (128 CTAs) 61 | 58 | 88    700 (192) 18.9 | 15.9 | 19.3    1000 after 3001 (256) 95 | 90 | 85
 //   1500 43.5 | 40.1 | 36.1    2048 65 | 62 | 51    4096 199 | 192 | 161    8192 688 | 665 | 570

@@ -37,7 +37,7 @@ struct GemmCfg {
   // token columns), so that two warps per scheduler hide each other's TMEM-load and FMA latencies.
   static constexpr int kEpiWarps = BT >= 64 ? 8 : 4;
   static constexpr int kCols = BT / (kEpiWarps / 4);   // token columns per epilogue thread
-  static constexpr int kThreads = 64 + 32 * kEpiWarps;
+  static constexpr int kThreads = 64 + 32 * kEpiWarps;  // the compiler spills 80 bytes with 64 tokens (two CTAs per SM), 68 with 128
   static constexpr int kXsBytes = kEpiWarps * kCols * 4;  // per-warp copy of the row multipliers of its token columns
   static constexpr int kWsMax = 256;                      // weight-block multipliers of a CTA's K range kept in smem
   static constexpr int kWsBytes = kWsMax * 4;

@@ -146,7 +146,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_trigger();  // TMEM is held by now: a successor that wants some waits for it, not the other way round
   // The register file is the scarce resource of the fold: the control warp group hands its registers to the epilogue
-  // groups, which then hold a thread's accumulators plus two chunks of raw columns.
+  // groups, which then hold a thread's accumulators plus two chunks of raw columns (with 256 tokens all but 44 bytes of it).
   if (warp < 4) {
   if constexpr (kTok) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   else asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");

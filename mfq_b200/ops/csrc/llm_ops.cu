@@ -206,8 +206,9 @@ __global__ void rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const 
 // divisions kept the issue slots two thirds busy), 1000 rows from 36 to 20.  With the gates by silu2 74 and 19, with all loads of a full row
 // requested before the first is used 69 and 18.
 // ---------------------------------------------------------------------------------------------
-// kFull: gated rows of kRowVecs vectors for every thread.  They need more registers, which the others do without: with 50 instead of 40 the CTAs of
-// the second product of 320 routes found no room beside this kernel's, and that layer took 148 us instead of 146.
+// kFull: gated rows of kRowVecs vectors for every thread.  They need 62 registers, which the others do without: three CTAs per SM, with 40 registers and
+// 16 bytes of spills, take 4096 gated rows of 11008 in 54.5 us and 1000 of 18944 in 39.4, two with 47 and none 61.3 and 43.4 (2000 rows of 512: 3.9
+// and 3.5).
 constexpr int kRowVecs = 4;
 template <int kMode, bool kFull = false>
 __global__ void __launch_bounds__(512, kFull ? 1 : 3) quant_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out,
