@@ -41,8 +41,8 @@ __device__ __forceinline__ void delta_stage(T* dst, const T* src, int n, int wid
 }
 
 __device__ __forceinline__ void delta_cluster_barrier() {
-  __syncwarp();  // the aligned form is for whole warps, and loops or branches of single lanes may come before
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();  // loops or branches of single lanes may come before
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ float delta_peer_load(const float* mine, uint32_t cta) {
   uint32_t a;

@@ -90,8 +90,8 @@ __device__ __forceinline__ DenseEpilogue dense_epilogue_at(const DenseParams& p,
 }
 
 __device__ __forceinline__ void dense_cluster_barrier() {
-  __syncwarp();  // the aligned form is for whole warps, and loops or branches of single lanes may come before
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();  // loops or branches of single lanes may come before
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t dense_cluster_addr(uint32_t addr, uint32_t cta) {
   uint32_t r;

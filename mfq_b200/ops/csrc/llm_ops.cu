@@ -383,7 +383,7 @@ __global__ void __cluster_dims__(kSwigluSplit, 1, 1) __launch_bounds__(256)
 silu_mul_quant_split_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out, float* __restrict__ scale_out,
                             int K, int in_stride) {
   pdl_trigger();
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
   __shared__ float red[33];
   __shared__ float maxima[kSwigluSplit];
   const size_t row = blockIdx.x / kSwigluSplit;
@@ -417,14 +417,14 @@ silu_mul_quant_split_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __rest
     }
   }
   amax = block_reduce<true>(amax, red);
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   if (threadIdx.x < kSwigluSplit) {
     uint32_t remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&maxima[part])), "r"(threadIdx.x));
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(amax) : "memory");
   }
   __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
   float row_max = maxima[0];
 #pragma unroll
   for (int r = 1; r < kSwigluSplit; ++r) row_max = fmaxf(row_max, maxima[r]);

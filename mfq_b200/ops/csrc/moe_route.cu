@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(128) moe_router_topk_warp_kernel(const RouterP
 }
 
 __device__ __forceinline__ void plan_cluster_barrier() {
-  __syncwarp();  // the aligned form is for whole warps, and loops or branches of single lanes may come before
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();  // loops or branches of single lanes may come before
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t plan_peer_load(const int* mine, int cta) {  // the same variable of another CTA of the cluster
   uint32_t addr, v;
